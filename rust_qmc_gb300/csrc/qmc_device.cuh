@@ -10,6 +10,7 @@
 #include <utility>
 #include <cuda_runtime.h>
 #include "qmc_ff.cuh"
+#include "qmc_fp64.cuh"
 
 namespace qmc {
 
@@ -89,23 +90,19 @@ template <int N, class F>
 __device__ __forceinline__ void static_for(F&& f) { unroll_impl<N>(f, std::make_integer_sequence<int, N>{}); }
 
 // ---------------------------------------------------------------------------
-// Math helpers (float paths use the hardware approximations).
+// Math helpers (float paths use the hardware approximations, double paths the
+// functions of qmc_fp64.cuh).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double fexp(double x) { return exp(x); }
+__device__ __forceinline__ double fexp(double x) { return d_exp(x); }
 __device__ __forceinline__ float fexp(float x) { return __expf(x); }
-__device__ __forceinline__ double flog(double x) { return log(x); }
+__device__ __forceinline__ double flog(double x) { return d_log(x); }
 __device__ __forceinline__ float flog(float x) { return __logf(x); }
-__device__ __forceinline__ double fsqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double fsqrt(double x) { return d_sqrt(x); }
 __device__ __forceinline__ float fsqrt(float x) { return sqrtf(x); }
-// Double-precision reciprocal and reciprocal square root: single-precision
-// hardware seed refined by one Newton-Raphson step, y1 = y0 (2 - x y0) and
-// y1 = y0 (3 - x y0^2) / 2, which squares the seed's ~2^-22 relative error
-// to ~1e-14.  Arguments are positive and within single-precision range here.
-__device__ __forceinline__ double frcp(double x) {
-    double y = (double)__fdividef(1.0f, (float)x);
-    double e = fma(-x, y, 1.0);
-    return fma(e, y, y);
-}
+// Reciprocal (and frsqrt below) of a positive double within single-precision
+// range: FP32 seed and one Newton-Raphson step, which squares the seed's
+// ~2^-22 relative error to ~1e-14.
+__device__ __forceinline__ double frcp(double x) { return d_rcp(x); }
 __device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
 // 2^x by the PTX approximate base-2 exponential (flush-to-zero).
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -143,15 +140,12 @@ __device__ __forceinline__ U4 rng_draw(uint64_t seed, uint32_t walker, uint64_t 
 // A single-electron move takes one Philox call: four 24-bit uniforms feed two
 // Box-Muller pairs (three displacement components are used) and the top
 // bytes of words 0-2 form the 24-bit acceptance uniform.
-__device__ __forceinline__ double u24(uint32_t k, double) { return ((double)k + 0.5) * (1.0 / 16777216.0); }
+__device__ __forceinline__ double u24(uint32_t k, double) { return d_u24(k); }
 __device__ __forceinline__ float u24(uint32_t k, float) { return ((float)k + 0.5f) * (1.0f / 16777216.0f); }
 template <class T>
 struct MoveDraw { T n0, n1, n2, uacc; };
 __device__ __forceinline__ void bm24(uint32_t a, uint32_t b, double& n0, double& n1) {
-    double r = sqrt(-2.0 * log(u24(a, 0.0)));
-    double s, c;
-    sincospi(2.0 * u24(b, 0.0), &s, &c);
-    n0 = r * c; n1 = r * s;
+    d_normals24(a, b, n0, n1);
 }
 __device__ __forceinline__ void bm24(uint32_t a, uint32_t b, float& n0, float& n1) {
     float r = sqrtf(-2.0f * __logf(u24(a, 0.0f)));
@@ -159,13 +153,10 @@ __device__ __forceinline__ void bm24(uint32_t a, uint32_t b, float& n0, float& n
     __sincosf(6.28318530717958647f * u24(b, 0.0f), &s, &c);
     n0 = r * c; n1 = r * s;
 }
-__device__ __forceinline__ double to_u01(uint32_t x, double) { return ((double)x + 0.5) * (1.0 / 4294967296.0); }
+__device__ __forceinline__ double to_u01(uint32_t x, double) { return d_u32(x); }
 __device__ __forceinline__ float to_u01(uint32_t x, float) { return ((float)(x >> 8) + 0.5f) * (1.0f / 16777216.0f); }
 __device__ __forceinline__ void bm(uint32_t a, uint32_t b, double& n0, double& n1) {
-    double r = sqrt(-2.0 * log(to_u01(a, 0.0)));
-    double s, c;
-    sincospi(2.0 * to_u01(b, 0.0), &s, &c);
-    n0 = r * c; n1 = r * s;
+    d_normals32(a, b, n0, n1);
 }
 __device__ __forceinline__ void bm(uint32_t a, uint32_t b, float& n0, float& n1) {
     float r = sqrtf(-2.0f * __logf(to_u01(a, 0.0f)));
@@ -370,11 +361,7 @@ struct MOEval {
 template <class T>
 __device__ __forceinline__ T frsqrt(T x);
 template <>
-__device__ __forceinline__ double frsqrt<double>(double x) {
-    double y = (double)rsqrtf((float)x);
-    double e = fma(-x * y, y, 1.0);
-    return fma(0.5 * e, y, y);
-}
+__device__ __forceinline__ double frsqrt<double>(double x) { return d_rsqrt(x); }
 template <>
 __device__ __forceinline__ float frsqrt<float>(float x) { return rsqrtf(x); }
 
@@ -384,6 +371,14 @@ __device__ __forceinline__ void dist(T r2, T& d, T& rinv) {
     rinv = r2 > T(0) ? frsqrt(r2) : T(0);
     d = r2 * rinv;
 }
+__device__ __forceinline__ void dist(double r2, double& d, double& rinv) {
+    rinv = d_positive(r2) ? d_rsqrt(r2) : 0.0;
+    d = r2 * rinv;
+}
+// d < c for a distance d (double: on the high words, no FP64 compare).
+template <class T>
+__device__ __forceinline__ bool closer(T d, double c) { return d < T(c); }
+__device__ __forceinline__ bool closer(double d, double c) { return d_below(d, c); }
 
 // upr = u'(r)/r, lt = u'' + 2u'/r.  rinv = 1/r (0 at r = 0).
 template <class T>
@@ -409,6 +404,14 @@ __device__ __forceinline__ void pade_ab(T a, T b, T d, T rinv, T& u, T& upr, T& 
 // 828-829).  A is destroyed; Ainv = A^-1.  Row swaps use selects so that
 // all indices stay compile-time.
 // ---------------------------------------------------------------------------
+// Pivot magnitudes are compared, and 1 / pivot is formed, in the cheapest form
+// of each type (double: the high words as integers, d_rcp_full).
+template <class T>
+__device__ __forceinline__ T pivot_mag(T a) { return fabs(a); }
+__device__ __forceinline__ int pivot_mag(double a) { return d_hi(a) & 0x7fffffff; }
+template <class T>
+__device__ __forceinline__ T recip_full(T a) { return T(1) / a; }
+__device__ __forceinline__ double recip_full(double a) { return d_rcp_full(a); }
 // on_pivot(|pivot|) receives each pivot magnitude for the determinant.
 template <int N, class T, class OnPivot>
 __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], int& sign, OnPivot on_pivot) {
@@ -421,10 +424,10 @@ __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], i
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         int p = k;
-        T best = fabs(A[k][k]);
+        auto best = pivot_mag(A[k][k]);
 #pragma unroll
         for (int i = k + 1; i < N; ++i) {
-            T a = fabs(A[i][k]);
+            const auto a = pivot_mag(A[i][k]);
             if (a > best) { best = a; p = i; }
         }
 #pragma unroll
@@ -443,7 +446,7 @@ __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], i
         if (!(piv != T(0))) { ok = false; piv = T(1); }
         if (piv < 0) sign = -sign;
         on_pivot(fabs(piv));
-        T ip = T(1) / piv;
+        T ip = recip_full(piv);
 #pragma unroll
         for (int j = 0; j < N; ++j) { A[k][j] *= ip; Ainv[k][j] *= ip; }
 #pragma unroll
@@ -460,7 +463,7 @@ __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], i
 template <int N, class T>
 __device__ __forceinline__ bool gj_inverse(T (&A)[N][N], T (&Ainv)[N][N], double& logdet, int& sign) {
     logdet = 0.0;
-    return gj_inverse_core<N, T>(A, Ainv, sign, [&](T p) { logdet += log((double)p); });
+    return gj_inverse_core<N, T>(A, Ainv, sign, [&](T p) { logdet += d_log((double)p); });
 }
 
 // Float-float form: |det| accumulated as a rescaled product (one logarithm

@@ -229,13 +229,12 @@ __host__ __device__ constexpr int sweep_words() {
 template <class T>
 __device__ __forceinline__ T sq3(T x, T y, T z) { return x * x + y * y + z * z; }
 
-// 1/r from r^2; +inf at r = 0, so that a / (b + 1/r) gives the r -> 0 limit 0.
-__device__ __forceinline__ float inv_r(float r2) { return rsqrtf(r2); }
-__device__ __forceinline__ double inv_r(double r2) { return r2 > 0.0 ? frsqrt(r2) : (double)INFINITY; }
-
-// Pade a r / (1 + b r) evaluated as a / (b + 1/r).
-template <class T>
-__device__ __forceinline__ T pade_value(T a, T b, T r2) { return a * frcp(b + inv_r(r2)); }
+// Pade a r / (1 + b r) evaluated as a / (b + 1/r), 0 at r = 0 (FP32: 1/r = +inf
+// there, double: selected).
+__device__ __forceinline__ float pade_value(float a, float b, float r2) { return a * frcp(b + rsqrtf(r2)); }
+__device__ __forceinline__ double pade_value(double a, double b, double r2) {
+    return d_positive(r2) ? a * d_rcp(b + d_rsqrt(r2)) : 0.0;
+}
 
 // Electron-electron u of one pair at squared distance r2.
 template <class SH, class T>
@@ -493,7 +492,7 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
             if (SH::JAS == JAS_PADE_F) pade_f(S.F, S.invF, d, ri, uu, upr, lt);
             else pade_ab(S.a_ee[c], S.b_ee[c], d, ri, uu, upr, lt);
             u += uu;
-            bool skip = (SH::JAS == JAS_PADE_EEN) ? (d < TC(1e-10)) : (d == TC(0));
+            bool skip = (SH::JAS == JAS_PADE_EEN) ? closer(d, 1e-10) : (d == TC(0));
             if (!skip) {
                 gx[i] += upr * dx; gy[i] += upr * dy; gz[i] += upr * dz;
                 gx[j] -= upr * dx; gy[j] -= upr * dy; gz[j] -= upr * dz;
@@ -502,7 +501,7 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
                 gsq[i] += up * up; gsq[j] += up * up;
             }
             if (WANT_O && SH::JAS == JAS_PADE_EEN) {
-                TC inv = TC(1) / (1 + S.b_ee[c] * d);
+                TC inv = recip_full(1 + S.b_ee[c] * d);
                 O[c] += -S.a_ee[c] * d * d * inv * inv;
                 O[2 + c] += d * inv;
             }
@@ -519,12 +518,12 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
             TC uu, upr, lt;
             pade_ab(S.enA[I], S.enB[I], d, ri, uu, upr, lt);
             u -= uu;
-            if (!(d < TC(1e-10))) {
+            if (!closer(d, 1e-10)) {
                 gx[i] -= upr * dx; gy[i] -= upr * dy; gz[i] -= upr * dz;
                 lu[i] -= lt;
             }
             if (WANT_O) {
-                TC inv = TC(1) / (1 + S.enB[I] * d);
+                TC inv = recip_full(1 + S.enB[I] * d);
                 TC dB = S.Aspec[I] * S.Z[I] * d * d * inv * inv;
                 TC dA = -S.Z[I] * d * inv;
                 if (S.species[I] == 0) { O[4] += dB; O[6] += dA; }
@@ -1498,7 +1497,7 @@ __global__ void __launch_bounds__(TPB) k_step_all(const __grid_constant__ SysT<S
         FullEval<SH, T, 0> ev;
         evaluate_config<SH, T, 0>(S, rn, ev, false, nostore, (T*)nullptr);
         U4 a = rng_draw(seed, (uint32_t)w, st, 0, TAG_ACCEPT);
-        double prob = exp(2.0 * (ev.logabs - lp));
+        double prob = d_exp(2.0 * (ev.logabs - lp));
         bool accept = act && ev.ok && (to_u01(a.x, 0.0) < prob);
         if (accept) {
 #pragma unroll
