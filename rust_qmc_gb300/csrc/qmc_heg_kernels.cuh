@@ -7,8 +7,8 @@
 // evaluates its own orbital e^{i k.r} (no AO contraction is needed).  The
 // FP64 measurement rebuilds the inverses by complex Gauss-Jordan elimination
 // and evaluates the Ewald sum: real-space pairs with images inside the erfc
-// cutoff, reciprocal sum over a half-space k list (rho_k built from per-lane
-// phase recursions and a warp reduction), and FP64 constants from the host.
+// cutoff, the reciprocal sum by octants of k vectors (a lane per octant vector,
+// per-electron phases in shared memory), and FP64 constants from the host.
 #pragma once
 #include <cstdio>
 #include <cmath>
@@ -18,6 +18,11 @@
 #include "qmc_device.cuh"
 
 namespace qmc {
+
+// A pair of scalars as one vector: complex inverse columns, phases.
+template <class T> struct HComplex;
+template <> struct HComplex<float> { using type = float2; };
+template <> struct HComplex<double> { using type = double2; };
 
 constexpr int HMAX_K = 1800;      // reciprocal half-space vectors (|n_i| <= 7 cube: 1687)
 
@@ -34,17 +39,26 @@ struct SysH {
     double ksum_const;             // added per walker with the reciprocal sum
     T k2sum;                       // (1/2) sum over occupied |k|^2 of both sectors
     T kvec[2][32][3];              // [sector][column][xyz]
-    int nk;
-    int kmax;                      // reciprocal cutoff |n| <= kmax (sphere) or |n_i| <= kmax (cube)
-    int kcube;                     // 1: the reference's full cube of integer vectors
+    int nt;                        // octant vectors of the reciprocal sum
+    int kmax;                      // their largest component
+    float aL, rc2u;                // alpha L and the squared real-space cutoff, in box units
+    ff a2l2;                       // (alpha L)^2 log2(e)
     int perm[64];                  // internal -> caller electron index
 };
 
-// Reciprocal-space table of the Ewald sum (global memory, read uniformly).
+// Intervals of the real-space erfc table: width 1/32 on [0, 6].
+constexpr int HERFC_N = 192;
+
+// Ewald tables (global memory).
 struct KTable {
-    int kint[HMAX_K][3];
+    // Octant vectors (a, b, c) >= 0 packed a | b << 8 | c << 16, and the Ewald
+    // weight times the number of half-space vectors (+-a, +-b, +-c) they stand for.
+    int tri[HMAX_K];
     double kw[HMAX_K];
     float2 kwf[HMAX_K];            // kw as a float-float pair (hi, lo)
+    // Taylor coefficients of erfc at the interval centres: orders 0..3 as
+    // float-float pairs, 4..7 as floats.
+    float4 erfc_tab[HERFC_N][3];
 };
 
 template <class T>
@@ -61,33 +75,61 @@ static bool fill_sysh(const HostSys& hs, int NE, int NUP, SysH<T>& S, KTable& KT
     S.quirk_cross = (hs.quirks & 8) ? 1 : 0;
     const bool qe = (hs.quirks & 4) != 0;
     const double alpha = qe ? 5.0 / L : hs.jas[4] / L;
-    const int K = qe ? 7 : (int)hs.jas[5];
+    const int K = reciprocal_kmax(hs);
     S.alpha = (T)alpha;
     S.real_images = qe ? 0 : 1;
     S.rcut = (T)(5.6 / alpha);
-    // the device sums the 27 nearest images: the cutoff must stay below 1.5 L
+    // the device sums the 27 nearest images: the cutoff must stay below 1.5 L (which
+    // also keeps alpha L above 3.73, the range of image_erfc's polynomial)
     if (!qe && 5.6 / alpha >= 1.5 * L) return false;
-    // reciprocal half space; weight (4 pi / V) e^{-k^2 / 4 alpha^2} / k^2
-    int nk = 0;
+    // reciprocal half space, by octants; weight (4 pi / V) e^{-k^2 / 4 alpha^2} / k^2
+    int nk = 0, nt = 0;
     double wsum = 0.0;
     const double dk = 2.0 * M_PI / L;
     for (int nx = 0; nx <= K; ++nx)
-        for (int ny = -K; ny <= K; ++ny)
-            for (int nz = -K; nz <= K; ++nz) {
-                if (nx == 0 && (ny < 0 || (ny == 0 && nz <= 0))) continue;
+        for (int ny = 0; ny <= K; ++ny)
+            for (int nz = 0; nz <= K; ++nz) {
+                if (nx == 0 && ny == 0 && nz == 0) continue;
                 if (!qe && nx * nx + ny * ny + nz * nz > K * K) continue;
-                if (nk >= HMAX_K) return false;
-                double k2 = dk * dk * (nx * nx + ny * ny + nz * nz);
-                KT.kint[nk][0] = nx; KT.kint[nk][1] = ny; KT.kint[nk][2] = nz;
-                KT.kw[nk] = 4.0 * M_PI / V * std::exp(-k2 / (4.0 * alpha * alpha)) / k2;
-                KT.kwf[nk].x = (float)KT.kw[nk];
-                KT.kwf[nk].y = (float)(KT.kw[nk] - (double)KT.kwf[nk].x);
-                wsum += KT.kw[nk];
-                ++nk;
+                const int signs = (nx ? 2 : 1) * (ny ? 2 : 1) * (nz ? 2 : 1);
+                nk += signs / 2;
+                if (nk > HMAX_K) return false;
+                const double k2 = dk * dk * (nx * nx + ny * ny + nz * nz);
+                const double w = 4.0 * M_PI / V * std::exp(-k2 / (4.0 * alpha * alpha)) / k2;
+                KT.tri[nt] = nx | (ny << 8) | (nz << 16);
+                KT.kw[nt] = w * (signs / 2);
+                KT.kwf[nt].x = (float)KT.kw[nt];
+                KT.kwf[nt].y = (float)(KT.kw[nt] - (double)KT.kwf[nt].x);
+                wsum += KT.kw[nt];
+                ++nt;
             }
-    S.nk = nk;
+    for (int j = 0; j < HERFC_N; ++j) {
+        // derivatives of erfc: f' = g = -2/sqrt(pi) e^{-x^2}, f^(n+1) = -2 x f^(n) - 2 (n-1) f^(n-1)
+        const double x = (j + 0.5) / 32.0;
+        double d[8];
+        d[0] = std::erfc(x);
+        d[1] = -2.0 / std::sqrt(M_PI) * std::exp(-x * x);
+        d[2] = -2.0 * x * d[1];
+        for (int n = 2; n < 7; ++n) d[n + 1] = -2.0 * x * d[n] - 2.0 * (n - 1) * d[n - 1];
+        double f = 1.0;
+        float c[12];
+        for (int n = 0; n < 8; ++n) {
+            if (n) f *= n;
+            const double v = d[n] / f;
+            if (n < 4) {
+                c[2 * n] = (float)v;
+                c[2 * n + 1] = (float)(v - (double)c[2 * n]);
+            } else {
+                c[4 + n] = (float)v;
+            }
+        }
+        for (int q = 0; q < 3; ++q) KT.erfc_tab[j][q] = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+    }
+    S.nt = nt;
     S.kmax = K;
-    S.kcube = qe ? 1 : 0;
+    S.aL = (float)(alpha * L);
+    S.a2l2 = ff(alpha * L * alpha * L * 1.4426950408889634);
+    S.rc2u = (float)(5.6 / (alpha * L) * (5.6 / (alpha * L)));
     const int N = hs.N;
     if (qe) {
         // heg.rs:526-581: (1/2) sum_k f_k (|rho_k|^2 - N) and -0.448 N / r_s
@@ -176,58 +218,95 @@ __device__ __forceinline__ void fsincos(ff x, ff* s, ff* c) {
     }
 }
 
-// erfc on [0, 6] in float-float arithmetic (0 beyond): the Chebyshev
-// interpolant erfc(x) = c_0 / 2 + sum_{k=1..42} c_k T_k(t), t = x / 3 - 1,
-// through 64 first-kind nodes (coefficients from gen_erfc_table.py, mpmath
-// at 40 digits; |c_k| < 2e-18 beyond k = 42), summed by Clenshaw's
-// recurrence: terms k >= 24 in FP32 (their partial sums stay below 1e-7),
-// the rest in float-float.  Absolute error below 2e-14 on [0, 6].
-static __constant__ const ff kErfcCheb[24] = {
-    ff(3.673991e-01f, -6.9200334e-09f),
-    ff(-3.3617035e-01f, 1.6510556e-09f),
-    ff(2.5549158e-01f, 9.960313e-09f),
-    ff(-1.5657288e-01f, 9.566121e-10f),
-    ff(7.125926e-02f, -5.790789e-10f),
-    ff(-1.7145663e-02f, 7.2621587e-10f),
-    ff(-5.9834975e-03f, -6.355615e-11f),
-    ff(9.309509e-03f, 1.6978224e-11f),
-    ff(-5.190865e-03f, 1.0619118e-10f),
-    ff(1.1763682e-03f, 4.8458522e-11f),
-    ff(5.319446e-04f, 3.415539e-13f),
-    ff(-6.203452e-04f, 1.8230945e-11f),
-    ff(2.4648002e-04f, 1.3352023e-11f),
-    ff(-4.3256662e-07f, -1.3714815e-14f),
-    ff(-5.34781e-05f, 3.0843093e-13f),
-    ff(2.795329e-05f, -6.6343177e-13f),
-    ff(-3.1002157e-06f, 4.7403328e-14f),
-    ff(-3.9868787e-06f, 1.6839862e-13f),
-    ff(2.4134415e-06f, 3.8801173e-14f),
-    ff(-3.3472375e-07f, 2.2182666e-15f),
-    ff(-2.8443293e-07f, 9.959113e-15f),
-    ff(1.730987e-07f, 5.6202656e-15f),
-    ff(-2.0892596e-08f, -6.1127414e-16f),
-    ff(-1.984897e-08f, -5.560824e-16f)};
-static __constant__ const float kErfcChebTail[19] = {1.05052615e-08f, -7.149105e-10f, -1.2955014e-09f, 5.301936e-10f, 9.567597e-12f, -7.440549e-11f, 2.116448e-11f, 3.314318e-12f, -3.5774686e-12f, 5.862873e-13f, 2.661633e-13f, -1.3746954e-13f, 4.9925553e-15f, 1.3928812e-14f, -3.9142388e-15f, -5.4379457e-16f, 5.295314e-16f, -6.445588e-17f, -3.8180913e-17f};
-__device__ __forceinline__ ff erfc_ff(ff x) {
+// erfc on [0, 6] in float-float arithmetic (0 beyond): Taylor series about the
+// centre of the argument's interval of width 1/32 (|d| <= 1/64: the truncated
+// order 8 is below 4e-17), orders 4..7 in FP32 (|d|^4 = 6e-8), the lower ones
+// in float-float.  Absolute error below 2e-14 on [0, 6].  A Chebyshev series
+// over the whole range took 23 float-float steps (about 720 instructions
+// against 75 and three 16-byte loads).
+__device__ __forceinline__ ff erfc_ff(const KTable* __restrict__ KT, ff x) {
     if (!(x.hi < 6.0f)) return ff(0.0f);
-    const ff t = x * ff(1.0 / 3.0) - ff(1.0f);
-    const float th2 = 2.0f * t.hi;
-    float b1 = 0.0f, b2 = 0.0f;
+    const int j = min((int)(x.hi * 32.0f), HERFC_N - 1);
+    const ff d = x + ff(-((float)j + 0.5f) * 0.03125f);
+    const float4 a = KT->erfc_tab[j][0], b = KT->erfc_tab[j][1], c = KT->erfc_tab[j][2];
+    const float t = __fmaf_rn(d.hi, __fmaf_rn(d.hi, __fmaf_rn(d.hi, c.w, c.z), c.y), c.x);
+    const ff p = ff_two_prod(d.hi, t);
+    ff s = ff_fast_two_sum(b.z, __fadd_rn(b.w, p.hi));
+    s = d * s + ff(b.x, b.y);
+    s = d * s + ff(a.z, a.w);
+    return d * s + ff(a.x, a.y);
+}
+
+// 2^-(q c) for FP32 q >= 0 with its rounding error qe and the constant c as a
+// float pair: the product in two parts, a degree-6 polynomial for the fraction (fitted at
+// Chebyshev nodes of |f| <= 1/2, 8e-8 with its rounding), the integer in the exponent.
+__device__ __forceinline__ float exp2_neg(float q, float qe, ff c) {
+    const float p = __fmul_rn(q, c.hi);
+    float pe = __fmaf_rn(q, c.hi, -p);
+    pe = __fmaf_rn(q, c.lo, pe);
+    pe = __fmaf_rn(qe, c.hi, pe);
+    const float n = fminf(rintf(p), 125.0f);
+    const float f = fmaxf(__fsub_rn(__fsub_rn(n, p), pe), -200.0f);   // clamped with n: the result underflows to 0
+    float r = __fmaf_rn(f, 0.00015461445f, 0.0013400428f);
+    r = __fmaf_rn(f, r, 0.009618057f);
+    r = __fmaf_rn(f, r, 0.05550327f);
+    r = __fmaf_rn(f, r, 0.2402265f);
+    r = __fmaf_rn(f, r, 0.6931472f);
+    r = __fmaf_rn(f, r, 1.0f);
+    return p > 125.0f ? 0.0f : __fmul_rn(r, __int_as_float((127 - (int)n) << 23));
+}
+
+// Sum over the 26 images n != 0 of erfc(aL |s + n|) / |s + n| inside the cutoff,
+// s the minimum-image separation in box units, in FP32.  erfc(x) = e^{-x^2}
+// Q(1/x^2) / x with Q a degree-8 polynomial fitted at Chebyshev nodes of 1/x^2 in
+// [1/36, 1/1.86^2] (7e-8 with its FP32 rounding), and e^{-x^2} is a product over
+// the axes, so 9 exponentials serve the 26 terms and no square root is left:
+// erfc(x) / d = e^{-x^2} Q(1/x^2) / (aL d^2).  Images with two axes shifted away
+// (d^2 > 2) are skipped when the cutoff excludes them for every pair.
+__device__ __forceinline__ float image_erfc(float sx, float sy, float sz, float aL, float rc2u, ff a2l2) {
+    float qx[3], qy[3], qz[3], ex[3], ey[3], ez[3];
+    // axis values ordered: no shift, shift towards the image (|s| - 1), shift away (|s| + 1)
+    auto axis = [&](float s, float (&q)[3], float (&e)[3]) {
+        const float a = fabsf(s);
 #pragma unroll
-    for (int k = 42; k >= 24; --k) {
-        const float b0 = __fmaf_rn(th2, b1, __fsub_rn(kErfcChebTail[k - 24], b2));
-        b2 = b1;
-        b1 = b0;
-    }
-    ff B1 = ff(b1), B2 = ff(b2);
-    const ff t2 = ff(2.0f * t.hi, 2.0f * t.lo);
+        for (int k = 0; k < 3; ++k) {
+            const float t = k == 0 ? a : (k == 1 ? __fsub_rn(a, 1.0f) : __fadd_rn(a, 1.0f));
+            q[k] = __fmul_rn(t, t);
+            e[k] = exp2_neg(q[k], __fmaf_rn(t, t, -q[k]), a2l2);
+        }
+    };
+    axis(sx, qx, ex);
+    axis(sy, qy, ey);
+    axis(sz, qz, ez);
+    const float ia = __fdividef(1.0f, aL), ia2 = ia * ia;
+    float acc = 0.0f;
 #pragma unroll
-    for (int k = 23; k >= 1; --k) {
-        const ff B0 = t2 * B1 + kErfcCheb[k] - B2;
-        B2 = B1;
-        B1 = B0;
-    }
-    return ff(0.5f * kErfcCheb[0].hi, 0.5f * kErfcCheb[0].lo) + t * B1 - B2;
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            if ((i == 2) + (j == 2) == 2 && rc2u <= 2.0f) continue;
+            const float qij = qx[i] + qy[j], eij = __fmul_rn(ex[i], ey[j]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (i + j + k == 0) continue;
+                if ((i == 2) + (j == 2) + (k == 2) >= 2 && rc2u <= 2.0f) continue;
+                const float d2 = qij + qz[k];
+                float id = __fdividef(1.0f, d2);
+                id = __fmaf_rn(__fmaf_rn(-d2, id, 1.0f), id, id);
+                const float w = id * ia2;
+                float g = __fmaf_rn(w, 12.996532f, -21.552807f);
+                g = __fmaf_rn(w, g, 16.388454f);
+                g = __fmaf_rn(w, g, -7.8752494f);
+                g = __fmaf_rn(w, g, 2.9005704f);
+                g = __fmaf_rn(w, g, -1.0063616f);
+                g = __fmaf_rn(w, g, 0.42103583f);
+                g = __fmaf_rn(w, g, -0.28204688f);
+                g = __fmaf_rn(w, g, 0.56418914f);
+                const float v = __fmul_rn(__fmul_rn(eij, ez[k]), __fmul_rn(g, id));
+                acc += d2 < rc2u ? v : 0.0f;
+            }
+        }
+    return __fmul_rn(acc, ia);
 }
 
 // Nearest integer of a float-float value (ties resolved by the leading part).
@@ -247,6 +326,36 @@ __device__ __forceinline__ T min_img(T d, const SysH<T>& S) { return d - S.L * r
 __device__ __forceinline__ float hshfl(float v, int s) { return __shfl_sync(0xffffffffu, v, s); }
 __device__ __forceinline__ double hshfl(double v, int s) { return __shfl_sync(0xffffffffu, v, s); }
 __device__ __forceinline__ ff hshfl(ff v, int s) { return wshfl(v, s); }
+
+// Two consecutive values of shared memory as one load.
+template <class T>
+__device__ __forceinline__ void load_pair(const T* p, T& a, T& b) {
+    const auto v = *reinterpret_cast<const typename HComplex<T>::type*>(p);
+    a = v.x; b = v.y;
+}
+__device__ __forceinline__ void load_pair(const ff* p, ff& a, ff& b) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a = ff(v.x, v.y); b = ff(v.z, v.w);
+}
+
+template <class T>
+__device__ __forceinline__ void store_pair(T* p, T a, T b) {
+    *reinterpret_cast<typename HComplex<T>::type*>(p) = {a, b};
+}
+__device__ __forceinline__ void store_pair(ff* p, ff a, ff b) {
+    *reinterpret_cast<float4*>(p) = make_float4(a.hi, a.lo, b.hi, b.lo);
+}
+
+// Exchange registers 0 and p (0 < p < N, the same on every lane): one case runs.
+template <int N, class T>
+__device__ __forceinline__ void swap_rows(int p, T (&a)[N], T (&b)[N]) {
+#pragma unroll
+    for (int r = 1; r < N; ++r)
+        if (p == r) {
+            T t = a[0]; a[0] = a[r]; a[r] = t;
+            t = b[0]; b[0] = b[r]; b[r] = t;
+        }
+}
 
 // |z|^2 of a pivot candidate on the leading parts (pivot choice only).
 __device__ __forceinline__ float pivot_mag(float r, float i) { return r * r + i * i; }
@@ -280,6 +389,80 @@ __device__ __forceinline__ void heg_u(const SysH<T>& S, T r, T a, T& u, T& du, T
         T d2 = a * ex / (S.F * S.F * op * op * op) * (-3 - 3 * x + x * x + x * x * x);
         lu = d2 + 2 / r * du;
     }
+}
+
+// Refresh pair geometry: minimum image of xi - xj.  FP32 walkers' positions are
+// floats (the low parts are zero), so the difference is one exact TwoSum.
+template <class T>
+__device__ __forceinline__ T pair_image(T a, T b, const SysH<T>& S) { return min_img(a - b, S); }
+__device__ __forceinline__ ff pair_image(ff a, ff b, const SysH<ff>& S) {
+    const ff d = ff_two_sum(a.hi, -b.hi);
+    const float n = rintf(__fmul_rn(d.hi, S.invL.hi));
+    return d + ff(__fmul_rn(-n, S.L.hi), __fmul_rn(-n, S.L.lo));
+}
+
+// Squared length; the float-float form sums the exact squares lazily.
+template <class T>
+__device__ __forceinline__ T length2(T x, T y, T z) { return x * x + y * y + z * z; }
+__device__ __forceinline__ ff length2(ff x, ff y, ff z) {
+    ff r = ff_two_prod(x.hi, x.hi);
+    r.lo = __fmaf_rn(2.0f * x.hi, x.lo, r.lo);
+    ff_fma_lazy(r, y, y);
+    ff_fma_lazy(r, z, z);
+    return ff_norm(r);
+}
+
+// Pair function of the refresh: u, u'(r)/r and u'' + 2u'/r of heg_u inside its
+// cutoff, from r, r^2 and 1/r, with one reciprocal for the RPA form.
+template <class T>
+__device__ __forceinline__ void heg_pair(const SysH<T>& S, T r, T r2, T ri, T a, T& u, T& f, T& lu) {
+    if (S.form != 1) {
+        T du;
+        heg_u(S, r, a, u, du, lu);
+        f = du * ri;
+        return;
+    }
+    const T cr = S.pc * r, cr2 = S.pc * r2, q = T(1) - cr2;
+    const T inv = frcp(T(1) + S.pb * r + cr2);
+    const T ai = a * inv, ai2 = ai * inv;
+    u = ai * r;
+    f = ai2 * q * ri;
+    // u'' + 2u'/r = 2 a inv^2 ( q / r - c r - q (b + 2 c r) inv )
+    lu = T(2) * ai2 * (q * ri - cr - q * (S.pb + T(2) * cr) * inv);
+    const bool in = r < S.halfL && r > T(1e-10);
+    u = in ? u : T(0);
+    f = in ? f : T(0);
+    lu = in ? lu : T(0);
+}
+
+// Phase of the reciprocal sum at coordinate x: (cos, sin)(2 pi x / L).
+template <class T>
+__device__ __forceinline__ void unit_phase(T x, const SysH<T>& S, T& c, T& s) {
+    double sd, cd;
+    sincos(2.0 * M_PI / (double)S.L * (double)x, &sd, &cd);
+    c = (T)cd;
+    s = (T)sd;
+}
+__device__ __forceinline__ void unit_phase(ff x, const SysH<ff>& S, ff& c, ff& s) {
+    ff t = x * S.invL;
+    t = t - rint(t);
+    fsincos(ff(6.283185307179586) * t, &s, &c);
+}
+
+// Product that is only multiplied or summed further (float-float: not renormalised).
+template <class T>
+__device__ __forceinline__ T mul_lazy(T a, T b) { return a * b; }
+__device__ __forceinline__ ff mul_lazy(ff a, ff b) {
+    const ff p = ff_two_prod(a.hi, b.hi);
+    return ff(p.hi, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, p.lo)));
+}
+
+// acc += x without renormalising (closed with macc_norm).
+template <class T>
+__device__ __forceinline__ T add_lazy(T acc, T x) { return acc + x; }
+__device__ __forceinline__ ff add_lazy(ff acc, ff x) {
+    const ff t = ff_two_sum(acc.hi, x.hi);
+    return ff(t.hi, __fadd_rn(acc.lo, __fadd_rn(t.lo, x.lo)));
 }
 
 template <class T, int NE>
@@ -396,9 +579,6 @@ __global__ void khw_init(const SysH<double>* __restrict__ S, TS* __restrict__ po
 }
 
 // Single-electron sweeps, one warp per walker.
-template <class T> struct HComplex;
-template <> struct HComplex<float> { using type = float2; };
-template <> struct HComplex<double> { using type = double2; };
 // Shared bytes per warp of the sweep's inverse columns (both sectors).
 template <int NM, class T>
 __host__ __device__ constexpr size_t hsweep_warp_bytes() { return sizeof(T) * 2 * 2 * NM * 32; }
@@ -650,6 +830,7 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
     constexpr int NM = NUP > NDN ? NUP : NDN;
     const int lane = threadIdx.x & 31;
     TC* Mi = Mr + NM * 32;                            // Mr: [re|im][row][lane]
+    TC* bc = Mr + 2 * NM * 32;                        // [row][re|im] of the pivot column
     double e_l = 0.0;
     if (act) {
         HLanePos<TC, NE> P;
@@ -706,32 +887,45 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
             int src = lane;
 #pragma unroll 1
             for (int k = 0; k < NS; ++k) {
-                // pivot: the largest |D[i][k]| over the rows not yet pivoted
-                // (leading parts; the first of equal ones)
-                int p = 0;
-                float best = pivot_mag(Ar[0], Ai[0]);
+                // column k, row by row, to the warp's broadcast buffer
+                if (lane == k) {
 #pragma unroll
-                for (int r = 1; r < NM; ++r) {
-                    const float m = pivot_mag(Ar[r], Ai[r]);
-                    if (r < NS - k && m > best) { best = m; p = r; }
+                    for (int i = 0; i < NM; ++i) store_pair(bc + 2 * i, Ar[i], Ai[i]);
                 }
-                p = __shfl_sync(0xffffffffu, p, k);
-#pragma unroll
-                for (int r = 1; r < NM; ++r) {
-                    const bool sw = (r == p);
-                    TC a = Ar[0], b = Ar[r]; Ar[0] = sw ? b : a; Ar[r] = sw ? a : b;
-                    a = Ai[0]; b = Ai[r]; Ai[0] = sw ? b : a; Ai[r] = sw ? a : b;
+                __syncwarp();
+                // pivot: the largest |D[i][k]| over the rows not yet pivoted, a row
+                // per lane (leading parts, whose bits order as integers; the first
+                // of equal ones)
+                unsigned key = 0;
+                if (lane < NS - k) {
+                    TC r, m;
+                    load_pair(bc + 2 * lane, r, m);
+                    key = __float_as_uint(pivot_mag(r, m));
+                }
+                const unsigned top = __reduce_max_sync(0xffffffffu, key);
+                const int p = __ffs(__ballot_sync(0xffffffffu, lane < NS - k && key == top)) - 1;
+                if (p != 0) {
+                    swap_rows<NM>(p, Ar, Ai);             // p is the same on every lane
+                    if (lane == 0) {
+                        TC r0, i0, rp, ip;
+                        load_pair(bc, r0, i0);
+                        load_pair(bc + 2 * p, rp, ip);
+                        store_pair(bc, rp, ip);
+                        store_pair(bc + 2 * p, r0, i0);
+                    }
+                    __syncwarp();
                 }
                 const int pk = k + p;
                 src = (src == k) ? pk : ((src == pk) ? k : src);
-                TC pr = hshfl(Ar[0], k), pi = hshfl(Ai[0], k);
+                TC pr, pi;
+                load_pair(bc, pr, pi);
                 TC pa = pr * pr + pi * pi;
                 if (!(pa > TC(0))) { ok = false; pr = 1; pi = 0; pa = 1; }
                 if constexpr (std::is_same<TC, ff>::value) {
                     pmag = pmag * pa;                  // |det|^2 as a rescaled product
                     ff_rescale(pmag, pexp);
                 } else {
-                    logdet += 0.5 * log((double)pa);
+                    logdet += 0.5 * d_log((double)pa);
                 }
                 const TC ipr = pr / pa, ipi = -pi / pa;           // 1/a
                 TC tr, ti;
@@ -745,9 +939,11 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
 #pragma unroll
                 for (int i = 1; i < NM; ++i) {
                     if (i >= NS) continue;
-                    TC fr = hshfl(Ar[i], k), fi = hshfl(Ai[i], k);
+                    TC fr, fi;
+                    load_pair(bc + 2 * i, fr, fi);
                     Ar[i] -= fr * tr - fi * ti; Ai[i] -= fr * ti + fi * tr;
                 }
+                __syncwarp();                             // bc is read
                 // rotate registers 0..NS-1 by one: the pivoted row goes last
                 const TC r0 = Ar[0], i0 = Ai[0];
 #pragma unroll
@@ -795,7 +991,7 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
             __syncwarp();
         }
         if constexpr (std::is_same<TC, ff>::value)
-            logdet = 0.5 * (log((double)pmag) + (double)pexp * 0.6931471805599453);
+            logdet = 0.5 * (d_log((double)pmag) + (double)pexp * 0.6931471805599453);
         }
         if constexpr (PART == 1) {
 #pragma unroll
@@ -829,66 +1025,39 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
             }
             logdet = a.log[w];
         }
-        // Jastrow for this lane's electrons (pairs from both ends)
+        // Jastrow and real-space Ewald, each unordered pair once, spread evenly
+        // over the lanes: pair p < NE (NE-1)/2 pairs electron i = p mod NE with
+        // j = i + p / NE + 1 (mod NE) for the first NE floor((NE-1)/2) pairs and
+        // i = p - that with i + NE/2 for the rest (even NE).  Consecutive pairs
+        // have distinct i and distinct j, so the lanes add the gradient and
+        // Laplacian terms of their i, and then of their j, to shared sums
+        // without conflicts.  Per-electron sums over all partners from both
+        // ends took 108 pair evaluations on 27 of 32 lanes against 45 here.
+        // The minimum image term is in the compute type (FP64 for FP32 compute);
+        // the other 26 images lie beyond L/2, where each term is below
+        // erfc(alpha L/2)/(L/2), and are summed in FP32.
         TC u = 0, kin = 0;
-#pragma unroll
-        for (int sig = 0; sig < 2; ++sig) {
-            const int NS = sig == 0 ? NUP : NDN;
-            const int i = sig * NUP + lane;
-            const bool own = lane < NS;
-            TC xi, yi, zi;
-            P.get_own(min(i, NE - 1), xi, yi, zi);
-            TC gx = 0, gy = 0, gz = 0, lu = 0;
-            for (int j = 0; j < NE; ++j) {
-                TC xj, yj, zj;
-                P.get(j, xj, yj, zj);
-                if (!own || j == i) continue;
-                const TC a = S.a_ee[((j < NUP) == (i < NUP)) ? 1 : 0];
-                TC dx = min_img(xi - xj, S), dy = min_img(yi - yj, S), dz = min_img(zi - zj, S);
-                TC r = fsqrt(dx * dx + dy * dy + dz * dz);
-                TC uu, du, l;
-                heg_u(S, r, a, uu, du, l);
-                u += TC(0.5) * uu;
-                if (r < S.halfL && r > TC(1e-10)) {
-                    TC f = du / r;
-                    gx += f * dx; gy += f * dy; gz += f * dz;
-                    lu += l;
-                }
-            }
-            if (own) {
-                TC cx = S.quirk_cross ? gqx[sig] : gdx[sig], cy = S.quirk_cross ? gqy[sig] : gdy[sig],
-                   cz = S.quirk_cross ? gqz[sig] : gdz[sig];
-                TC lp = ldet[sig] + lu + gx * gx + gy * gy + gz * gz + 2 * (cx * gx + cy * gy + cz * gz);
-                kin += lp;
-                if (a.grad) {
-                    a.grad[((size_t)w * NE + i) * 3 + 0] = (double)(gdx[sig] + gx);
-                    a.grad[((size_t)w * NE + i) * 3 + 1] = (double)(gdy[sig] + gy);
-                    a.grad[((size_t)w * NE + i) * 3 + 2] = (double)(gdz[sig] + gz);
-                }
-                if (a.lap) a.lap[(size_t)w * NE + i] = (double)lp;
-            }
-        }
-        // Real-space Ewald, each unordered pair once, spread evenly over the
-        // lanes: pair p < NE (NE-1)/2 pairs electron i = p mod NE with
-        // i + p / NE + 1 (mod NE) for the first NE floor((NE-1)/2) pairs and
-        // i = p - that with i + NE/2 for the rest (even NE).  The minimum
-        // image term is FP64; the other 26 images lie beyond L/2, where each
-        // term is below erfc(alpha L/2)/(L/2), and are summed in FP32.
         double vreal = 0.0;
         ff vreal_ff = ff(0.0f);
         {
-            TC* ps = Mr;                                  // the rows buffer is free again
+            TC* ps = Mr;                                  // [3][NE] positions, then [4][NE] sums
+            TC* sums = Mr + 3 * NE;
             __syncwarp();
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int j = lane + 32 * r;
-                if (j < NE) { ps[3 * j] = P.x[r]; ps[3 * j + 1] = P.y[r]; ps[3 * j + 2] = P.z[r]; }
+                if (j < NE) {
+                    ps[j] = P.x[r]; ps[NE + j] = P.y[r]; ps[2 * NE + j] = P.z[r];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) sums[c * NE + j] = TC(0);
+                }
             }
             __syncwarp();
+            static_assert(NE > 32, "the lanes of one round hold distinct electrons");
             constexpr int NPAIR = NE * (NE - 1) / 2, HALF = (NE - 1) / 2, FULL = NE * HALF;
-            const float aLf = (float)((double)S.alpha * (double)S.L);
-            const float rcu = (float)((double)S.rcut * (double)S.invL), rc2u = rcu * rcu;
-            for (int p = lane; p < NPAIR; p += 32) {
+            for (int p0 = 0; p0 < NPAIR; p0 += 32) {
+                const bool on = p0 + lane < NPAIR;
+                const int p = on ? p0 + lane : NPAIR - 1;
                 int i, j;
                 if (p < FULL) {
                     i = p % NE;
@@ -898,156 +1067,128 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
                     j = i + NE / 2;
                 }
                 if (j >= NE) j -= NE;
-                const TC dx = min_img(ps[3 * i] - ps[3 * j], S), dy = min_img(ps[3 * i + 1] - ps[3 * j + 1], S),
-                         dz = min_img(ps[3 * i + 2] - ps[3 * j + 2], S);
+                const TC dx = pair_image(ps[i], ps[j], S), dy = pair_image(ps[NE + i], ps[NE + j], S),
+                         dz = pair_image(ps[2 * NE + i], ps[2 * NE + j], S);
+                const TC r2 = length2(dx, dy, dz);
+                const TC r = fsqrt(r2);
+                const bool apart = on && r > TC(1e-10);
+                const TC ri = apart ? frcp(r) : TC(0);
+                TC uu, f, l;
+                heg_pair(S, r, r2, ri, S.a_ee[((j < NUP) == (i < NUP)) ? 1 : 0], uu, f, l);
+                if (on) u += uu;
+                const TC g[4] = {f * dx, f * dy, f * dz, l};
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (on) sums[c * NE + i] = add_lazy(sums[c * NE + i], g[c]);
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (on) sums[c * NE + j] = add_lazy(sums[c * NE + j], c < 3 ? -g[c] : g[c]);
+                __syncwarp();
                 if constexpr (std::is_same<TC, ff>::value) {
-                    // float-float minimum-image term: no FP64 in this phase
-                    const ff r = fsqrt(dx * dx + dy * dy + dz * dz);
-                    if (r.hi > 1e-10f) vreal_ff += erfc_ff(S.alpha * r) / r;
+                    if (apart) vreal_ff += erfc_ff(static_cast<const KTable*>(a.kt), S.alpha * r) * ri;
                 } else {
-                    const double r = sqrt((double)dx * (double)dx + (double)dy * (double)dy + (double)dz * (double)dz);
-                    if (r > 1e-10) vreal += erfc((double)S.alpha * r) / r;
+                    if (apart) vreal += erfc((double)S.alpha * (double)r) / (double)r;
                 }
                 if (S.real_images) {
-                    // box units: the image shift is an exact integer, alpha L is
-                    // exact in FP32 for the usual splittings, and sqrt and the
-                    // quotient are correctly rounded, so the rounding of each
-                    // term is unbiased; the sum is scaled by 1/L in FP64
-                    const float sx = (float)((double)dx * (double)S.invL), sy = (float)((double)dy * (double)S.invL),
-                                sz = (float)((double)dz * (double)S.invL);
-                    float acc = 0.0f;
-                    for (int ia = -1; ia <= 1; ++ia)
-                        for (int ib = -1; ib <= 1; ++ib)
-#pragma unroll
-                            for (int ic = -1; ic <= 1; ++ic) {
-                                if (!ia && !ib && !ic) continue;
-                                const float ex = sx + (float)ia, ey = sy + (float)ib, ez = sz + (float)ic;
-                                const float d2 = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
-                                if (d2 < rc2u) {
-                                    const float d = __fsqrt_rn(d2);
-                                    acc += __fdiv_rn(erfcf(__fmul_rn(aLf, d)), d);
-                                }
-                            }
-                    if constexpr (std::is_same<TC, ff>::value) vreal_ff += ff(acc) * S.invL;
-                    else vreal += (double)acc * (double)S.invL;
+                    // box units: the image shifts are exact integers; the sum is
+                    // scaled by 1/L in the compute type
+                    const float acc = image_erfc(lead(dx * S.invL), lead(dy * S.invL), lead(dz * S.invL), S.aL, S.rc2u,
+                                                 S.a2l2);
+                    if (on) {
+                        if constexpr (std::is_same<TC, ff>::value) vreal_ff += ff(acc) * S.invL;
+                        else vreal += (double)acc * (double)S.invL;
+                    }
                 }
             }
+#pragma unroll
+            for (int sig = 0; sig < 2; ++sig) {
+                const int NS = sig == 0 ? NUP : NDN;
+                const int i = sig * NUP + lane;
+                if (lane < NS) {
+                    const TC gx = macc_norm(sums[i]), gy = macc_norm(sums[NE + i]), gz = macc_norm(sums[2 * NE + i]),
+                             lu = macc_norm(sums[3 * NE + i]);
+                    TC cx = S.quirk_cross ? gqx[sig] : gdx[sig], cy = S.quirk_cross ? gqy[sig] : gdy[sig],
+                       cz = S.quirk_cross ? gqz[sig] : gdz[sig];
+                    TC lp = ldet[sig] + lu + gx * gx + gy * gy + gz * gz + TC(2) * (cx * gx + cy * gy + cz * gz);
+                    kin += lp;
+                    if (a.grad) {
+                        a.grad[((size_t)w * NE + i) * 3 + 0] = (double)(gdx[sig] + gx);
+                        a.grad[((size_t)w * NE + i) * 3 + 1] = (double)(gdy[sig] + gy);
+                        a.grad[((size_t)w * NE + i) * 3 + 2] = (double)(gdz[sig] + gz);
+                    }
+                    if (a.lap) a.lap[(size_t)w * NE + i] = (double)lp;
+                }
+            }
+            __syncwarp();
         }
-        // reciprocal Ewald: rho_k = sum_i e^{i k.r_i} over the half space of
-        // integer vectors n (k = 2 pi n / L), visited in the order of the
-        // host's weight table (nx, then ny, then nz ascending).  For each of
-        // its electrons a lane keeps the running phase e^{i k.r}, advanced by
-        // one complex multiply per step; one warp reduction per k.  Electrons
-        // a lane does not own start from zero phase and contribute nothing.
-        double vk = 0.0;
+        // Reciprocal Ewald: sum over the half space of integer vectors n of
+        // w_n |rho_n|^2, rho_n = sum_i e^{2 pi i n.r_i / L}.  With c, s the cosines
+        // and sines of an electron's phases (a x, b y, c z), the sums over the sign
+        // combinations of an octant vector (a, b, c) collapse: the cross terms of
+        // the eight sums T = sum_i {c,s}_x {c,s}_y {c,s}_z cancel and
+        // sum_{signs} |rho|^2 = (number of distinct signs) sum T^2.  A lane takes
+        // an octant vector and runs over the electrons, whose phases (powers
+        // 0..K of e^{2 pi i x / L} per axis) are in the warp's shared memory:
+        // 4 products and 8 multiply-adds per octant vector and electron for up
+        // to 4 half-space vectors, and no reduction between lanes.  A lane per
+        // electron, with a running phase and a warp reduction per vector, took
+        // about 275 000 sub-partition cycles per walker against 45 000 here.
+        TC vkt = TC(0);
         {
-            const double dk = 2.0 * M_PI / (double)S.L;
-            const int K = S.kmax;
-            TC exr[2], exi[2], eyr[2], eyi[2], ezr[2], ezi[2], ymr[2], ymi[2], zmr[2], zmi[2], pxr[2], pxi[2];
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const bool own = lane + 32 * r < NE;
-                double s, c;
-                sincos(dk * (double)P.x[r], &s, &c);
-                exr[r] = own ? TC(c) : TC(0); exi[r] = own ? TC(s) : TC(0);
-                sincos(dk * (double)P.y[r], &s, &c);
-                eyr[r] = own ? TC(c) : TC(0); eyi[r] = own ? TC(s) : TC(0);
-                sincos(dk * (double)P.z[r], &s, &c);
-                ezr[r] = own ? TC(c) : TC(0); ezi[r] = own ? TC(s) : TC(0);
-                // e^{-i K dk y}, e^{-i K dk z}: K multiplications by the conjugate
-                ymr[r] = own ? TC(1) : TC(0); ymi[r] = TC(0);
-                zmr[r] = own ? TC(1) : TC(0); zmi[r] = TC(0);
-                for (int m = 0; m < K; ++m) {
-                    TC t = ymr[r] * eyr[r] + ymi[r] * eyi[r];
-                    ymi[r] = ymi[r] * eyr[r] - ymr[r] * eyi[r]; ymr[r] = t;
-                    t = zmr[r] * ezr[r] + zmi[r] * ezi[r];
-                    zmi[r] = zmi[r] * ezr[r] - zmr[r] * ezi[r]; zmr[r] = t;
-                }
-                pxr[r] = TC(1); pxi[r] = TC(0);
-            }
-            TC vkt = TC(0);
-            int t = 0;
-            for (int nx = 0; nx <= K; ++nx) {
-                TC qr[2], qi[2];                              // e^{i (nx x + ny y) dk}, ny = -K
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    qr[r] = pxr[r] * ymr[r] - pxi[r] * ymi[r];
-                    qi[r] = pxr[r] * ymi[r] + pxi[r] * ymr[r];
-                }
-                for (int ny = -K; ny <= K; ++ny) {
-                    const int rest = K * K - nx * nx - ny * ny;
-                    if (!(nx == 0 && ny < 0) && (S.kcube || rest >= 0)) {
-                        TC tr[2], ti[2];                      // nz = -K
-#pragma unroll
-                        for (int r = 0; r < 2; ++r) {
-                            tr[r] = qr[r] * zmr[r] - qi[r] * zmi[r];
-                            ti[r] = qr[r] * zmi[r] + qi[r] * zmr[r];
-                        }
-                        // nz in chunks of four: the four lane partials of rho_k
-                        // are reduced together (butterfly reduce-scatter: two
-                        // exchanges at distance 16, one at 8, then a full
-                        // reduction over the low three lane bits), after which
-                        // lanes 0, 8, 16, 24 hold chunk values 0..3
-                        const int vi = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
-                        for (int nz0 = -K; nz0 <= K; nz0 += 4) {
-                            TC pr[4], pim[4];
-                            int tk[4];
-                            bool ok4[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const int nz = nz0 + j;
-                                ok4[j] = nz <= K && !(nx == 0 && ny == 0 && nz <= 0) && (S.kcube || nz * nz <= rest);
-                                tk[j] = t;
-                                t += ok4[j] ? 1 : 0;
-                                pr[j] = ok4[j] ? tr[0] + tr[1] : TC(0);
-                                pim[j] = ok4[j] ? ti[0] + ti[1] : TC(0);
-#pragma unroll
-                                for (int r = 0; r < 2; ++r) {
-                                    TC x = tr[r] * ezr[r] - ti[r] * ezi[r];
-                                    ti[r] = tr[r] * ezi[r] + ti[r] * ezr[r];
-                                    tr[r] = x;
-                                }
-                            }
-                            const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
-                            TC wr[2], wi[2];
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {            // distance 16: keep v_h or v_{h+2}
-                                const TC sr = b4 ? pr[h] : pr[h + 2], si = b4 ? pim[h] : pim[h + 2];
-                                wr[h] = (b4 ? pr[h + 2] : pr[h]) + hshfl_xor(sr, 16);
-                                wi[h] = (b4 ? pim[h + 2] : pim[h]) + hshfl_xor(si, 16);
-                            }
-                            const TC sr = b3 ? wr[0] : wr[1], si = b3 ? wi[0] : wi[1];   // distance 8
-                            TC vr = (b3 ? wr[1] : wr[0]) + hshfl_xor(sr, 8);
-                            TC vim = (b3 ? wi[1] : wi[0]) + hshfl_xor(si, 8);
-#pragma unroll
-                            for (int m = 4; m > 0; m >>= 1) {
-                                vr += hshfl_xor(vr, m);
-                                vim += hshfl_xor(vim, m);
-                            }
-                            const bool okv = vi == 0 ? ok4[0] : (vi == 1 ? ok4[1] : (vi == 2 ? ok4[2] : ok4[3]));
-                            const int tv = vi == 0 ? tk[0] : (vi == 1 ? tk[1] : (vi == 2 ? tk[2] : tk[3]));
-                            if ((lane & 7) == 0 && okv) vkt += kweight<TC>(static_cast<const KTable*>(a.kt), tv) * (vr * vr + vim * vim);
-                        }
-                    }
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        TC x = qr[r] * eyr[r] - qi[r] * eyi[r];
-                        qi[r] = qr[r] * eyi[r] + qi[r] * eyr[r];
-                        qr[r] = x;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    TC x = pxr[r] * exr[r] - pxi[r] * exi[r];
-                    pxi[r] = pxr[r] * exi[r] + pxi[r] * exr[r];
-                    pxr[r] = x;
+            const int K1 = S.kmax + 1;
+            TC* ph = Mr;                                  // [3 (K+1)][NE] pairs (cos, sin)
+            for (int it = lane; it < 3 * NE; it += 32) {
+                const int ax = it / NE, i = it - ax * NE;
+                TC c1, s1;
+                unit_phase((TC)a.pos[(3 * i + ax) * (size_t)a.Wcap + w], S, c1, s1);
+                TC c = TC(1), sn = TC(0);
+                TC* out = ph + 2 * ((size_t)ax * K1 * NE + i);
+                for (int n = 0; n < K1; ++n) {
+                    out[0] = c;
+                    out[1] = sn;
+                    out += 2 * NE;
+                    const TC t = c * c1 - sn * s1;
+                    sn = c * s1 + sn * c1;
+                    c = t;
                 }
             }
-            vk = (double)hsum(vkt);
+            __syncwarp();
+            const KTable* KT = static_cast<const KTable*>(a.kt);
+            for (int t = lane; t < S.nt; t += 32) {
+                const int v = KT->tri[t];
+                const TC* px = ph + 2 * NE * (v & 255);
+                const TC* py = ph + 2 * NE * (K1 + ((v >> 8) & 255));
+                const TC* pz = ph + 2 * NE * (2 * K1 + (v >> 16));
+                TC T[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) T[q] = TC(0);
+#pragma unroll 2
+                for (int i = 0; i < NE; ++i) {
+                    TC xc, xs, yc, ys, zc, zs;
+                    load_pair(px + 2 * i, xc, xs);
+                    load_pair(py + 2 * i, yc, ys);
+                    load_pair(pz + 2 * i, zc, zs);
+                    const TC cc = mul_lazy(xc, yc), cs = mul_lazy(xc, ys), sc = mul_lazy(xs, yc), ss = mul_lazy(xs, ys);
+                    macc(T[0], cc, zc); macc(T[1], cc, zs);
+                    macc(T[2], cs, zc); macc(T[3], cs, zs);
+                    macc(T[4], sc, zc); macc(T[5], sc, zs);
+                    macc(T[6], ss, zc); macc(T[7], ss, zs);
+                }
+                TC q = TC(0);
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const TC x = macc_norm(T[m]);
+                    q += x * x;
+                }
+                vkt += kweight<TC>(KT, t) * q;
+            }
         }
+        const double vk = (double)hsum(vkt);
         u = hsum(u);
         kin = hsum(kin);
-        vreal = hsum(vreal + (double)vreal_ff);
+        if constexpr (std::is_same<TC, ff>::value) vreal = (double)hsum(vreal_ff);
+        else vreal = hsum(vreal);
         double V = vreal + vk + S.ksum_const + S.e_const;
         e_l = -0.5 * (double)kin + V;
         if (lane == 0) {
@@ -1075,15 +1216,21 @@ __device__ __forceinline__ void hwarp_block_partial(double v, double* partial, i
     __syncthreads();
 }
 
-// Shared words per warp of a refresh launch: the orbital matrix rows for the
-// determinant half, the positions for the energy half alone.
+// Shared words per warp of a refresh launch: the orbital matrix rows of the
+// determinant half, and for the energy half the pair sums (positions and four
+// sums per electron), then the phase table of a reciprocal cutoff kmax.
 template <int NE, int NUP, int PART>
-__host__ __device__ constexpr int hmeasure_warp_words() {
-    return PART == 2 ? 3 * NE : 2 * (NUP > NE - NUP ? NUP : NE - NUP) * 32;
+__host__ __device__ constexpr int hmeasure_warp_words(int kmax) {
+    const int det = PART == 2 ? 0 : 2 * (NUP > NE - NUP ? NUP : NE - NUP) * 33;
+    const int pair = PART == 1 ? 0 : 7 * NE, ph = PART == 1 ? 0 : 6 * (kmax + 1) * NE;
+    const int e = pair > ph ? pair : ph;
+    return det > e ? det : e;
 }
+// Energy-half blocks per SM: 12 warps at up to 168 registers (the phase table
+// takes 73 KB a block at kmax = 6).
 
 template <int NE, int NUP, class TC, class TS, int WPB, int PART = 0>
-__global__ void __launch_bounds__(32 * WPB, PART == 2 ? 4 : 2) khw_measure(
+__global__ void __launch_bounds__(32 * WPB, PART == 2 ? 3 : 2) khw_measure(
     const SysH<TC>* __restrict__ Sg, const KTable* __restrict__ KT, const TS* __restrict__ gpos,
     TS* __restrict__ gdinv, double* __restrict__ glog, int* __restrict__ gsign, double* __restrict__ gel, int W,
     int Wcap, int write_state, double* __restrict__ out_grad, double* __restrict__ out_lap, double* partial,
@@ -1100,14 +1247,14 @@ __global__ void __launch_bounds__(32 * WPB, PART == 2 ? 4 : 2) khw_measure(
     const int wib = threadIdx.x >> 5;
     const int w = blockIdx.x * WPB + wib;
     double e_l = khw_measure_walker<NE, NUP, TC, TS, PART>(
-        S, a, rows + (size_t)wib * hmeasure_warp_words<NE, NUP, PART>(), w, w < W);
+        S, a, rows + (size_t)wib * hmeasure_warp_words<NE, NUP, PART>(S.kmax), w, w < W);
     if (PART != 1 && partial) hwarp_block_partial<WPB>(e_l, partial, blockIdx.x);
 }
 
 // Batched form (compute type TC, state written, per-tile E_L partials), one
 // block per tile.
 template <int NE, int NUP, class TC, class TS, int WPB, int PART = 0>
-__global__ void __launch_bounds__(32 * WPB, PART == 2 ? 4 : 2) khwb_measure(const BatchTile* __restrict__ tiles,
+__global__ void __launch_bounds__(32 * WPB, PART == 2 ? 3 : 2) khwb_measure(const BatchTile* __restrict__ tiles,
                                                                          int ntiles, const BatchRec* __restrict__ recs,
                                                                          double* tile_partial) {
     extern __shared__ __align__(16) unsigned char hsm[];
@@ -1122,7 +1269,7 @@ __global__ void __launch_bounds__(32 * WPB, PART == 2 ? 4 : 2) khwb_measure(cons
     const volatile MeasureArgs<TS>& a = args;
     const int w = tl.w0 + wib;
     double e_l = khw_measure_walker<NE, NUP, TC, TS, PART>(
-        S, a, rows + (size_t)wib * hmeasure_warp_words<NE, NUP, PART>(), w, w < a.W);
+        S, a, rows + (size_t)wib * hmeasure_warp_words<NE, NUP, PART>(S.kmax), w, w < a.W);
     if (PART != 1) hwarp_block_partial<WPB>(e_l, tile_partial, blockIdx.x);
 }
 
@@ -1207,16 +1354,16 @@ struct HegShapeOps {
     }
 
     template <class TC, class TS, int PART>
-    static size_t measure_smem() {
-        return ((sizeof(SysH<TC>) + 15) / 16) * 16 + sizeof(TC) * WPB * hmeasure_warp_words<NE, NUP, PART>();
+    static size_t measure_smem(int kmax) {
+        return ((sizeof(SysH<TC>) + 15) / 16) * 16 + sizeof(TC) * WPB * hmeasure_warp_words<NE, NUP, PART>(kmax);
     }
 
     template <class TC, class TS, int PART>
     static int batch_measure_t(const BatchClass& bc, cudaStream_t st, int* occ) {
-        const size_t smem = measure_smem<TC, TS, PART>();
+        const size_t smem = measure_smem<TC, TS, PART>(bc.kmax);
         auto kern = khwb_measure<NE, NUP, TC, TS, WPB, PART>;
-        static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
+        static size_t attr = 0;
+        if (attr < smem) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = smem; }
         if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, 32 * WPB, smem) == cudaSuccess ? 0 : 2;
         if (bc.ntiles == 0) return 0;
         kern<<<bc.ntiles, 32 * WPB, smem, st>>>(bc.tiles, bc.ntiles, bc.recs, bc.tile_partial);
@@ -1252,12 +1399,12 @@ struct HegShapeOps {
     }
 
     template <class TC, class TS, int PART>
-    static int launch_measure_part(const SysH<TC>* S, const KTable* KT, DevWalkers& dw, bool ws, const MeasureOut& out,
-                                   double* partial, int nb, cudaStream_t st) {
-        const size_t smem = measure_smem<TC, TS, PART>();
+    static int launch_measure_part(int kmax, const SysH<TC>* S, const KTable* KT, DevWalkers& dw, bool ws,
+                                   const MeasureOut& out, double* partial, int nb, cudaStream_t st) {
+        const size_t smem = measure_smem<TC, TS, PART>(kmax);
         auto kern = khw_measure<NE, NUP, TC, TS, WPB, PART>;
-        static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
+        static size_t attr = 0;
+        if (attr < smem) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = smem; }
         kern<<<nb, 32 * WPB, smem, st>>>(S, KT, (const TS*)dw.pos, (TS*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W,
                                          dw.Wcap, ws ? 1 : 0, out.grad, out.lap, partial, dw.flags, dw.rows);
         ++g_launch_count;
@@ -1276,11 +1423,11 @@ struct HegShapeOps {
         if constexpr (std::is_same<TC, ff>::value) two = ws && dw.rows && !out.grad && !out.lap;
         if (two) {
             if constexpr (std::is_same<TC, ff>::value) {
-                rc = launch_measure_part<TC, TS, 1>(S, KT, dw, ws, out, nullptr, nb, st);
-                if (!rc) rc = launch_measure_part<TC, TS, 2>(S, KT, dw, ws, out, partial, nb, st);
+                rc = launch_measure_part<TC, TS, 1>(reciprocal_kmax(hs), S, KT, dw, ws, out, nullptr, nb, st);
+                if (!rc) rc = launch_measure_part<TC, TS, 2>(reciprocal_kmax(hs), S, KT, dw, ws, out, partial, nb, st);
             }
         } else {
-            rc = launch_measure_part<TC, TS, 0>(S, KT, dw, ws, out, partial, nb, st);
+            rc = launch_measure_part<TC, TS, 0>(reciprocal_kmax(hs), S, KT, dw, ws, out, partial, nb, st);
         }
         if (rc) return rc;
         if (!partial) return 0;

@@ -102,6 +102,11 @@ struct MeasureOut {
     bool inverse_only = false;
 };
 
+// Electron gas: largest component of the Ewald sum's reciprocal vectors (0 for
+// other systems).
+inline int reciprocal_kmax(const HostSys& hs) {
+    return hs.shape != SHAPE_HEG54 ? 0 : ((hs.quirks & 4) ? 7 : (int)hs.jas[5]);
+}
 int nmax_of_shape(int shape);
 // Bytes per walker of the two-pass refresh scratch (0: the shape has none).
 size_t refresh_rows_bytes(int shape);
@@ -216,6 +221,7 @@ struct BatchClass {
     int nrec = 0;
     const int* tile_begin = nullptr;     // device [nrec + 1]
     double* tile_partial = nullptr;      // device [ntiles][2]
+    int kmax = 0;                        // electron gas: largest reciprocal component of the class's systems
     int grid_measure = 0;                // persistent refresh grid of the thread-per-walker shapes
                                          // (0: one block per tile); other launches: one block per tile
 };
@@ -227,7 +233,7 @@ int batch_tile_width(int shape);
 int launch_batch_sweep(const BatchClass& bc, int move_kind, const BatchCtl* ctl, cudaStream_t st);
 int launch_batch_measure(const BatchClass& bc, cudaStream_t st);
 // Resident blocks per SM of the class's batch kernels (occupancy query).
-int batch_occupancy(int shape, int prec, int move_kind, bool measure);
+int batch_occupancy(int shape, int prec, int move_kind, bool measure, int kmax = 0);
 // Device tables of a system for batched launches (cached in the HostSys).
 int batch_tables(const HostSys& hs, int prec, BatchRec& rec);
 // Per-system mean E_L of the class: sum of its tiles' partials / W, written to

@@ -448,8 +448,9 @@ int launch_batch_measure(const BatchClass& bc, cudaStream_t st) {
 #undef C_
 }
 
-int batch_occupancy(int shape, int prec, int move_kind, bool measure) {
+int batch_occupancy(int shape, int prec, int move_kind, bool measure, int kmax) {
     BatchClass bc;
+    bc.kmax = kmax;
     bc.shape = shape;
     bc.prec = prec;
     int occ = 0, rc = 7;
