@@ -1,7 +1,7 @@
 """Tables of the FP64 elementary functions of qmc_fp64.cuh, computed with
 mpmath at 40 digits and rounded to doubles (printed as hexadecimal literals):
 
-  kExp2T[j]   2^(j/256), j = 0..255
+  kExp2T[j]   2^(j/256), j = 0..255, as a double and what it leaves
   kLogT[i]    (1/c_i, log c_i) for the 128 intervals of z in [0.6875, 1.375)
               that the leading bits of z select; 1/c_i is the rounded
               reciprocal of the interval's midpoint and log c_i is
@@ -49,7 +49,8 @@ if __name__ == "__main__":
     print("// Written by gen_fp64_tables.py: tables of the functions of qmc_fp64.cuh.")
     print("#pragma once")
     print("namespace qmc {")
-    table("double", "kExp2T", [hexd(mp.mpf(2) ** (mp.mpf(j) / 256)) for j in range(256)], 4)
+    powers = [mp.mpf(2) ** (mp.mpf(j) / 256) for j in range(256)]
+    table("double2", "kExp2T", ["{%s, %s}" % (hexd(v), hexd(v - mp.mpf(float(v)))) for v in powers], 2)
     table("double2", "kLogT", ["{%s, %s}" % (hexd(a), hexd(b)) for a, b in log_rows()], 2)
     table("double2", "kSinCosT", ["{%s, %s}" % (hexd(mp.cos(2 * mp.pi * j / 256)), hexd(mp.sin(2 * mp.pi * j / 256)))
                                   for j in range(64)], 2)

@@ -18,8 +18,6 @@
 using namespace qmc;
 
 namespace qmc {
-int launch_step_all_recorded(const HostSys& hs, DevWalkers& dw, int move_kind, int n, uint64_t s0, double step,
-                             uint64_t seed, double* partial, cudaStream_t st);
 int launch_sum_partials(const double* partial, int nblk, int nrows, double* out, cudaStream_t st);
 int launch_scatter_positions(const double* src, DevWalkers& dw, const int* d_perm, int N, cudaStream_t st);
 int launch_gather_positions(const DevWalkers& dw, double* dst, const int* d_perm, int N, cudaStream_t st);
@@ -717,22 +715,22 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     if (warp && P != 8) return QMC_ERR_UNSUPPORTED;
     // device scratch: O [W][P], the SR sums and their block partials, the
     // Jastrow table (jas[8], nuclei [n_nuc][5]), then with dEL: dEL [W][P] and
-    // grad ln|psi| [W][N][3]
+    // (benzene) grad ln|psi| [W][N][3]
     const size_t base = (size_t)W * P + (size_t)M + 2 * (size_t)M * nblk + 64;
     const size_t ntab = 8 + 5 * (size_t)hs.n_nuc;
-    const size_t nd = dEL ? (size_t)W * P + (size_t)W * hs.N * 3 : 0;
+    const size_t nd = dEL ? (size_t)W * P + (warp ? (size_t)W * hs.N * 3 : 0) : 0;
     CK(upload_positions(wk, pos));
     CK(ensure_out(wk, base + ntab + nd));
     double* d_tab = wk->d_out + base;
     double* d_dEL = dEL ? d_tab + ntab : nullptr;
-    double* d_grad = dEL ? d_dEL + (size_t)W * P : nullptr;
+    double* d_grad = dEL && warp ? d_dEL + (size_t)W * P : nullptr;
     std::vector<double> tab(hs.jas, hs.jas + 8);
     for (int I = 0; I < hs.n_nuc; ++I) {
         for (int c = 0; c < 3; ++c) tab.push_back(hs.R[3 * I + c]);
         tab.push_back(hs.Z[I]);
         tab.push_back((double)hs.species[I]);
     }
-    if (warp || dEL) CU(cudaMemcpyAsync(d_tab, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice, st));
+    if (warp) CU(cudaMemcpyAsync(d_tab, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice, st));
     MeasureOut mo;
     mo.grad = d_grad;
     if (warp) {
@@ -742,15 +740,10 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
             return QMC_ERR_CUDA;
         mo.O = wk->d_out;
     } else {
-        // thread-per-walker shapes: O_p, E_L, grad and the rotation columns of
-        // dE_L/dp in one evaluation; the Jastrow columns of dE_L/dp from the
-        // gradient afterwards
+        // the molecules' team kernels: O_p, E_L and dE_L/dp in one evaluation
         mo.O = wk->d_out;
         mo.dEL = d_dEL;
         CK(launch_measure(hs, wk->dw, 0, true, mo, st));
-        if (dEL && launch_jastrow3_logderiv(wk->dw, hs.N, hs.n_up, hs.n_nuc, d_tab + 8, d_tab, P, nullptr, st, d_grad,
-                                            d_dEL))
-            return QMC_ERR_CUDA;
     }
     double* d_sums = wk->d_out + (size_t)W * P;
     double* d_scr = d_sums + M;
@@ -1042,7 +1035,8 @@ int qmc_vmc_run(qmc_sys_t s, const qmc_run_params* p, uint64_t seed, qmc_run_res
     if (p->move_kind == QMC_MOVE_ALL_GAUSS || p->move_kind == QMC_MOVE_ALL_BOX) {
         if (!(p->step > 0)) return QMC_ERR_ARG;
         const int total = p->n_burnin + p->n_steps;
-        int nblk = (wk->dw.W + 63) / 64;
+        const int nblk = step_all_blocks(hs, wk->dw);
+        if (nblk <= 0) return QMC_ERR_UNSUPPORTED;
         double* d_part = nullptr;
         double* d_mean = nullptr;
         CU(cudaMalloc((void**)&d_part, 16 * (size_t)nblk * p->n_steps));
@@ -1058,8 +1052,8 @@ int qmc_vmc_run(qmc_sys_t s, const qmc_run_params* p, uint64_t seed, qmc_run_res
             if (ad.on) end = std::min(end, (t / ad.interval + 1) * ad.interval);
             const int n = end - t;
             if (t >= p->n_burnin)
-                CK(launch_step_all_recorded(hs, wk->dw, p->move_kind, n, (uint64_t)t, ad.value, seed,
-                                            d_part + 2 * (size_t)nblk * (t - p->n_burnin), st));
+                CK(launch_step_all(hs, wk->dw, p->move_kind, n, (uint64_t)t, ad.value, seed,
+                                   d_part + 2 * (size_t)nblk * (t - p->n_burnin), st));
             else
                 CK(launch_sweep(hs, wk->dw, p->move_kind, n, (uint64_t)t, ad.value, 0, 0, seed, st));
             t = end;

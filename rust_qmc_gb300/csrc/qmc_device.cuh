@@ -58,14 +58,11 @@ struct SysT {
     T Z[SH::NNUC];
     T enA[SH::NNUC];          // A_species * Z_I (e-n Jastrow amplitude)
     T enB[SH::NNUC];          // B_species
-    T Aspec[SH::NNUC];        // A_species (unscaled)
-    int species[SH::NNUC];
     T F, invF;                // Pade-F parameter and 1/F
     T b_ee[2], a_ee[2];       // [0] antiparallel, [1] parallel
     T qa;                     // Jastrow2 gradient prefactor quirk (F or 1)
     int quirk_lap;            // Jastrow2 Laplacian quirk
     T v_nn;
-    int n_rot;
     int sh_start[SH::NNUC + 1];
     int sh_p0[SH::NSH], sh_np[SH::NSH];
     int sh_s0[SH::NSH], sh_s1[SH::NSH], sh_p[SH::NSH];
@@ -74,8 +71,6 @@ struct SysT {
     T cs0[SH::NPRIM], cs1[SH::NPRIM], cp[SH::NPRIM];
     int ppow[SH::NPRIM];
     T C[2][SH::NAO][SH::NMAX];      // [sector][internal AO][column]
-    T dC[SH::NROT][SH::NAO];        // d phi / d theta rows
-    int rot_col[SH::NROT][2];       // column of the rotated MO in each sector (-1 none)
     T init_sigma;
     int init_nuc[SH::NE];           // internal electron order
     int perm[SH::NE];               // internal -> caller electron index
@@ -200,7 +195,7 @@ __device__ __forceinline__ MoveDraw<T> draw_of(const MoveDraw<T>& d, int q) {
 // ---------------------------------------------------------------------------
 // Orbital evaluation: phi_k(r) = sum_a C[sig][a][k] chi_a(r) for the NS
 // columns of sector SIG, optionally with gradients (MODE >= 1) and
-// Laplacians (MODE >= 2), and NR extra rows (rotation derivatives, values).
+// Laplacians (MODE >= 2).
 // Shells are grouped by nucleus; each shell's primitive exponentials are
 // computed once and shared by its s-type AOs and p triplet
 // (src/systems/methane.rs:498-590 for Gaussians, src/wavefunction/slater.rs:
@@ -215,15 +210,10 @@ __device__ __forceinline__ float gauss_prim(const SysT<SH, float>& S, int p, flo
     return ex2_approx(S.pexp2[p] * r2);
 }
 
-// MODE 3 adds the gradients and Laplacians of the NR rotation rows (the
-// parameter derivatives of the local energy need them).
-template <class SH, class T, int SIG, int MODE, int NR>
+template <class SH, class T, int SIG, int MODE>
 struct MOEval {
     static constexpr int NS = SIG == 0 ? SH::NUP : SH::NDN;
-    static constexpr int NRD = (MODE >= 3 && NR > 0) ? NR : 1;
     T v[SH::NMAX], gx[SH::NMAX], gy[SH::NMAX], gz[SH::NMAX], l[SH::NMAX];
-    T dv[NR > 0 ? NR : 1];
-    T dgx[NRD], dgy[NRD], dgz[NRD], dl[NRD];
 
     __device__ __forceinline__ void add(const SysT<SH, T>& S, int a, T chi, T ax, T ay, T az, T la) {
 #pragma unroll
@@ -232,12 +222,6 @@ struct MOEval {
             v[k] += c * chi;
             if (MODE >= 1) { gx[k] += c * ax; gy[k] += c * ay; gz[k] += c * az; }
             if (MODE >= 2) l[k] += c * la;
-        }
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-            const T c = S.dC[q][a];
-            dv[q] += c * chi;
-            if (MODE >= 3) { dgx[q] += c * ax; dgy[q] += c * ay; dgz[q] += c * az; dl[q] += c * la; }
         }
     }
 
@@ -253,21 +237,15 @@ struct MOEval {
         }
     }
 
-    // only_nuc >= 0 restricts the sum to AOs centred on that nucleus.
-    __device__ __forceinline__ void run(const SysT<SH, T>& S, T x, T y, T z, int only_nuc = -1) {
+    __device__ __forceinline__ void run(const SysT<SH, T>& S, T x, T y, T z) {
 #pragma unroll
         for (int k = 0; k < SH::NMAX; ++k) { v[k] = 0; gx[k] = 0; gy[k] = 0; gz[k] = 0; l[k] = 0; }
-#pragma unroll
-        for (int q = 0; q < (NR > 0 ? NR : 1); ++q) dv[q] = 0;
-#pragma unroll
-        for (int q = 0; q < NRD; ++q) { dgx[q] = 0; dgy[q] = 0; dgz[q] = 0; dl[q] = 0; }
         if constexpr (!std::is_void<typename SH::Layout>::value) {
             using LY = typename SH::Layout;
 #pragma unroll
             for (int sh = 0; sh < LY::NSHELL; ++sh) {
                 const int I = LY::nuc(sh), p0 = LY::p0(sh), a = LY::ao0(sh);
                 const bool has_p = LY::kind(sh) == 2;
-                if (only_nuc >= 0 && only_nuc != I) continue;
                 T dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
                 T r2 = dx * dx + dy * dy + dz * dz;
                 T a0 = 0, b0 = 0, c0 = 0, ap = 0, bp = 0, cpp = 0;
@@ -289,15 +267,14 @@ struct MOEval {
                 gto_shell(S, a, has_p, a0, b0, c0, ap, bp, cpp, dx, dy, dz, r2);
             }
         } else {
-            run_tables(S, x, y, z, only_nuc);
+            run_tables(S, x, y, z);
         }
     }
 
     // Table-driven shells (runtime shell and primitive counts).
-    __device__ __forceinline__ void run_tables(const SysT<SH, T>& S, T x, T y, T z, int only_nuc) {
+    __device__ __forceinline__ void run_tables(const SysT<SH, T>& S, T x, T y, T z) {
 #pragma unroll
         for (int I = 0; I < SH::NNUC; ++I) {
-            if (only_nuc >= 0 && only_nuc != I) continue;
             T dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
             T r2 = dx * dx + dy * dy + dz * dz;
             for (int sh = S.sh_start[I]; sh < S.sh_start[I + 1]; ++sh) {

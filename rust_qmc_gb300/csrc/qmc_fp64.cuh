@@ -99,11 +99,11 @@ __device__ __forceinline__ double d_exp(double x) {
     const double kd = d_of_float(kf);
     double r = fma(kd, -0x1.62e42fee00000p-9, x);
     r = fma(kd, -0x1.a39ef35793c76p-41, r);
-    const double t = kExp2T[n & 255];
+    const double2 t = kExp2T[n & 255];
     double p = fma(r, 1.0 / 24.0, 1.0 / 6.0 + 1.3288e-8);
     p = fma(r, p, 0.5);
     const double s = fma(r * r, p, r);
-    const double v = d_scale(fma(t, s, t), n >> 8);
+    const double v = d_scale(t.x + fma(t.x, s, t.y), n >> 8);
     if (!out) return v;
     return mag > 0x7ff00000 ? x : (hi < 0 ? 0.0 : __hiloint2double(0x7ff00000, 0));
 }

@@ -52,9 +52,9 @@ struct HostSys {
     std::vector<double> kvec;            // periodic electron gas: [n_mo*3] orbital wave vectors
     int version = 0;                     // bumped when parameters or nuclei change
     // cached device copies of the system table per arithmetic type:
-    // [0] FP64, [1] FP32, [2] float-float
-    mutable void* dev_table[3] = {nullptr, nullptr, nullptr};
-    mutable int dev_table_version[3] = {-1, -1, -1};
+    // [0] FP64, [1] FP32, [2] float-float; [3] the FP64 team kernels' table
+    mutable void* dev_table[4] = {nullptr, nullptr, nullptr, nullptr};
+    mutable int dev_table_version[4] = {-1, -1, -1, -1};
 
     int n_params() const { return 8 + (int)rot_occ.size(); }
     // Effective (rotated) MO coefficients in caller AO order.
@@ -122,6 +122,11 @@ int launch_measure(const HostSys& hs, DevWalkers& dw, int compute_prec, bool wri
                    const MeasureOut& out, cudaStream_t st);
 int launch_sweep(const HostSys& hs, DevWalkers& dw, int move_kind, int n_sweeps, uint64_t step0,
                  double step, double tau, double max_drift, uint64_t seed, cudaStream_t st);
+// All-electron steps; with `partial` the per-step E_L sums of step_all_blocks()
+// blocks, [n][blocks] compensated pairs.
+int launch_step_all(const HostSys& hs, DevWalkers& dw, int move_kind, int n, uint64_t s0, double step, uint64_t seed,
+                    double* partial, cudaStream_t st);
+int step_all_blocks(const HostSys& hs, const DevWalkers& dw);
 // FP64 compensated sums.  Sums column c of X (row-major [W][ncol]) into
 // out[c]; when `products` is set also out[ncol + ...] = sum of the pairwise
 // products used by the SR matrices (see qmc_kernels.cu).

@@ -3,4 +3,5 @@
 
 namespace qmc {
 QMC_DEFINE_SHAPE_MEASURE(ch4min, ShapeCH4Min)
+QMC_DEFINE_SHAPE_TEAM_STEPS(ch4min, ShapeCH4Min)
 }  // namespace qmc

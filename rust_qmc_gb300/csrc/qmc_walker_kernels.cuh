@@ -2,14 +2,14 @@
 // (sm_103a), instantiated once per system shape in qmc_shape_*.cu.
 //
 //   k_init       MultiWfn::initialize for every walker (Philox, tag 3)
-//   k_measure    full evaluation from positions: AO->MO, Gauss-Jordan inverse
-//                and log-determinant, Jastrow, grad/Laplacian, E_L, optional
-//                parameter log-derivatives and nuclear forces.  In FP64 it is
-//                the refresh of the FP32 walkers (inverse + E_L every N sweeps)
+//   k_measure    plain FP32 evaluation from positions: AO->MO, Gauss-Jordan
+//                inverse and log-determinant, Jastrow, grad/Laplacian, E_L
+//                (FP64 walkers: qmc_team_kernels.cuh)
+//   k_rows, k_assemble  the FP64-class refresh of FP32 walkers
 //   k_sweep_one  single-electron Metropolis / Langevin sweeps with
 //                Sherman-Morrison inverse updates, n sweeps per launch, walker
 //                state resident in shared memory for the whole launch
-//   k_step_all   all-electron Metropolis steps (H2 path of MCMCSimulation)
+//   k_step_all   all-electron Metropolis steps of FP32 walkers (MCMCSimulation)
 #pragma once
 #include <cstdio>
 #include <cstring>
@@ -19,6 +19,7 @@
 #include <utility>
 #include "qmc_internal.h"
 #include "qmc_device.cuh"
+#include "qmc_team_kernels.cuh"
 
 namespace qmc {
 
@@ -35,8 +36,6 @@ static bool fill_sys(const HostSys& hs, SysT<SH, T>& S) {
         for (int c = 0; c < 3; ++c) S.nuc[I][c] = (T)hs.R[3 * I + c];
         S.Z[I] = (T)hs.Z[I];
         int sp = hs.species[I];
-        S.species[I] = sp;
-        S.Aspec[I] = (T)hs.jas[6 + sp];
         S.enA[I] = (T)(hs.jas[6 + sp] * hs.Z[I]);
         S.enB[I] = (T)hs.jas[4 + sp];
     }
@@ -47,7 +46,6 @@ static bool fill_sys(const HostSys& hs, SysT<SH, T>& S) {
     S.qa = (hs.quirks & 1) ? (T)hs.F : (T)1;
     S.quirk_lap = (hs.quirks & 2) ? 1 : 0;
     S.v_nn = (T)hs.v_nn;
-    S.n_rot = (int)hs.rot_occ.size();
     // shells (already sorted by nucleus)
     int np = 0;
     for (int I = 0; I <= SH::NNUC; ++I) S.sh_start[I] = 0;
@@ -81,20 +79,6 @@ static bool fill_sys(const HostSys& hs, SysT<SH, T>& S) {
             int k = hs.occ[e];
             for (int a = 0; a < hs.n_ao; ++a) S.C[sig][hs.ao_int[a]][col] = (T)Ce[(size_t)k * hs.n_ao + a];
             ++col;
-        }
-    }
-    std::vector<double> dC = hs.rotation_derivative_rows();
-    for (size_t q = 0; q < hs.rot_occ.size(); ++q) {
-        for (int a = 0; a < hs.n_ao; ++a) S.dC[q][hs.ao_int[a]] = (T)dC[q * hs.n_ao + a];
-        for (int sig = 0; sig < 2; ++sig) {
-            S.rot_col[q][sig] = -1;
-            int col = 0;
-            for (int ei = 0; ei < hs.N; ++ei) {
-                int e = hs.perm[ei];
-                if ((hs.spins[e] > 0) != (sig == 0)) continue;
-                if (hs.occ[e] == hs.rot_occ[q]) S.rot_col[q][sig] = col;
-                ++col;
-            }
         }
     }
     S.init_sigma = (T)hs.init_sigma;
@@ -328,54 +312,31 @@ __device__ __forceinline__ void pair_cache_store(T* pc, int e, const T (&un)[SH:
 // ---------------------------------------------------------------------------
 // Full evaluation of one configuration in precision TC.
 // ---------------------------------------------------------------------------
-template <class SH, class TC, int NR>
+template <class SH, class TC>
 struct FullEval {
     double logabs;
     int sign;
     bool ok;
     TC el;
     TC gx[SH::NE], gy[SH::NE], gz[SH::NE], lap[SH::NE];   // grad psi/psi, lap psi/psi
-    TC O[8 + (NR > 0 ? NR : 1)];
-    TC dE[NR > 0 ? NR : 1];                               // d E_L / d theta_q (DEL evaluations)
 };
 
-// One spin sector.  With DEL (and NR > 0) it also accumulates into dErot the
-// rotation-angle derivatives of the local energy: for column c of the sector
-// rotated by theta_q, with B = A^-1, beta = B (d phi_c / d theta)(r_.),
-//   d (X B)_ii = X_psi(r_i) B_ci - B_ci sum_k X_k(r_i) beta_k   (X = grad, lap),
-//   d E_L / d theta_q += -1/2 sum_i [ d (L B)_ii + 2 d (G B)_ii . j_i ],
-// j_i the Jastrow gradient of electron i (gjx, gjy, gjz).
-template <class SH, class TC, int SIG, int NR, class DinvStore, bool DEL = false>
+// One spin sector.
+template <class SH, class TC, int SIG, class DinvStore>
 __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], double& logdet,
                                             int& sg, bool& ok, TC (&gdx)[SH::NE], TC (&gdy)[SH::NE],
-                                            TC (&gdz)[SH::NE], TC (&ld)[SH::NE], TC* Orot,
-                                            DinvStore store, TC* omega, const TC* gjx = nullptr,
-                                            const TC* gjy = nullptr, const TC* gjz = nullptr,
-                                            TC* dErot = nullptr) {
+                                            TC (&gdz)[SH::NE], TC (&ld)[SH::NE], DinvStore store) {
     constexpr int NS = SIG == 0 ? SH::NUP : SH::NDN;
     if (NS == 0) return;
     constexpr int NSa = NS > 0 ? NS : 1;
-    constexpr bool WD = DEL && NR > 0;
-    constexpr int NRa = NR > 0 ? NR : 1;
-    constexpr int NRD = WD ? NRa : 1;
     TC D[NSa][NSa], Gx[NSa][NSa], Gy[NSa][NSa], Gz[NSa][NSa], L[NSa][NSa];
-    TC dvr[NSa][NRa];
-    TC dgxr[NSa][NRD], dgyr[NSa][NRD], dgzr[NSa][NRD], dlr[NSa][NRD];
 #pragma unroll 1
     for (int q = 0; q < NS; ++q) {
         const int e = SIG * SH::NUP + q;
-        MOEval<SH, TC, SIG, WD ? 3 : 2, NR> m;
+        MOEval<SH, TC, SIG, 2> m;
         m.run(S, r[e][0], r[e][1], r[e][2]);
 #pragma unroll
         for (int k = 0; k < NS; ++k) { D[q][k] = m.v[k]; Gx[q][k] = m.gx[k]; Gy[q][k] = m.gy[k]; Gz[q][k] = m.gz[k]; L[q][k] = m.l[k]; }
-#pragma unroll
-        for (int qq = 0; qq < NR; ++qq) dvr[q][qq] = m.dv[qq];
-        if constexpr (WD) {
-#pragma unroll
-            for (int qq = 0; qq < NR; ++qq) {
-                dgxr[q][qq] = m.dgx[qq]; dgyr[q][qq] = m.dgy[qq]; dgzr[q][qq] = m.dgz[qq]; dlr[q][qq] = m.dl[qq];
-            }
-        }
     }
     TC Di[NSa][NSa];
     double lg;
@@ -398,81 +359,15 @@ __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)
         }
         gdx[e] = ax; gdy[e] = ay; gdz[e] = az; ld[e] = al;
     }
-    if (NR > 0 && Orot) {
-#pragma unroll
-        for (int qq = 0; qq < NR; ++qq) {
-            if (qq >= S.n_rot) continue;
-            int c = S.rot_col[qq][SIG];
-            TC acc = 0;
-#pragma unroll
-            for (int cc = 0; cc < NS; ++cc) {
-                if (cc != c) continue;
-#pragma unroll
-                for (int row = 0; row < NS; ++row) acc += Di[cc][row] * dvr[row][qq];
-            }
-            Orot[qq] += acc;
-        }
-    }
-    if constexpr (WD) {
-#pragma unroll 1
-        for (int qq = 0; qq < NR; ++qq) {
-            if (qq >= S.n_rot) continue;
-            const int c = S.rot_col[qq][SIG];
-            if (c < 0) continue;
-            TC beta[NSa];
-#pragma unroll
-            for (int col = 0; col < NS; ++col) {
-                TC b = 0;
-#pragma unroll
-                for (int row = 0; row < NS; ++row) b += Di[col][row] * dvr[row][qq];
-                beta[col] = b;
-            }
-            TC acc = 0;
-#pragma unroll
-            for (int q = 0; q < NS; ++q) {
-                const int e = SIG * SH::NUP + q;
-                TC bci = 0;
-#pragma unroll
-                for (int cc = 0; cc < NS; ++cc) bci = (cc == c) ? Di[cc][q] : bci;
-                TC tx = 0, ty = 0, tz = 0, tl = 0;
-#pragma unroll
-                for (int col = 0; col < NS; ++col) {
-                    tx += Gx[q][col] * beta[col]; ty += Gy[q][col] * beta[col];
-                    tz += Gz[q][col] * beta[col]; tl += L[q][col] * beta[col];
-                }
-                const TC dgx = bci * (dgxr[q][qq] - tx), dgy = bci * (dgyr[q][qq] - ty);
-                const TC dgz = bci * (dgzr[q][qq] - tz), dl = bci * (dlr[q][qq] - tl);
-                acc += dl + 2 * (dgx * gjx[e] + dgy * gjy[e] + dgz * gjz[e]);
-            }
-            dErot[qq] += TC(-0.5) * acc;
-        }
-    }
-    if (omega) {
-        // d ln|D| / dR_I = -sum_rows sum_k Dinv[k][row] sum_{a on I} C[k][a] grad chi_a(r_row)
-#pragma unroll 1
-        for (int q = 0; q < NS; ++q) {
-            const int e = SIG * SH::NUP + q;
-#pragma unroll
-            for (int I = 0; I < SH::NNUC; ++I) {
-                MOEval<SH, TC, SIG, 1, 0> m;
-                m.run(S, r[e][0], r[e][1], r[e][2], I);
-                TC ox = 0, oy = 0, oz = 0;
-#pragma unroll
-                for (int k = 0; k < NS; ++k) { ox += Di[k][q] * m.gx[k]; oy += Di[k][q] * m.gy[k]; oz += Di[k][q] * m.gz[k]; }
-                omega[3 * I] -= ox; omega[3 * I + 1] -= oy; omega[3 * I + 2] -= oz;
-            }
-        }
-    }
 }
 
 // Jastrow over all pairs: u, grad_i u (true gradient), sum_j (u''+2u'/r),
-// sum_j u'^2 (for the per-pair Laplacian quirk), parameter derivatives, and
-// the Coulomb potential V_ee + V_en + V_nn from the same distances (one
+// sum_j u'^2 (for the per-pair Laplacian quirk), and the Coulomb potential V_ee + V_en + V_nn from the same distances (one
 // reciprocal square root per pair).
-template <class SH, class TC, bool WANT_O>
+template <class SH, class TC>
 __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], TC (&gx)[SH::NE],
                                               TC (&gy)[SH::NE], TC (&gz)[SH::NE], TC (&lu)[SH::NE],
-                                              TC (&gsq)[SH::NE], TC* O, TC& V) {
+                                              TC (&gsq)[SH::NE], TC& V) {
     TC u = 0;
     V = S.v_nn;
 #pragma unroll
@@ -500,11 +395,6 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
                 TC up = upr * d;
                 gsq[i] += up * up; gsq[j] += up * up;
             }
-            if (WANT_O && SH::JAS == JAS_PADE_EEN) {
-                TC inv = recip_full(1 + S.b_ee[c] * d);
-                O[c] += -S.a_ee[c] * d * d * inv * inv;
-                O[2 + c] += d * inv;
-            }
         }
 #pragma unroll
     for (int i = 0; i < SH::NE; ++i)
@@ -522,37 +412,22 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
                 gx[i] -= upr * dx; gy[i] -= upr * dy; gz[i] -= upr * dz;
                 lu[i] -= lt;
             }
-            if (WANT_O) {
-                TC inv = recip_full(1 + S.enB[I] * d);
-                TC dB = S.Aspec[I] * S.Z[I] * d * d * inv * inv;
-                TC dA = -S.Z[I] * d * inv;
-                if (S.species[I] == 0) { O[4] += dB; O[6] += dA; }
-                else { O[5] += dB; O[7] += dA; }
-            }
         }
     return u;
 }
 
-template <class SH, class TC, int NR, class DinvStore, bool DEL = false>
-__device__ __forceinline__ void evaluate_config(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3],
-                                                FullEval<SH, TC, NR>& out, bool want_o, DinvStore store,
-                                                TC* omega) {
+template <class SH, class TC, class DinvStore>
+__device__ __forceinline__ void evaluate_config(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], FullEval<SH, TC>& out,
+                                                DinvStore store) {
     TC gjx[SH::NE], gjy[SH::NE], gjz[SH::NE], lu[SH::NE], gsq[SH::NE];
-#pragma unroll
-    for (int p = 0; p < 8 + (NR > 0 ? NR : 1); ++p) out.O[p] = 0;
-    TC u, V;
-    if (NR > 0 || want_o) u = jastrow_coulomb<SH, TC, true>(S, r, gjx, gjy, gjz, lu, gsq, out.O, V);
-    else u = jastrow_coulomb<SH, TC, false>(S, r, gjx, gjy, gjz, lu, gsq, out.O, V);
+    TC V;
+    const TC u = jastrow_coulomb<SH, TC>(S, r, gjx, gjy, gjz, lu, gsq, V);
     TC gdx[SH::NE], gdy[SH::NE], gdz[SH::NE], ld[SH::NE];
     double logdet = 0.0;
     int sg = 1;
     bool ok = true;
-#pragma unroll
-    for (int q = 0; q < (NR > 0 ? NR : 1); ++q) out.dE[q] = 0;
-    eval_sector<SH, TC, 0, NR, DinvStore, DEL>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, out.O + 8, store, omega, gjx,
-                                              gjy, gjz, out.dE);
-    eval_sector<SH, TC, 1, NR, DinvStore, DEL>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, out.O + 8, store, omega, gjx,
-                                              gjy, gjz, out.dE);
+    eval_sector<SH, TC, 0>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
+    eval_sector<SH, TC, 1>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
     TC kin = 0;
 #pragma unroll
     for (int e = 0; e < SH::NE; ++e) {
@@ -591,15 +466,15 @@ __global__ void k_init(const __grid_constant__ SysT<SH, double> S, TS* __restric
     }
 }
 
-// Full evaluation of walker w (refresh of the inverse, log|psi|, E_L and the
-// requested extras); returns E_L (0 for an inactive lane, which still runs the
-// arithmetic on a dummy configuration so that the block stays converged).
-template <class SH, class TC, class TS, int NR, bool DEL = false>
+// Full evaluation of walker w in FP32 (the inverse, log|psi|, E_L and, when asked
+// for, gradients and Laplacians); returns E_L (0 for an inactive lane, which
+// still runs the arithmetic on a dummy configuration so that the block stays
+// converged).
+template <class SH, class TC, class TS>
 __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS* __restrict__ pos,
                                                  TS* __restrict__ dinv, double* __restrict__ logabs,
                                                  int* __restrict__ sign, double* __restrict__ el, int w, bool act,
-                                                 int Wcap, int write_state, const MeasureOut& out, int P,
-                                                 int* flags) {
+                                                 int Wcap, int write_state, const MeasureOut& out, int* flags) {
     TC r[SH::NE][3];
 #pragma unroll
     for (int e = 0; e < SH::NE; ++e)
@@ -609,12 +484,8 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
     auto store = [&](int sig, int k, int j, TC v) {
         if (act && write_state) dinv[((size_t)(sig * NM * NM + k * NM + j)) * Wcap + w] = (TS)v;
     };
-    TC omega[3 * SH::NNUC];
-#pragma unroll
-    for (int i = 0; i < 3 * SH::NNUC; ++i) omega[i] = 0;
-    FullEval<SH, TC, NR> ev;
-    evaluate_config<SH, TC, NR, decltype(store), DEL>(S, r, ev, out.O != nullptr, store,
-                                                      (act && out.omega) ? omega : (TC*)nullptr);
+    FullEval<SH, TC> ev;
+    evaluate_config<SH, TC>(S, r, ev, store);
     double e_l = (double)ev.el;
     if (act) {
         int fl = 0;
@@ -634,65 +505,18 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
 #pragma unroll
             for (int e = 0; e < SH::NE; ++e) out.lap[(size_t)w * SH::NE + e] = (double)ev.lap[e];
         }
-        if (out.O) {
-            for (int p = 0; p < P; ++p) out.O[(size_t)w * P + p] = (double)ev.O[p];
-        }
-        if (DEL && out.dEL) {
-            // rotation columns; the Jastrow columns 0..7 come from k_jastrow3_logderiv
-            for (int p = 8; p < P; ++p) out.dEL[(size_t)w * P + p] = (double)ev.dE[p - 8];
-        }
-        if (out.fhf) {
-#pragma unroll
-            for (int I = 0; I < SH::NNUC; ++I) {
-                TC fx = 0, fy = 0, fz = 0;
-#pragma unroll
-                for (int i = 0; i < SH::NE; ++i) {
-                    TC dx = r[i][0] - S.nuc[I][0], dy = r[i][1] - S.nuc[I][1], dz = r[i][2] - S.nuc[I][2];
-                    TC d = fsqrt(dx * dx + dy * dy + dz * dz);
-                    if (d > TC(1e-10)) { TC f = S.Z[I] / (d * d * d); fx += f * dx; fy += f * dy; fz += f * dz; }
-                }
-#pragma unroll
-                for (int J = 0; J < SH::NNUC; ++J) {
-                    if (J == I) continue;
-                    TC dx = S.nuc[I][0] - S.nuc[J][0], dy = S.nuc[I][1] - S.nuc[J][1], dz = S.nuc[I][2] - S.nuc[J][2];
-                    TC d = fsqrt(dx * dx + dy * dy + dz * dz);
-                    if (d > TC(1e-10)) { TC f = S.Z[I] * S.Z[J] / (d * d * d); fx -= f * dx; fy -= f * dy; fz -= f * dz; }
-                }
-                out.fhf[((size_t)w * SH::NNUC + I) * 3 + 0] = (double)fx;
-                out.fhf[((size_t)w * SH::NNUC + I) * 3 + 1] = (double)fy;
-                out.fhf[((size_t)w * SH::NNUC + I) * 3 + 2] = (double)fz;
-            }
-        }
-        if (out.omega) {
-            if (SH::JAS == JAS_PADE_EEN) {
-#pragma unroll
-                for (int I = 0; I < SH::NNUC; ++I)
-#pragma unroll
-                    for (int i = 0; i < SH::NE; ++i) {
-                        TC dx = r[i][0] - S.nuc[I][0], dy = r[i][1] - S.nuc[I][1], dz = r[i][2] - S.nuc[I][2];
-                        TC d = fsqrt(dx * dx + dy * dy + dz * dz);
-                        if (d < TC(1e-10)) continue;
-                        TC den = 1 + S.enB[I] * d;
-                        TC f = S.enA[I] / (d * den * den);
-                        omega[3 * I] += f * dx; omega[3 * I + 1] += f * dy; omega[3 * I + 2] += f * dz;
-                    }
-            }
-#pragma unroll
-            for (int i = 0; i < 3 * SH::NNUC; ++i) out.omega[(size_t)w * 3 * SH::NNUC + i] = (double)omega[i];
-        }
     }
     return act ? e_l : 0.0;
 }
 
-template <class SH, class TC, class TS, int TPB, int NR, bool DEL = false>
+template <class SH, class TC, class TS, int TPB>
 __global__ void __launch_bounds__(TPB) k_measure(const __grid_constant__ SysT<SH, TC> S,
                                                  const TS* __restrict__ pos, TS* __restrict__ dinv,
                                                  double* __restrict__ logabs, int* __restrict__ sign,
                                                  double* __restrict__ el, int W, int Wcap, int write_state,
-                                                 MeasureOut out, int P, double* partial, int* flags) {
+                                                 MeasureOut out, double* partial, int* flags) {
     const int w = blockIdx.x * TPB + threadIdx.x;
-    double e_l = measure_walker<SH, TC, TS, NR, DEL>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state,
-                                                     out, P, flags);
+    double e_l = measure_walker<SH, TC, TS>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out, flags);
     if (partial) block_partial<TPB>(e_l, partial, blockIdx.x);
 }
 
@@ -811,7 +635,7 @@ template <class SH, int SIG, int MODE>
 __device__ __forceinline__ void rows_orbitals(const SysT<SH, ff>& S, ff x, ff y, ff z, ff (&v)[SH::NMAX],
                                               ff (&gx)[SH::NMAX], ff (&gy)[SH::NMAX], ff (&gz)[SH::NMAX],
                                               ff (&l)[SH::NMAX]) {
-    MOEval<SH, ff, SIG, MODE, 0> m;
+    MOEval<SH, ff, SIG, MODE> m;
     m.run(S, x, y, z);
 #pragma unroll
     for (int k = 0; k < SH::NMAX; ++k) { v[k] = m.v[k]; gx[k] = m.gx[k]; gy[k] = m.gy[k]; gz[k] = m.gz[k]; l[k] = m.l[k]; }
@@ -1115,7 +939,7 @@ __device__ __forceinline__ void sweep_sector(const SysT<SH, T>& S, T* sp, T* sd,
         if (MOVE == MOVE_ONE_DRIFT) {
             // drift at the current position: grad ln D (from the current
             // inverse) + grad u; then the Langevin proposal
-            MOEval<SH, T, SIG, 1, 0> mc;
+            MOEval<SH, T, SIG, 1> mc;
             mc.run(S, rx, ry, rz);
             T ax = 0, ay = 0, az = 0;
 #pragma unroll
@@ -1128,7 +952,7 @@ __device__ __forceinline__ void sweep_sector(const SysT<SH, T>& S, T* sp, T* sd,
             if (m > maxd) { T s = maxd / m; dlx *= s; dly *= s; dlz *= s; }
             T sd2 = fsqrt(2 * tau);
             nx = rx + dlx + sd2 * n0; ny = ry + dly + sd2 * n1; nz = rz + dlz + sd2 * n2;
-            MOEval<SH, T, SIG, 1, 0> mn;
+            MOEval<SH, T, SIG, 1> mn;
             mn.run(S, nx, ny, nz);
 #pragma unroll
             for (int k = 0; k < NS; ++k) { R += mn.v[k] * DI(k, q); mv[k] = mn.v[k]; }
@@ -1146,7 +970,7 @@ __device__ __forceinline__ void sweep_sector(const SysT<SH, T>& S, T* sp, T* sd,
             logG = ((fx * fx + fy * fy + fz * fz) - (qx * qx + qy * qy + qz * qz)) / (4 * tau);
         } else {
             nx = rx + step * n0; ny = ry + step * n1; nz = rz + step * n2;
-            MOEval<SH, T, SIG, 0, 0> mn;
+            MOEval<SH, T, SIG, 0> mn;
             mn.run(S, nx, ny, nz);
 #pragma unroll
             for (int k = 0; k < NS; ++k) { R += mn.v[k] * DI(k, q); mv[k] = mn.v[k]; }
@@ -1427,32 +1251,7 @@ __global__ void __launch_bounds__(TPB, (sizeof(T) == 4 ? 512 : 256) / TPB) kb_sw
     if (flg) atomicOr(a.flags, flg);
 }
 
-// Batched refresh + E_L (compute type TC) with one compensated partial per tile.
-template <class SH, class TC, class TS, int TPB>
-__global__ void __launch_bounds__(TPB) kb_measure(const BatchTile* __restrict__ tiles, int ntiles,
-                                                  const BatchRec* __restrict__ recs, double* tile_partial) {
-    __shared__ __align__(16) unsigned char sraw[batch_table_bytes<SH, TC>()];
-    SysT<SH, TC>& S = *reinterpret_cast<SysT<SH, TC>*>(sraw);
-    int t0, t1;
-    batch_tile_range(ntiles, t0, t1);
-    int cur = -1;
-    for (int ti = t0; ti < t1; ++ti) {
-        const BatchTile tl = tiles[ti];
-        if (tl.rec != cur) {
-            stage_table(&S, recs[tl.rec].tab_d);   // block_partial ended the previous tile with a barrier
-            __syncthreads();
-            cur = tl.rec;
-        }
-        const BatchRec& R = recs[tl.rec];
-        const int w = tl.w0 + (int)threadIdx.x;
-        MeasureOut none;
-        double e_l = measure_walker<SH, TC, TS, 0>(S, (const TS*)R.pos, (TS*)R.dinv, R.logabs, R.sign, R.el, w,
-                                                   w < R.W, R.Wcap, 1, none, 0, R.flags);
-        block_partial<TPB>(e_l, tile_partial, ti);
-    }
-}
-
-// All-electron Metropolis steps (src/sampling/vmc.rs:95-119): every step
+// All-electron Metropolis steps of FP32 walkers (src/sampling/vmc.rs:95-119): every step
 // proposes all electrons, evaluates psi and E_L at the proposal from scratch,
 // accepts with min(1, psi'^2/psi^2).  Per-step block partial sums of E_L
 // (Neumaier pairs) are written to partial[step][block] when requested.
@@ -1494,8 +1293,8 @@ __global__ void __launch_bounds__(TPB) k_step_all(const __grid_constant__ SysT<S
                 rn[e][2] = r[e][2] + step * (to_u01(x.z, T(0)) - T(0.5));
             }
         }
-        FullEval<SH, T, 0> ev;
-        evaluate_config<SH, T, 0>(S, rn, ev, false, nostore, (T*)nullptr);
+        FullEval<SH, T> ev;
+        evaluate_config<SH, T>(S, rn, ev, nostore);
         U4 a = rng_draw(seed, (uint32_t)w, st, 0, TAG_ACCEPT);
         double prob = d_exp(2.0 * (ev.logabs - lp));
         bool accept = act && ev.ok && (to_u01(a.x, 0.0) < prob);
@@ -1550,17 +1349,17 @@ struct ShapeOps {
         return cuda_status(cudaGetLastError());
     }
 
-    template <class TC, class TS, int NR, bool DEL = false>
-    static int measure2(const HostSys& hs, DevWalkers& dw, bool write_state, const MeasureOut& out, cudaStream_t st) {
-        SysT<SH, TC> S;
+    // Plain FP32 evaluation of FP32 walkers.
+    static int measure1(const HostSys& hs, DevWalkers& dw, bool write_state, const MeasureOut& out, cudaStream_t st) {
+        SysT<SH, float> S;
         if (!fill_sys(hs, S)) return 7;
         constexpr int TPB = 64;
         int nb = (dw.W + TPB - 1) / TPB;
         double* partial = nullptr;
         if (write_state && dw.partial && dw.partial_cap >= 2 * nb + 1) partial = dw.partial;
-        k_measure<SH, TC, TS, TPB, NR, DEL><<<nb, TPB, 0, st>>>(S, (const TS*)dw.pos, (TS*)dw.dinv, dw.logabs, dw.sign,
-                                                            dw.el, dw.W, dw.Wcap, write_state ? 1 : 0, out,
-                                                            hs.n_params(), partial, dw.flags);
+        k_measure<SH, float, float, TPB><<<nb, TPB, 0, st>>>(S, (const float*)dw.pos, (float*)dw.dinv, dw.logabs,
+                                                             dw.sign, dw.el, dw.W, dw.Wcap, write_state ? 1 : 0, out,
+                                                             partial, dw.flags);
         ++g_launch_count;
         int rc = cuda_status(cudaGetLastError());
         if (rc || !partial) return rc;
@@ -1590,22 +1389,16 @@ struct ShapeOps {
         return launch_sum_partials(partial, nb, 1, dw.partial + dw.partial_cap - 1, st);
     }
 
+    // FP64 walkers: a team of lanes per walker (qmc_team_kernels.cuh).
+    using Teams = TeamOps<SH, SH::NE == 2 ? 4 : (SH::NE == 3 ? 8 : 32)>;
+
     static int measure(const HostSys& hs, DevWalkers& dw, int cp, bool ws, const MeasureOut& out, cudaStream_t st) {
-        if (out.O) {
-            if (SH::JAS != JAS_PADE_EEN || cp != 0 || dw.prec != 0) return 7;
-            if (out.dEL) return measure2<double, double, SH::NROT, true>(hs, dw, ws, out, st);
-            return measure2<double, double, SH::NROT>(hs, dw, ws, out, st);
-        }
-        if (cp == 0) {
-            if (dw.prec == 0) return measure2<double, double, 0>(hs, dw, ws, out, st);
-            // FP64-class refresh on the FP32 pipe: the two-pass form when only
-            // the walker state is wanted, else the single-kernel form
-            if (dw.rows && !out.grad && !out.lap && !out.fhf && !out.omega)
-                return out.inverse_only ? measure_split<true>(hs, dw, ws, st) : measure_split<false>(hs, dw, ws, st);
-            return measure2<ff, float, 0>(hs, dw, ws, out, st);
-        }
-        if (dw.prec == 1) return measure2<float, float, 0>(hs, dw, ws, out, st);
-        return 7;
+        if (cp == 0 && dw.prec == 0) return Teams::measure(hs, dw, ws, out, st);
+        if (dw.prec == 0 || out.O || out.fhf || out.omega) return 7;
+        if (cp != 0) return measure1(hs, dw, ws, out, st);
+        // FP64-class refresh on the FP32 pipe in two passes
+        if (!dw.rows || out.grad || out.lap) return 7;
+        return out.inverse_only ? measure_split<true>(hs, dw, ws, st) : measure_split<false>(hs, dw, ws, st);
     }
 
     template <class T, int MOVE>
@@ -1686,6 +1479,9 @@ struct ShapeOps {
         return true;
     }
 
+    // All-electron steps with E_L recorded in partial (block partials) when given.
+    static int step_blocks(const DevWalkers& dw) { return dw.prec == 0 ? Teams::step_blocks(dw.W) : (dw.W + 63) / 64; }
+
     template <class T, int MOVE>
     static int step_all(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, uint64_t seed,
                         cudaStream_t st, double* partial) {
@@ -1718,15 +1514,18 @@ struct ShapeOps {
         return 0;
     }
 
-    // tab_s: the sweep table (walker precision); tab_d: the refresh table
-    // (FP64 for FP64 walkers, float-float for FP32 walkers).
+    // tab_s: the sweep table (walker precision); tab_d: the refresh table (the
+    // team table for FP64 walkers, float-float for FP32 walkers).
     static int batch_tables(const HostSys& hs, int prec, BatchRec& r) {
         r.ktab = nullptr;
         if (prec == 0) {
             const SysT<SH, double>* d;
+            const TeamTab<SH>* t;
             int rc = table<double>(hs, &d);
+            if (!rc) rc = Teams::table(hs, &t);
             if (rc) return rc;
-            r.tab_d = r.tab_s = d;
+            r.tab_s = d;
+            r.tab_d = t;
             return 0;
         }
         const SysT<SH, ff>* m;
@@ -1771,18 +1570,6 @@ struct ShapeOps {
         return 7;
     }
 
-    template <class TC, class TS>
-    static int batch_measure_t(const BatchClass& bc, cudaStream_t st, int* occ) {
-        auto kern = kb_measure<SH, TC, TS, BTPB>;
-        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, BTPB, 0) == cudaSuccess ? 0 : 2;
-        if (bc.ntiles == 0) return 0;
-        const int grid =
-            bc.grid_measure > 0 ? (bc.grid_measure < bc.ntiles ? bc.grid_measure : bc.ntiles) : bc.ntiles;
-        kern<<<grid, BTPB, 0, st>>>(bc.tiles, bc.ntiles, bc.recs, bc.tile_partial);
-        ++g_launch_count;
-        return cuda_status(cudaGetLastError());
-    }
-
     // FP32 walkers: the two-pass float-float refresh (rows, then assembly).
     static int batch_measure_split(const BatchClass& bc, cudaStream_t st, int* occ) {
         auto k1 = kb_rows<SH, float, BTPB>;
@@ -1811,7 +1598,7 @@ struct ShapeOps {
     }
 
     static int batch_measure(const BatchClass& bc, cudaStream_t st, int* occ = nullptr) {
-        return bc.prec == 0 ? batch_measure_t<double, double>(bc, st, occ) : batch_measure_split(bc, st, occ);
+        return bc.prec == 0 ? Teams::template batch_measure<BTPB>(bc, st, occ) : batch_measure_split(bc, st, occ);
     }
 
     template <bool ALL>
@@ -1820,8 +1607,6 @@ struct ShapeOps {
         bool all = (mk == MOVE_ALL_GAUSS || mk == MOVE_ALL_BOX);
         if (all != ALL) return 1;
         if (ALL) {
-            if (dw.prec == 0) return mk == MOVE_ALL_BOX ? step_all<double, MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, st, partial)
-                                                        : step_all<double, MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, st, partial);
             return mk == MOVE_ALL_BOX ? step_all<float, MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, st, partial)
                                       : step_all<float, MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, st, partial);
         }
@@ -1862,6 +1647,15 @@ struct ShapeOps {
     }                                                                                                         \
     int shape_batch_width_##NAME() { return ShapeOps<SHAPE>::BTPB; }
 
+// All-electron steps: FP64 walkers by teams, FP32 walkers a thread per walker.
+#define QMC_DEFINE_SHAPE_TEAM_STEPS(NAME, SHAPE)                                                               \
+    int shape_team_steps_##NAME(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64_t s0, double step,  \
+                                uint64_t seed, cudaStream_t st, double* partial) {                            \
+        using TO = ShapeOps<SHAPE>::Teams;                                                                    \
+        return mk == MOVE_ALL_BOX ? TO::steps<MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, partial, st)           \
+                                  : TO::steps<MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, partial, st);        \
+    }                                                                                                         \
+    int shape_step_blocks_##NAME(const DevWalkers& dw) { return ShapeOps<SHAPE>::step_blocks(dw); }
 #define QMC_DEFINE_SHAPE_ALL(NAME, SHAPE)                                                                      \
     int shape_step_all_##NAME(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64_t s0, double step,    \
                               uint64_t seed, cudaStream_t st, double* partial) {                              \
