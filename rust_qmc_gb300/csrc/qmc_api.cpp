@@ -303,11 +303,12 @@ int ensure_dmc(qmc_walkers_s* wk) {
     DevBranch& b = wk->br;
     int cap = wk->dw.Wcap;
     cudaError_t e = cudaMalloc((void**)&b.counts, 4 * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b.offsets, 4 * (size_t)cap);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b.parent, 4 * (size_t)cap);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b.partial, 16 * (size_t)((cap + 255) / 256));
     if (e == cudaSuccess) e = cudaMalloc((void**)&b.el_old, 8 * (size_t)cap);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b.stats, 8 * 4);
     if (e != cudaSuccess) {
-        cudaFree(b.counts); cudaFree(b.offsets); cudaFree(b.el_old); cudaFree(b.stats);
+        cudaFree(b.counts); cudaFree(b.parent); cudaFree(b.partial); cudaFree(b.el_old); cudaFree(b.stats);
         b = DevBranch();
         free_dev(wk->alt);
         return cuda_rc(e);
@@ -321,7 +322,8 @@ void free_walkers(qmc_walkers_s* wk) {
     free_dev(wk->dw);
     if (wk->br.cap) {
         free_dev(wk->alt);
-        cudaFree(wk->br.counts); cudaFree(wk->br.offsets); cudaFree(wk->br.el_old); cudaFree(wk->br.stats);
+        cudaFree(wk->br.counts); cudaFree(wk->br.parent); cudaFree(wk->br.partial); cudaFree(wk->br.el_old);
+        cudaFree(wk->br.stats);
     }
     cudaFree(wk->d_stage);
     cudaFree(wk->d_out);
@@ -707,7 +709,7 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     const HostSys& hs = s->hs;
     int P = hs.n_params();
     int M = 2 + 2 * P + P * (P + 1) / 2;
-    int nblk = std::min(1024, std::max(1, (W + 255) / 256));
+    int nblk = sr_blocks(W);
     // benzene (OptimizableWfn of BenzeneGTO, src/systems/benzene.rs:726-756):
     // the warp kernels give E_L, a per-walker kernel the Jastrow derivatives;
     // MO-rotation angles would need the determinant and are not compiled

@@ -86,7 +86,8 @@ struct DevWalkers {
 struct DevBranch {
     int cap = 0;
     int* counts = nullptr;               // [cap] copies per walker
-    int* offsets = nullptr;              // [cap] exclusive scan
+    int* parent = nullptr;               // [cap] source walker of each new slot
+    double* partial = nullptr;           // [2 ceil(cap / 256)] block sums of copies x E_L
     double* el_old = nullptr;            // [cap] E_L before the sweep
     double* stats = nullptr;             // [4] total copies, sum m E (compensated), flags
 };
@@ -132,6 +133,10 @@ int step_all_blocks(const HostSys& hs, const DevWalkers& dw);
 // products used by the SR matrices (see qmc_kernels.cu).
 int launch_walker_sum(const double* X, int W, int ncol, double* d_out, double* d_scratch,
                       int scratch_cap, cudaStream_t st);
+// Chunks of walkers whose sums run as blocks of their own: 32 walkers each (a
+// block's serial chain of compensated FP64 additions is what an SR batch waits
+// for), 1024 at most.
+inline int sr_blocks(int W) { return W <= 32 ? 1 : (W >= 32768 ? 1024 : (W + 31) / 32); }
 int launch_sr_sums(const double* E, const double* O, int W, int P, double* d_out,
                    double* d_scratch, int scratch_cap, cudaStream_t st);
 int launch_flush(void* buf, size_t bytes, cudaStream_t st);

@@ -189,28 +189,33 @@ __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__
 
 // SR sums: quantity m over the walkers of chunk b, Neumaier-compensated,
 // fixed order.  Quantities: 0 E, 1 E^2, 2..2+P-1 O_p, 2+P..2+2P-1 E O_p,
-// then O_p O_q for p <= q (row-major upper triangle).
-__device__ __forceinline__ double sr_quantity(int m, int P, const double* E, const double* O, int w) {
-    double e = E[w];
-    if (m == 0) return e;
-    if (m == 1) return e * e;
-    if (m < 2 + P) return O[(size_t)w * P + (m - 2)];
-    if (m < 2 + 2 * P) return e * O[(size_t)w * P + (m - 2 - P)];
-    int k = m - 2 - 2 * P;
-    int p = 0;
-    while (k >= P - p) { k -= P - p; ++p; }
-    int q = p + k;
-    return O[(size_t)w * P + p] * O[(size_t)w * P + q];
-}
-
+// then O_p O_q for p <= q (row-major upper triangle): products of two of
+// 1, E and O_p.
 __global__ void k_sr_partials(const double* __restrict__ E, const double* __restrict__ O, int W, int P, int M,
                               int chunk, double* __restrict__ partial, int nblk) {
-    int m = threadIdx.x;
-    int b = blockIdx.x;
+    const int m = threadIdx.x;
+    const int b = blockIdx.x;
     if (m >= M) return;
-    int w0 = b * chunk, w1 = min(W, w0 + chunk);
+    // the factors' columns: -2 one, -1 E, p >= 0 O_p
+    int f = -2, g = -1;
+    if (m == 1) f = -1;
+    else if (m >= 2 && m < 2 + P) g = m - 2;
+    else if (m >= 2 + P && m < 2 + 2 * P) { f = -1; g = m - 2 - P; }
+    else if (m >= 2 + 2 * P) {
+        int k = m - 2 - 2 * P, p = 0;
+        while (k >= P - p) { k -= P - p; ++p; }
+        f = p;
+        g = p + k;
+    }
+    const double* pf = f < 0 ? E : O + f;
+    const double* pg = g < 0 ? E : O + g;
+    const size_t sf = f < 0 ? 1 : P, sg = g < 0 ? 1 : P;
+    const int w0 = b * chunk, w1 = min(W, w0 + chunk);
     Comp acc{0.0, 0.0};
-    for (int w = w0; w < w1; ++w) acc = comp_add(acc, Comp{sr_quantity(m, P, E, O, w), 0.0});
+    for (int w = w0; w < w1; ++w) {
+        const double x = pg[sg * w];
+        acc = comp_add(acc, Comp{f == -2 ? x : pf[sf * w] * x, 0.0});
+    }
     partial[((size_t)m * nblk + b) * 2] = acc.s;
     partial[((size_t)m * nblk + b) * 2 + 1] = acc.c;
 }
@@ -224,7 +229,7 @@ __global__ void k_flush(uint4* buf, size_t n, unsigned v) {
 int launch_sr_sums(const double* E, const double* O, int W, int P, double* d_out, double* d_scratch,
                    int scratch_cap, cudaStream_t st) {
     int M = 2 + 2 * P + P * (P + 1) / 2;
-    int nblk = std::min(1024, std::max(1, (W + 255) / 256));
+    int nblk = sr_blocks(W);
     int chunk = (W + nblk - 1) / nblk;
     nblk = (W + chunk - 1) / chunk;
     if ((size_t)2 * M * nblk > (size_t)scratch_cap) return 8;
@@ -543,43 +548,48 @@ int launch_sum_partials(const double* partial, int nblk, int nrows, double* out,
 // ---------------------------------------------------------------------------
 // Copies per walker: m = min(floor(exp(tau (E_ref - (E_L + E_old)/2)) + xi), 3),
 // FP64 log-weight, xi from the tag-4 Philox draw of (walker slot, step).
-// Walkers with a non-finite energy get no copy.
-__global__ void k_branch_counts(const double* __restrict__ el, const double* __restrict__ el_old, int W,
-                                double e_ref, double tau, double e_cut, uint64_t seed, uint64_t step,
-                                int* __restrict__ counts, int* flags) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= W) return;
-    double e = el[w], eo = el_old[w];
-    int m = 0;
-    if (isfinite(e) && isfinite(eo)) {
-        double eb = 0.5 * (e + eo);
-        if (e_cut > 0.0) eb = fmin(e_ref + e_cut, fmax(e_ref - e_cut, eb));
-        double logw = tau * (e_ref - eb);
-        U4 x = rng_draw(seed, (uint32_t)w, step, 0, TAG_BRANCH);
-        double f = floor(exp(logw) + to_u01(x.x, 0.0));
-        m = f >= 3.0 ? 3 : (f <= 0.0 ? 0 : (int)f);
-    } else {
-        atomicOr(flags, FLAG_NONFINITE);
+// Walkers with a non-finite energy get no copy.  Each block also leaves the
+// compensated sum of its copies x E_L (a block per 256 walkers: the FP64 work of
+// one block over all of them took 25 us at 8192 walkers).
+constexpr int BRANCH_TPB = 256;
+__global__ void __launch_bounds__(BRANCH_TPB) k_branch_counts(const double* __restrict__ el,
+                                                              const double* __restrict__ el_old, int W, double e_ref,
+                                                              double tau, double e_cut, uint64_t seed, uint64_t step,
+                                                              int* __restrict__ counts, double* __restrict__ partial,
+                                                              int* flags) {
+    const int w = blockIdx.x * BRANCH_TPB + threadIdx.x;
+    double me = 0.0;
+    if (w < W) {
+        const double e = el[w], eo = el_old[w];
+        int m = 0;
+        if (isfinite(e) && isfinite(eo)) {
+            double eb = 0.5 * (e + eo);
+            if (e_cut > 0.0) eb = fmin(e_ref + e_cut, fmax(e_ref - e_cut, eb));
+            const double logw = tau * (e_ref - eb);
+            const U4 x = rng_draw(seed, (uint32_t)w, step, 0, TAG_BRANCH);
+            const double f = floor(exp(logw) + to_u01(x.x, 0.0));
+            m = f >= 3.0 ? 3 : (f <= 0.0 ? 0 : (int)f);
+            if (m) me = (double)m * e;
+        } else {
+            atomicOr(flags, FLAG_NONFINITE);
+        }
+        counts[w] = m;
     }
-    counts[w] = m;
+    block_partial<BRANCH_TPB>(me, partial, blockIdx.x);
 }
 
-// One block: exclusive scan of the counts (offsets), the new population size
-// and the compensated sum of copies x E_L, in a fixed order.
-__global__ void __launch_bounds__(1024) k_branch_scan(const int* __restrict__ counts, const double* __restrict__ el,
-                                                      int W, int* __restrict__ offsets, double* __restrict__ stats) {
+// One block: exclusive scan of the counts, the source walker of every new slot
+// (parent), the new population size and, from the block partials, the
+// compensated sum of copies x E_L, in a fixed order.
+__global__ void __launch_bounds__(1024) k_branch_scan(const int* __restrict__ counts,
+                                                      const double* __restrict__ partial, int nblk, int W, int cap,
+                                                      int* __restrict__ parent, double* __restrict__ stats) {
     __shared__ int ssum[1024];
-    __shared__ double se[1024], sc[1024];
     const int t = threadIdx.x;
     const int per = (W + 1023) / 1024;
     const int b = min(W, t * per), e = min(W, b + per);
     int local = 0;
-    Comp ce{0.0, 0.0};
-    for (int i = b; i < e; ++i) {
-        int c = counts[i];
-        local += c;
-        if (c) ce = comp_add(ce, Comp{(double)c * el[i], 0.0});
-    }
+    for (int i = b; i < e; ++i) local += counts[i];
     ssum[t] = local;
     __syncthreads();
     for (int off = 1; off < 1024; off <<= 1) {
@@ -589,66 +599,71 @@ __global__ void __launch_bounds__(1024) k_branch_scan(const int* __restrict__ co
         __syncthreads();
     }
     int run = ssum[t] - local;
-    for (int i = b; i < e; ++i) { offsets[i] = run; run += counts[i]; }
-    se[t] = ce.s;
-    sc[t] = ce.c;
-    __syncthreads();
-    for (int o = 512; o > 0; o >>= 1) {
-        if (t < o) {
-            Comp x = comp_add(Comp{se[t], sc[t]}, Comp{se[t + o], sc[t + o]});
-            se[t] = x.s;
-            sc[t] = x.c;
+    for (int i = b; i < e; ++i)
+        for (int c = counts[i]; c > 0; --c, ++run)
+            if (run < cap) parent[run] = i;
+    if (t < 32) {
+        Comp c{0.0, 0.0};
+        for (int i = t; i < nblk; i += 32) c = comp_add(c, Comp{partial[2 * i], partial[2 * i + 1]});
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            c = comp_add(c, Comp{__shfl_down_sync(0xffffffffu, c.s, o), __shfl_down_sync(0xffffffffu, c.c, o)});
+        if (t == 0) {
+            stats[0] = (double)ssum[1023];
+            stats[1] = c.s + c.c;
         }
-        __syncthreads();
-    }
-    if (t == 0) {
-        stats[0] = (double)ssum[1023];
-        stats[1] = se[0] + sc[0];
     }
 }
 
-// Order-stable gather: destination slot d takes the walker w with
-// offsets[w] <= d < offsets[w] + counts[w] (the last w with offsets[w] <= d).
+// Order-stable gather of the new population: slot d takes walker parent[d],
+// GATHER_ROWS state rows per thread (one thread per walker for all 1008 rows of
+// a benzene walker left 65 blocks with serial copies: 286 us at 8192 walkers).
+constexpr int GATHER_ROWS = 8;
 template <class TS>
-__global__ void k_branch_gather(const int* __restrict__ offsets, int W, const double* __restrict__ stats, int cap,
-                                const TS* __restrict__ spos, const TS* __restrict__ sdinv,
-                                const double* __restrict__ slog, const int* __restrict__ ssign,
-                                const double* __restrict__ sel, int sWcap, TS* __restrict__ dpos,
-                                TS* __restrict__ ddinv, double* __restrict__ dlog, int* __restrict__ dsign,
-                                double* __restrict__ del, int dWcap, int npos, int ndinv) {
-    int d = blockIdx.x * blockDim.x + threadIdx.x;
-    int total = (int)stats[0];
+__global__ void __launch_bounds__(128) k_branch_gather(const int* __restrict__ parent, const double* __restrict__ stats,
+                                                       int cap, const TS* __restrict__ spos,
+                                                       const TS* __restrict__ sdinv, const double* __restrict__ slog,
+                                                       const int* __restrict__ ssign, const double* __restrict__ sel,
+                                                       int sWcap, TS* __restrict__ dpos, TS* __restrict__ ddinv,
+                                                       double* __restrict__ dlog, int* __restrict__ dsign,
+                                                       double* __restrict__ del, int dWcap, int npos, int ndinv) {
+    const int d = blockIdx.x * 128 + threadIdx.x;
+    const int total = (int)stats[0];
     if (d >= total || d >= cap) return;
-    int lo = 0, hi = W - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (offsets[mid] <= d) lo = mid; else hi = mid - 1;
+    const int w = parent[d];
+    const int r0 = blockIdx.y * GATHER_ROWS;
+#pragma unroll
+    for (int k = 0; k < GATHER_ROWS; ++k) {
+        const int i = r0 + k;
+        if (i < npos) dpos[(size_t)i * dWcap + d] = spos[(size_t)i * sWcap + w];
+        else if (i < npos + ndinv) ddinv[(size_t)(i - npos) * dWcap + d] = sdinv[(size_t)(i - npos) * sWcap + w];
     }
-    const int w = lo;
-    for (int i = 0; i < npos; ++i) dpos[(size_t)i * dWcap + d] = spos[(size_t)i * sWcap + w];
-    for (int i = 0; i < ndinv; ++i) ddinv[(size_t)i * dWcap + d] = sdinv[(size_t)i * sWcap + w];
-    dlog[d] = slog[w];
-    dsign[d] = ssign[w];
-    del[d] = sel[w];
+    if (blockIdx.y == 0) {
+        dlog[d] = slog[w];
+        dsign[d] = ssign[w];
+        del[d] = sel[w];
+    }
 }
 
 int launch_branch(DevWalkers& src, DevWalkers& dst, DevBranch& br, int n_elec, int nmax, double e_ref, double tau,
                   double e_cut, uint64_t seed, uint64_t step, cudaStream_t st) {
     int W = src.W;
     if (W <= 0 || W > br.cap) return 1;
-    k_branch_counts<<<(W + 255) / 256, 256, 0, st>>>(src.el, br.el_old, W, e_ref, tau, e_cut, seed, step,
-                                                       br.counts, src.flags);
-    k_branch_scan<<<1, 1024, 0, st>>>(br.counts, src.el, W, br.offsets, br.stats);
+    const int nb = (W + BRANCH_TPB - 1) / BRANCH_TPB;
+    k_branch_counts<<<nb, BRANCH_TPB, 0, st>>>(src.el, br.el_old, W, e_ref, tau, e_cut, seed, step, br.counts,
+                                               br.partial, src.flags);
+    k_branch_scan<<<1, 1024, 0, st>>>(br.counts, br.partial, nb, W, br.cap, br.parent, br.stats);
     int most = std::min(3 * W, dst.Wcap);
     int npos = 3 * n_elec, ndinv = nmax;   // caller passes the per-walker inverse-block size
+    const dim3 grid((most + 127) / 128, (npos + ndinv + GATHER_ROWS - 1) / GATHER_ROWS);
     if (src.prec == 0)
-        k_branch_gather<double><<<(most + 127) / 128, 128, 0, st>>>(
-            br.offsets, W, br.stats, dst.Wcap, (const double*)src.pos, (const double*)src.dinv, src.logabs,
+        k_branch_gather<double><<<grid, 128, 0, st>>>(
+            br.parent, br.stats, dst.Wcap, (const double*)src.pos, (const double*)src.dinv, src.logabs,
             src.sign, src.el, src.Wcap, (double*)dst.pos, (double*)dst.dinv, dst.logabs, dst.sign, dst.el, dst.Wcap,
             npos, ndinv);
     else
-        k_branch_gather<float><<<(most + 127) / 128, 128, 0, st>>>(
-            br.offsets, W, br.stats, dst.Wcap, (const float*)src.pos, (const float*)src.dinv, src.logabs,
+        k_branch_gather<float><<<grid, 128, 0, st>>>(
+            br.parent, br.stats, dst.Wcap, (const float*)src.pos, (const float*)src.dinv, src.logabs,
             src.sign, src.el, src.Wcap, (float*)dst.pos, (float*)dst.dinv, dst.logabs, dst.sign, dst.el, dst.Wcap,
             npos, ndinv);
     g_launch_count += 3;
