@@ -1511,15 +1511,24 @@ int batch_build(qmc_ctx_s* ctx, const std::vector<qmc_walkers_s*>& wk, bool owns
     } guard{b};
     int nsm = 0;
     CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    // classes by shape, precision and, for FP64 molecules, the kernels that the set
+    // takes by itself
     std::map<std::pair<int, int>, int> index;
     for (size_t i = 0; i < wk.size(); ++i) {
-        auto key = std::make_pair(wk[i]->sys->hs.shape, wk[i]->dw.prec);
+        const int shape = wk[i]->sys->hs.shape, prec = wk[i]->dw.prec;
+        const int W = wk[i]->dw.W;
+        const int team = prec == QMC_FP64 && has_team_kernels(shape)
+                             ? (team_sweeps(W, false) ? 1 : 0) | (team_sweeps(W, true) ? 2 : 0) |
+                                   (team_measures(W) ? 4 : 0)
+                             : 0;
+        auto key = std::make_pair(shape, 8 * prec + team);
         auto it = index.find(key);
         if (it == index.end()) {
             it = index.emplace(key, (int)b->cls.size()).first;
             b->cls.emplace_back();
-            b->cls.back().bc.shape = key.first;
-            b->cls.back().bc.prec = key.second;
+            b->cls.back().bc.shape = shape;
+            b->cls.back().bc.prec = prec;
+            b->cls.back().bc.team = team;
         }
         b->cls[it->second].members.push_back((int)i);
     }
@@ -1565,12 +1574,12 @@ int batch_build(qmc_ctx_s* ctx, const std::vector<qmc_walkers_s*>& wk, bool owns
         // sweeps run one block per tile; the occupancy queries set the kernels'
         // shared-memory attributes before any stream capture
         for (int m = 0; m < 2; ++m) {
-            int occ = batch_occupancy(c.bc.shape, c.bc.prec, QMC_MOVE_ONE_GAUSS + m, false);
+            int occ = batch_occupancy(c.bc.shape, c.bc.prec, QMC_MOVE_ONE_GAUSS + m, false, 0, c.bc.team);
             if (occ < 0) return -occ;
         }
         // persistent refresh grids of the thread-per-walker shapes: every
         // resident block slot of the GPU (occupancy x SMs)
-        int occ = batch_occupancy(c.bc.shape, c.bc.prec, 0, true);
+        int occ = batch_occupancy(c.bc.shape, c.bc.prec, 0, true, 0, c.bc.team);
         if (occ < 0) return -occ;
         c.grid_measure = std::max(1, occ) * nsm;
         c.bc.grid_measure = c.grid_measure;

@@ -231,11 +231,26 @@ struct BatchClass {
     int nrec = 0;
     const int* tile_begin = nullptr;     // device [nrec + 1]
     double* tile_partial = nullptr;      // device [ntiles][2]
+    int team = 0;                        // FP64 molecules by teams (bits): Gaussian (1), Langevin (2) sweeps, refresh (4)
     int kmax = 0;                        // electron gas: largest reciprocal component of the class's systems
     int grid_measure = 0;                // persistent refresh grid of the thread-per-walker shapes
                                          // (0: one block per tile); other launches: one block per tile
 };
 
+// FP64 sweeps of the molecules: a team of lanes per walker for smaller ensembles,
+// a thread per walker for larger ones, which fill the FP64 pipes by themselves.
+// Measured crossings (8 sweeps, team / thread): Gaussian moves 6700 (Li), 7500
+// (CH4), 8700 (H2); Langevin moves 10 300 (Li), 11 000 (H2), 11 700 - 12 300 (CH4).
+// At 2048 walkers CH4 6-31G: 1.03 / 2.48 ms and 1.67 / 8.11 ms; at 32 768: 11.4 /
+// 5.8 ms and 20.0 / 16.4 ms.
+inline bool team_sweeps(int W, bool drift) { return W <= (drift ? 10240 : 6144); }
+// FP64 refresh and recorded all-electron steps, the same choice (a team evaluates
+// every pair from both ends and a p triplet's radial part three times, which a
+// thread does not).  Measured crossings of the refresh: 8000 (H2) to 12 000 (CH4);
+// CH4 6-31G at 1000 walkers 0.08 ms by teams and 0.64 ms by threads, at 20 000
+// 1.15 and 0.9 ms.
+inline bool team_measures(int W) { return W <= 9216; }
+inline bool has_team_kernels(int shape) { return shape != SHAPE_C6H6 && shape != SHAPE_HEG54; }
 // Walkers per tile for a shape: threads per block for the thread-per-walker
 // shapes, a multiple of the warps per sweep block for the warp-per-walker ones.
 int batch_tile_width(int shape);
@@ -243,7 +258,7 @@ int batch_tile_width(int shape);
 int launch_batch_sweep(const BatchClass& bc, int move_kind, const BatchCtl* ctl, cudaStream_t st);
 int launch_batch_measure(const BatchClass& bc, cudaStream_t st);
 // Resident blocks per SM of the class's batch kernels (occupancy query).
-int batch_occupancy(int shape, int prec, int move_kind, bool measure, int kmax = 0);
+int batch_occupancy(int shape, int prec, int move_kind, bool measure, int kmax = 0, int team = 0);
 // Device tables of a system for batched launches (cached in the HostSys).
 int batch_tables(const HostSys& hs, int prec, BatchRec& rec);
 // Per-system mean E_L of the class: sum of its tiles' partials / W, written to

@@ -27,11 +27,8 @@ static int cuda_status(cudaError_t e) {
                                uint64_t, cudaStream_t);                                                      \
     int shape_step_all_##NAME(const HostSys&, DevWalkers&, int, int, uint64_t, double, uint64_t, cudaStream_t,\
                               double*);                                                                      \
+    int shape_step_blocks_##NAME(const DevWalkers&);                                                          \
     int shape_nmax_##NAME();
-#define QMC_DECLARE_TEAM(NAME)                                                                                \
-    int shape_team_steps_##NAME(const HostSys&, DevWalkers&, int, int, uint64_t, double, uint64_t,            \
-                                cudaStream_t, double*);                                                       \
-    int shape_step_blocks_##NAME(const DevWalkers&);
 #define QMC_DECLARE_BATCH(NAME)                                                                               \
     int shape_batch_sweep_##NAME(const BatchClass&, int, const BatchCtl*, cudaStream_t, int*);                \
     int shape_batch_measure_##NAME(const BatchClass&, cudaStream_t, int*);                                    \
@@ -43,10 +40,6 @@ QMC_DECLARE_BATCH(ch4)
 QMC_DECLARE_BATCH(ch4min)
 QMC_DECLARE_BATCH(c6h6)
 QMC_DECLARE_BATCH(heg)
-QMC_DECLARE_TEAM(h2)
-QMC_DECLARE_TEAM(li)
-QMC_DECLARE_TEAM(ch4)
-QMC_DECLARE_TEAM(ch4min)
 QMC_DECLARE_SHAPE(h2)
 QMC_DECLARE_SHAPE(li)
 QMC_DECLARE_SHAPE(ch4)
@@ -71,12 +64,6 @@ size_t refresh_rows_bytes(int shape) {
 int dinv_elems_of_shape(int shape) {
     int nm = nmax_of_shape(shape);
     return 2 * nm * nm * (shape == SHAPE_HEG54 ? 2 : 1);
-}
-
-// The compile-time CH4 layout has no FP32 all-electron kernels of its own.
-int shape_step_all_ch4min(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64_t s0, double step, uint64_t seed,
-                          cudaStream_t st, double* partial) {
-    return shape_step_all_ch4(hs, dw, mk, n, s0, step, seed, st, partial);
 }
 
 bool layout_matches_ch4min(const HostSys& hs) {
@@ -121,29 +108,14 @@ int launch_measure(const HostSys& hs, DevWalkers& dw, int compute_prec, bool wri
 #undef C_
 }
 
-// Shapes of the molecules, which have FP64 team kernels.
-#define QMC_TEAM_SWITCH(shape, CALL)                   \
-    switch (shape) {                                   \
-        case SHAPE_H2: return CALL(h2);                \
-        case SHAPE_LI: return CALL(li);                \
-        case SHAPE_CH4: return CALL(ch4);              \
-        case SHAPE_CH4MIN: return CALL(ch4min);        \
-    }
-
 int step_all_blocks(const HostSys& hs, const DevWalkers& dw) {
 #define C_(n) shape_step_blocks_##n(dw)
-    QMC_TEAM_SWITCH(hs.shape, C_)
+    QMC_SHAPE_SWITCH(hs.shape, C_)
 #undef C_
-    return 0;
 }
 
 int launch_step_all(const HostSys& hs, DevWalkers& dw, int move_kind, int n, uint64_t s0, double step, uint64_t seed,
                     double* partial, cudaStream_t st) {
-    if (dw.prec == 0) {
-#define C_(nm) shape_team_steps_##nm(hs, dw, move_kind, n, s0, step, seed, st, partial)
-        QMC_TEAM_SWITCH(hs.shape, C_)
-#undef C_
-    }
 #define C_(nm) shape_step_all_##nm(hs, dw, move_kind, n, s0, step, seed, st, partial)
     QMC_SHAPE_SWITCH(hs.shape, C_)
 #undef C_
@@ -475,9 +447,10 @@ int launch_batch_measure(const BatchClass& bc, cudaStream_t st) {
 #undef C_
 }
 
-int batch_occupancy(int shape, int prec, int move_kind, bool measure, int kmax) {
+int batch_occupancy(int shape, int prec, int move_kind, bool measure, int kmax, int team) {
     BatchClass bc;
     bc.kmax = kmax;
+    bc.team = team;
     bc.shape = shape;
     bc.prec = prec;
     int occ = 0, rc = 7;

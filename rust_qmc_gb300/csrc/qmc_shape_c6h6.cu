@@ -17,5 +17,6 @@ int shape_sweep_one_c6h6(const HostSys& hs, DevWalkers& dw, int mk, int n, uint6
 int shape_step_all_c6h6(const HostSys&, DevWalkers&, int, int, uint64_t, double, uint64_t, cudaStream_t, double*) {
     return 7;   // all-electron moves are not compiled for the benzene shape
 }
+int shape_step_blocks_c6h6(const DevWalkers&) { return 0; }
 int shape_nmax_c6h6() { return C6H6Ops::NM; }
 }  // namespace qmc

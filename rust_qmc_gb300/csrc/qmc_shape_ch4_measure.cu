@@ -3,5 +3,4 @@
 
 namespace qmc {
 QMC_DEFINE_SHAPE_MEASURE(ch4, ShapeCH4)
-QMC_DEFINE_SHAPE_TEAM_STEPS(ch4, ShapeCH4)
 }  // namespace qmc

@@ -3,7 +3,6 @@
 
 namespace qmc {
 QMC_DEFINE_SHAPE_MEASURE(h2, ShapeH2)
-QMC_DEFINE_SHAPE_TEAM_STEPS(h2, ShapeH2)
 QMC_DEFINE_SHAPE_ONE(h2, ShapeH2)
 QMC_DEFINE_SHAPE_ALL(h2, ShapeH2)
 QMC_DEFINE_SHAPE_BATCH_SWEEP(h2, ShapeH2)

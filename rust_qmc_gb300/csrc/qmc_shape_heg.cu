@@ -17,5 +17,6 @@ int shape_sweep_one_heg(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64
 int shape_step_all_heg(const HostSys&, DevWalkers&, int, int, uint64_t, double, uint64_t, cudaStream_t, double*) {
     return 7;   // all-electron moves are not compiled for the electron gas
 }
+int shape_step_blocks_heg(const DevWalkers&) { return 0; }
 int shape_nmax_heg() { return HegOps::NM; }
 }  // namespace qmc

@@ -3,7 +3,6 @@
 
 namespace qmc {
 QMC_DEFINE_SHAPE_MEASURE(li, ShapeLi)
-QMC_DEFINE_SHAPE_TEAM_STEPS(li, ShapeLi)
 QMC_DEFINE_SHAPE_ONE(li, ShapeLi)
 QMC_DEFINE_SHAPE_ALL(li, ShapeLi)
 QMC_DEFINE_SHAPE_BATCH_SWEEP(li, ShapeLi)

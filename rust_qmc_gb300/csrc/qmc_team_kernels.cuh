@@ -131,6 +131,68 @@ static bool fill_team(const HostSys& hs, TeamTab<SH>& S) {
     return true;
 }
 
+// AO a at (x, y, z): value and, with MODE >= 1 / 2, gradient / Laplacian; zero
+// unless ok.
+template <class SH, int MODE>
+__device__ __forceinline__ void team_ao(const TeamTab<SH>& S, int a, bool ok, double x, double y, double z, double& v,
+                                        double& gx, double& gy, double& gz, double& l) {
+    const int d = S.ao[ok ? a : 0];
+    const int I = d & 15, type = (d >> 4) & 15, np = (d >> 8) & 255, p0 = d >> 16;
+    const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    double s0 = 0, s1 = 0, s2 = 0;
+    if constexpr (SH::BASIS == BASIS_GTO) {
+        for (int p = p0; p < p0 + np; ++p) {
+            const double2 pr = S.prim[p];
+            const double f = pr.y * d_exp(-pr.x * r2);
+            s0 += f;
+            if (MODE >= 1) {
+                const double fa = pr.x * f;
+                s1 += fa;
+                if (MODE >= 2) s2 += pr.x * fa;
+            }
+        }
+        // s: chi = R0, grad = -2 R1 dr, lap = -6 R1 + 4 r^2 R2; p_m: chi = x_m R0,
+        // grad = x_m (-2 R1 dr) + e_m R0, lap = x_m (-10 R1 + 4 r^2 R2)
+        const double ang = type == 0 ? 1.0 : (type == 1 ? dx : (type == 2 ? dy : dz));
+        v = ang * s0;
+        if (MODE >= 1) {
+            const double g = -2.0 * s1 * ang;
+            gx = g * dx + (type == 1 ? s0 : 0.0);
+            gy = g * dy + (type == 2 ? s0 : 0.0);
+            gz = g * dz + (type == 3 ? s0 : 0.0);
+        }
+        if (MODE >= 2) l = ang * ((type == 0 ? -6.0 : -10.0) * s1 + 4.0 * r2 * s2);
+    } else {
+        // R(r) = sum c r^n e^{-zeta r}: with t = n/r - zeta a term's derivatives
+        // are f t and f (t^2 - n/r^2)
+        const double r = d_sqrt(r2);
+        const double id = d_positive(r) ? d_rcp(r) : 0.0;
+        for (int p = p0; p < p0 + np; ++p) {
+            const double2 pr = S.prim[p];
+            double f = pr.y * d_exp(-pr.x * r);
+            for (int m = S.powi[p]; m > 0; --m) f *= r;
+            s0 += f;
+            if (MODE >= 1) {
+                const double nr = S.pown[p] * id, u = nr - pr.x, fu = f * u;
+                s1 += fu;
+                if (MODE >= 2) s2 += f * (u * u - nr * id);
+            }
+        }
+        v = s0;
+        if (MODE >= 1) {
+            const double g = s1 * id;
+            gx = g * dx; gy = g * dy; gz = g * dz;
+            if (MODE >= 2) l = d_positive(r) ? s2 + 2.0 * g : 0.0;
+        }
+    }
+    if (!ok) {
+        v = 0;
+        if (MODE >= 1) { gx = 0; gy = 0; gz = 0; }
+        if (MODE >= 2) l = 0;
+    }
+}
+
 // Lanes of a walker (team) and the pieces of an evaluation.
 template <class SH, int G>
 struct Team {
@@ -174,67 +236,12 @@ struct Team {
         return r;
     }
 
-    // AO of this lane's slot at (x, y, z): value and, with DER, gradient and
-    // Laplacian (zero past the basis).
+    // AO of this lane's slot at (x, y, z) (zero past the basis).
     template <bool DER>
     __device__ __forceinline__ void ao(const Tab& S, int slot, double x, double y, double z, double& v, double& gx,
                                        double& gy, double& gz, double& l) const {
         const int a = slot * PARTS + part;
-        const bool ok = on && a < S.n_ao;
-        const int d = S.ao[ok ? a : 0];
-        const int I = d & 15, type = (d >> 4) & 15, np = (d >> 8) & 255, p0 = d >> 16;
-        const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        double s0 = 0, s1 = 0, s2 = 0;
-        if constexpr (SH::BASIS == BASIS_GTO) {
-            for (int p = p0; p < p0 + np; ++p) {
-                const double2 pr = S.prim[p];
-                const double f = pr.y * d_exp(-pr.x * r2);
-                s0 += f;
-                if (DER) {
-                    const double fa = pr.x * f;
-                    s1 += fa;
-                    s2 += pr.x * fa;
-                }
-            }
-            // s: chi = R0, grad = -2 R1 dr, lap = -6 R1 + 4 r^2 R2; p_m: chi = x_m R0,
-            // grad = x_m (-2 R1 dr) + e_m R0, lap = x_m (-10 R1 + 4 r^2 R2)
-            const double ang = type == 0 ? 1.0 : (type == 1 ? dx : (type == 2 ? dy : dz));
-            v = ang * s0;
-            if (DER) {
-                const double g = -2.0 * s1 * ang;
-                gx = g * dx + (type == 1 ? s0 : 0.0);
-                gy = g * dy + (type == 2 ? s0 : 0.0);
-                gz = g * dz + (type == 3 ? s0 : 0.0);
-                l = ang * ((type == 0 ? -6.0 : -10.0) * s1 + 4.0 * r2 * s2);
-            }
-        } else {
-            // R(r) = sum c r^n e^{-zeta r}: with t = n/r - zeta a term's derivatives
-            // are f t and f (t^2 - n/r^2)
-            const double r = d_sqrt(r2);
-            const double id = d_positive(r) ? d_rcp(r) : 0.0;
-            for (int p = p0; p < p0 + np; ++p) {
-                const double2 pr = S.prim[p];
-                double f = pr.y * d_exp(-pr.x * r);
-                for (int m = S.powi[p]; m > 0; --m) f *= r;
-                s0 += f;
-                if (DER) {
-                    const double nr = S.pown[p] * id, u = nr - pr.x, fu = f * u;
-                    s1 += fu;
-                    s2 += f * (u * u - nr * id);
-                }
-            }
-            v = s0;
-            if (DER) {
-                const double g = s1 * id;
-                gx = g * dx; gy = g * dy; gz = g * dz;
-                l = d_positive(r) ? s2 + 2.0 * g : 0.0;
-            }
-        }
-        if (!ok) {
-            v = 0;
-            if (DER) { gx = 0; gy = 0; gz = 0; l = 0; }
-        }
+        team_ao<SH, DER ? 2 : 0>(S, a, on && a < S.n_ao, x, y, z, v, gx, gy, gz, l);
     }
 
     // Determinants of both sectors from the electrons' orbital rows v (part 0's),
@@ -929,6 +936,292 @@ __global__ void __launch_bounds__(TPB) kb_team_measure(const BatchTile* __restri
     }
 }
 
+// ---------------------------------------------------------------------------
+// Single-electron sweeps of FP64 walkers, a team per walker: lane t takes the AOs
+// and the partners (electrons, then nuclei) t, t + G, ... of the moving electron
+// and column t of its sector's inverse; the walker is in shared memory.  Every
+// pair's u (and for drift moves its gradient, and every electron's AO gradients)
+// at the current positions is kept there, so a proposal evaluates only the new
+// position; c'_a = sum_k C[a][k] D^-1[k][q] turns grad ln D into one
+// multiply-add per AO and component.
+// ---------------------------------------------------------------------------
+template <class SH, int MOVE>
+struct SweepState {
+    static constexpr bool DRIFT = MOVE == MOVE_ONE_DRIFT;
+    static constexpr int NE = SH::NE, NM = SH::NMAX, NP = SH::NE + SH::NNUC;
+    double pos[NE][3];
+    double dinv[2][NM][NM];
+    double pu[NE][NP];                                  // u of (electron, partner), nuclei negative
+    double draw[NE][4];                                 // the sweep's normals and acceptance uniforms
+    double pf[DRIFT ? NE : 1][DRIFT ? NP : 1][3];       // grad_e u of (electron, partner)
+    double ga[DRIFT ? NE : 1][DRIFT ? SH::NAO : 1][3];  // AO gradients at the electron's position
+};
+
+template <class SH, int G, int MOVE>
+struct SweepTeam {
+    using St = SweepState<SH, MOVE>;
+    using Tab = TeamTab<SH>;
+    static constexpr bool DRIFT = St::DRIFT;
+    static constexpr int NE = SH::NE, NM = SH::NMAX, NNUC = SH::NNUC, NP = St::NP;
+    static constexpr int AS = (SH::NAO + G - 1) / G, PS = (NP + G - 1) / G;
+    static_assert(G >= NM, "a lane per column of the inverse");
+
+    static __device__ __forceinline__ double sum(double v) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    }
+
+    // u of electron e at (x, y, z) with partner m (nuclei: -u) and, for drift
+    // moves, its gradient; zero for e itself.
+    static __device__ __forceinline__ void pair(const Tab& S, const St& W, int e, int m, double x, double y, double z,
+                                                double& u, double (&f)[3]) {
+        u = 0;
+        f[0] = f[1] = f[2] = 0;
+        if (m >= NP || m == e) return;
+        const bool el = m < NE;
+        const int I = el ? 0 : m - NE;
+        if (SH::JAS != JAS_PADE_EEN && !el) return;
+        const double dx = x - (el ? W.pos[el ? m : 0][0] : S.nuc[I][0]), dy = y - (el ? W.pos[el ? m : 0][1] : S.nuc[I][1]),
+                     dz = z - (el ? W.pos[el ? m : 0][2] : S.nuc[I][2]);
+        double d, ri, g;
+        dist(dx * dx + dy * dy + dz * dz, d, ri);
+        if (SH::JAS == JAS_PADE_EEN) {
+            const int c = (m < SH::NUP) == (e < SH::NUP) ? 1 : 0;
+            const double a = el ? S.a_ee[c] : -S.enA[I], b = el ? S.b_ee[c] : S.enB[I];
+            const double inv = d_rcp(1.0 + b * d);
+            u = a * d * inv;
+            g = a * inv * inv * ri;
+        } else {
+            const double inv = d_rcp(1.0 + d * S.invF);
+            u = -0.5 * S.F * inv;
+            g = 0.5 * inv * inv * ri;
+        }
+        if (DRIFT) { f[0] = g * dx; f[1] = g * dy; f[2] = g * dz; }
+    }
+
+    // tau F capped at maxd.
+    static __device__ __forceinline__ void cap(double& x, double& y, double& z, double maxd) {
+        const double m = d_sqrt(x * x + y * y + z * z);
+        if (m > maxd) {
+            const double s = maxd * recip_full(m);
+            x *= s; y *= s; z *= s;
+        }
+    }
+
+    // n_sweeps sweeps of walker w; every lane of the warp calls it (idle teams,
+    // act false, run on a dummy configuration and store nothing).
+    static __device__ __forceinline__ void run(const Tab& S, St& W, int w, bool act, double* __restrict__ gpos,
+                                               double* __restrict__ gdinv, int* __restrict__ gsign, int Wcap,
+                                               int n_sweeps, uint64_t step0, double step, double tau, double maxd,
+                                               uint64_t seed, int fixed_node, unsigned long long* acc_out, int* flags) {
+        const int lane = threadIdx.x & 31, base = lane & ~(G - 1), t = lane - base;
+        for (int i = t; i < 3 * NE; i += G)
+            W.pos[i / 3][i % 3] = act ? gpos[(size_t)i * Wcap + w] : (i / 3 + 1) * (0.37 + i % 3);
+        for (int i = t; i < 2 * NM * NM; i += G) (&W.dinv[0][0][0])[i] = act ? gdinv[(size_t)i * Wcap + w] : 0.0;
+        __syncwarp();
+        double g0, g1, g2, gl;
+        for (int e = 0; e < NE; ++e) {
+            const double x = W.pos[e][0], y = W.pos[e][1], z = W.pos[e][2];
+            for (int m = t; m < NP; m += G) {
+                double u, f[3];
+                pair(S, W, e, m, x, y, z, u, f);
+                W.pu[e][m] = u;
+                if (DRIFT) { W.pf[e][m][0] = f[0]; W.pf[e][m][1] = f[1]; W.pf[e][m][2] = f[2]; }
+            }
+            if (DRIFT)
+                for (int a = t; a < SH::NAO; a += G) {
+                    double v;
+                    team_ao<SH, 1>(S, a, a < S.n_ao, x, y, z, v, g0, g1, g2, gl);
+                    W.ga[e][a][0] = g0; W.ga[e][a][1] = g1; W.ga[e][a][2] = g2;
+                }
+        }
+        int sgn = act ? gsign[w] : 1;
+        unsigned acc = 0;
+        int flg = 0;
+        const double sd2 = DRIFT ? d_sqrt(2.0 * tau) : step, i4t = DRIFT ? recip_full(4.0 * tau) : 0.0;
+        for (int it = 0; it < n_sweeps; ++it) {
+            __syncwarp();
+            // an electron's two Box-Muller pairs are two items of the lanes
+            for (int i = t; i < 2 * NE; i += G) {
+                const int e = i >> 1;
+                const U4 x = rng_draw(seed, (uint32_t)w, step0 + (uint64_t)it, (uint32_t)e, TAG_PROPOSE);
+                double n0, n1;
+                if (i & 1) {
+                    bm24(x.z & 0xFFFFFFu, x.w & 0xFFFFFFu, n0, n1);
+                    W.draw[e][2] = n0;
+                    W.draw[e][3] = u24((x.x >> 24) | ((x.y >> 24) << 8) | ((x.z >> 24) << 16), 0.0);
+                } else {
+                    bm24(x.x & 0xFFFFFFu, x.y & 0xFFFFFFu, n0, n1);
+                    W.draw[e][0] = n0;
+                    W.draw[e][1] = n1;
+                }
+            }
+            __syncwarp();
+            for (int e = 0; e < NE; ++e) {
+                const int sig = e < SH::NUP ? 0 : 1, q = e - sig * SH::NUP;
+                const int NS = sig == 0 ? SH::NUP : SH::NDN;
+                const double rx = W.pos[e][0], ry = W.pos[e][1], rz = W.pos[e][2];
+                double wq[NM];
+#pragma unroll
+                for (int k = 0; k < NM; ++k) wq[k] = k < NS ? W.dinv[sig][k][q] : 0.0;
+                double cw[AS], dlx = 0, dly = 0, dlz = 0;
+                if (DRIFT) {
+                    double gx = 0, gy = 0, gz = 0, jx = 0, jy = 0, jz = 0;
+#pragma unroll
+                    for (int s = 0; s < AS; ++s) {
+                        const int a = min(t + G * s, SH::NAO - 1);
+                        double c = 0;
+#pragma unroll
+                        for (int k = 0; k < NM; ++k) c += S.C[sig][a][k] * wq[k];
+                        cw[s] = t + G * s < S.n_ao ? c : 0.0;
+                        gx += cw[s] * W.ga[e][a][0]; gy += cw[s] * W.ga[e][a][1]; gz += cw[s] * W.ga[e][a][2];
+                    }
+#pragma unroll
+                    for (int r = 0; r < PS; ++r) {
+                        const int m = t + G * r;
+                        if (m < NP) { jx += W.pf[e][m][0]; jy += W.pf[e][m][1]; jz += W.pf[e][m][2]; }
+                    }
+                    gx = sum(gx + S.qa * jx); gy = sum(gy + S.qa * jy); gz = sum(gz + S.qa * jz);
+                    dlx = tau * (2.0 * gx); dly = tau * (2.0 * gy); dlz = tau * (2.0 * gz);
+                    cap(dlx, dly, dlz, maxd);
+                }
+                const double nx = rx + dlx + sd2 * W.draw[e][0], ny = ry + dly + sd2 * W.draw[e][1],
+                             nz = rz + dlz + sd2 * W.draw[e][2];
+                // AOs at r': orbital values on every lane, then t_j = sum_k phi_k D^-1[k][j]
+                double na[DRIFT ? AS : 1][3], phi[NM];
+#pragma unroll
+                for (int k = 0; k < NM; ++k) phi[k] = 0;
+#pragma unroll
+                for (int s = 0; s < AS; ++s) {
+                    const int a = t + G * s, ac = min(a, SH::NAO - 1);
+                    double v;
+                    team_ao<SH, DRIFT ? 1 : 0>(S, a, a < S.n_ao, nx, ny, nz, v, g0, g1, g2, gl);
+                    if (DRIFT) { na[s][0] = g0; na[s][1] = g1; na[s][2] = g2; }
+#pragma unroll
+                    for (int k = 0; k < NM; ++k) phi[k] += S.C[sig][ac][k] * v;
+                }
+                double tj = 0;
+                const int col = t < NS ? t : 0;
+#pragma unroll
+                for (int k = 0; k < NM; ++k) {
+                    phi[k] = sum(phi[k]);
+                    if (k < NS) tj += phi[k] * W.dinv[sig][k][col];
+                }
+                const double R = __shfl_sync(0xffffffffu, tj, base + q);
+                // Jastrow at r' against the kept terms at r
+                double un[PS], fn[PS][3], du = 0;
+#pragma unroll
+                for (int r = 0; r < PS; ++r) {
+                    const int m = t + G * r;
+                    pair(S, W, e, m, nx, ny, nz, un[r], fn[r]);
+                    du += m < NP ? un[r] - W.pu[e][m] : 0.0;
+                }
+                du = sum(du);
+                const bool zero = ((d_hi(R) & 0x7fffffff) | d_lo(R)) == 0;
+                const double iR = zero ? 0.0 : recip_full(R);
+                double lg = 2.0 * du;
+                if (DRIFT) {
+                    double bx = 0, by = 0, bz = 0, jx = 0, jy = 0, jz = 0;
+#pragma unroll
+                    for (int s = 0; s < AS; ++s) { bx += cw[s] * na[s][0]; by += cw[s] * na[s][1]; bz += cw[s] * na[s][2]; }
+#pragma unroll
+                    for (int r = 0; r < PS; ++r) { jx += fn[r][0]; jy += fn[r][1]; jz += fn[r][2]; }
+                    bx = sum(bx * iR + S.qa * jx); by = sum(by * iR + S.qa * jy); bz = sum(bz * iR + S.qa * jz);
+                    bx *= tau * 2.0; by *= tau * 2.0; bz *= tau * 2.0;
+                    cap(bx, by, bz, maxd);
+                    const double fx = nx - rx - dlx, fy = ny - ry - dly, fz = nz - rz - dlz;
+                    const double qx = rx - nx - bx, qy = ry - ny - by, qz = rz - nz - bz;
+                    lg += ((fx * fx + fy * fy + fz * fz) - (qx * qx + qy * qy + qz * qz)) * i4t;
+                }
+                const double prob = R * R * d_exp(lg);
+                if (prob != prob) flg |= FLAG_NONFINITE;
+                const int take = W.draw[e][3] < prob && !zero && !(fixed_node && d_hi(R) < 0);
+                if (__shfl_sync(0xffffffffu, take, base)) {
+                    if (t < NS) {
+#pragma unroll
+                        for (int k = 0; k < NM; ++k) {
+                            if (k >= NS) break;
+                            const double c = wq[k] * iR;
+                            W.dinv[sig][k][t] = t == q ? c : W.dinv[sig][k][t] - c * tj;
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < PS; ++r) {
+                        const int m = t + G * r;
+                        if (m >= NP) break;
+                        W.pu[e][m] = un[r];
+                        if (m < NE) W.pu[m][e] = un[r];
+                        if (DRIFT) {
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                W.pf[e][m][c] = fn[r][c];
+                                if (m < NE && m != e) W.pf[m][e][c] = -fn[r][c];
+                            }
+                        }
+                    }
+                    if (DRIFT) {
+#pragma unroll
+                        for (int s = 0; s < AS; ++s) {
+                            const int a = t + G * s;
+                            if (a >= SH::NAO) break;
+                            W.ga[e][a][0] = na[s][0]; W.ga[e][a][1] = na[s][1]; W.ga[e][a][2] = na[s][2];
+                        }
+                    }
+                    if (t == 0) { W.pos[e][0] = nx; W.pos[e][1] = ny; W.pos[e][2] = nz; }
+                    if (d_hi(R) < 0) sgn = -sgn;
+                    ++acc;
+                }
+                __syncwarp();
+            }
+        }
+        if (!act) return;
+        for (int i = t; i < 3 * NE; i += G) gpos[(size_t)i * Wcap + w] = W.pos[i / 3][i % 3];
+        for (int i = t; i < 2 * NM * NM; i += G) gdinv[(size_t)i * Wcap + w] = (&W.dinv[0][0][0])[i];
+        if (t == 0) {
+            gsign[w] = sgn;
+            if (acc) atomicAdd(acc_out, (unsigned long long)acc);
+        }
+        if (flg) atomicOr(flags, flg);
+    }
+};
+
+// A warp per block: the walkers' state is most of a block's shared memory.
+template <class SH, int G, int MOVE>
+__global__ void __launch_bounds__(32) k_team_sweep(const TeamTab<SH>* __restrict__ tab, double* __restrict__ gpos,
+                                                   double* __restrict__ gdinv, int* __restrict__ gsign, int W, int Wcap,
+                                                   int n_sweeps, uint64_t step0, double step, double tau, double maxd,
+                                                   uint64_t seed, unsigned long long* acc_out, int* flags,
+                                                   int fixed_node) {
+    constexpr int NT = 32 / G;
+    __shared__ TeamTab<SH> S;
+    __shared__ SweepState<SH, MOVE> st[NT];
+    stage_team(&S, tab);
+    const int tm = threadIdx.x / G, w = blockIdx.x * NT + tm;
+    SweepTeam<SH, G, MOVE>::run(S, st[tm], w, w < W, gpos, gdinv, gsign, Wcap, n_sweeps, step0, step, tau, maxd, seed,
+                                fixed_node, acc_out, flags);
+}
+
+// Batched form: TW / NT blocks per (system, TW-walker tile).
+template <class SH, int G, int MOVE, int TW>
+__global__ void __launch_bounds__(32) kb_team_sweep(const BatchTile* __restrict__ tiles, int ntiles,
+                                                    const BatchRec* __restrict__ recs,
+                                                    const BatchCtl* __restrict__ ctl) {
+    constexpr int NT = 32 / G, BPT = TW / NT;
+    static_assert(TW % NT == 0, "a tile splits into whole blocks");
+    __shared__ TeamTab<SH> S;
+    __shared__ SweepState<SH, MOVE> st[NT];
+    if ((int)blockIdx.x >= ntiles * BPT) return;
+    const BatchTile tl = tiles[blockIdx.x / BPT];
+    const BatchRec& R = recs[tl.rec];
+    const int tm = threadIdx.x / G, w0 = tl.w0 + (int)(blockIdx.x % BPT) * NT, w = w0 + tm;
+    if (w0 >= R.W) return;                              // the whole block
+    stage_team(&S, static_cast<const TeamTab<SH>*>(R.tab_d));
+    SweepTeam<SH, G, MOVE>::run(S, st[tm], w, w < R.W, (double*)R.pos, (double*)R.dinv, R.sign, R.Wcap, ctl->n_sweeps,
+                                ctl->step, ctl->step_size, ctl->tau, ctl->max_drift,
+                                batch_system_seed(ctl->seed, R.index), R.fixed_node, R.acc, R.flags);
+}
+
 // Launchers of a shape with teams of G lanes.
 template <class SH, int G>
 struct TeamOps {
@@ -1003,6 +1296,31 @@ struct TeamOps {
         }
         if (out.fhf || out.omega) return measure_t<0, false, true>(hs, dw, ws, out, st);
         return measure_t<0, false, false>(hs, dw, ws, out, st);
+    }
+
+    // Lanes per walker of the sweeps.
+    static constexpr int GS = SH::NE <= 3 ? 4 : 8;
+    template <int MOVE>
+    static int sweep(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, double tau, double maxd,
+                     uint64_t seed, cudaStream_t st) {
+        constexpr int NT = 32 / GS;
+        const TeamTab<SH>* tab;
+        const int rc = table(hs, &tab);
+        if (rc) return rc;
+        k_team_sweep<SH, GS, MOVE><<<(dw.W + NT - 1) / NT, 32, 0, st>>>(
+            tab, (double*)dw.pos, (double*)dw.dinv, dw.sign, dw.W, dw.Wcap, n, s0, step, tau, maxd, seed, dw.acc,
+            dw.flags, dw.fixed_node);
+        ++g_launch_count;
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
+    }
+    template <int MOVE, int TW>
+    static int batch_sweep(const BatchClass& bc, const BatchCtl* ctl, cudaStream_t st, int* occ) {
+        auto kern = kb_team_sweep<SH, GS, MOVE, TW>;
+        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, 32, 0) == cudaSuccess ? 0 : 2;
+        if (bc.ntiles == 0) return 0;
+        kern<<<bc.ntiles * (TW * GS / 32), 32, 0, st>>>(bc.tiles, bc.ntiles, bc.recs, ctl);
+        ++g_launch_count;
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
     }
 
     template <int TW>

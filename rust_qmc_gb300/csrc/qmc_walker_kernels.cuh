@@ -2,14 +2,15 @@
 // (sm_103a), instantiated once per system shape in qmc_shape_*.cu.
 //
 //   k_init       MultiWfn::initialize for every walker (Philox, tag 3)
-//   k_measure    plain FP32 evaluation from positions: AO->MO, Gauss-Jordan
-//                inverse and log-determinant, Jastrow, grad/Laplacian, E_L
-//                (FP64 walkers: qmc_team_kernels.cuh)
+//   k_measure    evaluation from positions in the walkers' precision: AO->MO,
+//                Gauss-Jordan inverse and log-determinant, Jastrow,
+//                grad/Laplacian, E_L (FP64: large ensembles; smaller ones, and
+//                the extra outputs, in qmc_team_kernels.cuh)
 //   k_rows, k_assemble  the FP64-class refresh of FP32 walkers
 //   k_sweep_one  single-electron Metropolis / Langevin sweeps with
 //                Sherman-Morrison inverse updates, n sweeps per launch, walker
 //                state resident in shared memory for the whole launch
-//   k_step_all   all-electron Metropolis steps of FP32 walkers (MCMCSimulation)
+//   k_step_all   all-electron Metropolis steps (MCMCSimulation), as k_measure
 #pragma once
 #include <cstdio>
 #include <cstring>
@@ -466,8 +467,8 @@ __global__ void k_init(const __grid_constant__ SysT<SH, double> S, TS* __restric
     }
 }
 
-// Full evaluation of walker w in FP32 (the inverse, log|psi|, E_L and, when asked
-// for, gradients and Laplacians); returns E_L (0 for an inactive lane, which
+// Full evaluation of walker w by one thread (the inverse, log|psi|, E_L and, when
+// asked for, gradients and Laplacians); returns E_L (0 for an inactive lane, which
 // still runs the arithmetic on a dummy configuration so that the block stays
 // converged).
 template <class SH, class TC, class TS>
@@ -509,14 +510,14 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
     return act ? e_l : 0.0;
 }
 
-template <class SH, class TC, class TS, int TPB>
-__global__ void __launch_bounds__(TPB) k_measure(const __grid_constant__ SysT<SH, TC> S,
-                                                 const TS* __restrict__ pos, TS* __restrict__ dinv,
+template <class SH, class T, int TPB>
+__global__ void __launch_bounds__(TPB) k_measure(const __grid_constant__ SysT<SH, T> S,
+                                                 const T* __restrict__ pos, T* __restrict__ dinv,
                                                  double* __restrict__ logabs, int* __restrict__ sign,
                                                  double* __restrict__ el, int W, int Wcap, int write_state,
                                                  MeasureOut out, double* partial, int* flags) {
     const int w = blockIdx.x * TPB + threadIdx.x;
-    double e_l = measure_walker<SH, TC, TS>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out, flags);
+    double e_l = measure_walker<SH, T, T>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out, flags);
     if (partial) block_partial<TPB>(e_l, partial, blockIdx.x);
 }
 
@@ -1251,7 +1252,25 @@ __global__ void __launch_bounds__(TPB, (sizeof(T) == 4 ? 512 : 256) / TPB) kb_sw
     if (flg) atomicOr(a.flags, flg);
 }
 
-// All-electron Metropolis steps of FP32 walkers (src/sampling/vmc.rs:95-119): every step
+// Batched FP64 refresh of large sets, one block per TPB-walker tile.
+template <class SH, class T, int TPB>
+__global__ void __launch_bounds__(TPB) kb_measure(const BatchTile* __restrict__ tiles, int ntiles,
+                                                  const BatchRec* __restrict__ recs, double* tile_partial) {
+    __shared__ __align__(16) unsigned char sraw[batch_table_bytes<SH, T>()];
+    SysT<SH, T>& S = *reinterpret_cast<SysT<SH, T>*>(sraw);
+    if ((int)blockIdx.x >= ntiles) return;
+    const BatchTile tl = tiles[blockIdx.x];
+    const BatchRec& R = recs[tl.rec];
+    stage_table(&S, R.tab_s);
+    __syncthreads();
+    const int w = tl.w0 + (int)threadIdx.x;
+    const MeasureOut none;
+    const double e_l = measure_walker<SH, T, T>(S, (const T*)R.pos, (T*)R.dinv, R.logabs, R.sign, R.el, w, w < R.W,
+                                                R.Wcap, 1, none, R.flags);
+    block_partial<TPB>(e_l, tile_partial, blockIdx.x);
+}
+
+// All-electron Metropolis steps, a thread per walker (src/sampling/vmc.rs:95-119): every step
 // proposes all electrons, evaluates psi and E_L at the proposal from scratch,
 // accepts with min(1, psi'^2/psi^2).  Per-step block partial sums of E_L
 // (Neumaier pairs) are written to partial[step][block] when requested.
@@ -1349,17 +1368,17 @@ struct ShapeOps {
         return cuda_status(cudaGetLastError());
     }
 
-    // Plain FP32 evaluation of FP32 walkers.
+    // Evaluation in the walkers' precision, a thread per walker.
+    template <class T>
     static int measure1(const HostSys& hs, DevWalkers& dw, bool write_state, const MeasureOut& out, cudaStream_t st) {
-        SysT<SH, float> S;
+        SysT<SH, T> S;
         if (!fill_sys(hs, S)) return 7;
         constexpr int TPB = 64;
         int nb = (dw.W + TPB - 1) / TPB;
         double* partial = nullptr;
         if (write_state && dw.partial && dw.partial_cap >= 2 * nb + 1) partial = dw.partial;
-        k_measure<SH, float, float, TPB><<<nb, TPB, 0, st>>>(S, (const float*)dw.pos, (float*)dw.dinv, dw.logabs,
-                                                             dw.sign, dw.el, dw.W, dw.Wcap, write_state ? 1 : 0, out,
-                                                             partial, dw.flags);
+        k_measure<SH, T, TPB><<<nb, TPB, 0, st>>>(S, (const T*)dw.pos, (T*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W,
+                                                  dw.Wcap, write_state ? 1 : 0, out, partial, dw.flags);
         ++g_launch_count;
         int rc = cuda_status(cudaGetLastError());
         if (rc || !partial) return rc;
@@ -1393,9 +1412,13 @@ struct ShapeOps {
     using Teams = TeamOps<SH, SH::NE == 2 ? 4 : (SH::NE == 3 ? 8 : 32)>;
 
     static int measure(const HostSys& hs, DevWalkers& dw, int cp, bool ws, const MeasureOut& out, cudaStream_t st) {
-        if (cp == 0 && dw.prec == 0) return Teams::measure(hs, dw, ws, out, st);
+        if (cp == 0 && dw.prec == 0) {
+            const bool plain = !out.O && !out.fhf && !out.omega;
+            return plain && !team_measures(dw.W) ? measure1<double>(hs, dw, ws, out, st)
+                                                 : Teams::measure(hs, dw, ws, out, st);
+        }
         if (dw.prec == 0 || out.O || out.fhf || out.omega) return 7;
-        if (cp != 0) return measure1(hs, dw, ws, out, st);
+        if (cp != 0) return measure1<float>(hs, dw, ws, out, st);
         // FP64-class refresh on the FP32 pipe in two passes
         if (!dw.rows || out.grad || out.lap) return 7;
         return out.inverse_only ? measure_split<true>(hs, dw, ws, st) : measure_split<false>(hs, dw, ws, st);
@@ -1480,7 +1503,9 @@ struct ShapeOps {
     }
 
     // All-electron steps with E_L recorded in partial (block partials) when given.
-    static int step_blocks(const DevWalkers& dw) { return dw.prec == 0 ? Teams::step_blocks(dw.W) : (dw.W + 63) / 64; }
+    static int step_blocks(const DevWalkers& dw) {
+        return dw.prec == 0 && team_measures(dw.W) ? Teams::step_blocks(dw.W) : (dw.W + 63) / 64;
+    }
 
     template <class T, int MOVE>
     static int step_all(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, uint64_t seed,
@@ -1561,6 +1586,8 @@ struct ShapeOps {
 
     // occ != nullptr: report resident blocks per SM instead of launching.
     static int batch_sweep(const BatchClass& bc, int mk, const BatchCtl* ctl, cudaStream_t st, int* occ = nullptr) {
+        if (mk == MOVE_ONE_GAUSS && (bc.team & 1)) return Teams::template batch_sweep<MOVE_ONE_GAUSS, BTPB>(bc, ctl, st, occ);
+        if (mk == MOVE_ONE_DRIFT && (bc.team & 2)) return Teams::template batch_sweep<MOVE_ONE_DRIFT, BTPB>(bc, ctl, st, occ);
         if (mk == MOVE_ONE_GAUSS)
             return bc.prec == 0 ? batch_sweep_t<double, MOVE_ONE_GAUSS>(bc, ctl, st, occ)
                                 : batch_sweep_t<float, MOVE_ONE_GAUSS>(bc, ctl, st, occ);
@@ -1598,7 +1625,14 @@ struct ShapeOps {
     }
 
     static int batch_measure(const BatchClass& bc, cudaStream_t st, int* occ = nullptr) {
-        return bc.prec == 0 ? Teams::template batch_measure<BTPB>(bc, st, occ) : batch_measure_split(bc, st, occ);
+        if (bc.prec != 0) return batch_measure_split(bc, st, occ);
+        if (bc.team & 4) return Teams::template batch_measure<BTPB>(bc, st, occ);
+        auto kern = kb_measure<SH, double, BTPB>;
+        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, BTPB, 0) == cudaSuccess ? 0 : 2;
+        if (bc.ntiles == 0) return 0;
+        kern<<<bc.ntiles, BTPB, 0, st>>>(bc.tiles, bc.ntiles, bc.recs, bc.tile_partial);
+        ++g_launch_count;
+        return cuda_status(cudaGetLastError());
     }
 
     template <bool ALL>
@@ -1607,9 +1641,19 @@ struct ShapeOps {
         bool all = (mk == MOVE_ALL_GAUSS || mk == MOVE_ALL_BOX);
         if (all != ALL) return 1;
         if (ALL) {
+            // FP64 steps without a record need log|psi| alone: teams at any size
+            if (dw.prec == 0 && (!partial || team_measures(dw.W)))
+                return mk == MOVE_ALL_BOX ? Teams::template steps<MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, partial, st)
+                                          : Teams::template steps<MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, partial, st);
+            if (dw.prec == 0)
+                return mk == MOVE_ALL_BOX ? step_all<double, MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, st, partial)
+                                          : step_all<double, MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, st, partial);
             return mk == MOVE_ALL_BOX ? step_all<float, MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, st, partial)
                                       : step_all<float, MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, st, partial);
         }
+        if (dw.prec == 0 && team_sweeps(dw.W, mk == MOVE_ONE_DRIFT))
+            return mk == MOVE_ONE_DRIFT ? Teams::template sweep<MOVE_ONE_DRIFT>(hs, dw, n, s0, step, tau, maxd, seed, st)
+                                        : Teams::template sweep<MOVE_ONE_GAUSS>(hs, dw, n, s0, step, tau, maxd, seed, st);
         if (dw.prec == 0) return mk == MOVE_ONE_DRIFT ? sweep_one<double, MOVE_ONE_DRIFT>(hs, dw, n, s0, step, tau, maxd, seed, st)
                                                       : sweep_one<double, MOVE_ONE_GAUSS>(hs, dw, n, s0, step, tau, maxd, seed, st);
         return mk == MOVE_ONE_DRIFT ? sweep_one<float, MOVE_ONE_DRIFT>(hs, dw, n, s0, step, tau, maxd, seed, st)
@@ -1647,19 +1691,11 @@ struct ShapeOps {
     }                                                                                                         \
     int shape_batch_width_##NAME() { return ShapeOps<SHAPE>::BTPB; }
 
-// All-electron steps: FP64 walkers by teams, FP32 walkers a thread per walker.
-#define QMC_DEFINE_SHAPE_TEAM_STEPS(NAME, SHAPE)                                                               \
-    int shape_team_steps_##NAME(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64_t s0, double step,  \
-                                uint64_t seed, cudaStream_t st, double* partial) {                            \
-        using TO = ShapeOps<SHAPE>::Teams;                                                                    \
-        return mk == MOVE_ALL_BOX ? TO::steps<MOVE_ALL_BOX>(hs, dw, n, s0, step, seed, partial, st)           \
-                                  : TO::steps<MOVE_ALL_GAUSS>(hs, dw, n, s0, step, seed, partial, st);        \
-    }                                                                                                         \
-    int shape_step_blocks_##NAME(const DevWalkers& dw) { return ShapeOps<SHAPE>::step_blocks(dw); }
 #define QMC_DEFINE_SHAPE_ALL(NAME, SHAPE)                                                                      \
     int shape_step_all_##NAME(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64_t s0, double step,    \
                               uint64_t seed, cudaStream_t st, double* partial) {                              \
         return ShapeOps<SHAPE>::template sweep_part<true>(hs, dw, mk, n, s0, step, 0.0, 0.0, seed, st, partial);                  \
-    }
+    }                                                                                                         \
+    int shape_step_blocks_##NAME(const DevWalkers& dw) { return ShapeOps<SHAPE>::step_blocks(dw); }
 
 }  // namespace qmc

@@ -80,3 +80,54 @@ def test_recorded_energies_are_the_steps_means(ctx, name, W, steps):
     np.testing.assert_allclose(r["energies"], means, rtol=1e-11, atol=0)
     wk.close()
     sysh.close()
+
+
+@pytest.mark.parametrize("move", [L.QMC_MOVE_ONE_GAUSS, L.QMC_MOVE_ONE_DRIFT])
+@pytest.mark.parametrize("name, W", [("h2", 1), ("h2", 6144), ("h2", 6145), ("h2", 10240), ("h2", 10241), ("li", 9),
+                                     ("ch4_gto", 5), ("ch4_min", 3), ("ch4_min", 130)])
+def test_sweeps_match_oracle(ctx, oracle, name, W, move):
+    """Single-electron sweeps on both sides of the size where a thread per walker
+    takes over (6144 Gaussian, 10 240 Langevin), and with partly filled warps."""
+    spec = SPECS[name]()
+    sysh = Q.System(ctx, spec)
+    wk = Q.Walkers(sysh, W, L.QMC_FP64)
+    pos = random_configs(spec, W, seed=11)
+    wk.set_positions(pos)
+    wk.refresh()
+    n, seed = 3, 77
+    acc = wk.sweep(move, n, 4, seed=seed, step=0.3, tau=0.02)
+    want, acc_o, _ = oracle.sweeps(spec, pos, n, 4, move, seed, step=0.3, tau=0.02, want_energy=False)
+    got = wk.get_positions()
+    same = np.all(np.abs(got - want) < 1e-9, axis=(1, 2))
+    assert same.mean() >= 0.98, same.mean()
+    if same.all():
+        assert acc == acc_o.sum()
+    # the updated inverse gives the sign a rebuild gives
+    s0 = wk.state()[1]
+    wk.rebuild_inverse()
+    assert np.array_equal(s0, wk.state()[1])
+    assert wk.status() == 0
+    wk.close()
+    sysh.close()
+
+
+@pytest.mark.parametrize("name, W", [("h2", 9216), ("h2", 9217), ("li", 9217), ("ch4_min", 9217)])
+def test_refresh_and_recorded_steps_across_the_size_rule(ctx, oracle, name, W):
+    """Refresh and recorded steps on both sides of 9216 walkers: E_L of the first
+    and last walkers against the oracle, the recorded means against single steps."""
+    spec = SPECS[name]()
+    sysh = Q.System(ctx, spec)
+    wk = Q.Walkers(sysh, W, L.QMC_FP64)
+    wk.init(seed=5)
+    s, el = wk.refresh(want_energies=True)
+    pick = np.r_[0:40, W - 40:W]
+    _close(el[pick], oracle.evaluate(spec, wk.get_positions()[pick])["e_local"])
+    np.testing.assert_allclose(s, el.sum(), rtol=1e-11)
+    r = Q.vmc_run(sysh, n_walkers=W, n_steps=3, move_kind=L.QMC_MOVE_ALL_GAUSS, step=0.4, seed=5)
+    means = []
+    for t in range(3):
+        wk.sweep(L.QMC_MOVE_ALL_GAUSS, 1, t, seed=5, step=0.4)
+        means.append(wk.state()[2].mean())
+    np.testing.assert_allclose(r["energies"], means, rtol=1e-9, atol=0)
+    wk.close()
+    sysh.close()
