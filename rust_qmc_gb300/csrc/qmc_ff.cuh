@@ -37,6 +37,33 @@ struct ff {
     __host__ __device__ explicit constexpr operator float() const { return hi + lo; }
 };
 
+// ---- packed FP32 -------------------------------------------------------------
+// Two FP32 values in a 64-bit register, for the packed instructions (one issue
+// for two IEEE operations; subnormals are flushed, as the library's FP32 code is
+// compiled).
+struct F2 {
+    unsigned long long v;
+    F2() = default;
+    __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ explicit F2(float a) : F2(a, a) {}
+    __device__ __forceinline__ void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+};
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
 // ---- error-free transformations ---------------------------------------------
 __device__ __forceinline__ ff ff_two_sum(float a, float b) {
     float s = __fadd_rn(a, b);

@@ -579,9 +579,232 @@ __global__ void khw_init(const SysH<double>* __restrict__ S, TS* __restrict__ po
 }
 
 // Single-electron sweeps, one warp per walker.
-// Shared bytes per warp of the sweep's inverse columns (both sectors).
+// Shared bytes per warp of the generic sweep's inverse columns (both sectors).
 template <int NM, class T>
 __host__ __device__ constexpr size_t hsweep_warp_bytes() { return sizeof(T) * 2 * 2 * NM * 32; }
+
+// The FP32 Gaussian sweep's shared rows: both sectors' inverses in row pairs, a
+// column per electron of the sector, then two columns for each of two proposals'
+// phases.
+template <int NM>
+__host__ __device__ constexpr int hgauss_rows() { return (NM + 1) / 2; }
+template <int NM>
+__host__ __device__ constexpr int hgauss_cols() { return NM + 4; }
+template <int NM>
+__host__ __device__ constexpr size_t hgauss_warp_bytes() { return 16 * 2 * hgauss_rows<NM>() * hgauss_cols<NM>(); }
+
+// Jastrow change of the RPA form for electron e moving o -> n, both partner rounds
+// of a lane in packed instructions: hjastrow_delta<..., false>'s operations in its
+// order (rint by adding and subtracting 1.5 2^23, which rounds the same way).
+template <int NE, int NUP>
+__device__ __forceinline__ float hjastrow_delta_rpa(const SysH<float>& S, const HLanePos<float, NE>& P, int lane, int e,
+                                                    float ox, float oy, float oz, float nx, float ny, float nz) {
+    const F2 a(S.a_ee[((lane < NUP) == (e < NUP)) ? 1 : 0], S.a_ee[((lane + 32 < NUP) == (e < NUP)) ? 1 : 0]);
+    const F2 px(P.x[0], P.x[1]), py(P.y[0], P.y[1]), pz(P.z[0], P.z[1]);
+    const F2 one(1.0f), neg(-1.0f), iL(S.invL), nL(-S.L), big(12582912.0f), nbig(-12582912.0f), pb(S.pb), pc(S.pc);
+    auto image = [&](float o, F2 q) -> F2 {
+        const F2 d = fma2(q, neg, F2(o));
+        return fma2(nL, add2(add2(mul2(d, iL), big), nbig), d);
+    };
+    auto value = [&](float x, float y, float z, float (&u)[2]) {
+        const F2 dx = image(x, px), dy = image(y, py), dz = image(z, pz);
+        float r2[2], r[2], n[2], den[2];
+        fma2(dz, dz, fma2(dx, dx, mul2(dy, dy))).get(r2[0], r2[1]);
+        r[0] = fsqrt(r2[0]);
+        r[1] = fsqrt(r2[1]);
+        const F2 rr(r[0], r[1]);
+        fma2(mul2(pc, rr), rr, fma2(pb, rr, one)).get(den[0], den[1]);
+        mul2(a, rr).get(n[0], n[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float v = n[k] / den[k];
+            u[k] = (r[k] < S.halfL && r[k] > 1e-10f) ? v : 0.0f;
+        }
+    };
+    float uo[2], un[2];
+    value(ox, oy, oz, uo);
+    value(nx, ny, nz, un);
+    float du = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int j = lane + 32 * k;
+        const float d = un[k] - uo[k];
+        du += (j < NE && j != e) ? d : 0.0f;
+    }
+    return hsum(du);
+}
+
+// FP32 Gaussian sweeps.  The generic form below does the same arithmetic in the
+// same order; here a lane's inverse column lies in row pairs (re, re', im, im'), so
+// that a ratio and an update take two rows per 16-byte access and packed FP32
+// instruction, and the proposal's phases and the moving electron's column are read
+// from shared memory as broadcasts instead of two shuffles a row.  The next
+// proposal's phases (its electron has not moved yet) are written while this one is
+// decided.
+template <int NE, int NUP, class A>
+__device__ __forceinline__ void khw_gauss_walker(const SysH<float>& S, A& a, float4* Dsh, int w) {
+    constexpr int NDN = NE - NUP;
+    constexpr int NM = NUP > NDN ? NUP : NDN, NR = hgauss_rows<NM>(), NC = hgauss_cols<NM>();
+    static_assert(NUP <= 32 && NDN <= 32 && NC <= 32, "one lane per sector electron");
+    const int lane = threadIdx.x & 31;
+    const int col = min(lane, NC - 1);                    // spare lanes read along and store nothing
+    HLanePos<float, NE> P;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int j = lane + 32 * r;
+        const bool ok = j < NE;
+        P.x[r] = ok ? a.pos[(3 * j + 0) * (size_t)a.Wcap + w] : 0.0f;
+        P.y[r] = ok ? a.pos[(3 * j + 1) * (size_t)a.Wcap + w] : 0.0f;
+        P.z[r] = ok ? a.pos[(3 * j + 2) * (size_t)a.Wcap + w] : 0.0f;
+    }
+    auto row = [&](int sig, int k, bool im) -> size_t {
+        return (((size_t)(sig * NM * NM + k * NM + lane)) * 2 + (im ? 1 : 0)) * a.Wcap + w;
+    };
+#pragma unroll
+    for (int sig = 0; sig < 2; ++sig) {
+        const bool own = lane < (sig == 0 ? NUP : NDN);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const bool two = 2 * r + 1 < NM;
+            float4 d;
+            d.x = own ? a.dinv[row(sig, 2 * r, false)] : 0.0f;
+            d.y = own && two ? a.dinv[row(sig, two ? 2 * r + 1 : 0, false)] : 0.0f;
+            d.z = own ? a.dinv[row(sig, 2 * r, true)] : 0.0f;
+            d.w = own && two ? a.dinv[row(sig, two ? 2 * r + 1 : 0, true)] : 0.0f;
+            if (lane < NM) Dsh[(sig * NR + r) * NC + lane] = d;
+        }
+    }
+    unsigned acc = 0;
+    int flg = 0;
+    for (int it = 0; it < a.n_sweeps; ++it) {
+        const uint64_t st = a.step0 + (uint64_t)it;
+#pragma unroll 1
+        for (int sig = 0; sig < 2; ++sig) {
+            float4* D = Dsh + sig * NR * NC;
+            const int NS = sig == 0 ? NUP : NDN;
+            const float kx = S.kvec[sig][lane][0], ky = S.kvec[sig][lane][1], kz = S.kvec[sig][lane][2];
+            const MoveDraw<float> draws = sector_draws<float>(a.seed, (uint32_t)w, st, sig * NUP, NS, lane);
+            float csr = 1, csi = 0;                        // pending complex scale of this lane's column
+            // proposal q: old and new position, and the phase of row `lane` (zero past
+            // the sector) into columns NM + 2 (q mod 2), (cos, cos', sin, sin') of a row
+            // pair, and the one after, (-sin, -sin')
+            float rx, ry, rz, nx, ny, nz, uacc;
+            auto propose = [&](int q) {
+                P.get(sig * NUP + q, rx, ry, rz);
+                const MoveDraw<float> md = draw_of(draws, q);
+                const float step = a.step;
+                nx = rx + step * md.n0; ny = ry + step * md.n1; nz = rz + step * md.n2;
+                uacc = md.uacc;
+                float ps, pc;
+                fsincos(kx * nx + ky * ny + kz * nz, &ps, &pc);
+                if (lane < 2 * NR) {
+                    const bool own = lane < NS;
+                    float* f = reinterpret_cast<float*>(D + (lane >> 1) * NC + NM + 2 * (q & 1)) + (lane & 1);
+                    f[0] = own ? pc : 0.0f;
+                    f[2] = own ? ps : 0.0f;
+                    f[4] = own ? -ps : 0.0f;
+                }
+            };
+            propose(0);
+            __syncwarp();
+            for (int q = 0; q < NS; ++q) {
+                const int e = sig * NUP + q;
+                const float4* ph = D + NM + 2 * (q & 1);
+                const float cx = rx, cy = ry, cz = rz, mx = nx, my = ny, mz = nz, ua = uacc;
+                if (q + 1 < NS) propose(q + 1);
+                // t_l = sum_j phi_j Dinv[j][l]; R = t_q
+                float tr = 0, ti = 0;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    const float4 p = ph[r * NC], d = D[r * NC + col];
+                    const float2 n = *reinterpret_cast<const float2*>(ph + r * NC + 1);
+                    const F2 pr(p.x, p.y), pi(p.z, p.w), np(n.x, n.y), dx(d.x, d.y), dy(d.z, d.w);
+                    float a0, a1, b0, b1;
+                    fma2(pr, dx, mul2(np, dy)).get(a0, a1);
+                    fma2(pr, dy, mul2(pi, dx)).get(b0, b1);
+                    tr += a0; ti += b0;
+                    if (2 * r + 1 < NM) { tr += a1; ti += b1; }
+                }
+                const float Rr = __shfl_sync(0xffffffffu, tr, q), Ri = __shfl_sync(0xffffffffu, ti, q);
+                const float R2 = Rr * Rr + Ri * Ri;
+                float du, g0[3], gn[3];
+                if (S.form == 1) du = hjastrow_delta_rpa<NE, NUP>(S, P, lane, e, cx, cy, cz, mx, my, mz);
+                else du = hjastrow_delta<NE, NUP, float, false>(S, P, lane, e, cx, cy, cz, mx, my, mz, g0, gn);
+                const float prob = R2 * fexp(2 * du);
+                if (prob != prob) flg |= FLAG_NONFINITE;
+                if (ua < prob && R2 > 0.0f) {
+                    // wrap the new position into the box
+                    const float wx = mx - S.L * floor(mx * S.invL), wy = my - S.L * floor(my * S.invL),
+                                wz = mz - S.L * floor(mz * S.invL);
+                    if ((e & 31) == lane) {
+                        if (e < 32) { P.x[0] = wx; P.y[0] = wy; P.z[0] = wz; }
+                        else { P.x[1] = wx; P.y[1] = wy; P.z[1] = wz; }
+                    }
+                    // complex Sherman-Morrison: D'[k][l] = D[k][l] - D[k][q] t_l / R; column q
+                    // keeps its values and takes the factor 1/R when the sector ends (a
+                    // column's scale is 1 until its own electron moves, so t_q and R are
+                    // read unscaled), so it is not written while the others read it
+                    const float iR2 = 1.0f / R2;
+                    const float iRr = Rr * iR2, iRi = -Ri * iR2;              // 1/R
+                    const float fr = tr * iRr - ti * iRi, fi = tr * iRi + ti * iRr;   // t_l / R
+                    if (lane == q) { csr = iRr; csi = iRi; }
+                    const bool store = lane < NM && lane != q;
+                    const F2 f(fi), nfr(-fr), nfi(-fi);
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        const float4 c = D[r * NC + q];
+                        float4 d = D[r * NC + col];
+                        const F2 qr(c.x, c.y), qi(c.z, c.w);
+                        // d - (qr fr - qi fi) and d - (qr fi + qi fr)
+                        const F2 x = add2(F2(d.x, d.y), fma2(qr, nfr, mul2(qi, f)));
+                        const F2 y = add2(F2(d.z, d.w), fma2(qr, nfi, mul2(qi, nfr)));
+                        x.get(d.x, d.y);
+                        y.get(d.z, d.w);
+                        if (store) D[r * NC + lane] = d;
+                    }
+                    ++acc;
+                }
+                __syncwarp();                          // this proposal's reads before the next one's writes
+            }
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const float4 d = D[r * NC + col];
+                float4 n;
+                n.x = d.x * csr - d.z * csi; n.z = d.x * csi + d.z * csr;
+                n.y = d.y * csr - d.w * csi; n.w = d.y * csi + d.w * csr;
+                if (lane < NM) D[r * NC + lane] = n;
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int j = lane + 32 * r;
+        if (j < NE) {
+            a.pos[(3 * j + 0) * (size_t)a.Wcap + w] = P.x[r];
+            a.pos[(3 * j + 1) * (size_t)a.Wcap + w] = P.y[r];
+            a.pos[(3 * j + 2) * (size_t)a.Wcap + w] = P.z[r];
+        }
+    }
+#pragma unroll
+    for (int sig = 0; sig < 2; ++sig) {
+        if (lane >= (sig == 0 ? NUP : NDN)) continue;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const float4 d = Dsh[(sig * NR + r) * NC + lane];
+            a.dinv[row(sig, 2 * r, false)] = d.x;
+            a.dinv[row(sig, 2 * r, true)] = d.z;
+            if (2 * r + 1 < NM) {
+                a.dinv[row(sig, 2 * r + 1, false)] = d.y;
+                a.dinv[row(sig, 2 * r + 1, true)] = d.w;
+            }
+        }
+    }
+    if (lane == 0) {
+        if (acc) atomicAdd(a.acc, (unsigned long long)acc);
+        if (flg) atomicOr(a.flags, flg);
+    }
+}
 
 // A is const volatile SweepArgs<T> (block-shared; see SweepArgs).
 template <int NE, int NUP, class T, int MOVE, class A>
@@ -774,6 +997,21 @@ __device__ __forceinline__ void khw_sweep_walker(const SysH<T>& S, A& a, typenam
     }
 }
 
+// Sweeps of walker w by its warp, with the block's dynamic shared memory.
+template <int NM, class T, int MOVE>
+__host__ __device__ constexpr size_t hsweep_bytes() {
+    return std::is_same<T, float>::value && MOVE == MOVE_ONE_GAUSS ? hgauss_warp_bytes<NM>() : hsweep_warp_bytes<NM, T>();
+}
+template <int NE, int NUP, class T, int MOVE>
+__device__ __forceinline__ void hsweep_walker(const SysH<T>& S, const volatile SweepArgs<T>& a, unsigned char* sm, int w) {
+    constexpr int NM = NUP > NE - NUP ? NUP : NE - NUP;
+    unsigned char* mine = sm + (size_t)(threadIdx.x >> 5) * hsweep_bytes<NM, T, MOVE>();
+    if constexpr (std::is_same<T, float>::value && MOVE == MOVE_ONE_GAUSS)
+        khw_gauss_walker<NE, NUP>(S, a, reinterpret_cast<float4*>(mine), w);
+    else
+        khw_sweep_walker<NE, NUP, T, MOVE>(S, a, reinterpret_cast<typename HComplex<T>::type*>(mine), w);
+}
+
 template <int NE, int NUP, class T, int MOVE, int WPB>
 // 16 warps per SM for FP32 walkers (four blocks of four: 56 KB of shared
 // memory each, at most 128 registers), 8 for FP64 walkers.
@@ -781,7 +1019,6 @@ __global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 ? 16 : 8) / WPB) khw
                                                       T* __restrict__ gdinv, int W, int Wcap, int n_sweeps,
                                                       uint64_t step0, T step, T tau, T maxd, uint64_t seed,
                                                       unsigned long long* acc_out, int* flags) {
-    constexpr int NM = NUP > NE - NUP ? NUP : NE - NUP;
     __shared__ SysH<T> S;
     __shared__ SweepArgs<T> args;
     extern __shared__ __align__(16) unsigned char hsm[];
@@ -790,9 +1027,7 @@ __global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 ? 16 : 8) / WPB) khw
     load_sysh(&S, Sg, (int)sizeof(SysH<T>));   // ends with a block barrier
     const int w = blockIdx.x * WPB + (threadIdx.x >> 5);
     if (w >= W) return;
-    auto* Dsh = reinterpret_cast<typename HComplex<T>::type*>(hsm) + (size_t)(threadIdx.x >> 5) * 2 * NM * 32;
-    const volatile SweepArgs<T>& a = args;
-    khw_sweep_walker<NE, NUP, T, MOVE>(S, a, Dsh, w);
+    hsweep_walker<NE, NUP, T, MOVE>(S, args, hsm, w);
 }
 
 // Batched form: one block per (system, WPB-walker tile); the hardware block
@@ -801,19 +1036,224 @@ template <int NE, int NUP, class T, int MOVE, int WPB>
 __global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 ? 16 : 8) / WPB) khwb_sweep(const BatchTile* __restrict__ tiles, int ntiles,
                                                        const BatchRec* __restrict__ recs,
                                                        const BatchCtl* __restrict__ ctl) {
-    constexpr int NM = NUP > NE - NUP ? NUP : NE - NUP;
     __shared__ SysH<T> S;
     __shared__ SweepArgs<T> args;
     extern __shared__ __align__(16) unsigned char hsm[];
     if ((int)blockIdx.x >= ntiles) return;
-    auto* Dsh = reinterpret_cast<typename HComplex<T>::type*>(hsm) + (size_t)(threadIdx.x >> 5) * 2 * NM * 32;
     const BatchTile tl = tiles[blockIdx.x];
     if (threadIdx.x == 0) args = sweep_args<T>(recs[tl.rec], *ctl);
     load_sysh(&S, static_cast<const SysH<T>*>(recs[tl.rec].tab_s), (int)sizeof(SysH<T>));   // ends with a barrier
-    const volatile SweepArgs<T>& a = args;
     const int w = tl.w0 + (int)(threadIdx.x >> 5);
-    if (w >= a.W) return;
-    khw_sweep_walker<NE, NUP, T, MOVE>(S, a, Dsh, w);
+    if (w >= args.W) return;
+    hsweep_walker<NE, NUP, T, MOVE>(S, args, hsm, w);
+}
+
+// Inverse of one sector's complex orbital matrix (rows in Mr, Mi) by the warp: lane j
+// ends with column j.  |det| goes into (pmag, pexp) (float-float: |det|^2) or logdet.
+template <int NM, class TC>
+__device__ __forceinline__ void invert_sector(const TC* Mr, const TC* Mi, TC* bc, int NS, int lane, TC (&Ar)[NM],
+                                              TC (&Ai)[NM], ff& pmag, int& pexp, double& logdet, bool& ok) {
+                #pragma unroll
+                for (int i = 0; i < NM; ++i) {
+                    bool in = i < NS && lane < NS;
+                    Ar[i] = in ? Mr[i * 32 + lane] : TC(i == lane ? 1 : 0);
+                    Ai[i] = in ? Mi[i * 32 + lane] : TC(0);
+                }
+                int src = lane;
+#pragma unroll 1
+                for (int k = 0; k < NS; ++k) {
+                    // column k, row by row, to the warp's broadcast buffer
+                    if (lane == k) {
+#pragma unroll
+                        for (int i = 0; i < NM; ++i) store_pair(bc + 2 * i, Ar[i], Ai[i]);
+                    }
+                    __syncwarp();
+                    // pivot: the largest |D[i][k]| over the rows not yet pivoted, a row
+                    // per lane (leading parts, whose bits order as integers; the first
+                    // of equal ones)
+                    unsigned key = 0;
+                    if (lane < NS - k) {
+                        TC r, m;
+                        load_pair(bc + 2 * lane, r, m);
+                        key = __float_as_uint(pivot_mag(r, m));
+                    }
+                    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+                    const int p = __ffs(__ballot_sync(0xffffffffu, lane < NS - k && key == top)) - 1;
+                    if (p != 0) {
+                        swap_rows<NM>(p, Ar, Ai);             // p is the same on every lane
+                        if (lane == 0) {
+                            TC r0, i0, rp, ip;
+                            load_pair(bc, r0, i0);
+                            load_pair(bc + 2 * p, rp, ip);
+                            store_pair(bc, rp, ip);
+                            store_pair(bc + 2 * p, r0, i0);
+                        }
+                        __syncwarp();
+                    }
+                    const int pk = k + p;
+                    src = (src == k) ? pk : ((src == pk) ? k : src);
+                    TC pr, pi;
+                    load_pair(bc, pr, pi);
+                    TC pa = pr * pr + pi * pi;
+                    if (!(pa > TC(0))) { ok = false; pr = 1; pi = 0; pa = 1; }
+                    if constexpr (std::is_same<TC, ff>::value) {
+                        pmag = pmag * pa;                  // |det|^2 as a rescaled product
+                        ff_rescale(pmag, pexp);
+                    } else {
+                        logdet += 0.5 * d_log((double)pa);
+                    }
+                    const TC ipr = pr / pa, ipi = -pi / pa;           // 1/a
+                    TC tr, ti;
+                    if (lane == k) {
+                        tr = TC(1) + ipr; ti = ipi;
+                        Ar[0] = ipr; Ai[0] = ipi;
+                    } else {
+                        tr = Ar[0] * ipr - Ai[0] * ipi; ti = Ar[0] * ipi + Ai[0] * ipr;
+                        Ar[0] = tr; Ai[0] = ti;
+                    }
+#pragma unroll
+                    for (int i = 1; i < NM; ++i) {
+                        if (i >= NS) continue;
+                        TC fr, fi;
+                        load_pair(bc + 2 * i, fr, fi);
+                        Ar[i] -= fr * tr - fi * ti; Ai[i] -= fr * ti + fi * tr;
+                    }
+                    __syncwarp();                             // bc is read
+                    // rotate registers 0..NS-1 by one: the pivoted row goes last
+                    const TC r0 = Ar[0], i0 = Ai[0];
+#pragma unroll
+                    for (int i = 0; i + 1 < NM; ++i) {
+                        if (i + 1 < NS) { Ar[i] = Ar[i + 1]; Ai[i] = Ai[i + 1]; }
+                        else if (i + 1 == NS) { Ar[i] = r0; Ai[i] = i0; }
+                    }
+                    if (NS == NM) { Ar[NM - 1] = r0; Ai[NM - 1] = i0; }
+                }
+                // unscramble: lane j takes column src(j)
+#pragma unroll
+                for (int i = 0; i < NM; ++i) {
+                    if (i >= NS) break;
+                    Ar[i] = hshfl(Ar[i], src);
+                    Ai[i] = hshfl(Ai[i], src);
+                }
+}
+
+// The float-float form: a row's real and imaginary parts share packed instructions,
+// in the operations and the order of the generic form (a product's low part and a
+// subtraction's operand are carried negated, which rounds the same way).  Half the
+// instructions also keep the pivot loop's body inside the instruction cache, whose
+// misses were 45 % of the generic form's stalls.
+struct C2 { F2 hi, lo; };                             // complex float-float: (re, im) of both parts
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, F2(-1.0f), a); }   // a - b
+// a + b as operator+(ff, ff)
+__device__ __forceinline__ C2 add_c2(C2 a, C2 b) {
+    const F2 s = add2(a.hi, b.hi), bb = sub2(s, a.hi);
+    const F2 e = add2(sub2(a.hi, sub2(s, bb)), sub2(b.hi, bb));
+    const F2 t = add2(e, add2(a.lo, b.lo));
+    const F2 h = add2(s, t);
+    return {h, sub2(t, sub2(h, s))};
+}
+// -(f t) for a splatted factor -f (nfh, nfl) and -t (nth, ntl), t.hi = th; low part negated
+__device__ __forceinline__ C2 mul_neg(F2 nfh, F2 nfl, F2 th, F2 nth, F2 ntl) {
+    const F2 q = mul2(nfh, th);
+    F2 ne = fma2(nfh, nth, q);
+    ne = fma2(nfh, ntl, ne);
+    ne = fma2(nfl, nth, ne);
+    const F2 h = sub2(q, ne);
+    return {h, add2(ne, sub2(h, q))};
+}
+template <int NM>
+__device__ __forceinline__ void invert_sector(const ff* Mr, const ff* Mi, ff* bc, int NS, int lane, ff (&Ar)[NM],
+                                              ff (&Ai)[NM], ff& pmag, int& pexp, double&, bool& ok) {
+    C2 A[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        const bool in = i < NS && lane < NS;
+        const ff r = in ? Mr[i * 32 + lane] : ff(i == lane ? 1 : 0), m = in ? Mi[i * 32 + lane] : ff(0);
+        A[i] = {F2(r.hi, m.hi), F2(r.lo, m.lo)};
+    }
+    float4* b4 = reinterpret_cast<float4*>(bc);        // [row](re.hi, im.hi, re.lo, im.lo), negated
+    int src = lane;
+#pragma unroll 1
+    for (int k = 0; k < NS; ++k) {
+        if (lane == k) {
+#pragma unroll
+            for (int i = 0; i < NM; ++i) {
+                float4 v;
+                A[i].hi.get(v.x, v.y);
+                A[i].lo.get(v.z, v.w);
+                b4[i] = make_float4(-v.x, -v.y, -v.z, -v.w);
+            }
+        }
+        __syncwarp();
+        unsigned key = 0;
+        if (lane < NS - k) {
+            const float4 v = b4[lane];
+            key = __float_as_uint(pivot_mag(ff(v.x, v.z), ff(v.y, v.w)));
+        }
+        const unsigned top = __reduce_max_sync(0xffffffffu, key);
+        const int p = __ffs(__ballot_sync(0xffffffffu, lane < NS - k && key == top)) - 1;
+        if (p != 0) {
+#pragma unroll
+            for (int r = 1; r < NM; ++r)
+                if (p == r) { const C2 t = A[0]; A[0] = A[r]; A[r] = t; }   // the same row on every lane
+            if (lane == 0) {
+                const float4 u = b4[0], v = b4[p];
+                b4[0] = v;
+                b4[p] = u;
+            }
+            __syncwarp();
+        }
+        const int pk = k + p;
+        src = (src == k) ? pk : ((src == pk) ? k : src);
+        const float4 pv = b4[0];
+        ff pr(-pv.x, -pv.z), pi(-pv.y, -pv.w);
+        ff pa = pr * pr + pi * pi;
+        if (!(pa > ff(0))) { ok = false; pr = 1; pi = 0; pa = 1; }
+        pmag = pmag * pa;                              // |det|^2 as a rescaled product
+        ff_rescale(pmag, pexp);
+        const ff ipr = pr / pa, ipi = -pi / pa;        // 1/a
+        ff ar, ai, tr, ti;
+        A[0].hi.get(ar.hi, ai.hi);
+        A[0].lo.get(ar.lo, ai.lo);
+        if (lane == k) {
+            tr = ff(1) + ipr; ti = ipi;
+            ar = ipr; ai = ipi;
+        } else {
+            tr = ar * ipr - ai * ipi; ti = ar * ipi + ai * ipr;
+            ar = tr; ai = ti;
+        }
+        // -(f t) = (-fr)(tr, ti) + (-fi)(-ti, tr)
+        const F2 th(tr.hi, ti.hi), nth(-tr.hi, -ti.hi), ntl(-tr.lo, -ti.lo);
+        const F2 uh(-ti.hi, tr.hi), nuh(ti.hi, -tr.hi), nul(ti.lo, -tr.lo);
+        const C2 first{F2(ar.hi, ai.hi), F2(ar.lo, ai.lo)};
+        // rows 1..NS-1 lose f x row k and move one register down; row k goes last
+#pragma unroll
+        for (int i = 1; i < NM; ++i) {
+            if (i == NS) A[i - 1] = first;
+            if (i >= NS) continue;
+            const float4 f = b4[i];
+            const C2 x = mul_neg(F2(f.x), F2(f.z), th, nth, ntl), y = mul_neg(F2(f.y), F2(f.w), uh, nuh, nul);
+            // x + y with both low parts negated: e - (x.lo + y.lo)
+            const F2 s = add2(x.hi, y.hi), bb = sub2(s, x.hi);
+            const F2 e = add2(sub2(x.hi, sub2(s, bb)), sub2(y.hi, bb));
+            const F2 t = sub2(e, add2(x.lo, y.lo)), h = add2(s, t);
+            A[i - 1] = add_c2(A[i], C2{h, sub2(t, sub2(h, s))});
+        }
+        if (NS == NM) A[NM - 1] = first;
+        __syncwarp();                                  // bc is read
+    }
+    // unscramble: lane j takes column src(j)
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        float a0, a1, b0, b1;
+        A[i].hi.get(a0, a1);
+        A[i].lo.get(b0, b1);
+        Ar[i] = ff(a0, b0);
+        Ai[i] = ff(a1, b1);
+        if (i >= NS) continue;
+        Ar[i] = hshfl(Ar[i], src);
+        Ai[i] = hshfl(Ai[i], src);
+    }
 }
 
 // FP64 (or FP32) full evaluation: complex Gauss-Jordan, kinetic terms, Ewald.
@@ -878,88 +1318,7 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
             // register 0 to the back.  After NS steps the order is row k in
             // register k again.
             TC Ar[NM], Ai[NM];
-#pragma unroll
-            for (int i = 0; i < NM; ++i) {
-                bool in = i < NS && lane < NS;
-                Ar[i] = in ? Mr[i * 32 + lane] : TC(i == lane ? 1 : 0);
-                Ai[i] = in ? Mi[i * 32 + lane] : TC(0);
-            }
-            int src = lane;
-#pragma unroll 1
-            for (int k = 0; k < NS; ++k) {
-                // column k, row by row, to the warp's broadcast buffer
-                if (lane == k) {
-#pragma unroll
-                    for (int i = 0; i < NM; ++i) store_pair(bc + 2 * i, Ar[i], Ai[i]);
-                }
-                __syncwarp();
-                // pivot: the largest |D[i][k]| over the rows not yet pivoted, a row
-                // per lane (leading parts, whose bits order as integers; the first
-                // of equal ones)
-                unsigned key = 0;
-                if (lane < NS - k) {
-                    TC r, m;
-                    load_pair(bc + 2 * lane, r, m);
-                    key = __float_as_uint(pivot_mag(r, m));
-                }
-                const unsigned top = __reduce_max_sync(0xffffffffu, key);
-                const int p = __ffs(__ballot_sync(0xffffffffu, lane < NS - k && key == top)) - 1;
-                if (p != 0) {
-                    swap_rows<NM>(p, Ar, Ai);             // p is the same on every lane
-                    if (lane == 0) {
-                        TC r0, i0, rp, ip;
-                        load_pair(bc, r0, i0);
-                        load_pair(bc + 2 * p, rp, ip);
-                        store_pair(bc, rp, ip);
-                        store_pair(bc + 2 * p, r0, i0);
-                    }
-                    __syncwarp();
-                }
-                const int pk = k + p;
-                src = (src == k) ? pk : ((src == pk) ? k : src);
-                TC pr, pi;
-                load_pair(bc, pr, pi);
-                TC pa = pr * pr + pi * pi;
-                if (!(pa > TC(0))) { ok = false; pr = 1; pi = 0; pa = 1; }
-                if constexpr (std::is_same<TC, ff>::value) {
-                    pmag = pmag * pa;                  // |det|^2 as a rescaled product
-                    ff_rescale(pmag, pexp);
-                } else {
-                    logdet += 0.5 * d_log((double)pa);
-                }
-                const TC ipr = pr / pa, ipi = -pi / pa;           // 1/a
-                TC tr, ti;
-                if (lane == k) {
-                    tr = TC(1) + ipr; ti = ipi;
-                    Ar[0] = ipr; Ai[0] = ipi;
-                } else {
-                    tr = Ar[0] * ipr - Ai[0] * ipi; ti = Ar[0] * ipi + Ai[0] * ipr;
-                    Ar[0] = tr; Ai[0] = ti;
-                }
-#pragma unroll
-                for (int i = 1; i < NM; ++i) {
-                    if (i >= NS) continue;
-                    TC fr, fi;
-                    load_pair(bc + 2 * i, fr, fi);
-                    Ar[i] -= fr * tr - fi * ti; Ai[i] -= fr * ti + fi * tr;
-                }
-                __syncwarp();                             // bc is read
-                // rotate registers 0..NS-1 by one: the pivoted row goes last
-                const TC r0 = Ar[0], i0 = Ai[0];
-#pragma unroll
-                for (int i = 0; i + 1 < NM; ++i) {
-                    if (i + 1 < NS) { Ar[i] = Ar[i + 1]; Ai[i] = Ai[i + 1]; }
-                    else if (i + 1 == NS) { Ar[i] = r0; Ai[i] = i0; }
-                }
-                if (NS == NM) { Ar[NM - 1] = r0; Ai[NM - 1] = i0; }
-            }
-            // unscramble: lane j takes column src(j)
-#pragma unroll
-            for (int i = 0; i < NM; ++i) {
-                if (i >= NS) break;
-                Ar[i] = hshfl(Ar[i], src);
-                Ai[i] = hshfl(Ai[i], src);
-            }
+            invert_sector<NM>(Mr, Mi, bc, NS, lane, Ar, Ai, pmag, pexp, logdet, ok);
             TC (&Ir)[NM] = Ar;
             TC (&Ii)[NM] = Ai;
             if (a.write_state && lane < NS) {
@@ -1327,7 +1686,7 @@ struct HegShapeOps {
     template <class T, int MOVE>
     static int batch_sweep_t(const BatchClass& bc, const BatchCtl* ctl, cudaStream_t st, int* occ) {
         auto kern = khwb_sweep<NE, NUP, T, MOVE, WPB>;
-        const size_t smem = WPB * hsweep_warp_bytes<NM, T>();
+        const size_t smem = WPB * hsweep_bytes<NM, T, MOVE>();
         static bool attr = false;
         if (!attr) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -1451,7 +1810,7 @@ struct HegShapeOps {
         if (rc) return rc;
         int nb = (dw.W + WPB - 1) / WPB;
         auto kern = khw_sweep<NE, NUP, T, MOVE, WPB>;
-        const size_t smem = WPB * hsweep_warp_bytes<NM, T>();
+        const size_t smem = WPB * hsweep_bytes<NM, T, MOVE>();
         static bool attr = false;
         if (!attr) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
