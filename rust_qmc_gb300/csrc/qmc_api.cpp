@@ -1530,6 +1530,10 @@ int batch_build(qmc_ctx_s* ctx, const std::vector<qmc_walkers_s*>& wk, bool owns
             b->cls.back().bc.prec = prec;
             b->cls.back().bc.team = team;
         }
+        {
+            int& n = b->cls[it->second].bc.n_ao;
+            n = std::max(n, wk[i]->sys->hs.n_ao);
+        }
         b->cls[it->second].members.push_back((int)i);
     }
     for (auto& c : b->cls) {

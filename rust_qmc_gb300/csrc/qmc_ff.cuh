@@ -244,4 +244,106 @@ __device__ __forceinline__ ff shfl_xor(ff v, int m) {
     return ff(__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m));
 }
 
+
+// ---- two float-float values in packed instructions -----------------------------
+// The same operations in the same order as ff's on both components, so each
+// component has the same bits; seeds, exponents and comparisons go component by
+// component.  (sub2 and the negations of two-products are exact.)
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, F2(-1.0f), a); }   // a - b
+__device__ __forceinline__ F2 neg2(F2 a) { return mul2(a, F2(-1.0f)); }
+
+struct ff2 {
+    F2 hi, lo;
+    ff2() = default;
+    __device__ __forceinline__ ff2(F2 h, F2 l) : hi(h), lo(l) {}
+    __device__ __forceinline__ ff2(ff a, ff b) : hi(a.hi, b.hi), lo(a.lo, b.lo) {}
+    __device__ __forceinline__ explicit ff2(ff a) : hi(a.hi), lo(a.lo) {}
+    __device__ __forceinline__ explicit ff2(float a) : hi(a), lo(0.0f) {}
+    __device__ __forceinline__ void get(ff& a, ff& b) const {
+        hi.get(a.hi, b.hi);
+        lo.get(a.lo, b.lo);
+    }
+};
+__device__ __forceinline__ ff2 ff2_fast_two_sum(F2 a, F2 b) {
+    const F2 s = add2(a, b);
+    return ff2(s, sub2(b, sub2(s, a)));
+}
+__device__ __forceinline__ ff2 ff2_two_sum(F2 a, F2 b) {
+    const F2 s = add2(a, b), bb = sub2(s, a);
+    return ff2(s, add2(sub2(a, sub2(s, bb)), sub2(b, bb)));
+}
+__device__ __forceinline__ ff2 operator+(ff2 a, ff2 b) {
+    const ff2 s = ff2_two_sum(a.hi, b.hi);
+    return ff2_fast_two_sum(s.hi, add2(s.lo, add2(a.lo, b.lo)));
+}
+__device__ __forceinline__ ff2 operator-(ff2 a, ff2 b) {
+    const F2 s = sub2(a.hi, b.hi), bb = sub2(s, a.hi);
+    // (a - (s - bb)) + (-b - bb)
+    const F2 e = sub2(sub2(a.hi, sub2(s, bb)), add2(b.hi, bb));
+    return ff2_fast_two_sum(s, add2(e, sub2(a.lo, b.lo)));
+}
+__device__ __forceinline__ ff2 operator*(ff2 a, ff2 b) {
+    const F2 p = mul2(a.hi, b.hi);
+    F2 e = fma2(a.hi, b.hi, neg2(p));
+    e = fma2(a.hi, b.lo, e);
+    e = fma2(a.lo, b.hi, e);
+    return ff2_fast_two_sum(p, e);
+}
+__device__ __forceinline__ ff2 ff2_mul_f(ff2 a, F2 b) {
+    const F2 p = mul2(a.hi, b);
+    return ff2_fast_two_sum(p, fma2(a.lo, b, fma2(a.hi, b, neg2(p))));
+}
+__device__ __forceinline__ ff2& operator+=(ff2& a, ff2 b) { return a = a + b; }
+__device__ __forceinline__ ff2& operator-=(ff2& a, ff2 b) { return a = a - b; }
+// acc += c x as ff_fma_lazy, acc += x as a lazy sum; closed with ff2_norm.
+__device__ __forceinline__ void ff2_fma_lazy(ff2& acc, ff2 c, ff2 x) {
+    const F2 p = mul2(c.hi, x.hi);
+    F2 e = fma2(c.hi, x.hi, neg2(p));
+    e = fma2(c.hi, x.lo, e);
+    e = fma2(c.lo, x.hi, e);
+    const ff2 s = ff2_two_sum(acc.hi, p);
+    acc.hi = s.hi;
+    acc.lo = add2(acc.lo, add2(s.lo, e));
+}
+__device__ __forceinline__ ff2 ff2_norm(ff2 a) { return ff2_fast_two_sum(a.hi, a.lo); }
+__device__ __forceinline__ ff2 ff2_frcp(ff2 b) {
+    float b0, b1;
+    b.hi.get(b0, b1);
+    const F2 x(__frcp_rn(b0), __frcp_rn(b1));
+    const ff2 e = ff2(1.0f) - ff2_mul_f(b, x);
+    return ff2_fast_two_sum(x, mul2(e.hi, x));
+}
+__device__ __forceinline__ ff2 ff2_frsqrt(ff2 a) {      // positive components
+    float a0, a1;
+    a.hi.get(a0, a1);
+    const F2 x(rsqrtf(a0), rsqrtf(a1));
+    const ff2 e = ff2(1.0f) - ff2_mul_f(ff2_mul_f(a, x), x);
+    return ff2_fast_two_sum(x, mul2(e.hi, mul2(F2(0.5f), x)));
+}
+__device__ __forceinline__ ff2 ff2_fexp(ff2 a) {
+    constexpr ff ln2_32 = ff(0.02166084939249829);
+    float a0, a1;
+    a.hi.get(a0, a1);
+    a.hi = F2(a0 < -88.0f ? -88.0f : a0, a1 < -88.0f ? -88.0f : a1);   // returned as 0 below
+    // the nearest integer by adding 1.5 2^23: its low bits are the integer
+    const F2 big = add2(mul2(a.hi, F2(46.166241308446828f)), F2(12582912.0f)), nf = sub2(big, F2(12582912.0f));
+    const F2 lh(ln2_32.hi), p = mul2(lh, nf);
+    const ff2 r = a - ff2_fast_two_sum(p, fma2(F2(ln2_32.lo), nf, fma2(lh, nf, neg2(p))));
+    const F2 q = mul2(r.hi, r.hi), ql = fma2(r.hi, r.hi, neg2(q)), half(0.5f);
+    const ff2 h(mul2(q, half), mul2(fma2(mul2(F2(2.0f), r.hi), r.lo, ql), half));
+    const F2 poly = fma2(r.hi, fma2(r.hi, F2(1.0f / 60.0f), F2(1.0f / 12.0f)), F2(1.0f / 3.0f));
+    const F2 tail = mul2(mul2(h.hi, r.hi), poly);
+    ff2 s = ff2_two_sum(h.hi, tail);
+    s = ff2_fast_two_sum(s.hi, add2(s.lo, h.lo));       // h + tail
+    s = r + s;
+    s = ff2(1.0f) + s;
+    float b0, b1;
+    big.get(b0, b1);
+    const int n0 = __float_as_int(b0) - 0x4b400000, n1 = __float_as_int(b1) - 0x4b400000;
+    const ff2 m = s * ff2(kExp2Frac[n0 & 31], kExp2Frac[n1 & 31]);
+    const F2 sc(a0 < -87.0f ? 0.0f : __int_as_float(((n0 >> 5) + 127) << 23),
+                a1 < -87.0f ? 0.0f : __int_as_float(((n1 >> 5) + 127) << 23));
+    return ff2(mul2(m.hi, sc), mul2(m.lo, sc));
+}
+
 }  // namespace qmc

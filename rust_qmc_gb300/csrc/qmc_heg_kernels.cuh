@@ -1143,7 +1143,6 @@ __device__ __forceinline__ void invert_sector(const TC* Mr, const TC* Mi, TC* bc
 // instructions also keep the pivot loop's body inside the instruction cache, whose
 // misses were 45 % of the generic form's stalls.
 struct C2 { F2 hi, lo; };                             // complex float-float: (re, im) of both parts
-__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, F2(-1.0f), a); }   // a - b
 // a + b as operator+(ff, ff)
 __device__ __forceinline__ C2 add_c2(C2 a, C2 b) {
     const F2 s = add2(a.hi, b.hi), bb = sub2(s, a.hi);

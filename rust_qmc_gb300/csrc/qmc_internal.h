@@ -232,6 +232,7 @@ struct BatchClass {
     const int* tile_begin = nullptr;     // device [nrec + 1]
     double* tile_partial = nullptr;      // device [ntiles][2]
     int team = 0;                        // FP64 molecules by teams (bits): Gaussian (1), Langevin (2) sweeps, refresh (4)
+    int n_ao = 0;                        // largest basis of the class's systems (benzene: table size)
     int kmax = 0;                        // electron gas: largest reciprocal component of the class's systems
     int grid_measure = 0;                // persistent refresh grid of the thread-per-walker shapes
                                          // (0: one block per tile); other launches: one block per tile

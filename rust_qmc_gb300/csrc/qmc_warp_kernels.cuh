@@ -10,6 +10,7 @@
 // Gauss-Jordan elimination in which lane j carries column j of [D | I] and
 // ends holding column j of D^-1 -- exactly the sweep kernel's layout.
 #pragma once
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -1038,6 +1039,459 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
     return act ? e_l : 0.0;
 }
 
+// ---------------------------------------------------------------------------
+// Float-float refresh of FP32 walkers, both spin sectors at once: the sectors have
+// the same size and the same walk over the basis, so sector 0 and sector 1 are the
+// two components of packed instructions (ff2), lane q holding electrons q and
+// NUP + q.  Orbital values and the inversion keep the rounding of the one-sector
+// form, component by component, so the inverses the sweeps start from are its bits;
+// pairs are evaluated once, two per lane and instruction.  The kernel is an
+// instruction stream of several loops, each longer than the instruction cache likes
+// to hold beside the others: the block's warps (one block per SM) walk the phases
+// together, so that one loop is in use at a time.
+// ---------------------------------------------------------------------------
+struct PairTabHead {                // sizes and scalars; the arrays follow in the block's shared memory
+    int n_ao, n_grp, quirk_lap, pad;
+    ff qa, v_nn;
+    ff b_ee[2], a_ee[2];
+};
+// Device table: head, nuclei [NNUC] (x, y, z, Z, enA, enB as ff), groups [WMAX_AO],
+// primitives (exponent, coefficient) [WMAX_PRIM], then the coefficients [n_ao][NM] of
+// both sectors as (hi, hi', lo, lo').
+template <int NNUC, int NM>
+struct PairTab {
+    PairTabHead head;
+    ff nuc[NNUC][6];
+    int grp[WMAX_AO];
+    float4 prim[WMAX_PRIM];
+    float4 C[WMAX_AO][NM];
+    __host__ __device__ static size_t bytes(int n_ao) { return offsetof(PairTab, C) + sizeof(float4) * NM * (size_t)n_ao; }
+};
+
+template <int NNUC, int NM>
+static void fill_pairtab(const SysW<ff>& w, PairTab<NNUC, NM>& S) {
+    std::memset(static_cast<void*>(&S), 0, sizeof(S));
+    S.head.n_ao = w.n_ao;
+    S.head.n_grp = w.n_grp;
+    S.head.quirk_lap = w.quirk_lap;
+    S.head.qa = w.qa;
+    S.head.v_nn = w.v_nn;
+    for (int c = 0; c < 2; ++c) { S.head.b_ee[c] = w.b_ee[c]; S.head.a_ee[c] = w.a_ee[c]; }
+    for (int I = 0; I < NNUC; ++I) {
+        const ff v[6] = {w.nuc[I][0], w.nuc[I][1], w.nuc[I][2], w.Z[I], w.enA[I], w.enB[I]};
+        for (int c = 0; c < 6; ++c) S.nuc[I][c] = v[c];
+    }
+    for (int g = 0; g < w.n_grp; ++g) S.grp[g] = w.grp[g];
+    for (int p = 0; p < WMAX_PRIM; ++p)
+        S.prim[p] = make_float4(w.prim[p][0].hi, w.prim[p][0].lo, w.prim[p][1].hi, w.prim[p][1].lo);
+    for (int a = 0; a < w.n_ao; ++a)
+        for (int k = 0; k < NM; ++k) {
+            const ff c0 = w.C[0][a][k], c1 = w.C[1][a][k];
+            S.C[a][k] = make_float4(c0.hi, c1.hi, c0.lo, c1.lo);
+        }
+}
+
+__device__ __forceinline__ ff2 load_ff2(const float4* p) {
+    const float4 v = *p;
+    return ff2(F2(v.x, v.y), F2(v.z, v.w));
+}
+__device__ __forceinline__ void store_ff2(float4* p, ff2 v) {
+    float4 t;
+    v.hi.get(t.x, t.y);
+    v.lo.get(t.z, t.w);
+    *p = t;
+}
+
+// Shared float4 of a warp: the sectors' rows (row q at q NM), then, over the same
+// storage, positions [3][NE] and sums [5][NE] of the pair pass as ff.
+template <int NE, int NM>
+__host__ __device__ constexpr int pair_scratch() {
+    return NM * NM > (8 * NE + 1) / 2 ? NM * NM : (8 * NE + 1) / 2;
+}
+
+// Pade pair terms of two pairs at separations (dx, dy, dz): u = a r / (1 + b r),
+// u'/r, u'' + 2u'/r, 1/r (0 at r = 0) and the distances' leading parts.
+__device__ __forceinline__ void pair_terms(ff2 dx, ff2 dy, ff2 dz, ff2 a, ff2 b, ff2& u, ff2& f, ff2& l, ff2& ri,
+                                           float (&d)[2]) {
+    const ff2 r2 = dx * dx + dy * dy + dz * dz;
+    float h0, h1;
+    r2.hi.get(h0, h1);
+    if (!(h0 > 0.0f && h1 > 0.0f)) {
+        // 1/r = 0 at a vanishing distance (and NaN stays NaN through r^2)
+        const ff2 s = ff2_frsqrt(ff2(F2(h0 > 0.0f ? h0 : 1.0f, h1 > 0.0f ? h1 : 1.0f), r2.lo));
+        const F2 m(h0 > 0.0f ? 1.0f : 0.0f, h1 > 0.0f ? 1.0f : 0.0f);
+        ri = ff2(mul2(s.hi, m), mul2(s.lo, m));
+    } else {
+        ri = ff2_frsqrt(r2);
+    }
+    const ff2 r = r2 * ri;
+    const ff2 inv = ff2_frcp(ff2(1.0f) + b * r), ai = a * inv, up = ai * inv;
+    u = ai * r;
+    f = up * ri;
+    // 2 (u'/r - a b inv^3)
+    l = f - up * (b * inv);
+    l = ff2(add2(l.hi, l.hi), add2(l.lo, l.lo));
+    r.hi.get(d[0], d[1]);
+}
+
+template <int NE, int NUP, int NNUC>
+__device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S, float4* scr,
+                                                    const float* __restrict__ gpos, float* __restrict__ gdinv,
+                                                    double* __restrict__ glog, int* __restrict__ gsign,
+                                                    double* __restrict__ gel, int w, bool act, int Wcap,
+                                                    int write_state, int* flags) {
+    static_assert(NE == 2 * NUP && NUP <= 32, "equal sectors, an electron of each per lane");
+    constexpr int NM = NUP;
+    const int lane = threadIdx.x & 31;
+    const int q = min(lane, NM - 1);                        // spare lanes repeat the last electron
+    float px[2], py[2], pz[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const size_t i = (size_t)(3 * (s * NUP + q)) * Wcap + w;
+        px[s] = gpos[i];
+        py[s] = gpos[i + Wcap];
+        pz[s] = gpos[i + 2 * (size_t)Wcap];
+    }
+    const ff2 x{ff(px[0]), ff(px[1])}, y{ff(py[0]), ff(py[1])}, z{ff(pz[0]), ff(pz[1])};
+    // orbital values of the lane's electrons, row q of both matrices
+    __syncthreads();
+    {
+        ff2 v[NM];
+#pragma unroll
+        for (int k = 0; k < NM; ++k) v[k] = ff2(0.0f);
+        for (int g = 0; g < S.head.n_grp; ++g) {
+            const int d = S.grp[g];
+            const int I = d & 15, kind = (d >> 4) & 1, np = (d >> 5) & 15, p0 = (d >> 9) & 255, a0 = grp_a0(d);
+            const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
+            const ff2 r2 = dx * dx + dy * dy + dz * dz;
+            ff2 s0(0.0f);
+            for (int p = p0; p < p0 + np; ++p) {
+                const float4 t = S.prim[p];
+                s0 += ff2(ff(t.z, t.w)) * ff2_fexp(ff2(ff(-t.x, -t.y)) * r2);
+            }
+            for (int m = 0; m < (kind ? 3 : 1); ++m) {
+                const ff2 chi = kind ? (m == 0 ? dx : (m == 1 ? dy : dz)) * s0 : s0;
+                const F2 nh = neg2(chi.hi), nl = neg2(chi.lo);
+                const float4* c = S.C[a0 + m];
+                // ff_fma_lazy(v[k], c[k], chi) with the error term carried negated
+#pragma unroll
+                for (int k = 0; k < NM; ++k) {
+                    const ff2 ck = load_ff2(c + k);
+                    const F2 t = mul2(ck.hi, chi.hi);
+                    F2 ne = fma2(ck.hi, nh, t);
+                    ne = fma2(ck.hi, nl, ne);
+                    ne = fma2(ck.lo, nh, ne);
+                    const ff2 u = ff2_two_sum(v[k].hi, t);
+                    v[k] = ff2(u.hi, add2(v[k].lo, sub2(u.lo, ne)));
+                }
+            }
+        }
+        if (lane < NM) {
+#pragma unroll
+            for (int k = 0; k < NM; ++k) store_ff2(scr + lane * NM + k, ff2_norm(v[k]));
+        }
+    }
+    __syncwarp();
+    // Gauss-Jordan of both matrices in place (kw_measure_walker's steps): the pivot
+    // column goes through the warp's shared memory, negated, which also lets a lane
+    // per row search the pivots
+    __syncthreads();
+    ff2 A[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        A[i] = load_ff2(scr + i * NM + q);
+        if (lane >= NM) A[i] = ff2(0.0f);
+    }
+    __syncwarp();
+    ff pm0 = ff(1.0f), pm1 = ff(1.0f);
+    int pe = 0, sg = 1, src0 = lane, src1 = lane;
+    bool ok = true;
+#pragma unroll 1
+    for (int k = 0; k < NM; ++k) {
+        if (lane == k) {
+#pragma unroll
+            for (int i = 0; i < NM; ++i) {
+                float4 t;
+                A[i].hi.get(t.x, t.y);
+                A[i].lo.get(t.z, t.w);
+                scr[i] = make_float4(-t.x, -t.y, -t.z, -t.w);
+            }
+        }
+        __syncwarp();
+        // the largest |D[i][k]| over the rows not yet pivoted; the first of equal ones
+        unsigned k0 = 0, k1 = 0;
+        const bool cand = lane < NM - k;
+        if (cand) {
+            const float4 t = scr[lane];
+            k0 = __float_as_uint(t.x) & 0x7fffffffu;
+            k1 = __float_as_uint(t.y) & 0x7fffffffu;
+        }
+        const unsigned m0 = __reduce_max_sync(0xffffffffu, k0), m1 = __reduce_max_sync(0xffffffffu, k1);
+        const int p0 = __ffs(__ballot_sync(0xffffffffu, cand && k0 == m0)) - 1;
+        const int p1 = __ffs(__ballot_sync(0xffffffffu, cand && k1 == m1)) - 1;
+        if (p0 != 0 || p1 != 0) {
+            // the same rows on every lane
+#pragma unroll
+            for (int r = 1; r < NM; ++r)
+                if (p0 == r || p1 == r) {
+                    float a0, a1, b0, b1, c0, c1, d0, d1;
+                    A[0].hi.get(a0, a1); A[0].lo.get(b0, b1);
+                    A[r].hi.get(c0, c1); A[r].lo.get(d0, d1);
+                    if (p0 == r) { float t = a0; a0 = c0; c0 = t; t = b0; b0 = d0; d0 = t; }
+                    if (p1 == r) { float t = a1; a1 = c1; c1 = t; t = b1; b1 = d1; d1 = t; }
+                    A[0] = ff2(F2(a0, a1), F2(b0, b1));
+                    A[r] = ff2(F2(c0, c1), F2(d0, d1));
+                }
+            if (lane == 0) {
+                float4 t = scr[0], u = scr[p0];
+                scr[p0] = make_float4(t.x, u.y, t.z, u.w);
+                t.x = u.x; t.z = u.z;
+                scr[0] = t;
+                t = scr[0]; u = scr[p1];
+                scr[p1] = make_float4(u.x, t.y, u.z, t.w);
+                t = scr[0];
+                if (p1 != 0) { t.y = u.y; t.w = u.w; }
+                scr[0] = t;
+            }
+            __syncwarp();
+        }
+        if (p0 != 0) sg = -sg;
+        if (p1 != 0) sg = -sg;
+        const int q0 = k + p0, q1 = k + p1;
+        src0 = src0 == k ? q0 : (src0 == q0 ? k : src0);
+        src1 = src1 == k ? q1 : (src1 == q1 ? k : src1);
+        const float4 pv = scr[0];
+        ff v0(-pv.x, -pv.z), v1(-pv.y, -pv.w);
+        if (!(v0 != ff(0))) { ok = false; v0 = ff(1); }
+        if (!(v1 != ff(0))) { ok = false; v1 = ff(1); }
+        if (v0.hi < 0.0f) sg = -sg;
+        if (v1.hi < 0.0f) sg = -sg;
+        pm0 = pm0 * fabs(v0);                              // |det| as rescaled products
+        pm1 = pm1 * fabs(v1);
+        ff_rescale(pm0, pe);
+        ff_rescale(pm1, pe);
+        const ff2 ip(ff(1) / v0, ff(1) / v1);
+        const ff2 scaled = A[0] * ip, own = ff2(1.0f) + ip;
+        const bool me = lane == k;
+        const ff2 t = me ? own : scaled, first = me ? ip : scaled;
+        const F2 nth = neg2(t.hi), ntl = neg2(t.lo);
+        // rows 1.. lose f x row k and move one register down; row k goes last
+#pragma unroll
+        for (int i = 1; i < NM; ++i) {
+            const ff2 f = load_ff2(scr + i);               // -f
+            const F2 m = mul2(f.hi, t.hi);
+            F2 ne = fma2(f.hi, nth, m);
+            ne = fma2(f.hi, ntl, ne);
+            ne = fma2(f.lo, nth, ne);
+            const F2 h = sub2(m, ne), nl = add2(ne, sub2(h, m));   // -(f t), low part negated
+            const ff2 s = ff2_two_sum(A[i].hi, h);
+            A[i - 1] = ff2_fast_two_sum(s.hi, add2(s.lo, sub2(A[i].lo, nl)));
+        }
+        A[NM - 1] = first;
+        __syncwarp();                                      // the column is read
+    }
+    // unscramble: lane j takes columns src(j); then A[k] = D^-1[k][lane]
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        ff a, b;
+        A[i].get(a, b);
+        a = wshfl(a, src0);
+        b = wshfl(b, src1);
+        A[i] = ff2(a, b);
+        if (act && write_state && lane < NM) {
+            gdinv[((size_t)(i * NM + lane)) * Wcap + w] = (float)a;
+            gdinv[((size_t)(NM * NM + i * NM + lane)) * Wcap + w] = (float)b;
+        }
+    }
+    // grad ln D and lap D / D of the lane's electrons: sum_a c'_a (grad, lap) chi_a with
+    // c'_a = sum_k C[a][k] D^-1[k][q].  s: grad = -2 R1 dr, lap = -6 R1 + 4 r^2 R2; a p
+    // triplet takes its three c' as a vector c: grad = -2 R1 (c.dr) dr + R0 c,
+    // lap = (c.dr)(-10 R1 + 4 r^2 R2).  The nuclei's pair terms follow from the
+    // distances at hand only in part, so they have a loop of their own.
+    __syncthreads();
+    ff2 gx(0.0f), gy(0.0f), gz(0.0f), ld(0.0f);
+    for (int g = 0; g < S.head.n_grp; ++g) {
+        const int d = S.grp[g];
+        const int I = d & 15, kind = (d >> 4) & 1, np = (d >> 5) & 15, p0 = (d >> 9) & 255, a0 = grp_a0(d);
+        const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
+        const ff2 r2 = dx * dx + dy * dy + dz * dz;
+        ff2 s0(0.0f), s1(0.0f), s2(0.0f);
+        for (int p = p0; p < p0 + np; ++p) {
+            const float4 t = S.prim[p];
+            const ff2 al(ff(t.x, t.y));
+            const ff2 e = ff2(ff(t.z, t.w)) * ff2_fexp(ff2(ff(-t.x, -t.y)) * r2), ea = al * e;
+            s0 += e;
+            s1 += ea;
+            ff2_fma_lazy(s2, al, ea);
+        }
+        s2 = ff2_norm(s2);
+        const ff2 two(F2(-2.0f), F2(0.0f)), l4 = ff2(4.0f) * r2 * s2, t1 = two * s1;
+        // cd: c' of an s AO, (c'.dr) of a p triplet
+        ff2 cd(0.0f);
+#pragma unroll 1
+        for (int m = 0; m < (kind ? 3 : 1); ++m) {
+            const float4* c = S.C[a0 + m];
+            ff2 cw(0.0f);
+#pragma unroll
+            for (int k = 0; k < NM; ++k) ff2_fma_lazy(cw, load_ff2(c + k), A[k]);
+            cw = ff2_norm(cw);
+            if (!kind) {
+                cd = cw;
+            } else {
+                ff2_fma_lazy(cd, cw, m == 0 ? dx : (m == 1 ? dy : dz));
+                ff2 o = m == 0 ? gx : (m == 1 ? gy : gz);
+                ff2_fma_lazy(o, s0, cw);
+                if (m == 0) gx = o;
+                else if (m == 1) gy = o;
+                else gz = o;
+            }
+        }
+        cd = ff2_norm(cd);
+        const ff2 t = t1 * cd;
+        ff2_fma_lazy(gx, t, dx); ff2_fma_lazy(gy, t, dy); ff2_fma_lazy(gz, t, dz);
+        ff2_fma_lazy(ld, cd, l4 - (kind ? ff2(10.0f) : ff2(6.0f)) * s1);
+    }
+    gx = ff2_norm(gx); gy = ff2_norm(gy); gz = ff2_norm(gz); ld = ff2_norm(ld);
+    // electron pairs, each once, two per lane: pair p joins electron i = p mod NE with
+    // i + p / NE + 1 (mod NE), the last NE / 2 pairs i with i + NE / 2; 32 consecutive
+    // pairs have distinct i and distinct j, so their sums need no atomics
+    ff* pos = reinterpret_cast<ff*>(scr);
+    ff* sums = pos + 3 * NE;
+    __syncthreads();
+    if (lane < NM) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const int e = s * NUP + lane;
+            pos[e] = ff(px[s]); pos[NE + e] = ff(py[s]); pos[2 * NE + e] = ff(pz[s]);
+#pragma unroll
+            for (int c = 0; c < 5; ++c) sums[c * NE + e] = ff(0.0f);
+        }
+    }
+    __syncwarp();
+    ff2 u(0.0f), V(0.0f);
+    constexpr int NPAIR = NE * (NE - 1) / 2, FULL = NE * ((NE - 1) / 2);
+    static_assert(NE > 32 && NE % 2 == 0, "the pairs of one round hold distinct electrons");
+    for (int r0 = 0; r0 < NPAIR; r0 += 64) {
+        int i[2], j[2];
+        bool on[2];
+        float d0[2], d1[2], d2[2];
+        ff pa[2], pb[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            on[s] = r0 + 32 * s + lane < NPAIR;
+            const int p = on[s] ? r0 + 32 * s + lane : NPAIR - 1;
+            i[s] = p < FULL ? p % NE : p - FULL;
+            j[s] = p < FULL ? i[s] + p / NE + 1 : i[s] + NE / 2;
+            if (j[s] >= NE) j[s] -= NE;
+            d0[s] = pos[i[s]].hi; d1[s] = pos[NE + i[s]].hi; d2[s] = pos[2 * NE + i[s]].hi;
+            const int c = (j[s] < NUP) == (i[s] < NUP) ? 1 : 0;
+            pa[s] = S.head.a_ee[c]; pb[s] = S.head.b_ee[c];
+        }
+        // positions are floats: the differences are exact pairs
+        const ff2 dx = ff2_two_sum(F2(d0[0], d0[1]), F2(-pos[j[0]].hi, -pos[j[1]].hi));
+        const ff2 dy = ff2_two_sum(F2(d1[0], d1[1]), F2(-pos[NE + j[0]].hi, -pos[NE + j[1]].hi));
+        const ff2 dz = ff2_two_sum(F2(d2[0], d2[1]), F2(-pos[2 * NE + j[0]].hi, -pos[2 * NE + j[1]].hi));
+        ff2 uu, f, l, ri;
+        float dd[2];
+        pair_terms(dx, dy, dz, ff2(pa[0], pa[1]), ff2(pb[0], pb[1]), uu, f, l, ri, dd);
+        const ff2 fx = f * dx, fy = f * dy, fz = f * dz;
+        ff2 sq(0.0f);
+        if (S.head.quirk_lap) {
+            const ff2 up2 = f * f;
+            sq = up2 * (dx * dx + dy * dy + dz * dz);
+        }
+        ff t[7][2];
+        uu.get(t[0][0], t[0][1]); ri.get(t[1][0], t[1][1]);
+        fx.get(t[2][0], t[2][1]); fy.get(t[3][0], t[3][1]); fz.get(t[4][0], t[4][1]);
+        l.get(t[5][0], t[5][1]); sq.get(t[6][0], t[6][1]);
+        u += ff2(on[0] ? t[0][0] : ff(0.0f), on[1] ? t[0][1] : ff(0.0f));
+        V += ff2(on[0] ? t[1][0] : ff(0.0f), on[1] ? t[1][1] : ff(0.0f));
+        const int nq = S.head.quirk_lap ? 5 : 4;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const bool use = on[s] && !(dd[s] < 1e-10f);
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int e = side ? j[s] : i[s];
+                if (use) {
+#pragma unroll
+                    for (int c = 0; c < 5; ++c) {
+                        if (c >= nq) break;
+                        const ff v = t[2 + c][s];
+                        const ff o = sums[c * NE + e], n = ff_two_sum(o.hi, side && c < 3 ? -v.hi : v.hi);
+                        sums[c * NE + e] = ff(n.hi, __fadd_rn(o.lo, __fadd_rn(n.lo, side && c < 3 ? -v.lo : v.lo)));
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    // the lane's electrons: sums over electrons, then the nuclei
+    auto both = [&](int c) {
+        return ff2(ff_norm(sums[c * NE + q]), ff_norm(sums[c * NE + NUP + q]));
+    };
+    ff2 jx = both(0), jy = both(1), jz = both(2), lu = both(3);
+    const ff2 gsq = both(4);
+    ff2 un(0.0f), Vn(0.0f);
+    for (int I = 0; I < NNUC; ++I) {
+        const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
+        ff2 uu, f, l, ri;
+        float dd[2];
+        pair_terms(dx, dy, dz, ff2(S.nuc[I][4]), ff2(S.nuc[I][5]), uu, f, l, ri, dd);
+        un -= uu;
+        Vn -= ff2(S.nuc[I][3]) * ri;
+        if (dd[0] < 1e-10f || dd[1] < 1e-10f) {            // a coincident nucleus: no gradient terms
+            ff a, b;
+            f.get(a, b);
+            f = ff2(dd[0] < 1e-10f ? ff(0.0f) : a, dd[1] < 1e-10f ? ff(0.0f) : b);
+            l.get(a, b);
+            l = ff2(dd[0] < 1e-10f ? ff(0.0f) : a, dd[1] < 1e-10f ? ff(0.0f) : b);
+        }
+        jx -= f * dx; jy -= f * dy; jz -= f * dz;
+        lu -= l;
+    }
+    const ff2 qa(S.head.qa);
+    const ff2 lj = S.head.quirk_lap ? lu + gsq : lu + jx * jx + jy * jy + jz * jz;
+    const ff2 lp = ld + ff2(2.0f) * (qa * (gx * jx + gy * jy + gz * jz)) + lj;
+    const bool mine = lane < NM;
+    ff a, b;
+    u.get(a, b);
+    ff us = a + b;
+    un.get(a, b);
+    us = mine ? us + (a + b) : us;
+    V.get(a, b);
+    ff Vs = a + b;
+    Vn.get(a, b);
+    Vs = mine ? Vs + (a + b) : Vs;
+    lp.get(a, b);
+    if (mine) Vs = Vs - ff(0.5f) * (a + b);
+    us = wsum(us);
+    Vs = wsum(Vs);
+    const double e_l = (double)(Vs + S.head.v_nn);
+    if (act && lane == 0) {
+        int fl = 0;
+        if (!ok) fl |= FLAG_SINGULAR;
+        if (!isfinite(e_l)) fl |= FLAG_NONFINITE;
+        if (fl) atomicOr(flags, fl);
+        if (write_state) {
+            glog[w] = d_log((double)(pm0 * pm1)) + (double)pe * 0.6931471805599453 + (double)us;
+            gsign[w] = sg;
+            gel[w] = e_l;
+        }
+    }
+    return act ? e_l : 0.0;
+}
+
+// Whole-block copy of the table (n_ao rows of coefficients) into shared memory.
+template <class TAB>
+__device__ __forceinline__ void load_pairtab(TAB* dst, const TAB* __restrict__ src) {
+    const int n = (int)(TAB::bytes(src->head.n_ao) / sizeof(float4));
+    const float4* s = reinterpret_cast<const float4*>(src);
+    float4* d = reinterpret_cast<float4*>(dst);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = s[i];
+    __syncthreads();
+}
+
 // Compensated sum of the block's per-warp values (lane 0 of each warp) into
 // partial[2 slot], partial[2 slot + 1]; ends with a block barrier.
 template <int WPB>
@@ -1092,6 +1546,41 @@ __global__ void __launch_bounds__(32 * WPB) kwb_measure(const BatchTile* __restr
     warp_block_partial<WPB>(e_l, tile_partial, blockIdx.x);
 }
 
+// Float-float refresh of FP32 walkers: standalone and batched.
+template <int NE, int NUP, int NNUC, int WPB>
+__global__ void __launch_bounds__(32 * WPB, 12 / WPB) kw_refresh(const PairTab<NNUC, NUP>* __restrict__ Sg,
+                                                                const float* __restrict__ gpos,
+                                                                float* __restrict__ gdinv, double* __restrict__ glog,
+                                                                int* __restrict__ gsign, double* __restrict__ gel, int W,
+                                                                int Wcap, int write_state, double* partial, int* flags) {
+    extern __shared__ __align__(16) unsigned char wsm[];
+    const int wib = threadIdx.x >> 5, w = blockIdx.x * WPB + wib;
+    float4* scr = reinterpret_cast<float4*>(wsm) + (size_t)wib * pair_scratch<NE, NUP>();
+    auto& S = *reinterpret_cast<PairTab<NNUC, NUP>*>(wsm + sizeof(float4) * WPB * pair_scratch<NE, NUP>());
+    load_pairtab(&S, Sg);
+    // warps past the last walker repeat it and store nothing
+    const double e_l = kw_refresh_walker<NE, NUP, NNUC>(S, scr, gpos, gdinv, glog, gsign, gel, min(w, W - 1), w < W,
+                                                        Wcap, write_state, flags);
+    if (partial) warp_block_partial<WPB>(e_l, partial, blockIdx.x);
+}
+template <int NE, int NUP, int NNUC, int WPB>
+__global__ void __launch_bounds__(32 * WPB, 12 / WPB) kwb_refresh(const BatchTile* __restrict__ tiles, int ntiles,
+                                                                 const BatchRec* __restrict__ recs,
+                                                                 double* tile_partial) {
+    extern __shared__ __align__(16) unsigned char wsm[];
+    if ((int)blockIdx.x >= ntiles) return;
+    const int wib = threadIdx.x >> 5;
+    float4* scr = reinterpret_cast<float4*>(wsm) + (size_t)wib * pair_scratch<NE, NUP>();
+    auto& S = *reinterpret_cast<PairTab<NNUC, NUP>*>(wsm + sizeof(float4) * WPB * pair_scratch<NE, NUP>());
+    const BatchTile tl = tiles[blockIdx.x];
+    const BatchRec& R = recs[tl.rec];
+    load_pairtab(&S, static_cast<const PairTab<NNUC, NUP>*>(R.tab_d));
+    const int w = tl.w0 + wib;
+    const double e_l = kw_refresh_walker<NE, NUP, NNUC>(S, scr, (const float*)R.pos, (float*)R.dinv, R.logabs, R.sign,
+                                                        R.el, min(w, R.W - 1), w < R.W, R.Wcap, 1, R.flags);
+    warp_block_partial<WPB>(e_l, tile_partial, blockIdx.x);
+}
+
 int launch_sum_partials(const double* partial, int nblk, int nrows, double* out, cudaStream_t st);
 
 // Per-shape launchers for the warp kernels.
@@ -1099,10 +1588,11 @@ template <int NE, int NUP, int NNUC>
 struct WarpShapeOps {
     static constexpr int NM = NUP > NE - NUP ? NUP : NE - NUP;
     static constexpr int WPB = 4;
+    // Warps of a float-float refresh block, one block per SM (168 registers).
+    static constexpr int RWPB = 12;
     // Batch tiles hold BTW walkers: BTW / WPB sweep blocks each, and one
-    // refresh block of BTW warps (the wider refresh block shares the large
-    // shared-memory table among more warps).
-    static constexpr int BTW = 8;
+    // refresh block of BTW warps.
+    static constexpr int BTW = RWPB;
     // dynamic shared memory of a sweep block: the WPB warps' proposal rows
     template <class T>
     static constexpr size_t sweep_smem() { return sizeof(T) * WPB * (size_t)sweep_scratch_elems<NE, NUP>(); }
@@ -1161,54 +1651,56 @@ struct WarpShapeOps {
         return launch_sum_partials(partial, nb, 1, dw.partial + dw.partial_cap - 1, st);
     }
 
-    // Walkers per block of the standalone refresh, 4 or 8, chosen by timing.
-    // The system table is per block and the row scratch per warp, so the two
-    // shapes trade the table's fixed shared-memory cost against registers
-    // per block; which keeps more warps resident and issues faster depends
-    // on the arithmetic type.  A refresh recomputes the same state whatever
-    // the block shape, so the first refresh of at least 1024 walkers per
-    // arithmetic type (outside stream capture) runs both shapes, times each
-    // once after a warm-up launch, and keeps the faster.
-    static constexpr int WB_A = 4, WB_B = 8;
-
-    template <class TC, class TS>
-    static int measure2(const HostSys& hs, DevWalkers& dw, bool ws, const MeasureOut& out, cudaStream_t st) {
-        static int best = 0;
-        if (best == 0) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            if (dw.W < 1024 || cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
-                return measure_w<TC, TS, WB_A>(hs, dw, ws, out, st);
-            cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-            int rc = 0;
-            for (auto& e : ev)
-                if (!rc && cudaEventCreate(&e) != cudaSuccess) rc = 2;
-            if (!rc) rc = measure_w<TC, TS, WB_A>(hs, dw, ws, out, st);
-            if (!rc) rc = measure_w<TC, TS, WB_B>(hs, dw, ws, out, st);
-            if (!rc && cudaEventRecord(ev[0], st) != cudaSuccess) rc = 2;
-            if (!rc) rc = measure_w<TC, TS, WB_A>(hs, dw, ws, out, st);
-            if (!rc && cudaEventRecord(ev[1], st) != cudaSuccess) rc = 2;
-            if (!rc) rc = measure_w<TC, TS, WB_B>(hs, dw, ws, out, st);
-            if (!rc && cudaEventRecord(ev[2], st) != cudaSuccess) rc = 2;
-            float ta = 0.0f, tb = 0.0f;
-            if (!rc && cudaEventSynchronize(ev[2]) != cudaSuccess) rc = 2;
-            if (!rc && (cudaEventElapsedTime(&ta, ev[0], ev[1]) != cudaSuccess ||
-                        cudaEventElapsedTime(&tb, ev[1], ev[2]) != cudaSuccess))
-                rc = 2;
-            for (auto e : ev)
-                if (e) cudaEventDestroy(e);
-            if (!rc) best = tb < ta ? WB_B : WB_A;
-            return rc;
+    // Refresh of FP32 walkers: its table (device copy cached like the others) and
+    // shared memory.  12 warps per SM at up to 168 registers.
+    using PT = PairTab<NNUC, NUP>;
+    static int pair_table(const HostSys& hs, const PT** out) {
+        constexpr int slot = 2;
+        if (!hs.dev_table[slot] || hs.dev_table_version[slot] != hs.version) {
+            SysW<ff>* w = new SysW<ff>;
+            PT* h = new PT;
+            const bool good = fill_sysw<ff>(hs, NE, NUP, NNUC, *w);
+            if (good) fill_pairtab<NNUC, NUP>(*w, *h);
+            int rc = good ? 0 : 7;
+            if (!rc && !hs.dev_table[slot] && cudaMalloc(&hs.dev_table[slot], sizeof(PT)) != cudaSuccess) rc = 8;
+            if (!rc && cudaMemcpy(hs.dev_table[slot], h, sizeof(PT), cudaMemcpyHostToDevice) != cudaSuccess) rc = 2;
+            delete w;
+            delete h;
+            if (rc) return rc;
+            hs.dev_table_version[slot] = hs.version;
         }
-        return best == WB_B ? measure_w<TC, TS, WB_B>(hs, dw, ws, out, st)
-                            : measure_w<TC, TS, WB_A>(hs, dw, ws, out, st);
+        *out = static_cast<const PT*>(hs.dev_table[slot]);
+        return 0;
+    }
+    static size_t refresh_smem(int n_ao) { return sizeof(float4) * RWPB * pair_scratch<NE, NUP>() + PT::bytes(n_ao); }
+
+    static int refresh(const HostSys& hs, DevWalkers& dw, bool ws, cudaStream_t st) {
+        const PT* S;
+        const int rc = pair_table(hs, &S);
+        if (rc) return rc;
+        const int nb = (dw.W + RWPB - 1) / RWPB;
+        auto kern = kw_refresh<NE, NUP, NNUC, RWPB>;
+        static bool attr = false;
+        if (!attr) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)refresh_smem(WMAX_AO)) != cudaSuccess)
+                return 2;
+            attr = true;
+        }
+        double* partial = (ws && dw.partial && dw.partial_cap >= 2 * nb + 1) ? dw.partial : nullptr;
+        kern<<<nb, 32 * RWPB, refresh_smem(hs.n_ao), st>>>(S, (const float*)dw.pos, (float*)dw.dinv, dw.logabs, dw.sign, dw.el,
+                                                          dw.W, dw.Wcap, ws ? 1 : 0, partial, dw.flags);
+        ++g_launch_count;
+        if (cudaGetLastError() != cudaSuccess) return 2;
+        if (!partial) return 0;
+        return launch_sum_partials(partial, nb, 1, dw.partial + dw.partial_cap - 1, st);
     }
 
     static int measure(const HostSys& hs, DevWalkers& dw, int cp, bool ws, const MeasureOut& out, cudaStream_t st) {
         if (out.O || out.fhf || out.omega) return 7;
         // FP32 walkers refresh in float-float arithmetic on the FP32 pipe
-        if (cp == 0) return dw.prec == 0 ? measure2<double, double>(hs, dw, ws, out, st)
-                                         : measure2<ff, float>(hs, dw, ws, out, st);
-        if (dw.prec == 1) return measure2<float, float>(hs, dw, ws, out, st);
+        if (cp == 0 && dw.prec == 0) return measure_w<double, double, WPB>(hs, dw, ws, out, st);
+        if (cp == 0) return out.grad || out.lap ? 7 : refresh(hs, dw, ws, st);
+        if (dw.prec == 1) return measure_w<float, float, WPB>(hs, dw, ws, out, st);
         return 7;
     }
 
@@ -1245,9 +1737,9 @@ struct WarpShapeOps {
             r.tab_d = r.tab_s = d;
             return 0;
         }
-        const SysW<ff>* m;
+        const PT* m;
         const SysW<float>* f;
-        int rc = table<ff>(hs, &m);
+        int rc = pair_table(hs, &m);
         if (!rc) rc = table<float>(hs, &f);
         if (rc) return rc;
         r.tab_d = m;
@@ -1300,7 +1792,19 @@ struct WarpShapeOps {
     }
 
     static int batch_measure(const BatchClass& bc, cudaStream_t st, int* occ = nullptr) {
-        return bc.prec == 0 ? batch_measure_t<double, double>(bc, st, occ) : batch_measure_t<ff, float>(bc, st, occ);
+        if (bc.prec == 0) return batch_measure_t<double, double>(bc, st, occ);
+        auto kern = kwb_refresh<NE, NUP, NNUC, RWPB>;
+        const size_t smem = refresh_smem(WMAX_AO);
+        static bool attr = false;
+        if (!attr) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
+            attr = true;
+        }
+        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, 32 * RWPB, smem) == cudaSuccess ? 0 : 2;
+        if (bc.ntiles == 0) return 0;
+        kern<<<bc.ntiles, 32 * RWPB, refresh_smem(bc.n_ao), st>>>(bc.tiles, bc.ntiles, bc.recs, bc.tile_partial);
+        ++g_launch_count;
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
     }
 
     static int sweep(const HostSys& hs, DevWalkers& dw, int mk, int n, uint64_t s0, double step, double tau,
