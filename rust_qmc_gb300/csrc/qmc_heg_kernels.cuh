@@ -39,6 +39,7 @@ struct SysH {
     double ksum_const;             // added per walker with the reciprocal sum
     T k2sum;                       // (1/2) sum over occupied |k|^2 of both sectors
     T kvec[2][32][3];              // [sector][column][xyz]
+    T k2[2][32];                   // |k|^2 of each
     int nt;                        // octant vectors of the reciprocal sum
     int kmax;                      // their largest component
     float aL, rc2u;                // alpha L and the squared real-space cutoff, in box units
@@ -158,8 +159,10 @@ static bool fill_sysh(const HostSys& hs, int NE, int NUP, SysH<T>& S, KTable& KT
             int k = hs.occ[e];
             if (col >= 32) return false;
             for (int c = 0; c < 3; ++c) S.kvec[sig][col][c] = (T)hs.kvec[3 * k + c];
-            k2s += hs.kvec[3 * k] * hs.kvec[3 * k] + hs.kvec[3 * k + 1] * hs.kvec[3 * k + 1] +
-                   hs.kvec[3 * k + 2] * hs.kvec[3 * k + 2];
+            const double k2 = hs.kvec[3 * k] * hs.kvec[3 * k] + hs.kvec[3 * k + 1] * hs.kvec[3 * k + 1] +
+                              hs.kvec[3 * k + 2] * hs.kvec[3 * k + 2];
+            S.k2[sig][col] = (T)k2;
+            k2s += k2;
             ++col;
         }
     }
@@ -1048,6 +1051,10 @@ __global__ void __launch_bounds__(32 * WPB, (sizeof(T) == 4 ? 16 : 8) / WPB) khw
     hsweep_walker<NE, NUP, T, MOVE>(S, args, hsm, w);
 }
 
+// Row stride of the refresh's matrix scratch (odd: rows and columns read without
+// bank conflicts).
+constexpr int HRS = 33;
+
 // Inverse of one sector's complex orbital matrix (rows in Mr, Mi) by the warp: lane j
 // ends with column j.  |det| goes into (pmag, pexp) (float-float: |det|^2) or logdet.
 template <int NM, class TC>
@@ -1056,8 +1063,8 @@ __device__ __forceinline__ void invert_sector(const TC* Mr, const TC* Mi, TC* bc
                 #pragma unroll
                 for (int i = 0; i < NM; ++i) {
                     bool in = i < NS && lane < NS;
-                    Ar[i] = in ? Mr[i * 32 + lane] : TC(i == lane ? 1 : 0);
-                    Ai[i] = in ? Mi[i * 32 + lane] : TC(0);
+                    Ar[i] = in ? Mr[i * HRS + lane] : TC(i == lane ? 1 : 0);
+                    Ai[i] = in ? Mi[i * HRS + lane] : TC(0);
                 }
                 int src = lane;
 #pragma unroll 1
@@ -1167,7 +1174,7 @@ __device__ __forceinline__ void invert_sector(const ff* Mr, const ff* Mi, ff* bc
 #pragma unroll
     for (int i = 0; i < NM; ++i) {
         const bool in = i < NS && lane < NS;
-        const ff r = in ? Mr[i * 32 + lane] : ff(i == lane ? 1 : 0), m = in ? Mi[i * 32 + lane] : ff(0);
+        const ff r = in ? Mr[i * HRS + lane] : ff(i == lane ? 1 : 0), m = in ? Mi[i * HRS + lane] : ff(0);
         A[i] = {F2(r.hi, m.hi), F2(r.lo, m.lo)};
     }
     float4* b4 = reinterpret_cast<float4*>(bc);        // [row](re.hi, im.hi, re.lo, im.lo), negated
@@ -1268,8 +1275,8 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
     constexpr int NDN = NE - NUP;
     constexpr int NM = NUP > NDN ? NUP : NDN;
     const int lane = threadIdx.x & 31;
-    TC* Mi = Mr + NM * 32;                            // Mr: [re|im][row][lane]
-    TC* bc = Mr + 2 * NM * 32;                        // [row][re|im] of the pivot column
+    TC* Mi = Mr + NM * HRS;                           // Mr: [re|im][row][lane]
+    TC* bc = Mr + 2 * NM * HRS;                       // [row][re|im] of the pivot column
     double e_l = 0.0;
     if (act) {
         HLanePos<TC, NE> P;
@@ -1288,17 +1295,18 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
         TC gdx[2] = {0, 0}, gdy[2] = {0, 0}, gdz[2] = {0, 0}, gqx[2] = {0, 0}, gqy[2] = {0, 0}, gqz[2] = {0, 0};
         TC ldet[2] = {0, 0};
         if constexpr (PART != 2) {
-#pragma unroll
+        // one copy of the sector's code, for the instruction cache
+#pragma unroll 1
         for (int sig = 0; sig < 2; ++sig) {
-            const int NS = sig == 0 ? NUP : NDN;
+            const int NS = NUP == NDN || sig == 0 ? NUP : NDN;
             const TC kx = S.kvec[sig][lane][0], ky = S.kvec[sig][lane][1], kz = S.kvec[sig][lane][2];
             for (int q = 0; q < NS; ++q) {
                 TC rx, ry, rz;
                 P.get(sig * NUP + q, rx, ry, rz);
                 TC s, c;
                 fsincos(kx * rx + ky * ry + kz * rz, &s, &c);
-                Mr[q * 32 + lane] = c;
-                Mi[q * 32 + lane] = s;
+                Mr[q * HRS + lane] = c;
+                Mi[q * HRS + lane] = s;
             }
             __syncwarp();
             // complex Gauss-Jordan in place: lane j carries column j of D and
@@ -1330,18 +1338,28 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
                 }
             }
             // lane = electron row q: grad ln D = sum_j Dinv[j][q] i k_j phi_j(r_q); lap D / D = -sum_j Dinv phi k^2
+            // (a rolled loop over a thread-local copy of the column: unrolled it is
+            // longer than the instruction cache)
             if (lane < NS) {
-                TC ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0, lr = 0;
+                TC Dr[NM], Dm[NM];
 #pragma unroll
-                for (int j = 0; j < NM; ++j) {
-                    if (j >= NS) break;
-                    TC pr = Mr[lane * 32 + j], pi = Mi[lane * 32 + j];
-                    TC re = pr * Ir[j] - pi * Ii[j], im = pr * Ii[j] + pi * Ir[j];
-                    TC kjx = S.kvec[sig][j][0], kjy = S.kvec[sig][j][1], kjz = S.kvec[sig][j][2];
-                    ax -= kjx * im; ay -= kjy * im; az -= kjz * im;                 // Re(i k w phi)
-                    bx -= kjx * Ii[j]; by -= kjy * Ii[j]; bz -= kjz * Ii[j];         // Re(i k w), reference form
-                    lr -= (kjx * kjx + kjy * kjy + kjz * kjz) * re;
+                for (int j = 0; j < NM; ++j) { Dr[j] = Ir[j]; Dm[j] = Ii[j]; }
+                TC ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0, lr = 0;
+#pragma unroll 1
+                for (int j = 0; j < NS; ++j) {
+                    const TC pr = Mr[lane * HRS + j], pi = Mi[lane * HRS + j], dr = Dr[j], di = Dm[j];
+                    TC re = mul_lazy(pr, dr), im = mul_lazy(pr, di);
+                    macc(re, -pi, di);
+                    macc(im, pi, dr);
+                    re = macc_norm(re);
+                    im = macc_norm(im);
+                    const TC kjx = -S.kvec[sig][j][0], kjy = -S.kvec[sig][j][1], kjz = -S.kvec[sig][j][2];
+                    macc(ax, kjx, im); macc(ay, kjy, im); macc(az, kjz, im);        // Re(i k w phi)
+                    if (S.quirk_cross) { macc(bx, kjx, di); macc(by, kjy, di); macc(bz, kjz, di); }   // Re(i k w), reference form
+                    macc(lr, -S.k2[sig][j], re);
                 }
+                ax = macc_norm(ax); ay = macc_norm(ay); az = macc_norm(az);
+                bx = macc_norm(bx); by = macc_norm(by); bz = macc_norm(bz); lr = macc_norm(lr);
                 gdx[sig] = ax; gdy[sig] = ay; gdz[sig] = az;
                 gqx[sig] = bx; gqy[sig] = by; gqz[sig] = bz;
                 ldet[sig] = lr;
@@ -1579,7 +1597,7 @@ __device__ __forceinline__ void hwarp_block_partial(double v, double* partial, i
 // sums per electron), then the phase table of a reciprocal cutoff kmax.
 template <int NE, int NUP, int PART>
 __host__ __device__ constexpr int hmeasure_warp_words(int kmax) {
-    const int det = PART == 2 ? 0 : 2 * (NUP > NE - NUP ? NUP : NE - NUP) * 33;
+    const int det = PART == 2 ? 0 : 2 * (NUP > NE - NUP ? NUP : NE - NUP) * (HRS + 1);
     const int pair = PART == 1 ? 0 : 7 * NE, ph = PART == 1 ? 0 : 6 * (kmax + 1) * NE;
     const int e = pair > ph ? pair : ph;
     return det > e ? det : e;
