@@ -52,9 +52,10 @@ struct HostSys {
     std::vector<double> kvec;            // periodic electron gas: [n_mo*3] orbital wave vectors
     int version = 0;                     // bumped when parameters or nuclei change
     // cached device copies of the system table per arithmetic type:
-    // [0] FP64, [1] FP32, [2] float-float; [3] the FP64 team kernels' table
-    mutable void* dev_table[4] = {nullptr, nullptr, nullptr, nullptr};
-    mutable int dev_table_version[4] = {-1, -1, -1, -1};
+    // [0] FP64, [1] FP32, [2] float-float; [3] the FP64 team kernels' table;
+    // [4] the FP32 Gaussian sweep's (benzene)
+    mutable void* dev_table[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    mutable int dev_table_version[5] = {-1, -1, -1, -1, -1};
 
     int n_params() const { return 8 + (int)rot_occ.size(); }
     // Effective (rotated) MO coefficients in caller AO order.
@@ -190,6 +191,7 @@ QMC_HD inline uint64_t batch_system_seed(uint64_t seed, int s) {
 struct BatchRec {
     const void* tab_d = nullptr;         // system table, FP64 form (shape-specific type)
     const void* tab_s = nullptr;         // system table in the walkers' precision
+    const void* tab_g = nullptr;         // table of the FP32 Gaussian sweep where it has its own (benzene), else null
     const void* ktab = nullptr;          // reciprocal-space table (electron gas), else null
     void* pos = nullptr;
     void* dinv = nullptr;

@@ -141,6 +141,17 @@ __device__ __forceinline__ void load_sysw(SysW<T>* dst, const SysW<T>* __restric
     __syncthreads();
 }
 
+// Used part of a table (a whole number of 16-byte words) into the block's shared
+// memory; ends with a block barrier.
+template <class TAB>
+__device__ __forceinline__ void load_tab(TAB* dst, const TAB* __restrict__ src) {
+    const int n = (int)(TAB::used(src) / sizeof(float4));
+    const float4* s = reinterpret_cast<const float4*>(src);
+    float4* d = reinterpret_cast<float4*>(dst);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = s[i];
+    __syncthreads();
+}
+
 // (exponent, coefficient) pair of a primitive: one 8- or 16-byte shared load.
 template <class T>
 __device__ __forceinline__ void load2(const T (&p)[2], T& a, T& b) { a = p[0]; b = p[1]; }
@@ -246,6 +257,15 @@ __device__ __forceinline__ int pair_slot(int i, int j) {
 template <int NE, int NUP>
 __host__ __device__ constexpr int sweep_scratch_elems() {
     return (NUP > NE - NUP ? NUP : NE - NUP) * WNCOL + jcache_elems<NE>();
+}
+// The FP32 Gaussian sweep's (kw_gauss_walker): per sector and proposal a row of
+// WNCOL orbital values, then the proposed position and the acceptance draw (a stride
+// of 7 16-byte words: row stores of neighbouring lanes fall on different banks); one
+// column of the inverse; the Jastrow cache.
+constexpr int GRS = WNCOL + 4;
+template <int NE, int NUP>
+__host__ __device__ constexpr int gauss_scratch_elems() {
+    return 2 * (NUP > NE - NUP ? NUP : NE - NUP) * GRS + WNCOL + jcache_elems<NE>();
 }
 
 // MO contraction: lane k receives phi_k = sum_a C[sig][a][k] chi_a (and
@@ -711,6 +731,399 @@ __device__ __forceinline__ void kw_sweep_walker(const SysW<T>& S, A& a, int w, T
     }
 }
 
+// An inverse column in registers: rows 2v and 2v + 1 in p[v], the last row of an odd
+// sector in t.
+template <int NM>
+struct ColF2 {
+    F2 p[NM / 2 > 0 ? NM / 2 : 1];
+    float t;
+};
+
+// Table of the FP32 Gaussian sweep: groups as (nucleus x, y, z, descriptor bits),
+// primitives (exponent, coefficient), coefficients of both sectors side by side, the
+// columns padded to pairs.
+template <int NNUC, int NM>
+struct GaussTab {
+    static constexpr int NC = (NM + 1) / 2 * 2;
+    int n_ao, n_grp;
+    float a_ee[2], b_ee[2];
+    float pad[2];
+    float nuc[NNUC][4];                       // x, y, z, unused
+    float en[NNUC][2];                        // A, B
+    alignas(16) float4 grp[WMAX_AO];
+    float2 prim[WMAX_PRIM];
+    float2 C[WMAX_AO][NC];
+    __host__ __device__ static size_t bytes(int n_ao) { return offsetof(GaussTab, C) + sizeof(float2) * NC * (size_t)n_ao; }
+    __device__ static size_t used(const GaussTab* t) { return bytes(t->n_ao); }
+};
+
+template <int NNUC, int NM>
+static void fill_gausstab(const SysW<float>& w, GaussTab<NNUC, NM>& S) {
+    std::memset(static_cast<void*>(&S), 0, sizeof(S));
+    S.n_ao = w.n_ao;
+    S.n_grp = w.n_grp;
+    for (int c = 0; c < 2; ++c) { S.a_ee[c] = w.a_ee[c]; S.b_ee[c] = w.b_ee[c]; }
+    for (int I = 0; I < NNUC; ++I) {
+        for (int c = 0; c < 3; ++c) S.nuc[I][c] = w.nuc[I][c];
+        S.en[I][0] = w.enA[I];
+        S.en[I][1] = w.enB[I];
+    }
+    for (int g = 0; g < w.n_grp; ++g) {
+        const int I = w.grp[g] & 15;
+        float bits;
+        std::memcpy(&bits, &w.grp[g], sizeof bits);
+        S.grp[g] = make_float4(w.nuc[I][0], w.nuc[I][1], w.nuc[I][2], bits);
+    }
+    for (int p = 0; p < WMAX_PRIM; ++p) S.prim[p] = make_float2(w.prim[p][0], w.prim[p][1]);
+    for (int a = 0; a < w.n_ao; ++a)
+        for (int k = 0; k < NM; ++k) S.C[a][k] = make_float2(w.C[0][a][k], w.C[1][a][k]);
+}
+
+// Orbital values of one proposal of each sector (x, y, z: the up sector's coordinate,
+// the down sector's) in packed instructions: proposal_orbitals' operations in the same
+// order on each.  Written to out0[k] and out1[k].
+template <int NNUC, int NM>
+__device__ __forceinline__ void proposal_orbitals2(const GaussTab<NNUC, NM>& S, F2 x, F2 y, F2 z, float* out0, float* out1) {
+    F2 acc[NM];
+#pragma unroll
+    for (int k = 0; k < NM; ++k) acc[k] = F2(0.0f);
+    auto axpy = [&](const float2* c, F2 chi) {
+#pragma unroll
+        for (int k = 0; k < NM; k += 2) {
+            const float4 v = *reinterpret_cast<const float4*>(c + k);
+            acc[k] = fma2(F2(v.x, v.y), chi, acc[k]);
+            if (k + 1 < NM) acc[k + 1 < NM ? k + 1 : 0] = fma2(F2(v.z, v.w), chi, acc[k + 1 < NM ? k + 1 : 0]);
+        }
+    };
+#pragma unroll 1
+    for (int g = 0; g < S.n_grp; ++g) {
+        const float4 G = S.grp[g];
+        const int d = __float_as_int(G.w);
+        const int np = (d >> 5) & 15;
+        const float2* prim = S.prim + ((d >> 9) & 255);
+        const float2* c = S.C[grp_a0(d)];
+        const F2 dx = add2(x, F2(-G.x)), dy = add2(y, F2(-G.y)), dz = add2(z, F2(-G.z));
+        const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+        F2 s0(0.0f);
+#pragma unroll 3
+        for (int p = 0; p < np; ++p) {
+            const float2 t = prim[p];
+            float e0, e1;
+            mul2(F2(-t.x), r2).get(e0, e1);
+            s0 = fma2(F2(t.y), F2(fexp(e0), fexp(e1)), s0);
+        }
+        if (d & 16) {
+            axpy(c, mul2(dx, s0));
+            axpy(c + S.NC, mul2(dy, s0));
+            axpy(c + 2 * S.NC, mul2(dz, s0));
+        } else {
+            axpy(c, s0);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NM; k += 4) {
+        float4 u, v;
+        acc[k].get(u.x, v.x);
+        acc[k + 1 < NM ? k + 1 : k].get(u.y, v.y);
+        acc[k + 2 < NM ? k + 2 : k].get(u.z, v.z);
+        acc[k + 3 < NM ? k + 3 : k].get(u.w, v.w);
+        *reinterpret_cast<float4*>(out0 + k) = u;
+        *reinterpret_cast<float4*>(out1 + k) = v;
+    }
+}
+
+// FP32 Gaussian sweeps.  kw_sweep_walker's operations in its order on every value;
+// here a lane's inverse columns lie in row pairs, so that ratio, update, orbital
+// contraction and the two rounds of Jastrow partners take packed FP32 instructions,
+// and a proposal's position and draw and the moving electron's column are read from
+// shared memory as broadcasts instead of a shuffle per value.
+template <int NE, int NUP, int NNUC, class TAB, class A>
+__device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float* ph) {
+    constexpr int NDN = NE - NUP;
+    constexpr int NM = NUP > NDN ? NUP : NDN;
+    constexpr int NE1 = NE > 32 ? NE - 32 : 0;   // partner electrons of the second round
+    constexpr int NPAIR = NE * (NE - 1) / 2;
+    static_assert(NE <= 64 && NE1 + NNUC <= 32, "second round: electrons 32.. and the nuclei share the lanes");
+    static_assert(NUP <= 32 && NDN <= 32, "one lane per sector electron");
+    const int lane = threadIdx.x & 31;
+    float* colq = ph + 2 * NM * GRS;                  // column q of the inverse
+    float* jc = colq + WNCOL;
+    const bool is_el = lane < NE1, is_nuc = !is_el && lane - NE1 < NNUC;
+    // partner positions: electron `lane`; electron 32 + lane or nucleus lane - NE1
+    // (the lanes past both repeat a partner and are masked)
+    const int j0 = lane < NE ? lane : NE - 1, j1 = is_el ? 32 + lane : 0, I1 = is_nuc ? lane - NE1 : 0;
+    auto load = [&](int j, int c) -> float { return a.pos[(3 * j + c) * (size_t)a.Wcap + w]; };
+    // p1 = (x, y'), p2 = (y, x'), pz = (z, z'), the second partner primed: its squared
+    // distance sums in the order y, x, z and the first one's in the order x, y, z
+    F2 p1(lane < NE ? load(j0, 0) : 0.0f, is_el ? load(j1, 1) : S.nuc[I1][1]),
+       p2(lane < NE ? load(j0, 1) : 0.0f, is_el ? load(j1, 0) : S.nuc[I1][0]),
+       pz(lane < NE ? load(j0, 2) : 0.0f, is_el ? load(j1, 2) : S.nuc[I1][2]);
+    ColF2<NM> D0, D1;
+    {
+        auto row = [&](int sig, int k) -> float {
+            return lane < (sig == 0 ? NUP : NDN) ? a.dinv[((size_t)(sig * NM * NM + k * NM + lane)) * a.Wcap + w] : 0.0f;
+        };
+#pragma unroll
+        for (int v = 0; v < NM / 2; ++v) {
+            D0.p[v] = F2(row(0, 2 * v), row(0, 2 * v + 1));
+            D1.p[v] = F2(row(1, 2 * v), row(1, 2 * v + 1));
+        }
+        if constexpr (NM % 2) { D0.t = row(0, NM - 1); D1.t = row(1, NM - 1); }
+    }
+    int sgn = a.sign[w];
+    unsigned acc = 0;
+    int flg = 0;
+    const bool fixed = a.fixed_node;
+    // position of electron e (any lane's own choice) from the lane that holds it
+    auto get = [&](int e, float& x, float& y, float& z) {
+        float a0, a1, b0, b1, c0, c1;
+        p1.get(a0, b1);
+        p2.get(b0, a1);
+        pz.get(c0, c1);
+        const int s = e & 31;
+        a0 = wshfl(a0, s); a1 = wshfl(a1, s); b0 = wshfl(b0, s); b1 = wshfl(b1, s); c0 = wshfl(c0, s); c1 = wshfl(c1, s);
+        x = e < 32 ? a0 : a1; y = e < 32 ? b0 : b1; z = e < 32 ? c0 : c1;
+    };
+    // the Jastrow cache (see kw_sweep_walker)
+    for (int i = 0; i < NE; ++i) {
+        float xi, yi, zi;
+        get(i, xi, yi, zi);
+        auto value = [&](float x, float y, float z, float A, float B) -> float {
+            const float dx = xi - x, dy = yi - y, dz = zi - z;
+            float d, ri, uu, upr, lt;
+            dist(dx * dx + dy * dy + dz * dz, d, ri);
+            pade_ab(A, B, d, ri, uu, upr, lt);
+            return uu;
+        };
+        float x[2], y[2], z[2];
+        p1.get(x[0], y[1]);
+        p2.get(y[0], x[1]);
+        pz.get(z[0], z[1]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int j = lane + 32 * r, c = ((j < NUP) == (i < NUP)) ? 1 : 0;
+            if (j < NE && j > i) jc[pair_slot(i, j)] = value(x[r], y[r], z[r], S.a_ee[c], S.b_ee[c]);
+        }
+        float en = 0;
+        if (lane < NNUC) en = value(S.nuc[lane][0], S.nuc[lane][1], S.nuc[lane][2], S.en[lane][0], S.en[lane][1]);
+        en = wsum(en);
+        if (lane == 0) jc[NPAIR + i] = en;
+    }
+    const int t0 = j0 * (j0 - 1) / 2, t1 = j1 * (j1 - 1) / 2;   // pair_slot of a larger partner, less e
+    for (int it = 0; it < a.n_sweeps; ++it) {
+        const uint64_t st = a.step0 + (uint64_t)it;
+        // Proposals of both sectors: an electron keeps its position until its own
+        // proposal, so all of them are known when the sweep starts.  Lane i evaluates the
+        // orbitals at proposal i of either sector.
+        __syncwarp();                                  // the previous sweep's rows are read
+        {
+            const float step = a.step;
+            const MoveDraw<float> du = sector_draws<float>(a.seed, (uint32_t)w, st, 0, NUP, lane),
+                                  dd = sector_draws<float>(a.seed, (uint32_t)w, st, NUP, NDN, lane);
+            const int eu = min(lane, NE - 1), ed = min(NUP + lane, NE - 1);
+            float ux, uy, uz, vx, vy, vz;
+            get(eu, ux, uy, uz);
+            get(ed, vx, vy, vz);
+            ux += step * du.n0; uy += step * du.n1; uz += step * du.n2;
+            vx += step * dd.n0; vy += step * dd.n1; vz += step * dd.n2;
+            if (lane < NM) {
+                float *r0 = ph + lane * GRS, *r1 = r0 + NM * GRS;
+                *reinterpret_cast<float4*>(r0 + WNCOL) = make_float4(ux, uy, uz, du.uacc);
+                *reinterpret_cast<float4*>(r1 + WNCOL) = make_float4(vx, vy, vz, dd.uacc);
+                proposal_orbitals2(S, F2(ux, vx), F2(uy, vy), F2(uz, vz), r0, r1);
+            }
+        }
+#pragma unroll
+        for (int sig = 0; sig < 2; ++sig) {
+            ColF2<NM>& D = sig == 0 ? D0 : D1;
+            const int NS = sig == 0 ? NUP : NDN;
+            // Padé parameters of the lane's two partners
+            const int c0 = ((j0 < NUP) == (sig == 0)) ? 1 : 0, c1 = ((j1 < NUP) == (sig == 0)) ? 1 : 0;
+            const F2 pa(S.a_ee[c0], is_el ? S.a_ee[c1] : S.en[I1][0]), pb(S.b_ee[c0], is_el ? S.b_ee[c1] : S.en[I1][1]);
+            float csc = 1;                             // pending scale of this lane's column
+            const float* row = ph + sig * NM * GRS;
+            for (int q = 0; q < NS; ++q, row += GRS) {
+                const int e = sig * NUP + q;
+                if (lane == q) {
+#pragma unroll
+                    for (int v = 0; v < NM / 4; ++v) {
+                        float4 c;
+                        D.p[2 * v].get(c.x, c.y);
+                        D.p[2 * v + 1].get(c.z, c.w);
+                        reinterpret_cast<float4*>(colq)[v] = c;
+                    }
+                    if constexpr (NM % 4 >= 2) {
+                        float2 c;
+                        D.p[NM / 2 - 1].get(c.x, c.y);
+                        *reinterpret_cast<float2*>(colq + NM / 4 * 4) = c;
+                    }
+                    if constexpr (NM % 2) colq[NM - 1] = D.t;
+                }
+                __syncwarp();                          // column and rows before their reads
+                const float4 np = *reinterpret_cast<const float4*>(row + WNCOL);
+                // t_j = sum_k phi_k Dinv[k][j], even and odd rows apart; R = t_q
+                F2 t2(0.0f);
+                float ta, tb;
+#pragma unroll
+                for (int v = 0; v < NM / 4; ++v) {
+                    const float4 f = reinterpret_cast<const float4*>(row)[v];
+                    t2 = fma2(F2(f.x, f.y), D.p[2 * v], t2);
+                    t2 = fma2(F2(f.z, f.w), D.p[2 * v + 1], t2);
+                }
+                if constexpr (NM % 4 >= 2) {
+                    const float2 f = *reinterpret_cast<const float2*>(row + NM / 4 * 4);
+                    t2 = fma2(F2(f.x, f.y), D.p[NM / 2 - 1], t2);
+                }
+                t2.get(ta, tb);
+                if constexpr (NM % 2) ta += row[NM - 1] * D.t;
+                const float tj = ta + tb;
+                const float R = wshfl(tj, q);
+                // the moving electron's new Jastrow terms against the cached old ones
+                // (unused terms are masked out; their lanes read a valid cache slot and may
+                // compute non-finite values)
+                const int et = e * (e - 1) / 2;
+                float *s0, *s1;
+                float u0, u1;
+                {
+                    const F2 neg(-1.0f);
+                    const F2 d1 = fma2(p1, neg, F2(np.x, np.y)), d2 = fma2(p2, neg, F2(np.y, np.x)), dz = fma2(pz, neg, F2(np.z));
+                    float ra, rb, da, db;
+                    fma2(dz, dz, fma2(d1, d1, mul2(d2, d2))).get(ra, rb);
+                    float ia, ib;
+                    dist(ra, da, ia);
+                    dist(rb, db, ib);
+                    const F2 d(da, db);
+                    float na, nb;
+                    fma2(pb, d, F2(1.0f)).get(na, nb);
+                    const F2 ad = mul2(pa, d), inv(frcp(na), frcp(nb));
+                    mul2(ad, inv).get(u0, u1);
+                    s0 = jc + (j0 < e ? et + j0 : t0 + e);
+                    s1 = jc + (j1 < e ? et + j1 : t1 + e);
+                }
+                const bool on0 = lane < NE && lane != e, on1 = is_el && j1 != e;
+                const float enn = is_nuc ? u1 : 0.0f;
+                float ds = on0 ? u0 - *s0 : 0.0f;
+                ds += on1 ? u1 - *s1 : 0.0f;
+                ds -= enn;
+                const float du = wsum(ds) + jc[NPAIR + e];
+                const float ratio = R * fexp(du);
+                const float prob = ratio * ratio;
+                if (prob != prob) flg |= FLAG_NONFINITE;
+                if (np.w < prob && R != 0.0f && !(fixed && R < 0.0f)) {
+                    // the lane that holds e takes the new position
+                    if ((e & 31) == lane) {
+                        float a0, a1, b0, b1, c0, c1;
+                        p1.get(a0, b1);
+                        p2.get(b0, a1);
+                        pz.get(c0, c1);
+                        if (e < 32) { a0 = np.x; b0 = np.y; c0 = np.z; }
+                        else { a1 = np.x; b1 = np.y; c1 = np.z; }
+                        p1 = F2(a0, b1); p2 = F2(b0, a1); pz = F2(c0, c1);
+                    }
+                    const float iR = 1.0f / R;
+                    // column q keeps its values and takes the factor 1/R when the sector
+                    // ends; the others take t_j / R times column q
+                    const float f = lane == q ? 0.0f : tj * iR;
+                    if (lane == q) csc = iR;
+                    const F2 nf(-f);
+#pragma unroll
+                    for (int v = 0; v < NM / 4; ++v) {
+                        const float4 c = reinterpret_cast<const float4*>(colq)[v];
+                        D.p[2 * v] = fma2(F2(c.x, c.y), nf, D.p[2 * v]);
+                        D.p[2 * v + 1] = fma2(F2(c.z, c.w), nf, D.p[2 * v + 1]);
+                    }
+                    if constexpr (NM % 4 >= 2) {
+                        const float2 c = *reinterpret_cast<const float2*>(colq + NM / 4 * 4);
+                        D.p[NM / 2 - 1] = fma2(F2(c.x, c.y), nf, D.p[NM / 2 - 1]);
+                    }
+                    if constexpr (NM % 2) D.t -= colq[NM - 1] * f;
+                    if (R < 0) sgn = -sgn;
+                    ++acc;
+                    if (on0) *s0 = u0;
+                    if (on1) *s1 = u1;
+                    const float us = wsum(enn);
+                    if (lane == 0) jc[NPAIR + e] = us;
+                }
+                __syncwarp();                          // this proposal's reads before the next one's writes
+            }
+            const F2 sc(csc);
+#pragma unroll
+            for (int v = 0; v < NM / 2; ++v) D.p[v] = mul2(D.p[v], sc);
+            if constexpr (NM % 2) D.t *= csc;
+        }
+    }
+    {
+        float x[2], y[2], z[2];
+        p1.get(x[0], y[1]);
+        p2.get(y[0], x[1]);
+        pz.get(z[0], z[1]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            if (r == 0 ? lane < NE : is_el) {
+                const int j = lane + 32 * r;
+                a.pos[(3 * j + 0) * (size_t)a.Wcap + w] = x[r];
+                a.pos[(3 * j + 1) * (size_t)a.Wcap + w] = y[r];
+                a.pos[(3 * j + 2) * (size_t)a.Wcap + w] = z[r];
+            }
+    }
+#pragma unroll
+    for (int sig = 0; sig < 2; ++sig) {
+        const ColF2<NM>& D = sig == 0 ? D0 : D1;
+        if (lane >= (sig == 0 ? NUP : NDN)) continue;
+        float* out = a.dinv + ((size_t)sig * NM * NM + lane) * a.Wcap + w;
+        const size_t rs = (size_t)NM * a.Wcap;
+#pragma unroll
+        for (int v = 0; v < NM / 2; ++v) {
+            float lo, hi;
+            D.p[v].get(lo, hi);
+            out[2 * v * rs] = lo;
+            out[(2 * v + 1) * rs] = hi;
+        }
+        if constexpr (NM % 2) out[(NM - 1) * rs] = D.t;
+    }
+    if (lane == 0) {
+        a.sign[w] = sgn;
+        if (acc) atomicAdd(a.acc, (unsigned long long)acc);
+        if (flg) atomicOr(a.flags, flg);
+    }
+}
+
+// Block size of the FP32 Gaussian sweep in dynamic shared memory.
+template <int NE, int NUP, int NNUC, int WPB>
+static size_t gauss_smem(int n_ao) {
+    return GaussTab<NNUC, (NUP > NE - NUP ? NUP : NE - NUP)>::bytes(n_ao) + sizeof(float) * WPB * gauss_scratch_elems<NE, NUP>();
+}
+// Dynamic shared memory: the table's used part, then the warps' scratch.
+template <int NE, int NUP, int NNUC, class TAB>
+__device__ __forceinline__ void gauss_block(const TAB* __restrict__ Sg, const volatile SweepArgs<float>& a, unsigned char* sm,
+                                            int w) {
+    TAB& S = *reinterpret_cast<TAB*>(sm);
+    load_tab(&S, Sg);                      // ends with a block barrier
+    if (w >= a.W) return;                      // whole warps only; no block barrier below
+    kw_gauss_walker<NE, NUP, NNUC>(S, a, w, reinterpret_cast<float*>(sm + TAB::bytes(S.n_ao)) +
+                                                (size_t)(threadIdx.x >> 5) * gauss_scratch_elems<NE, NUP>());
+}
+template <int NE, int NUP, int NNUC, int WPB, class TAB>
+__global__ void __launch_bounds__(32 * WPB, 16 / WPB) kw_gauss(const TAB* __restrict__ Sg, const __grid_constant__ SweepArgs<float> args0) {
+    __shared__ SweepArgs<float> args;
+    extern __shared__ __align__(16) unsigned char wsm[];
+    if (threadIdx.x == 0) args = args0;
+    gauss_block<NE, NUP, NNUC>(Sg, args, wsm, (int)blockIdx.x * WPB + (int)(threadIdx.x >> 5));
+}
+template <int NE, int NUP, int NNUC, int WPB, int TW, class TAB>
+__global__ void __launch_bounds__(32 * WPB, 16 / WPB) kwb_gauss(const BatchTile* __restrict__ tiles, int ntiles,
+                                                                const BatchRec* __restrict__ recs, const BatchCtl* __restrict__ ctl) {
+    static_assert(TW % WPB == 0, "a tile splits into whole blocks");
+    constexpr int BPT = TW / WPB;
+    __shared__ SweepArgs<float> args;
+    extern __shared__ __align__(16) unsigned char wsm[];
+    if ((int)blockIdx.x >= ntiles * BPT) return;
+    const BatchTile tl = tiles[blockIdx.x / BPT];
+    if (threadIdx.x == 0) args = sweep_args<float>(recs[tl.rec], *ctl);
+    gauss_block<NE, NUP, NNUC>(static_cast<const TAB*>(recs[tl.rec].tab_g), args, wsm,
+                               tl.w0 + (int)(blockIdx.x % BPT) * WPB + (int)(threadIdx.x >> 5));
+}
+
 // FP32: four 4-walker blocks per SM (<= 128 registers)
 template <int NE, int NUP, int NNUC, class T, int MOVE, int WPB>
 __global__ void __launch_bounds__(32 * WPB, sizeof(T) == 4 ? 16 / WPB : 1) kw_sweep(const SysW<T>* __restrict__ Sg, T* __restrict__ gpos,
@@ -1066,6 +1479,7 @@ struct PairTab {
     float4 prim[WMAX_PRIM];
     float4 C[WMAX_AO][NM];
     __host__ __device__ static size_t bytes(int n_ao) { return offsetof(PairTab, C) + sizeof(float4) * NM * (size_t)n_ao; }
+    __device__ static size_t used(const PairTab* t) { return bytes(t->head.n_ao); }
 };
 
 template <int NNUC, int NM>
@@ -1482,16 +1896,6 @@ __device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S,
     return act ? e_l : 0.0;
 }
 
-// Whole-block copy of the table (n_ao rows of coefficients) into shared memory.
-template <class TAB>
-__device__ __forceinline__ void load_pairtab(TAB* dst, const TAB* __restrict__ src) {
-    const int n = (int)(TAB::bytes(src->head.n_ao) / sizeof(float4));
-    const float4* s = reinterpret_cast<const float4*>(src);
-    float4* d = reinterpret_cast<float4*>(dst);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = s[i];
-    __syncthreads();
-}
-
 // Compensated sum of the block's per-warp values (lane 0 of each warp) into
 // partial[2 slot], partial[2 slot + 1]; ends with a block barrier.
 template <int WPB>
@@ -1557,7 +1961,7 @@ __global__ void __launch_bounds__(32 * WPB, 12 / WPB) kw_refresh(const PairTab<N
     const int wib = threadIdx.x >> 5, w = blockIdx.x * WPB + wib;
     float4* scr = reinterpret_cast<float4*>(wsm) + (size_t)wib * pair_scratch<NE, NUP>();
     auto& S = *reinterpret_cast<PairTab<NNUC, NUP>*>(wsm + sizeof(float4) * WPB * pair_scratch<NE, NUP>());
-    load_pairtab(&S, Sg);
+    load_tab(&S, Sg);
     // warps past the last walker repeat it and store nothing
     const double e_l = kw_refresh_walker<NE, NUP, NNUC>(S, scr, gpos, gdinv, glog, gsign, gel, min(w, W - 1), w < W,
                                                         Wcap, write_state, flags);
@@ -1574,7 +1978,7 @@ __global__ void __launch_bounds__(32 * WPB, 12 / WPB) kwb_refresh(const BatchTil
     auto& S = *reinterpret_cast<PairTab<NNUC, NUP>*>(wsm + sizeof(float4) * WPB * pair_scratch<NE, NUP>());
     const BatchTile tl = tiles[blockIdx.x];
     const BatchRec& R = recs[tl.rec];
-    load_pairtab(&S, static_cast<const PairTab<NNUC, NUP>*>(R.tab_d));
+    load_tab(&S, static_cast<const PairTab<NNUC, NUP>*>(R.tab_d));
     const int w = tl.w0 + wib;
     const double e_l = kw_refresh_walker<NE, NUP, NNUC>(S, scr, (const float*)R.pos, (float*)R.dinv, R.logabs, R.sign,
                                                         R.el, min(w, R.W - 1), w < R.W, R.Wcap, 1, R.flags);
@@ -1672,6 +2076,59 @@ struct WarpShapeOps {
         *out = static_cast<const PT*>(hs.dev_table[slot]);
         return 0;
     }
+    // FP32 Gaussian sweeps: their table and launches.
+    using GT = GaussTab<NNUC, NM>;
+    static int gauss_table(const HostSys& hs, const GT** out) {
+        constexpr int slot = 4;
+        if (!hs.dev_table[slot] || hs.dev_table_version[slot] != hs.version) {
+            SysW<float>* w = new SysW<float>;
+            GT* h = new GT;
+            const bool good = fill_sysw<float>(hs, NE, NUP, NNUC, *w);
+            if (good) fill_gausstab<NNUC, NM>(*w, *h);
+            int rc = good ? 0 : 7;
+            if (!rc && !hs.dev_table[slot] && cudaMalloc(&hs.dev_table[slot], sizeof(GT)) != cudaSuccess) rc = 8;
+            if (!rc && cudaMemcpy(hs.dev_table[slot], h, sizeof(GT), cudaMemcpyHostToDevice) != cudaSuccess) rc = 2;
+            delete w;
+            delete h;
+            if (rc) return rc;
+            hs.dev_table_version[slot] = hs.version;
+        }
+        *out = static_cast<const GT*>(hs.dev_table[slot]);
+        return 0;
+    }
+    static int gauss(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, uint64_t seed, cudaStream_t st) {
+        const GT* S;
+        const int rc = gauss_table(hs, &S);
+        if (rc) return rc;
+        auto kern = kw_gauss<NE, NUP, NNUC, WPB, GT>;
+        static bool attr = false;
+        if (!attr) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)gauss_smem<NE, NUP, NNUC, WPB>(WMAX_AO)) != cudaSuccess)
+                return 2;
+            attr = true;
+        }
+        const SweepArgs<float> a{(float*)dw.pos, (float*)dw.dinv, dw.sign, dw.acc, dw.flags, s0, seed,
+                                 (float)step, 0.0f, 0.0f, dw.W, dw.Wcap, n, dw.fixed_node};
+        kern<<<(dw.W + WPB - 1) / WPB, 32 * WPB, gauss_smem<NE, NUP, NNUC, WPB>(hs.n_ao), st>>>(S, a);
+        ++g_launch_count;
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
+    }
+    static int batch_gauss(const BatchClass& bc, const BatchCtl* ctl, cudaStream_t st, int* occ) {
+        auto kern = kwb_gauss<NE, NUP, NNUC, WPB, BTW, GT>;
+        const size_t smem = gauss_smem<NE, NUP, NNUC, WPB>(WMAX_AO);
+        static bool attr = false;
+        if (!attr) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
+            attr = true;
+        }
+        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, 32 * WPB, smem) == cudaSuccess ? 0 : 2;
+        if (bc.ntiles == 0) return 0;
+        kern<<<bc.ntiles * (BTW / WPB), 32 * WPB, smem, st>>>(bc.tiles, bc.ntiles, bc.recs, ctl);
+        ++g_launch_count;
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
+    }
+
     static size_t refresh_smem(int n_ao) { return sizeof(float4) * RWPB * pair_scratch<NE, NUP>() + PT::bytes(n_ao); }
 
     static int refresh(const HostSys& hs, DevWalkers& dw, bool ws, cudaStream_t st) {
@@ -1740,10 +2197,13 @@ struct WarpShapeOps {
         const PT* m;
         const SysW<float>* f;
         int rc = pair_table(hs, &m);
+        const GT* g;
         if (!rc) rc = table<float>(hs, &f);
+        if (!rc) rc = gauss_table(hs, &g);
         if (rc) return rc;
         r.tab_d = m;
         r.tab_s = f;
+        r.tab_g = g;
         return 0;
     }
 
@@ -1767,7 +2227,7 @@ struct WarpShapeOps {
     static int batch_sweep(const BatchClass& bc, int mk, const BatchCtl* ctl, cudaStream_t st, int* occ = nullptr) {
         if (mk == MOVE_ONE_GAUSS)
             return bc.prec == 0 ? batch_sweep_t<double, MOVE_ONE_GAUSS>(bc, ctl, st, occ)
-                                : batch_sweep_t<float, MOVE_ONE_GAUSS>(bc, ctl, st, occ);
+                                : batch_gauss(bc, ctl, st, occ);
         if (mk == MOVE_ONE_DRIFT)
             return bc.prec == 0 ? batch_sweep_t<double, MOVE_ONE_DRIFT>(bc, ctl, st, occ)
                                 : batch_sweep_t<float, MOVE_ONE_DRIFT>(bc, ctl, st, occ);
@@ -1811,7 +2271,7 @@ struct WarpShapeOps {
                      double maxd, uint64_t seed, cudaStream_t st) {
         if (mk == MOVE_ONE_GAUSS)
             return dw.prec == 0 ? sweep_t<double, MOVE_ONE_GAUSS>(hs, dw, n, s0, step, tau, maxd, seed, st)
-                                : sweep_t<float, MOVE_ONE_GAUSS>(hs, dw, n, s0, step, tau, maxd, seed, st);
+                                : gauss(hs, dw, n, s0, step, seed, st);
         if (mk == MOVE_ONE_DRIFT)
             return dw.prec == 0 ? sweep_t<double, MOVE_ONE_DRIFT>(hs, dw, n, s0, step, tau, maxd, seed, st)
                                 : sweep_t<float, MOVE_ONE_DRIFT>(hs, dw, n, s0, step, tau, maxd, seed, st);
