@@ -260,12 +260,12 @@ __host__ __device__ constexpr int sweep_scratch_elems() {
 }
 // The FP32 Gaussian sweep's (kw_gauss_walker): per sector and proposal a row of
 // WNCOL orbital values, then the proposed position and the acceptance draw (a stride
-// of 7 16-byte words: row stores of neighbouring lanes fall on different banks); one
-// column of the inverse; the Jastrow cache.
+// of 7 16-byte words: row stores of neighbouring lanes fall on different banks); two
+// columns of the inverse; the Jastrow cache.
 constexpr int GRS = WNCOL + 4;
 template <int NE, int NUP>
 __host__ __device__ constexpr int gauss_scratch_elems() {
-    return 2 * (NUP > NE - NUP ? NUP : NE - NUP) * GRS + WNCOL + jcache_elems<NE>();
+    return 2 * (NUP > NE - NUP ? NUP : NE - NUP) * GRS + 2 * WNCOL + jcache_elems<NE>();
 }
 
 // MO contraction: lane k receives phi_k = sum_a C[sig][a][k] chi_a (and
@@ -739,9 +739,10 @@ struct ColF2 {
     float t;
 };
 
-// Table of the FP32 Gaussian sweep: groups as (nucleus x, y, z, descriptor bits),
-// primitives (exponent, coefficient), coefficients of both sectors side by side, the
-// columns padded to pairs.
+// Table of the FP32 Gaussian sweep, values of both halves of a packed instruction
+// doubled: groups as (-x, -x, -y, -y), (-z, -z, descriptor bits, 0) of the nucleus,
+// primitives (-exponent, -exponent, coefficient, coefficient), coefficients of both
+// sectors side by side, the columns padded to pairs.
 template <int NNUC, int NM>
 struct GaussTab {
     static constexpr int NC = (NM + 1) / 2 * 2;
@@ -750,8 +751,8 @@ struct GaussTab {
     float pad[2];
     float nuc[NNUC][4];                       // x, y, z, unused
     float en[NNUC][2];                        // A, B
-    alignas(16) float4 grp[WMAX_AO];
-    float2 prim[WMAX_PRIM];
+    alignas(16) float4 grp[WMAX_AO][2];
+    float4 prim[WMAX_PRIM];
     float2 C[WMAX_AO][NC];
     __host__ __device__ static size_t bytes(int n_ao) { return offsetof(GaussTab, C) + sizeof(float2) * NC * (size_t)n_ao; }
     __device__ static size_t used(const GaussTab* t) { return bytes(t->n_ao); }
@@ -772,9 +773,10 @@ static void fill_gausstab(const SysW<float>& w, GaussTab<NNUC, NM>& S) {
         const int I = w.grp[g] & 15;
         float bits;
         std::memcpy(&bits, &w.grp[g], sizeof bits);
-        S.grp[g] = make_float4(w.nuc[I][0], w.nuc[I][1], w.nuc[I][2], bits);
+        S.grp[g][0] = make_float4(-w.nuc[I][0], -w.nuc[I][0], -w.nuc[I][1], -w.nuc[I][1]);
+        S.grp[g][1] = make_float4(-w.nuc[I][2], -w.nuc[I][2], bits, 0.0f);
     }
-    for (int p = 0; p < WMAX_PRIM; ++p) S.prim[p] = make_float2(w.prim[p][0], w.prim[p][1]);
+    for (int p = 0; p < WMAX_PRIM; ++p) S.prim[p] = make_float4(-w.prim[p][0], -w.prim[p][0], w.prim[p][1], w.prim[p][1]);
     for (int a = 0; a < w.n_ao; ++a)
         for (int k = 0; k < NM; ++k) S.C[a][k] = make_float2(w.C[0][a][k], w.C[1][a][k]);
 }
@@ -797,20 +799,20 @@ __device__ __forceinline__ void proposal_orbitals2(const GaussTab<NNUC, NM>& S, 
     };
 #pragma unroll 1
     for (int g = 0; g < S.n_grp; ++g) {
-        const float4 G = S.grp[g];
-        const int d = __float_as_int(G.w);
+        const float4 G = S.grp[g][0], H = S.grp[g][1];
+        const int d = __float_as_int(H.z);
         const int np = (d >> 5) & 15;
-        const float2* prim = S.prim + ((d >> 9) & 255);
+        const float4* prim = S.prim + ((d >> 9) & 255);
         const float2* c = S.C[grp_a0(d)];
-        const F2 dx = add2(x, F2(-G.x)), dy = add2(y, F2(-G.y)), dz = add2(z, F2(-G.z));
+        const F2 dx = add2(x, F2(G.x, G.y)), dy = add2(y, F2(G.z, G.w)), dz = add2(z, F2(H.x, H.y));
         const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
         F2 s0(0.0f);
 #pragma unroll 3
         for (int p = 0; p < np; ++p) {
-            const float2 t = prim[p];
+            const float4 t = prim[p];
             float e0, e1;
-            mul2(F2(-t.x), r2).get(e0, e1);
-            s0 = fma2(F2(t.y), F2(fexp(e0), fexp(e1)), s0);
+            mul2(F2(t.x, t.y), r2).get(e0, e1);
+            s0 = fma2(F2(t.z, t.w), F2(fexp(e0), fexp(e1)), s0);
         }
         if (d & 16) {
             axpy(c, mul2(dx, s0));
@@ -832,6 +834,27 @@ __device__ __forceinline__ void proposal_orbitals2(const GaussTab<NNUC, NM>& S, 
     }
 }
 
+// v[0] + ... + v[N - 1] in the order of wsum with v[i] on lane L0 + i (N <= 32 - L0) and
+// zeros elsewhere, which are left out.
+template <int L0, int N>
+__device__ __forceinline__ float wsum_order(const float* v) {
+    float s[32];
+    bool on[32];
+#pragma unroll
+    for (int l = 0; l < 32; ++l) {
+        on[l] = l >= L0 && l < L0 + N;
+        s[l] = on[l] ? v[on[l] ? l - L0 : 0] : 0.0f;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+#pragma unroll
+        for (int l = 0; l < o; ++l) {
+            s[l] = on[l] && on[l + o] ? s[l] + s[l + o] : (on[l] ? s[l] : s[l + o]);
+            on[l] = on[l] || on[l + o];
+        }
+    return s[0];
+}
+
 // FP32 Gaussian sweeps.  kw_sweep_walker's operations in its order on every value;
 // here a lane's inverse columns lie in row pairs, so that ratio, update, orbital
 // contraction and the two rounds of Jastrow partners take packed FP32 instructions,
@@ -845,9 +868,10 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
     constexpr int NPAIR = NE * (NE - 1) / 2;
     static_assert(NE <= 64 && NE1 + NNUC <= 32, "second round: electrons 32.. and the nuclei share the lanes");
     static_assert(NUP <= 32 && NDN <= 32, "one lane per sector electron");
+    static_assert(NNUC <= WNCOL, "a row takes the nuclei's terms");
     const int lane = threadIdx.x & 31;
-    float* colq = ph + 2 * NM * GRS;                  // column q of the inverse
-    float* jc = colq + WNCOL;
+    float* cols = ph + 2 * NM * GRS;              // column q of the inverse, at (q mod 2) WNCOL
+    float* jc = cols + 2 * WNCOL;
     const bool is_el = lane < NE1, is_nuc = !is_el && lane - NE1 < NNUC;
     // partner positions: electron `lane`; electron 32 + lane or nucleus lane - NE1
     // (the lanes past both repeat a partner and are masked)
@@ -909,7 +933,6 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
         en = wsum(en);
         if (lane == 0) jc[NPAIR + i] = en;
     }
-    const int t0 = j0 * (j0 - 1) / 2, t1 = j1 * (j1 - 1) / 2;   // pair_slot of a larger partner, less e
     for (int it = 0; it < a.n_sweeps; ++it) {
         const uint64_t st = a.step0 + (uint64_t)it;
         // Proposals of both sectors: an electron keeps its position until its own
@@ -941,9 +964,14 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
             const int c0 = ((j0 < NUP) == (sig == 0)) ? 1 : 0, c1 = ((j1 < NUP) == (sig == 0)) ? 1 : 0;
             const F2 pa(S.a_ee[c0], is_el ? S.a_ee[c1] : S.en[I1][0]), pb(S.b_ee[c0], is_el ? S.b_ee[c1] : S.en[I1][1]);
             float csc = 1;                             // pending scale of this lane's column
-            const float* row = ph + sig * NM * GRS;
-            for (int q = 0; q < NS; ++q, row += GRS) {
+            float* row = ph + sig * NM * GRS;
+            unsigned moved = 0;                        // accepted proposals of the sector
+            // the cache slots of e and the two partners: pair_slot, which grows by 1 while
+            // e < j and by e from there on
+            float *s0 = jc + pair_slot(sig * NUP, j0), *s1 = jc + pair_slot(sig * NUP, j1);
+            for (int q = 0; q < NS; ++q) {
                 const int e = sig * NUP + q;
+                float* colq = cols + (q & 1) * WNCOL;
                 if (lane == q) {
 #pragma unroll
                     for (int v = 0; v < NM / 4; ++v) {
@@ -981,8 +1009,6 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
                 // the moving electron's new Jastrow terms against the cached old ones
                 // (unused terms are masked out; their lanes read a valid cache slot and may
                 // compute non-finite values)
-                const int et = e * (e - 1) / 2;
-                float *s0, *s1;
                 float u0, u1;
                 {
                     const F2 neg(-1.0f);
@@ -997,8 +1023,6 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
                     fma2(pb, d, F2(1.0f)).get(na, nb);
                     const F2 ad = mul2(pa, d), inv(frcp(na), frcp(nb));
                     mul2(ad, inv).get(u0, u1);
-                    s0 = jc + (j0 < e ? et + j0 : t0 + e);
-                    s1 = jc + (j1 < e ? et + j1 : t1 + e);
                 }
                 const bool on0 = lane < NE && lane != e, on1 = is_el && j1 != e;
                 const float enn = is_nuc ? u1 : 0.0f;
@@ -1011,13 +1035,14 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
                 if (prob != prob) flg |= FLAG_NONFINITE;
                 if (np.w < prob && R != 0.0f && !(fixed && R < 0.0f)) {
                     // the lane that holds e takes the new position
-                    if ((e & 31) == lane) {
+                    {
                         float a0, a1, b0, b1, c0, c1;
                         p1.get(a0, b1);
                         p2.get(b0, a1);
                         pz.get(c0, c1);
-                        if (e < 32) { a0 = np.x; b0 = np.y; c0 = np.z; }
-                        else { a1 = np.x; b1 = np.y; c1 = np.z; }
+                        const bool h0 = lane == e, h1 = lane + 32 == e;
+                        a0 = h0 ? np.x : a0; b0 = h0 ? np.y : b0; c0 = h0 ? np.z : c0;
+                        a1 = h1 ? np.x : a1; b1 = h1 ? np.y : b1; c1 = h1 ? np.z : c1;
                         p1 = F2(a0, b1); p2 = F2(b0, a1); pz = F2(c0, c1);
                     }
                     const float iR = 1.0f / R;
@@ -1041,11 +1066,19 @@ __device__ __forceinline__ void kw_gauss_walker(const TAB& S, A& a, int w, float
                     ++acc;
                     if (on0) *s0 = u0;
                     if (on1) *s1 = u1;
-                    const float us = wsum(enn);
-                    if (lane == 0) jc[NPAIR + e] = us;
+                    // the one-body terms wait in the proposal's row, which has been read
+                    if (is_nuc) row[lane - NE1] = enn;
+                    moved |= 1u << q;
                 }
-                __syncwarp();                          // this proposal's reads before the next one's writes
+                s0 += e < j0 ? 1 : e;
+                s1 += e < j1 ? 1 : e;
+                row += GRS;
             }
+            __syncwarp();
+            // one-body sums of the moved electrons, by their lanes, as the warp sum over the
+            // nuclei's lanes adds them
+            if (moved >> lane & 1) jc[NPAIR + sig * NUP + lane] = wsum_order<NE1, NNUC>(ph + (sig * NM + lane) * GRS);
+            __syncwarp();
             const F2 sc(csc);
 #pragma unroll
             for (int v = 0; v < NM / 2; ++v) D.p[v] = mul2(D.p[v], sc);
@@ -2116,10 +2149,12 @@ struct WarpShapeOps {
     }
     static int batch_gauss(const BatchClass& bc, const BatchCtl* ctl, cudaStream_t st, int* occ) {
         auto kern = kwb_gauss<NE, NUP, NNUC, WPB, BTW, GT>;
-        const size_t smem = gauss_smem<NE, NUP, NNUC, WPB>(WMAX_AO);
+        const size_t smem = gauss_smem<NE, NUP, NNUC, WPB>(bc.n_ao);
         static bool attr = false;
         if (!attr) {
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)gauss_smem<NE, NUP, NNUC, WPB>(WMAX_AO)) != cudaSuccess)
+                return 2;
             attr = true;
         }
         if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, 32 * WPB, smem) == cudaSuccess ? 0 : 2;
