@@ -1606,7 +1606,7 @@ __host__ __device__ constexpr int hmeasure_warp_words(int kmax) {
 // takes 73 KB a block at kmax = 6).
 
 template <int NE, int NUP, class TC, class TS, int WPB, int PART = 0>
-__global__ void __launch_bounds__(32 * WPB, PART == 2 ? 3 : 2) khw_measure(
+__global__ void __launch_bounds__(32 * WPB, PART == 0 ? 2 : 3) khw_measure(
     const SysH<TC>* __restrict__ Sg, const KTable* __restrict__ KT, const TS* __restrict__ gpos,
     TS* __restrict__ gdinv, double* __restrict__ glog, int* __restrict__ gsign, double* __restrict__ gel, int W,
     int Wcap, int write_state, double* __restrict__ out_grad, double* __restrict__ out_lap, double* partial,
@@ -1630,7 +1630,7 @@ __global__ void __launch_bounds__(32 * WPB, PART == 2 ? 3 : 2) khw_measure(
 // Batched form (compute type TC, state written, per-tile E_L partials), one
 // block per tile.
 template <int NE, int NUP, class TC, class TS, int WPB, int PART = 0>
-__global__ void __launch_bounds__(32 * WPB, PART == 2 ? 3 : 2) khwb_measure(const BatchTile* __restrict__ tiles,
+__global__ void __launch_bounds__(32 * WPB, PART == 0 ? 2 : 3) khwb_measure(const BatchTile* __restrict__ tiles,
                                                                          int ntiles, const BatchRec* __restrict__ recs,
                                                                          double* tile_partial) {
     extern __shared__ __align__(16) unsigned char hsm[];

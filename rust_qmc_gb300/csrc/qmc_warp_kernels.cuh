@@ -224,6 +224,35 @@ __device__ __forceinline__ T wsum(T v) {
     return v;
 }
 
+// v[i] = wsum(v[i]) for N <= 8 values at once.  The two halves of a warp hold the same
+// partial sums after a butterfly step, so each step that is left over folds two values
+// into one: 9 shuffles and additions and 8 broadcasts for 8 values instead of 40 of
+// each.  The same additions, hence the same bits.
+template <int N, class T>
+__device__ __forceinline__ void wsum_n(T (&v)[N], int lane) {
+    static_assert(N <= 8, "three folds");
+    T a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (2 * i >= N) break;
+        const T x = v[2 * i], y = 2 * i + 1 < N ? v[2 * i + 1 < N ? 2 * i + 1 : 0] : T(0);
+        a[i] = (lane & 16 ? y : x) + wshfl_xor(lane & 16 ? x : y, 16);
+    }
+    constexpr int NA = (N + 1) / 2, NB = (NA + 1) / 2;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const T x = a[2 * i], y = 2 * i + 1 < NA ? a[2 * i + 1 < NA ? 2 * i + 1 : 0] : T(0);
+        b[i] = (lane & 8 ? y : x) + wshfl_xor(lane & 8 ? x : y, 8);
+    }
+    T c;
+    if constexpr (NB > 1) c = (lane & 4 ? b[1] : b[0]) + wshfl_xor(lane & 4 ? b[0] : b[1], 4);
+    else c = b[0] + wshfl_xor(b[0], 4);
+    c += wshfl_xor(c, 2);
+    c += wshfl_xor(c, 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = wshfl(c, (i & 1) << 4 | (i >> 1 & 1) << 3 | (i >> 2) << 2);
+}
+
 // Four consecutive elements of 16-byte-aligned shared memory as one vector
 // access (two for double).
 __device__ __forceinline__ void load4(const float* p, float& a, float& b, float& c, float& d) {
@@ -252,11 +281,14 @@ __device__ __forceinline__ int pair_slot(int i, int j) {
     return b * (b - 1) / 2 + a;
 }
 
-// Elements of the per-warp scratch of the single-electron sweep: one row of
-// WNCOL orbital values per proposal of a sector, then the Jastrow cache.
-template <int NE, int NUP>
+// Elements of the per-warp scratch of the single-electron sweep.  Gaussian moves: one
+// row of WNCOL orbital values per proposal of a sector, then the Jastrow cache.
+// Drift-diffusion moves: a column of the inverse, the proposal's orbital values and
+// its AO values, then the sector's draws.
+template <int NE, int NUP, int MOVE>
 __host__ __device__ constexpr int sweep_scratch_elems() {
-    return (NUP > NE - NUP ? NUP : NE - NUP) * WNCOL + jcache_elems<NE>();
+    constexpr int NM = NUP > NE - NUP ? NUP : NE - NUP;
+    return MOVE == MOVE_ONE_GAUSS ? NM * WNCOL + jcache_elems<NE>() : 2 * WNCOL + WMAX_AO + 4 * NM;
 }
 // The FP32 Gaussian sweep's (kw_gauss_walker): per sector and proposal a row of
 // WNCOL orbital values, then the proposed position and the acceptance draw (a stride
@@ -268,47 +300,40 @@ __host__ __device__ constexpr int gauss_scratch_elems() {
     return 2 * (NUP > NE - NUP ? NUP : NE - NUP) * GRS + 2 * WNCOL + jcache_elems<NE>();
 }
 
-// MO contraction: lane k receives phi_k = sum_a C[sig][a][k] chi_a (and
-// gradient / Laplacian), chi_a broadcast from lane a % 32; lanes past the
-// table's columns accumulate zeros.
-template <class T, int MODE>
-__device__ __forceinline__ void mo_lane(const SysW<T>& S, int sig, int lane, const AOLane<T, MODE>& ao, T& v, T& gx,
-                                        T& gy, T& gz, T& l) {
-    v = 0; gx = 0; gy = 0; gz = 0; l = 0;
-    const bool own = lane < WNCOL;
-    const int col = own ? lane : 0;
-#pragma unroll
-    for (int r = 0; r < WAO_ROUNDS; ++r) {
-        const int base = 32 * r;
-        if (base >= S.n_ao) break;
-        const int cnt = min(32, S.n_ao - base);
-        for (int t = 0; t < cnt; ++t) {
-            const T cl = S.C[sig][base + t][col];
-            const T c = own ? cl : T(0);
-            if (MODE != 3) v += c * wshfl(ao.v[r], t);
-            if (MODE >= 1) {
-                gx += c * wshfl(ao.gx[r], t);
-                gy += c * wshfl(ao.gy[r], t);
-                gz += c * wshfl(ao.gz[r], t);
-            }
-            if (MODE >= 2) l += c * wshfl(ao.l[r], t);
-        }
+// MO contraction: lane k < WNCOL receives phi_k = sum_a C[sig][a][k] chi_a, chi in
+// shared memory (16-byte aligned); lanes past the table's columns repeat column 0.
+template <class T>
+__device__ __forceinline__ T mo_lane(const SysW<T>& S, int sig, int lane, const T* chi) {
+    T v = 0;
+    const T* c = S.C[sig][0] + (lane < WNCOL ? lane : 0);
+    const int n4 = S.n_ao / 4 * 4;
+#pragma unroll 3
+    for (int t = 0; t < n4; t += 4) {
+        T x0, x1, x2, x3;
+        load4(chi + t, x0, x1, x2, x3);
+        v += c[t * WNCOL] * x0;
+        v += c[(t + 1) * WNCOL] * x1;
+        v += c[(t + 2) * WNCOL] * x2;
+        v += c[(t + 3) * WNCOL] * x3;
     }
+    for (int t = n4; t < S.n_ao; ++t) v += c[t * WNCOL] * chi[t];
+    return v;
 }
 
-// c'_a = sum_k C[sig][a][k] Dinv[k][q] for the lane's AOs a = lane + 32 r: column q of
-// the inverse (lane q's registers) broadcast four entries at a time, the lane's
-// coefficient rows read as 16-byte vectors.  Lanes past the basis get 0.
+// c'_a = sum_k C[sig][a][k] Dinv[k][q] for the lane's AOs a = lane + 32 r, column q of
+// the inverse in shared memory (col), the lane's coefficient rows read as 16-byte
+// vectors.  Lanes past the basis get 0.
 template <class T, int NM>
-__device__ __forceinline__ void inverse_column_coefficients(const SysW<T>& S, int sig, int lane, const T (&D)[NM],
-                                                            int q, T (&cw)[WAO_ROUNDS]) {
+__device__ __forceinline__ void inverse_column_coefficients(const SysW<T>& S, int sig, int lane, const T* col,
+                                                            T (&cw)[WAO_ROUNDS]) {
 #pragma unroll
     for (int r = 0; r < WAO_ROUNDS; ++r) cw[r] = 0;
 #pragma unroll
     for (int k0 = 0; k0 < NM; k0 += 4) {
         T dq[4];
+        load4(col + k0, dq[0], dq[1], dq[2], dq[3]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) dq[i] = (k0 + i < NM) ? wshfl(D[k0 + i < NM ? k0 + i : 0], q) : T(0);
+        for (int i = 0; i < 4; ++i) dq[i] = k0 + i < NM ? dq[i] : T(0);
 #pragma unroll
         for (int r = 0; r < WAO_ROUNDS; ++r) {
             if (32 * r >= S.n_ao) break;
@@ -495,6 +520,8 @@ __device__ __forceinline__ void kw_sweep_walker(const SysW<T>& S, A& a, int w, T
     // distance as a recomputation, hence the same value.
     constexpr int NPAIR = NE * (NE - 1) / 2;
     T* jc = ph + NM * PHS;
+    // drift moves: column q of the inverse, the proposal's orbital and AO values, draws
+    T *colq = ph, *phs = ph + WNCOL, *aos = ph + 2 * WNCOL, *drw = aos + WMAX_AO;
     if constexpr (MOVE == MOVE_ONE_GAUSS) {
         for (int i = 0; i < NE; ++i) {
             T xi, yi, zi;
@@ -542,30 +569,44 @@ __device__ __forceinline__ void kw_sweep_walker(const SysW<T>& S, A& a, int w, T
                 if (lane < NS) proposal_orbitals<T, NM>(S, sig, pnx, pny, pnz, ph + lane * PHS);
                 __syncwarp();
             }
+            if constexpr (MOVE == MOVE_ONE_DRIFT) {
+                if (lane < NS) store4(drw + 4 * lane, draws.n0, draws.n1, draws.n2, draws.uacc);
+                __syncwarp();
+            }
             T csc = 1;                                 // pending scale of this lane's column (Gaussian moves)
             for (int q = 0; q < NS; ++q) {
                 const int e = sig * NUP + q;
                 T rx, ry, rz;
                 P.get(e, rx, ry, rz);
-                const MoveDraw<T> md = draw_of(draws, q);
+                MoveDraw<T> md;
+                if constexpr (MOVE == MOVE_ONE_DRIFT) load4(drw + 4 * q, md.n0, md.n1, md.n2, md.uacc);
+                else md = draw_of(draws, q);
                 T nx, ny, nz, logG = 0, dlx = 0, dly = 0, dlz = 0;
                 // drift: c'_a = sum_k C[sig][a][k] Dinv[k][q] on the lanes of AO a, so that
                 // grad ln D at r and at r' are sums over the AOs (warp sums)
                 T cw[WAO_ROUNDS];
                 T u_old = 0;                           // drift: this lane's Jastrow terms at r
                 if constexpr (MOVE == MOVE_ONE_DRIFT) {
-                    inverse_column_coefficients<T, NM>(S, sig, lane, D, q, cw);
+                    if (lane == q) {
+#pragma unroll
+                        for (int k = 0; k < NM; k += 4)
+                            store4(colq + k, D[k], D[k + 1 < NM ? k + 1 : k], D[k + 2 < NM ? k + 2 : k], D[k + 3 < NM ? k + 3 : k]);
+                    }
+                    __syncwarp();
+                    inverse_column_coefficients<T, NM>(S, sig, lane, colq, cw);
                     AOLane<T, 1> ao;
                     ao_lane<T, 1>(S, rx, ry, rz, lane, ao);
                     T ax = 0, ay = 0, az = 0;
 #pragma unroll
                     for (int r = 0; r < WAO_ROUNDS; ++r) { ax += cw[r] * ao.gx[r]; ay += cw[r] * ao.gy[r]; az += cw[r] * ao.gz[r]; }
-                    ax = wsum(ax); ay = wsum(ay); az = wsum(az);
                     T gl[3];
                     wjastrow_lane_terms<NE, NUP, NNUC, T>(S, P, lane, e, rx, ry, rz, u_old, gl);
+                    T sm[6] = {ax, ay, az, gl[0], gl[1], gl[2]};
+                    wsum_n(sm, lane);
+                    ax = sm[0]; ay = sm[1]; az = sm[2];
                     T g0[3];
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) g0[c] = wsum(gl[c]) * S.qa;
+                    for (int c = 0; c < 3; ++c) g0[c] = sm[3 + c] * S.qa;
                     const T tau = a.tau, maxd = a.maxd;
                     dlx = tau * 2 * (ax + g0[0]); dly = tau * 2 * (ay + g0[1]); dlz = tau * 2 * (az + g0[2]);
                     T m = fsqrt(dlx * dlx + dly * dly + dlz * dlz);
@@ -582,16 +623,24 @@ __device__ __forceinline__ void kw_sweep_walker(const SysW<T>& S, A& a, int w, T
                     ao_lane<T, 1>(S, nx, ny, nz, lane, ao);
                     // orbital values at r' (every t_j is needed for the update), the
                     // gradient term of column q from c'
-                    AOLane<T, 0> av;
 #pragma unroll
-                    for (int r = 0; r < WAO_ROUNDS; ++r) av.v[r] = ao.v[r];
-                    T phi, pgx, pgy, pgz, pl;
-                    mo_lane<T, 0>(S, sig, lane, av, phi, pgx, pgy, pgz, pl);
+                    for (int r = 0; r < WAO_ROUNDS; ++r)
+                        if (lane + 32 * r < S.n_ao) aos[lane + 32 * r] = ao.v[r];
+                    __syncwarp();
+                    const T phi = mo_lane(S, sig, lane, aos);
+                    if (lane < NM) phs[lane] = phi;
+                    __syncwarp();
 #pragma unroll
-                    for (int k = 0; k < NM; ++k) tj += wshfl(phi, k) * D[k];
+                    for (int k = 0; k < NM; k += 4) {
+                        T f0, f1, f2, f3;
+                        load4(phs + k, f0, f1, f2, f3);
+                        tj += f0 * D[k];
+                        if (k + 1 < NM) tj += f1 * D[k + 1 < NM ? k + 1 : 0];
+                        if (k + 2 < NM) tj += f2 * D[k + 2 < NM ? k + 2 : 0];
+                        if (k + 3 < NM) tj += f3 * D[k + 3 < NM ? k + 3 : 0];
+                    }
 #pragma unroll
                     for (int r = 0; r < WAO_ROUNDS; ++r) { bx += cw[r] * ao.gx[r]; by += cw[r] * ao.gy[r]; bz += cw[r] * ao.gz[r]; }
-                    bx = wsum(bx); by = wsum(by); bz = wsum(bz);
                 } else {
                     const T* row = ph + q * PHS;
                     T t0 = 0, t1 = 0;
@@ -651,9 +700,12 @@ __device__ __forceinline__ void kw_sweep_walker(const SysW<T>& S, A& a, int w, T
                     // new position's terms against the old position's (kept from the drift)
                     T un, gl[3];
                     wjastrow_lane_terms<NE, NUP, NNUC, T>(S, P, lane, e, nx, ny, nz, un, gl);
-                    du = wsum(un - u_old);
+                    T sm[7] = {bx, by, bz, gl[0], gl[1], gl[2], un - u_old};
+                    wsum_n(sm, lane);
+                    bx = sm[0]; by = sm[1]; bz = sm[2];
+                    du = sm[6];
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) gn[c] = wsum(gl[c]) * S.qa;
+                    for (int c = 0; c < 3; ++c) gn[c] = sm[3 + c] * S.qa;
                 }
                 if constexpr (MOVE == MOVE_ONE_DRIFT) {
                     const T tau = a.tau, maxd = a.maxd;
@@ -688,9 +740,15 @@ __device__ __forceinline__ void kw_sweep_walker(const SysW<T>& S, A& a, int w, T
                     } else {
                         const T f = tj * iR;
 #pragma unroll
-                        for (int k = 0; k < NM; ++k) {
-                            T dq = wshfl(D[k], q);
-                            D[k] = (lane == q) ? dq * iR : D[k] - dq * f;
+                        for (int k = 0; k < NM; k += 4) {
+                            T dq[4];
+                            load4(colq + k, dq[0], dq[1], dq[2], dq[3]);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (k + i < NM) {
+                                    T& d = D[k + i < NM ? k + i : 0];
+                                    d = (lane == q) ? dq[i] * iR : d - dq[i] * f;
+                                }
                         }
                     }
                     if (R < 0) sgn = -sgn;
@@ -1174,7 +1232,7 @@ __global__ void __launch_bounds__(32 * WPB, sizeof(T) == 4 ? 16 / WPB : 1) kw_sw
     const int w = blockIdx.x * WPB + (threadIdx.x >> 5);
     if (w >= W) return;                        // whole warps only; no block barrier below
     const volatile SweepArgs<T>& a = args;
-    T* ph = reinterpret_cast<T*>(wsm) + (size_t)(threadIdx.x >> 5) * sweep_scratch_elems<NE, NUP>();
+    T* ph = reinterpret_cast<T*>(wsm) + (size_t)(threadIdx.x >> 5) * sweep_scratch_elems<NE, NUP, MOVE>();
     kw_sweep_walker<NE, NUP, NNUC, T, MOVE>(S, a, w, ph);
 }
 
@@ -1198,7 +1256,7 @@ __global__ void __launch_bounds__(32 * WPB, sizeof(T) == 4 ? 16 / WPB : 1) kwb_s
     const volatile SweepArgs<T>& a = args;
     const int w = tl.w0 + (int)(blockIdx.x % BPT) * WPB + (int)(threadIdx.x >> 5);
     if (w >= a.W) return;                      // whole warps only; no block barrier below
-    T* ph = reinterpret_cast<T*>(wsm) + (size_t)(threadIdx.x >> 5) * sweep_scratch_elems<NE, NUP>();
+    T* ph = reinterpret_cast<T*>(wsm) + (size_t)(threadIdx.x >> 5) * sweep_scratch_elems<NE, NUP, MOVE>();
     kw_sweep_walker<NE, NUP, NNUC, T, MOVE>(S, a, w, ph);
 }
 
@@ -2031,8 +2089,8 @@ struct WarpShapeOps {
     // refresh block of BTW warps.
     static constexpr int BTW = RWPB;
     // dynamic shared memory of a sweep block: the WPB warps' proposal rows
-    template <class T>
-    static constexpr size_t sweep_smem() { return sizeof(T) * WPB * (size_t)sweep_scratch_elems<NE, NUP>(); }
+    template <class T, int MOVE>
+    static constexpr size_t sweep_smem() { return sizeof(T) * WPB * (size_t)sweep_scratch_elems<NE, NUP, MOVE>(); }
 
     template <class T>
     static int table(const HostSys& hs, const SysW<T>** out) {
@@ -2204,7 +2262,7 @@ struct WarpShapeOps {
         if (rc) return rc;
         int nb = (dw.W + WPB - 1) / WPB;
         auto kern = kw_sweep<NE, NUP, NNUC, T, MOVE, WPB>;
-        const size_t smem = sweep_smem<T>();
+        const size_t smem = sweep_smem<T, MOVE>();
         static bool attr = false;
         if (!attr) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -2245,7 +2303,7 @@ struct WarpShapeOps {
     template <class T, int MOVE>
     static int batch_sweep_t(const BatchClass& bc, const BatchCtl* ctl, cudaStream_t st, int* occ) {
         auto kern = kwb_sweep<NE, NUP, NNUC, T, MOVE, WPB, BTW>;
-        const size_t smem = sweep_smem<T>();
+        const size_t smem = sweep_smem<T, MOVE>();
         static bool attr = false;
         if (!attr) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
