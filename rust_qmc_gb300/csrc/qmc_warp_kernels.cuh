@@ -10,6 +10,7 @@
 // Gauss-Jordan elimination in which lane j carries column j of [D | I] and
 // ends holding column j of D^-1 -- exactly the sweep kernel's layout.
 #pragma once
+#include <algorithm>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -126,6 +127,46 @@ static bool fill_sysw(const HostSys& hs, int NE, int NUP, int NNUC, SysW<T>& S) 
     }
     return true;
 }
+
+// Shells of a table's basis: consecutive radial groups as they stand, but an s group
+// and the p triplet after it on the same nucleus with the same exponents (the sp
+// shells of Pople's sets) as one, whose exponentials are evaluated once.
+// Descriptor: nucleus (bits 0-3), s (bit 4), p triplet (bit 5), primitive count (bits
+// 6-9), first primitive (bits 10-17), first AO (bits 18-24).
+constexpr int SHELL_S = 16, SHELL_P = 32;
+__host__ __device__ constexpr int shell_pack(int nuc, int kind, int np, int p0, int a0) {
+    return nuc | kind | (np << 6) | (p0 << 10) | (a0 << 18);
+}
+__host__ __device__ constexpr int shell_nuc(int d) { return d & 15; }
+__host__ __device__ constexpr int shell_np(int d) { return (d >> 6) & 15; }
+__host__ __device__ constexpr int shell_p0(int d) { return (d >> 10) & 255; }
+__host__ __device__ constexpr int shell_a0(int d) { return d >> 18; }
+
+template <class T>
+struct ShellList {
+    std::vector<int> desc;                     // in AO order
+    std::vector<T> al, c, cp;                  // exponent; the s or lone p coefficient; an sp shell's p coefficient
+    explicit ShellList(const SysW<T>& S) {
+        for (int g = 0; g < S.n_grp; ++g) {
+            const int d = S.grp[g], I = d & 15, np = (d >> 5) & 15, q0 = (d >> 9) & 255, a0 = grp_a0(d);
+            const bool p = (d >> 4) & 1;
+            int q1 = -1;
+            if (!p && g + 1 < S.n_grp) {
+                const int n = S.grp[g + 1];
+                bool same = (n & 15) == I && ((n >> 4) & 1) && ((n >> 5) & 15) == np && grp_a0(n) == a0 + 1;
+                for (int i = 0; same && i < np; ++i)
+                    same = (double)S.prim[q0 + i][0] == (double)S.prim[((n >> 9) & 255) + i][0];
+                if (same) { q1 = (n >> 9) & 255; ++g; }
+            }
+            desc.push_back(shell_pack(I, p ? SHELL_P : (q1 >= 0 ? SHELL_S | SHELL_P : SHELL_S), np, (int)al.size(), a0));
+            for (int i = 0; i < np; ++i) {
+                al.push_back(S.prim[q0 + i][0]);
+                c.push_back(S.prim[q0 + i][1]);
+                cp.push_back(S.prim[(q1 >= 0 ? q1 : q0) + i][1]);
+            }
+        }
+    }
+};
 
 // Copy the table from global to shared memory (whole block).
 template <class T>
@@ -798,19 +839,20 @@ struct ColF2 {
 };
 
 // Table of the FP32 Gaussian sweep, values of both halves of a packed instruction
-// doubled: groups as (-x, -x, -y, -y), (-z, -z, descriptor bits, 0) of the nucleus,
-// primitives (-exponent, -exponent, coefficient, coefficient), coefficients of both
-// sectors side by side, the columns padded to pairs.
+// doubled: shells as (-x, -x, -y, -y), (-z, -z, descriptor bits, 0) of the nucleus,
+// primitives (-exponent, -exponent, c, c) and (p coefficient of an sp shell twice),
+// coefficients of both sectors side by side, the columns padded to pairs.
 template <int NNUC, int NM>
 struct GaussTab {
     static constexpr int NC = (NM + 1) / 2 * 2;
-    int n_ao, n_grp;
+    int n_ao, n_sh;
     float a_ee[2], b_ee[2];
     float pad[2];
     float nuc[NNUC][4];                       // x, y, z, unused
     float en[NNUC][2];                        // A, B
-    alignas(16) float4 grp[WMAX_AO][2];
+    alignas(16) float4 sh[WMAX_AO][2];
     float4 prim[WMAX_PRIM];
+    float2 prim_p[WMAX_PRIM];
     float2 C[WMAX_AO][NC];
     __host__ __device__ static size_t bytes(int n_ao) { return offsetof(GaussTab, C) + sizeof(float2) * NC * (size_t)n_ao; }
     __device__ static size_t used(const GaussTab* t) { return bytes(t->n_ao); }
@@ -819,29 +861,33 @@ struct GaussTab {
 template <int NNUC, int NM>
 static void fill_gausstab(const SysW<float>& w, GaussTab<NNUC, NM>& S) {
     std::memset(static_cast<void*>(&S), 0, sizeof(S));
+    const ShellList<float> L(w);
     S.n_ao = w.n_ao;
-    S.n_grp = w.n_grp;
+    S.n_sh = (int)L.desc.size();
     for (int c = 0; c < 2; ++c) { S.a_ee[c] = w.a_ee[c]; S.b_ee[c] = w.b_ee[c]; }
     for (int I = 0; I < NNUC; ++I) {
         for (int c = 0; c < 3; ++c) S.nuc[I][c] = w.nuc[I][c];
         S.en[I][0] = w.enA[I];
         S.en[I][1] = w.enB[I];
     }
-    for (int g = 0; g < w.n_grp; ++g) {
-        const int I = w.grp[g] & 15;
+    for (int g = 0; g < S.n_sh; ++g) {
+        const int I = shell_nuc(L.desc[g]);
         float bits;
-        std::memcpy(&bits, &w.grp[g], sizeof bits);
-        S.grp[g][0] = make_float4(-w.nuc[I][0], -w.nuc[I][0], -w.nuc[I][1], -w.nuc[I][1]);
-        S.grp[g][1] = make_float4(-w.nuc[I][2], -w.nuc[I][2], bits, 0.0f);
+        std::memcpy(&bits, &L.desc[g], sizeof bits);
+        S.sh[g][0] = make_float4(-w.nuc[I][0], -w.nuc[I][0], -w.nuc[I][1], -w.nuc[I][1]);
+        S.sh[g][1] = make_float4(-w.nuc[I][2], -w.nuc[I][2], bits, 0.0f);
     }
-    for (int p = 0; p < WMAX_PRIM; ++p) S.prim[p] = make_float4(-w.prim[p][0], -w.prim[p][0], w.prim[p][1], w.prim[p][1]);
+    for (size_t p = 0; p < L.al.size(); ++p) {
+        S.prim[p] = make_float4(-L.al[p], -L.al[p], L.c[p], L.c[p]);
+        S.prim_p[p] = make_float2(L.cp[p], L.cp[p]);
+    }
     for (int a = 0; a < w.n_ao; ++a)
         for (int k = 0; k < NM; ++k) S.C[a][k] = make_float2(w.C[0][a][k], w.C[1][a][k]);
 }
 
 // Orbital values of one proposal of each sector (x, y, z: the up sector's coordinate,
 // the down sector's) in packed instructions: proposal_orbitals' operations in the same
-// order on each.  Written to out0[k] and out1[k].
+// order on each, an sp shell's exponentials once.  Written to out0[k] and out1[k].
 template <int NNUC, int NM>
 __device__ __forceinline__ void proposal_orbitals2(const GaussTab<NNUC, NM>& S, F2 x, F2 y, F2 z, float* out0, float* out1) {
     F2 acc[NM];
@@ -856,28 +902,35 @@ __device__ __forceinline__ void proposal_orbitals2(const GaussTab<NNUC, NM>& S, 
         }
     };
 #pragma unroll 1
-    for (int g = 0; g < S.n_grp; ++g) {
-        const float4 G = S.grp[g][0], H = S.grp[g][1];
+    for (int g = 0; g < S.n_sh; ++g) {
+        const float4 G = S.sh[g][0], H = S.sh[g][1];
         const int d = __float_as_int(H.z);
-        const int np = (d >> 5) & 15;
-        const float4* prim = S.prim + ((d >> 9) & 255);
-        const float2* c = S.C[grp_a0(d)];
+        const int np = shell_np(d);
+        const float4* prim = S.prim + shell_p0(d);
+        const float2* prim_p = S.prim_p + shell_p0(d);
+        const float2* c = S.C[shell_a0(d)];
         const F2 dx = add2(x, F2(G.x, G.y)), dy = add2(y, F2(G.z, G.w)), dz = add2(z, F2(H.x, H.y));
         const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
-        F2 s0(0.0f);
+        // s0: the s (or lone p) radial part, s1: an sp shell's p part
+        F2 s0(0.0f), s1(0.0f);
 #pragma unroll 3
         for (int p = 0; p < np; ++p) {
             const float4 t = prim[p];
+            const float2 u = prim_p[p];
             float e0, e1;
             mul2(F2(t.x, t.y), r2).get(e0, e1);
-            s0 = fma2(F2(t.z, t.w), F2(fexp(e0), fexp(e1)), s0);
+            const F2 e(fexp(e0), fexp(e1));
+            s0 = fma2(F2(t.z, t.w), e, s0);
+            s1 = fma2(F2(u.x, u.y), e, s1);
         }
-        if (d & 16) {
-            axpy(c, mul2(dx, s0));
-            axpy(c + S.NC, mul2(dy, s0));
-            axpy(c + 2 * S.NC, mul2(dz, s0));
-        } else {
+        if (d & SHELL_S) {
             axpy(c, s0);
+            c += S.NC;
+        }
+        if (d & SHELL_P) {
+            axpy(c, mul2(dx, s1));
+            axpy(c + S.NC, mul2(dy, s1));
+            axpy(c + 2 * S.NC, mul2(dz, s1));
         }
     }
 #pragma unroll
@@ -1555,19 +1608,22 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
 // together, so that one loop is in use at a time.
 // ---------------------------------------------------------------------------
 struct PairTabHead {                // sizes and scalars; the arrays follow in the block's shared memory
-    int n_ao, n_grp, quirk_lap, pad;
+    int n_ao, n_sh, n_third, quirk_lap;
     ff qa, v_nn;
     ff b_ee[2], a_ee[2];
 };
-// Device table: head, nuclei [NNUC] (x, y, z, Z, enA, enB as ff), groups [WMAX_AO],
-// primitives (exponent, coefficient) [WMAX_PRIM], then the coefficients [n_ao][NM] of
-// both sectors as (hi, hi', lo, lo').
+// Device table: head, nuclei [NNUC] (x, y, z, Z, enA, enB as ff), shells in AO order,
+// the same dealt into three lists of equal kinds (third t's shell i at 3 i + t; rows
+// are filled up with shells without primitives), primitives (exponent, coefficient)
+// and (c a, c a^2) of each, an sp shell's p coefficients beside them, then the
+// coefficients [n_ao][NM] of both sectors as (hi, hi', lo, lo').
 template <int NNUC, int NM>
 struct PairTab {
     PairTabHead head;
     ff nuc[NNUC][6];
-    int grp[WMAX_AO];
-    float4 prim[WMAX_PRIM];
+    int sh[WMAX_AO], third[WMAX_AO + 12];
+    float4 prim[WMAX_PRIM], primd[WMAX_PRIM];      // s or lone p
+    float4 prim_p[WMAX_PRIM], primd_p[WMAX_PRIM];  // p of an sp shell
     float4 C[WMAX_AO][NM];
     __host__ __device__ static size_t bytes(int n_ao) { return offsetof(PairTab, C) + sizeof(float4) * NM * (size_t)n_ao; }
     __device__ static size_t used(const PairTab* t) { return bytes(t->head.n_ao); }
@@ -1577,7 +1633,18 @@ template <int NNUC, int NM>
 static void fill_pairtab(const SysW<ff>& w, PairTab<NNUC, NM>& S) {
     std::memset(static_cast<void*>(&S), 0, sizeof(S));
     S.head.n_ao = w.n_ao;
-    S.head.n_grp = w.n_grp;
+    const ShellList<ff> L(w);
+    S.head.n_sh = (int)L.desc.size();
+    // thirds: shells of one kind, by primitive count, dealt in rows of three
+    std::vector<int> by[3];
+    for (int d : L.desc) by[(d & SHELL_S) ? ((d & SHELL_P) ? 2 : 0) : 1].push_back(d);
+    int nt = 0;
+    for (auto& v : by) {
+        std::stable_sort(v.begin(), v.end(), [](int a, int b) { return shell_np(a) < shell_np(b); });
+        for (size_t i = 0; i < (v.size() + 2) / 3 * 3; ++i)
+            S.third[nt++] = i < v.size() ? v[i] : shell_pack(0, v[0] & (SHELL_S | SHELL_P), 0, 0, 0);
+    }
+    S.head.n_third = nt / 3;
     S.head.quirk_lap = w.quirk_lap;
     S.head.qa = w.qa;
     S.head.v_nn = w.v_nn;
@@ -1586,9 +1653,16 @@ static void fill_pairtab(const SysW<ff>& w, PairTab<NNUC, NM>& S) {
         const ff v[6] = {w.nuc[I][0], w.nuc[I][1], w.nuc[I][2], w.Z[I], w.enA[I], w.enB[I]};
         for (int c = 0; c < 6; ++c) S.nuc[I][c] = v[c];
     }
-    for (int g = 0; g < w.n_grp; ++g) S.grp[g] = w.grp[g];
-    for (int p = 0; p < WMAX_PRIM; ++p)
-        S.prim[p] = make_float4(w.prim[p][0].hi, w.prim[p][0].lo, w.prim[p][1].hi, w.prim[p][1].lo);
+    for (int g = 0; g < S.head.n_sh; ++g) S.sh[g] = L.desc[g];
+    auto two = [](ff a, ff b) { return make_float4(a.hi, a.lo, b.hi, b.lo); };
+    for (size_t p = 0; p < L.al.size(); ++p) {
+        const double al = (double)L.al[p];
+        for (int k = 0; k < 2; ++k) {
+            const ff c = k ? L.cp[p] : L.c[p];
+            (k ? S.prim_p : S.prim)[p] = two(L.al[p], c);
+            (k ? S.primd_p : S.primd)[p] = two(ff((double)c * al), ff((double)c * al * al));
+        }
+    }
     for (int a = 0; a < w.n_ao; ++a)
         for (int k = 0; k < NM; ++k) {
             const ff c0 = w.C[0][a][k], c1 = w.C[1][a][k];
@@ -1608,10 +1682,13 @@ __device__ __forceinline__ void store_ff2(float4* p, ff2 v) {
 }
 
 // Shared float4 of a warp: the sectors' rows (row q at q NM), then, over the same
-// storage, positions [3][NE] and sums [5][NE] of the pair pass as ff.
+// storage, the inverse's columns, then positions [3][NE] and sums [5][NE] of the pair
+// pass as ff; after it the derivative sums [round][4][lane].
+template <int NE, int NM>
+__host__ __device__ constexpr int pair_rows() { return NM * NM > (8 * NE + 1) / 2 ? NM * NM : (8 * NE + 1) / 2; }
 template <int NE, int NM>
 __host__ __device__ constexpr int pair_scratch() {
-    return NM * NM > (8 * NE + 1) / 2 ? NM * NM : (8 * NE + 1) / 2;
+    return pair_rows<NE, NM>() + 2 * 4 * 32;
 }
 
 // Pade pair terms of two pairs at separations (dx, dy, dz): u = a r / (1 + b r),
@@ -1649,33 +1726,39 @@ __device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S,
     constexpr int NM = NUP;
     const int lane = threadIdx.x & 31;
     const int q = min(lane, NM - 1);                        // spare lanes repeat the last electron
-    float px[2], py[2], pz[2];
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        const size_t i = (size_t)(3 * (s * NUP + q)) * Wcap + w;
-        px[s] = gpos[i];
-        py[s] = gpos[i + Wcap];
-        pz[s] = gpos[i + 2 * (size_t)Wcap];
-    }
-    const ff2 x{ff(px[0]), ff(px[1])}, y{ff(py[0]), ff(py[1])}, z{ff(pz[0]), ff(pz[1])};
+    // coordinate c of electron pair e
+    auto coord = [&](int e, int c) {
+        return ff2(F2(gpos[(size_t)(3 * e + c) * Wcap + w], gpos[(size_t)(3 * (NUP + e) + c) * Wcap + w]), F2(0.0f));
+    };
     // orbital values of the lane's electrons, row q of both matrices
     __syncthreads();
     {
+        const ff2 x = coord(q, 0), y = coord(q, 1), z = coord(q, 2);
         ff2 v[NM];
 #pragma unroll
         for (int k = 0; k < NM; ++k) v[k] = ff2(0.0f);
-        for (int g = 0; g < S.head.n_grp; ++g) {
-            const int d = S.grp[g];
-            const int I = d & 15, kind = (d >> 4) & 1, np = (d >> 5) & 15, p0 = (d >> 9) & 255, a0 = grp_a0(d);
+        for (int g = 0; g < S.head.n_sh; ++g) {
+            const int d = S.sh[g];
+            const int I = shell_nuc(d), np = shell_np(d), p0 = shell_p0(d), a0 = shell_a0(d);
+            const int ns = (d & SHELL_S) ? 1 : 0, na = ns + ((d & SHELL_P) ? 3 : 0);
+            const bool sp = na == 4;
             const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
             const ff2 r2 = dx * dx + dy * dy + dz * dz;
-            ff2 s0(0.0f);
+            ff2 s0(0.0f), s1(0.0f);
             for (int p = p0; p < p0 + np; ++p) {
                 const float4 t = S.prim[p];
-                s0 += ff2(ff(t.z, t.w)) * ff2_fexp(ff2(ff(-t.x, -t.y)) * r2);
+                const ff2 e = ff2_fexp(ff2(ff(-t.x, -t.y)) * r2);
+                s0 += ff2(ff(t.z, t.w)) * e;
+                if (sp) {
+                    const float4 u = S.prim_p[p];
+                    s1 += ff2(ff(u.z, u.w)) * e;
+                }
             }
-            for (int m = 0; m < (kind ? 3 : 1); ++m) {
-                const ff2 chi = kind ? (m == 0 ? dx : (m == 1 ? dy : dz)) * s0 : s0;
+            if (!sp) s1 = s0;
+#pragma unroll 1
+            for (int m = 0; m < na; ++m) {
+                const int c3 = m - ns;
+                const ff2 chi = c3 < 0 ? s0 : (c3 == 0 ? dx : (c3 == 1 ? dy : dz)) * s1;
                 const F2 nh = neg2(chi.hi), nl = neg2(chi.lo);
                 const float4* c = S.C[a0 + m];
                 // ff_fma_lazy(v[k], c[k], chi) with the error term carried negated
@@ -1811,52 +1894,85 @@ __device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S,
     // grad ln D and lap D / D of the lane's electrons: sum_a c'_a (grad, lap) chi_a with
     // c'_a = sum_k C[a][k] D^-1[k][q].  s: grad = -2 R1 dr, lap = -6 R1 + 4 r^2 R2; a p
     // triplet takes its three c' as a vector c: grad = -2 R1 (c.dr) dr + R0 c,
-    // lap = (c.dr)(-10 R1 + 4 r^2 R2).  The nuclei's pair terms follow from the
-    // distances at hand only in part, so they have a loop of their own.
+    // lap = (c.dr)(-10 R1 + 4 r^2 R2).  The work is 3 NM (electron pair, third of the
+    // shells) tasks in two rounds of 32 lanes, two thirds of the time of one round of NM
+    // lanes over all shells: round 0 takes third 0 of every pair and third 1 of the first
+    // R1, round 1 the rest.  The inverse's columns go through the warp's shared memory.
     __syncthreads();
-    ff2 gx(0.0f), gy(0.0f), gz(0.0f), ld(0.0f);
-    for (int g = 0; g < S.head.n_grp; ++g) {
-        const int d = S.grp[g];
-        const int I = d & 15, kind = (d >> 4) & 1, np = (d >> 5) & 15, p0 = (d >> 9) & 255, a0 = grp_a0(d);
-        const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
-        const ff2 r2 = dx * dx + dy * dy + dz * dz;
-        ff2 s0(0.0f), s1(0.0f), s2(0.0f);
-        for (int p = p0; p < p0 + np; ++p) {
-            const float4 t = S.prim[p];
-            const ff2 al(ff(t.x, t.y));
-            const ff2 e = ff2(ff(t.z, t.w)) * ff2_fexp(ff2(ff(-t.x, -t.y)) * r2), ea = al * e;
-            s0 += e;
-            s1 += ea;
-            ff2_fma_lazy(s2, al, ea);
-        }
-        s2 = ff2_norm(s2);
-        const ff2 two(F2(-2.0f), F2(0.0f)), l4 = ff2(4.0f) * r2 * s2, t1 = two * s1;
-        // cd: c' of an s AO, (c'.dr) of a p triplet
-        ff2 cd(0.0f);
-#pragma unroll 1
-        for (int m = 0; m < (kind ? 3 : 1); ++m) {
-            const float4* c = S.C[a0 + m];
-            ff2 cw(0.0f);
+    static_assert(3 * NM <= 64 && NM <= 32, "three tasks per electron pair in two rounds");
+    constexpr int R1 = 32 - NM;
+    if (lane < NM) {
 #pragma unroll
-            for (int k = 0; k < NM; ++k) ff2_fma_lazy(cw, load_ff2(c + k), A[k]);
-            cw = ff2_norm(cw);
-            if (!kind) {
-                cd = cw;
-            } else {
-                ff2_fma_lazy(cd, cw, m == 0 ? dx : (m == 1 ? dy : dz));
-                ff2 o = m == 0 ? gx : (m == 1 ? gy : gz);
-                ff2_fma_lazy(o, s0, cw);
-                if (m == 0) gx = o;
-                else if (m == 1) gy = o;
-                else gz = o;
+        for (int k = 0; k < NM; ++k) store_ff2(scr + k * NM + lane, A[k]);
+    }
+    __syncwarp();
+    float4* part = scr + pair_rows<NE, NM>();
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+        const int t3 = round == 0 ? (lane < NM ? 0 : 1) : (lane < NM - R1 ? 1 : 2);
+        const int tq = min(round == 0 ? (lane < NM ? lane : lane - NM) : (lane < NM - R1 ? R1 + lane : lane - (NM - R1)), NM - 1);
+        const ff2 x = coord(tq, 0), y = coord(tq, 1), z = coord(tq, 2);
+#pragma unroll
+        for (int k = 0; k < NM; ++k) A[k] = load_ff2(scr + k * NM + tq);
+        ff2 gx(0.0f), gy(0.0f), gz(0.0f), ld(0.0f);
+        for (int g = 0; g < S.head.n_third; ++g) {
+            const int d = S.third[3 * g + t3];
+            const int I = shell_nuc(d), np = shell_np(d), p0 = shell_p0(d), a0 = shell_a0(d);
+            const int ns = (d & SHELL_S) ? 1 : 0, na = ns + ((d & SHELL_P) ? 3 : 0);
+            const bool sp = na == 4;
+            const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
+            const ff2 r2 = dx * dx + dy * dy + dz * dz;
+            ff2 s0(0.0f), s1(0.0f), s2(0.0f), p_0(0.0f), p_1(0.0f), p_2(0.0f);
+            for (int p = p0; p < p0 + np; ++p) {
+                const float4 t = S.prim[p], u = S.primd[p];
+                const ff2 e = ff2_fexp(ff2(ff(-t.x, -t.y)) * r2);
+                ff2_fma_lazy(s0, ff2(ff(t.z, t.w)), e);
+                ff2_fma_lazy(s1, ff2(ff(u.x, u.y)), e);
+                ff2_fma_lazy(s2, ff2(ff(u.z, u.w)), e);
+                if (sp) {
+                    const float4 tp = S.prim_p[p], up = S.primd_p[p];
+                    ff2_fma_lazy(p_0, ff2(ff(tp.z, tp.w)), e);
+                    ff2_fma_lazy(p_1, ff2(ff(up.x, up.y)), e);
+                    ff2_fma_lazy(p_2, ff2(ff(up.z, up.w)), e);
+                }
+            }
+            const ff2 two(F2(-2.0f), F2(0.0f)), r4 = ff2(F2(4.0f), F2(0.0f)) * r2;
+            s0 = ff2_norm(s0); s1 = ff2_norm(s1); s2 = ff2_norm(s2);
+            // cd: c' of an s AO, then (c'.dr) of a p triplet; a triplet's radial parts
+            // replace the s AO's once that is added
+            ff2 cd(0.0f);
+#pragma unroll 1
+            for (int m = 0; m < na; ++m) {
+                const float4* c = S.C[a0 + m];
+                ff2 cw(0.0f);
+#pragma unroll
+                for (int k = 0; k < NM; ++k) ff2_fma_lazy(cw, load_ff2(c + k), A[k]);
+                cw = ff2_norm(cw);
+                const int c3 = m - ns;
+                if (c3 < 0) {
+                    cd = cw;
+                } else {
+                    if (c3 == 0 && sp) { s0 = ff2_norm(p_0); s1 = ff2_norm(p_1); s2 = ff2_norm(p_2); cd = ff2(0.0f); }
+                    ff2_fma_lazy(cd, cw, c3 == 0 ? dx : (c3 == 1 ? dy : dz));
+                    ff2 o = c3 == 0 ? gx : (c3 == 1 ? gy : gz);
+                    ff2_fma_lazy(o, s0, cw);
+                    if (c3 == 0) gx = o;
+                    else if (c3 == 1) gy = o;
+                    else gz = o;
+                }
+                if (c3 < 0 || c3 == 2) {
+                    cd = ff2_norm(cd);
+                    const ff2 t = two * s1 * cd;
+                    ff2_fma_lazy(gx, t, dx); ff2_fma_lazy(gy, t, dy); ff2_fma_lazy(gz, t, dz);
+                    ff2_fma_lazy(ld, cd, r4 * s2 - ff2(F2(c3 < 0 ? 6.0f : 10.0f), F2(0.0f)) * s1);
+                }
             }
         }
-        cd = ff2_norm(cd);
-        const ff2 t = t1 * cd;
-        ff2_fma_lazy(gx, t, dx); ff2_fma_lazy(gy, t, dy); ff2_fma_lazy(gz, t, dz);
-        ff2_fma_lazy(ld, cd, l4 - (kind ? ff2(10.0f) : ff2(6.0f)) * s1);
+        store_ff2(part + (4 * round + 0) * 32 + lane, ff2_norm(gx));
+        store_ff2(part + (4 * round + 1) * 32 + lane, ff2_norm(gy));
+        store_ff2(part + (4 * round + 2) * 32 + lane, ff2_norm(gz));
+        store_ff2(part + (4 * round + 3) * 32 + lane, ff2_norm(ld));
     }
-    gx = ff2_norm(gx); gy = ff2_norm(gy); gz = ff2_norm(gz); ld = ff2_norm(ld);
     // electron pairs, each once, two per lane: pair p joins electron i = p mod NE with
     // i + p / NE + 1 (mod NE), the last NE / 2 pairs i with i + NE / 2; 32 consecutive
     // pairs have distinct i and distinct j, so their sums need no atomics
@@ -1867,7 +1983,8 @@ __device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S,
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const int e = s * NUP + lane;
-            pos[e] = ff(px[s]); pos[NE + e] = ff(py[s]); pos[2 * NE + e] = ff(pz[s]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) pos[c * NE + e] = ff(gpos[(size_t)(3 * e + c) * Wcap + w]);
 #pragma unroll
             for (int c = 0; c < 5; ++c) sums[c * NE + e] = ff(0.0f);
         }
@@ -1937,6 +2054,7 @@ __device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S,
     };
     ff2 jx = both(0), jy = both(1), jz = both(2), lu = both(3);
     const ff2 gsq = both(4);
+    const ff2 x = coord(q, 0), y = coord(q, 1), z = coord(q, 2);
     ff2 un(0.0f), Vn(0.0f);
     for (int I = 0; I < NNUC; ++I) {
         const ff2 dx = x - ff2(S.nuc[I][0]), dy = y - ff2(S.nuc[I][1]), dz = z - ff2(S.nuc[I][2]);
@@ -1955,6 +2073,13 @@ __device__ __forceinline__ double kw_refresh_walker(const PairTab<NNUC, NUP>& S,
         jx -= f * dx; jy -= f * dy; jz -= f * dz;
         lu -= l;
     }
+    // the pair's thirds: its own lane's, and the lanes that took the other two
+    ff2 dsum[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        dsum[c] = load_ff2(part + c * 32 + q) + load_ff2(part + (q < R1 ? c * 32 + NM + q : (4 + c) * 32 + q - R1)) +
+                  load_ff2(part + (4 + c) * 32 + NM - R1 + q);
+    const ff2 gx = dsum[0], gy = dsum[1], gz = dsum[2], ld = dsum[3];
     const ff2 qa(S.head.qa);
     const ff2 lj = S.head.quirk_lap ? lu + gsq : lu + jx * jx + jy * jy + jz * jz;
     const ff2 lp = ld + ff2(2.0f) * (qa * (gx * jx + gy * jy + gz * jz)) + lj;
