@@ -53,9 +53,9 @@ struct HostSys {
     int version = 0;                     // bumped when parameters or nuclei change
     // cached device copies of the system table per arithmetic type:
     // [0] FP64, [1] FP32, [2] float-float; [3] the FP64 team kernels' table;
-    // [4] the FP32 Gaussian sweep's (benzene)
-    mutable void* dev_table[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    mutable int dev_table_version[5] = {-1, -1, -1, -1, -1};
+    // [4] the FP32 Gaussian sweep's and [5] the FP64 evaluation's (benzene)
+    mutable void* dev_table[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    mutable int dev_table_version[6] = {-1, -1, -1, -1, -1, -1};
 
     int n_params() const { return 8 + (int)rot_occ.size(); }
     // Effective (rotated) MO coefficients in caller AO order.

@@ -168,6 +168,21 @@ struct ShellList {
     }
 };
 
+// Shells dealt into three lists of equal kinds, by primitive count: out[3 i + t] is
+// third t's shell i, rows filled up with shells without primitives; returns the rows.
+constexpr int WMAX_THIRD = WMAX_AO + 12;
+static int deal_thirds(const std::vector<int>& shells, int (&out)[WMAX_THIRD]) {
+    std::vector<int> by[3];
+    for (int d : shells) by[(d & SHELL_S) ? ((d & SHELL_P) ? 2 : 0) : 1].push_back(d);
+    int n = 0;
+    for (auto& v : by) {
+        std::stable_sort(v.begin(), v.end(), [](int a, int b) { return shell_np(a) < shell_np(b); });
+        for (size_t i = 0; i < (v.size() + 2) / 3 * 3; ++i)
+            out[n++] = i < v.size() ? v[i] : shell_pack(0, v[0] & (SHELL_S | SHELL_P), 0, 0, 0);
+    }
+    return n / 3;
+}
+
 // Copy the table from global to shared memory (whole block).
 template <class T>
 __device__ __forceinline__ void load_sysw(SysW<T>* dst, const SysW<T>* __restrict__ src) {
@@ -1597,6 +1612,346 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
 }
 
 // ---------------------------------------------------------------------------
+// FP64 evaluation and refresh, one warp per walker.  An FP64 instruction holds its
+// sub-partition for 64 cycles however many of its lanes are active, so the work is
+// laid out to fill lanes: the orbital values and the derivative sums are (electron,
+// third of the shells) tasks in rounds of 32, 126 tasks for benzene's 42 electrons,
+// where one lane per electron of a sector took two rounds of 21 lanes over all
+// shells; pairs and nucleus terms are evaluated once each and added to per-electron
+// sums; pivots are compared, and |det| is kept, on exponent and high-word bits, with
+// one logarithm a walker.
+// ---------------------------------------------------------------------------
+template <int NNUC, int NM>
+struct EvalTab {
+    int n_ao, n_third, quirk_lap, pad;
+    double qa, v_nn, a_ee[2], b_ee[2];
+    double nuc[NNUC][6];                      // x, y, z, Z, enA, enB
+    int third[WMAX_THIRD];
+    // exponent; c, c a, c a^2 of the s or lone p part; the same of an sp shell's p part
+    alignas(16) double prim[WMAX_PRIM][8];
+    double C[WMAX_AO][2][NM + 1];             // [AO][sector][column], rows of whole 16-byte words
+    __host__ __device__ static size_t bytes(int n_ao) {
+        return offsetof(EvalTab, C) + sizeof(double) * 2 * (NM + 1) * (size_t)n_ao;
+    }
+    __device__ static size_t used(const EvalTab* t) { return bytes(t->n_ao); }
+};
+
+template <int NNUC, int NM>
+static void fill_evaltab(const SysW<double>& w, EvalTab<NNUC, NM>& S) {
+    static_assert(NM % 2 == 1, "padded rows are 16-byte words");
+    std::memset(static_cast<void*>(&S), 0, sizeof(S));
+    const ShellList<double> L(w);
+    S.n_ao = w.n_ao;
+    S.n_third = deal_thirds(L.desc, S.third);
+    S.quirk_lap = w.quirk_lap;
+    S.qa = w.qa;
+    S.v_nn = w.v_nn;
+    for (int c = 0; c < 2; ++c) { S.a_ee[c] = w.a_ee[c]; S.b_ee[c] = w.b_ee[c]; }
+    for (int I = 0; I < NNUC; ++I) {
+        const double v[6] = {w.nuc[I][0], w.nuc[I][1], w.nuc[I][2], w.Z[I], w.enA[I], w.enB[I]};
+        for (int c = 0; c < 6; ++c) S.nuc[I][c] = v[c];
+    }
+    for (size_t p = 0; p < L.al.size(); ++p) {
+        const double a = L.al[p], v[7] = {a, L.c[p], L.c[p] * a, L.c[p] * a * a, L.cp[p], L.cp[p] * a, L.cp[p] * a * a};
+        for (int c = 0; c < 7; ++c) S.prim[p][c] = v[c];
+    }
+    for (int a = 0; a < w.n_ao; ++a)
+        for (int sig = 0; sig < 2; ++sig)
+            for (int k = 0; k < NM; ++k) S.C[a][sig][k] = w.C[sig][a][k];
+}
+
+// Shared doubles of a warp: row e of the electron's orbital values, then of its column
+// of the inverse, later positions [3][NE] and sums [5][NE] over the same storage; then
+// the derivative sums [4][NE].
+template <int NE, int NM>
+__host__ __device__ constexpr int eval_rows() { return (NE * NM > 8 * NE ? NE * NM : 8 * NE) + (NE * NM) % 2; }
+template <int NE, int NM>
+__host__ __device__ constexpr int eval_scratch() { return eval_rows<NE, NM>() + 4 * NE; }
+
+template <int NE, int NUP, int NNUC, class TAB>
+__device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, const double* __restrict__ gpos,
+                                                 double* __restrict__ gdinv, double* __restrict__ glog,
+                                                 int* __restrict__ gsign, double* __restrict__ gel, int w, int Wcap,
+                                                 int write_state, double* __restrict__ out_grad,
+                                                 double* __restrict__ out_lap, int* flags) {
+    static_assert(NE == 2 * NUP && NUP <= 32 && NE >= 32, "equal sectors; a round's tasks are of distinct electrons");
+    constexpr int NM = NUP, ROUNDS = (3 * NE + 31) / 32;
+    const int lane = threadIdx.x & 31;
+    double* der = scr + eval_rows<NE, NM>();
+    // task of this lane in a round (the spare lanes of the last round repeat the last task)
+    auto task_of = [&](int round, int& e, int& t3) {
+        const int task = min(32 * round + lane, 3 * NE - 1);
+        t3 = task / NE;
+        e = task - t3 * NE;
+        return 32 * round + lane < 3 * NE;
+    };
+    auto coord = [&](int e, int c) { return gpos[(size_t)(3 * e + c) * Wcap + w]; };
+    // orbital values, row e of the electron's matrix
+#pragma unroll 1
+    for (int round = 0; round < ROUNDS; ++round) {
+        int e, t3;
+        const bool on = task_of(round, e, t3);
+        const int sig = e >= NUP;
+        const double x = coord(e, 0), y = coord(e, 1), z = coord(e, 2);
+        double v[NM];
+#pragma unroll
+        for (int k = 0; k < NM; ++k) v[k] = 0;
+#pragma unroll 1
+        for (int g = 0; g < S.n_third; ++g) {
+            const int d = S.third[3 * g + t3];
+            const int I = shell_nuc(d), np = shell_np(d), p0 = shell_p0(d), a0 = shell_a0(d);
+            const int ns = (d & SHELL_S) ? 1 : 0, na = ns + ((d & SHELL_P) ? 3 : 0);
+            const bool sp = na == 4;
+            const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            double s0 = 0, s1 = 0;
+            for (int p = p0; p < p0 + np; ++p) {
+                const double ex = d_exp(-S.prim[p][0] * r2);
+                s0 += S.prim[p][1] * ex;
+                if (sp) s1 += S.prim[p][4] * ex;
+            }
+            if (!sp) s1 = s0;
+#pragma unroll 1
+            for (int m = 0; m < na; ++m) {
+                const int c3 = m - ns;
+                const double chi = c3 < 0 ? s0 : (c3 == 0 ? dx : (c3 == 1 ? dy : dz)) * s1;
+                const double* c = S.C[a0 + m][sig];
+#pragma unroll
+                for (int k = 0; k < NM; ++k) v[k] += c[k] * chi;
+            }
+        }
+        if (on) {
+#pragma unroll
+            for (int k = 0; k < NM; ++k) scr[e * NM + k] = t3 == 0 ? v[k] : scr[e * NM + k] + v[k];
+        }
+        __syncwarp();
+    }
+    // Gauss-Jordan of each sector (kw_measure_walker's steps), lane j with column j
+    double det = 1.0, logdet = 0.0;            // |det| = det 2^ex exp(logdet)
+    int ex = 0, sg = 1;
+    bool ok = true;
+#pragma unroll 1
+    for (int sig = 0; sig < 2; ++sig) {
+        double* M = scr + sig * NM * NM;
+        double A[NM];
+#pragma unroll
+        for (int i = 0; i < NM; ++i) A[i] = lane < NM ? M[i * NM + lane] : 0.0;
+        __syncwarp();
+        int src = lane;
+#pragma unroll 1
+        for (int k = 0; k < NM; ++k) {
+            int p = 0, best = d_hi(A[0]) & 0x7fffffff;
+#pragma unroll
+            for (int r = 1; r < NM; ++r) {
+                const int m = d_hi(A[r]) & 0x7fffffff;
+                if (r < NM - k && m > best) { best = m; p = r; }
+            }
+            p = wshfl(p, k);
+#pragma unroll
+            for (int r = 1; r < NM; ++r) {
+                const bool sw = r == p;
+                const double a = A[0], b = A[r];
+                A[0] = sw ? b : a;
+                A[r] = sw ? a : b;
+            }
+            if (p != 0) sg = -sg;
+            const int pk = k + p;
+            src = src == k ? pk : (src == pk ? k : src);
+            double piv = wshfl(A[0], k);
+            if (((d_hi(piv) & 0x7fffffff) | d_lo(piv)) == 0) { ok = false; piv = 1.0; }
+            const int h = d_hi(piv), f = (h >> 20) & 0x7ff;
+            if (h < 0) sg = -sg;
+            if (f == 0 || f == 0x7ff) {
+                logdet += log(fabs(piv));
+            } else {
+                det *= __hiloint2double((h & 0x000fffff) | 0x3ff00000, d_lo(piv));
+                ex += f - 1023;
+            }
+            const double ip = d_rcp_full(piv);
+            const double t = lane == k ? 1.0 + ip : A[0] * ip, first = lane == k ? ip : t;
+#pragma unroll
+            for (int i = 1; i < NM; ++i) A[i - 1] = A[i] - wshfl(A[i], k) * t;
+            A[NM - 1] = first;
+        }
+#pragma unroll
+        for (int i = 0; i < NM; ++i) A[i] = wshfl(A[i], src);
+        if (lane < NM) {
+#pragma unroll
+            for (int k = 0; k < NM; ++k) {
+                M[lane * NM + k] = A[k];
+                if (write_state) gdinv[((size_t)(sig * NM * NM + k * NM + lane)) * Wcap + w] = A[k];
+            }
+        }
+    }
+    logdet += d_log(det) + (double)ex * 0.6931471805599453;
+    __syncwarp();
+    // grad ln D and lap D / D of each electron: sum_a c'_a (grad, lap) chi_a with
+    // c'_a = sum_k C[a][k] D^-1[k][q] (kw_refresh_walker has the formulas)
+#pragma unroll 1
+    for (int round = 0; round < ROUNDS; ++round) {
+        int e, t3;
+        const bool on = task_of(round, e, t3);
+        const int sig = e >= NUP;
+        const double x = coord(e, 0), y = coord(e, 1), z = coord(e, 2);
+        double A[NM];
+#pragma unroll
+        for (int k = 0; k < NM; ++k) A[k] = scr[e * NM + k];
+        double gx = 0, gy = 0, gz = 0, ld = 0;
+#pragma unroll 1
+        for (int g = 0; g < S.n_third; ++g) {
+            const int d = S.third[3 * g + t3];
+            const int I = shell_nuc(d), np = shell_np(d), p0 = shell_p0(d), a0 = shell_a0(d);
+            const int ns = (d & SHELL_S) ? 1 : 0, na = ns + ((d & SHELL_P) ? 3 : 0);
+            const bool sp = na == 4;
+            const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
+            const double r2 = dx * dx + dy * dy + dz * dz, r4 = 4.0 * r2;
+            double s0 = 0, s1 = 0, s2 = 0, q0 = 0, q1 = 0, q2 = 0;
+            for (int p = p0; p < p0 + np; ++p) {
+                const double* t = S.prim[p];
+                const double E = d_exp(-t[0] * r2);
+                s0 += t[1] * E;
+                s1 += t[2] * E;
+                s2 += t[3] * E;
+                if (sp) {
+                    q0 += t[4] * E;
+                    q1 += t[5] * E;
+                    q2 += t[6] * E;
+                }
+            }
+            double cd = 0;
+#pragma unroll 1
+            for (int m = 0; m < na; ++m) {
+                const double* c = S.C[a0 + m][sig];
+                // two sums, for the latency of the chain
+                double c0 = 0, c1 = 0;
+#pragma unroll
+                for (int k = 0; k + 1 < NM; k += 2) { c0 += c[k] * A[k]; c1 += c[k + 1] * A[k + 1]; }
+                if (NM % 2) c0 += c[NM - 1] * A[NM - 1];
+                const double cw = c0 + c1;
+                const int c3 = m - ns;
+                if (c3 < 0) {
+                    cd = cw;
+                } else {
+                    if (c3 == 0 && sp) { s0 = q0; s1 = q1; s2 = q2; cd = 0; }
+                    cd += cw * (c3 == 0 ? dx : (c3 == 1 ? dy : dz));
+                    const double o = s0 * cw;
+                    if (c3 == 0) gx += o;
+                    else if (c3 == 1) gy += o;
+                    else gz += o;
+                }
+                if (c3 < 0 || c3 == 2) {
+                    const double t = -2.0 * s1 * cd;
+                    gx += t * dx; gy += t * dy; gz += t * dz;
+                    ld += cd * (r4 * s2 - (c3 < 0 ? 6.0 : 10.0) * s1);
+                }
+            }
+        }
+        if (on) {
+            const double v[4] = {gx, gy, gz, ld};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) der[c * NE + e] = t3 == 0 ? v[c] : der[c * NE + e] + v[c];
+        }
+        __syncwarp();
+    }
+    // Jastrow and Coulomb terms: pair p joins electron i = p mod NE with i + p / NE + 1
+    // (mod NE), the last NE / 2 pairs i with i + NE / 2; 32 consecutive pairs have
+    // distinct i and distinct j, so the sums need no atomics
+    double *pos = scr, *sums = scr + 3 * NE;
+    for (int e = lane; e < NE; e += 32) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) pos[c * NE + e] = coord(e, c);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) sums[c * NE + e] = 0.0;
+    }
+    __syncwarp();
+    double u = 0, V = 0;
+    // terms at separation r2: u, u'/r, u'' + 2u'/r, 1/r (0 at r = 0) and r
+    auto pade = [](double a, double b, double r2, double& uu, double& f, double& l, double& ri, double& r) {
+        dist(r2, r, ri);
+        const double inv = frcp(1.0 + b * r), ai = a * inv, up = ai * inv;
+        uu = ai * r;
+        f = up * ri;
+        l = 2.0 * (f - up * (b * inv));
+    };
+    constexpr int NPAIR = NE * (NE - 1) / 2, FULL = NE * ((NE - 1) / 2);
+    static_assert(NE % 2 == 0, "the last NE / 2 pairs join opposite electrons");
+#pragma unroll 1
+    for (int r0 = 0; r0 < NPAIR; r0 += 32) {
+        const bool on = r0 + lane < NPAIR;
+        const int p = on ? r0 + lane : NPAIR - 1;
+        const int i = p < FULL ? p % NE : p - FULL;
+        int j = p < FULL ? i + p / NE + 1 : i + NE / 2;
+        if (j >= NE) j -= NE;
+        const double dx = pos[i] - pos[j], dy = pos[NE + i] - pos[NE + j], dz = pos[2 * NE + i] - pos[2 * NE + j];
+        const int c = (j < NUP) == (i < NUP) ? 1 : 0;
+        double uu, f, l, ri, r;
+        pade(S.a_ee[c], S.b_ee[c], dx * dx + dy * dy + dz * dz, uu, f, l, ri, r);
+        if (on) { u += uu; V += ri; }
+        const bool use = on && !closer(r, 1e-10);
+        const double fx = f * dx, fy = f * dy, fz = f * dz;
+        if (use) {
+            sums[i] += fx; sums[NE + i] += fy; sums[2 * NE + i] += fz; sums[3 * NE + i] += l;
+        }
+        __syncwarp();
+        if (use) {
+            sums[j] -= fx; sums[NE + j] -= fy; sums[2 * NE + j] -= fz; sums[3 * NE + j] += l;
+        }
+        if (S.quirk_lap) {
+            const double up = f * r, sq = up * up;
+            if (use) sums[4 * NE + i] += sq;
+            __syncwarp();
+            if (use) sums[4 * NE + j] += sq;
+        }
+        __syncwarp();
+    }
+#pragma unroll 1
+    for (int r0 = 0; r0 < NE * NNUC; r0 += 32) {
+        const bool on = r0 + lane < NE * NNUC;
+        const int p = on ? r0 + lane : NE * NNUC - 1, I = p / NE, e = p - I * NE;
+        const double dx = pos[e] - S.nuc[I][0], dy = pos[NE + e] - S.nuc[I][1], dz = pos[2 * NE + e] - S.nuc[I][2];
+        double uu, f, l, ri, r;
+        pade(S.nuc[I][4], S.nuc[I][5], dx * dx + dy * dy + dz * dz, uu, f, l, ri, r);
+        if (on) {
+            u -= uu;
+            V -= S.nuc[I][3] * ri;
+            if (!closer(r, 1e-10)) {
+                sums[e] -= f * dx; sums[NE + e] -= f * dy; sums[2 * NE + e] -= f * dz; sums[3 * NE + e] -= l;
+            }
+        }
+        __syncwarp();
+    }
+    double kin = 0;
+#pragma unroll 1
+    for (int e = lane; e < NE; e += 32) {
+        const double jx = sums[e], jy = sums[NE + e], jz = sums[2 * NE + e], lu = sums[3 * NE + e];
+        const double gx = der[e], gy = der[NE + e], gz = der[2 * NE + e];
+        const double ax = S.qa * jx, ay = S.qa * jy, az = S.qa * jz;
+        const double lj = S.quirk_lap ? lu + sums[4 * NE + e] : lu + jx * jx + jy * jy + jz * jz;
+        const double lp = der[3 * NE + e] + 2.0 * (gx * ax + gy * ay + gz * az) + lj;
+        kin += lp;
+        if (out_grad) {                         // internal order; the host permutes to the caller's
+            double* o = out_grad + ((size_t)w * NE + e) * 3;
+            o[0] = gx + ax;
+            o[1] = gy + ay;
+            o[2] = gz + az;
+        }
+        if (out_lap) out_lap[(size_t)w * NE + e] = lp;
+    }
+    V += -0.5 * kin;
+    u = wsum(u);
+    V = wsum(V);
+    const double e_l = V + S.v_nn;
+    if (lane == 0) {
+        int fl = 0;
+        if (!ok) fl |= FLAG_SINGULAR;
+        if (!isfinite(e_l)) fl |= FLAG_NONFINITE;
+        if (fl) atomicOr(flags, fl);
+        if (write_state) { glog[w] = logdet + u; gsign[w] = sg; gel[w] = e_l; }
+    }
+    return e_l;
+}
+
+// ---------------------------------------------------------------------------
 // Float-float refresh of FP32 walkers, both spin sectors at once: the sectors have
 // the same size and the same walk over the basis, so sector 0 and sector 1 are the
 // two components of packed instructions (ff2), lane q holding electrons q and
@@ -1613,15 +1968,14 @@ struct PairTabHead {                // sizes and scalars; the arrays follow in t
     ff b_ee[2], a_ee[2];
 };
 // Device table: head, nuclei [NNUC] (x, y, z, Z, enA, enB as ff), shells in AO order,
-// the same dealt into three lists of equal kinds (third t's shell i at 3 i + t; rows
-// are filled up with shells without primitives), primitives (exponent, coefficient)
-// and (c a, c a^2) of each, an sp shell's p coefficients beside them, then the
+// the same in thirds (deal_thirds), primitives (exponent, coefficient) and (c a,
+// c a^2) of each, an sp shell's p coefficients beside them, then the
 // coefficients [n_ao][NM] of both sectors as (hi, hi', lo, lo').
 template <int NNUC, int NM>
 struct PairTab {
     PairTabHead head;
     ff nuc[NNUC][6];
-    int sh[WMAX_AO], third[WMAX_AO + 12];
+    int sh[WMAX_AO], third[WMAX_THIRD];
     float4 prim[WMAX_PRIM], primd[WMAX_PRIM];      // s or lone p
     float4 prim_p[WMAX_PRIM], primd_p[WMAX_PRIM];  // p of an sp shell
     float4 C[WMAX_AO][NM];
@@ -1635,16 +1989,7 @@ static void fill_pairtab(const SysW<ff>& w, PairTab<NNUC, NM>& S) {
     S.head.n_ao = w.n_ao;
     const ShellList<ff> L(w);
     S.head.n_sh = (int)L.desc.size();
-    // thirds: shells of one kind, by primitive count, dealt in rows of three
-    std::vector<int> by[3];
-    for (int d : L.desc) by[(d & SHELL_S) ? ((d & SHELL_P) ? 2 : 0) : 1].push_back(d);
-    int nt = 0;
-    for (auto& v : by) {
-        std::stable_sort(v.begin(), v.end(), [](int a, int b) { return shell_np(a) < shell_np(b); });
-        for (size_t i = 0; i < (v.size() + 2) / 3 * 3; ++i)
-            S.third[nt++] = i < v.size() ? v[i] : shell_pack(0, v[0] & (SHELL_S | SHELL_P), 0, 0, 0);
-    }
-    S.head.n_third = nt / 3;
+    S.head.n_third = deal_thirds(L.desc, S.third);
     S.head.quirk_lap = w.quirk_lap;
     S.head.qa = w.qa;
     S.head.v_nn = w.v_nn;
@@ -2146,23 +2491,47 @@ __global__ void __launch_bounds__(32 * WPB) kw_measure(const SysW<TC>* __restric
     if (partial) warp_block_partial<WPB>(e_l, partial, blockIdx.x);
 }
 
-// Batched form (compute type TC, state written, per-tile E_L partials), one
-// block of WPB warps per WPB-walker tile.
-template <int NE, int NUP, int NNUC, class TC, class TS, int WPB>
-__global__ void __launch_bounds__(32 * WPB) kwb_measure(const BatchTile* __restrict__ tiles, int ntiles,
-                                                        const BatchRec* __restrict__ recs, double* tile_partial) {
-    constexpr int NM = NUP > NE - NUP ? NUP : NE - NUP;
-    __shared__ SysW<TC> S;
+// FP64 evaluation, standalone and batched (state written, per-tile E_L partials; one
+// block of WPB warps per WPB-walker tile).  Dynamic shared memory: the table's used
+// part, then the warps' scratch.
+template <int NE, int NUP, int NNUC, int WPB>
+static size_t eval_smem(int n_ao) {
+    return EvalTab<NNUC, NUP>::bytes(n_ao) + sizeof(double) * WPB * eval_scratch<NE, NUP>();
+}
+template <int NE, int NUP, int NNUC, int WPB>
+__global__ void __launch_bounds__(32 * WPB) kw_eval(const EvalTab<NNUC, NUP>* __restrict__ Sg, const double* __restrict__ gpos,
+                                                    double* __restrict__ gdinv, double* __restrict__ glog,
+                                                    int* __restrict__ gsign, double* __restrict__ gel, int W, int Wcap,
+                                                    int write_state, double* __restrict__ out_grad,
+                                                    double* __restrict__ out_lap, double* partial, int* flags) {
+    using TAB = EvalTab<NNUC, NUP>;
+    extern __shared__ __align__(16) unsigned char wsm[];
+    TAB& S = *reinterpret_cast<TAB*>(wsm);
+    load_tab(&S, Sg);
+    const int wib = threadIdx.x >> 5, w = blockIdx.x * WPB + wib;
+    double* scr = reinterpret_cast<double*>(wsm + TAB::bytes(S.n_ao)) + (size_t)wib * eval_scratch<NE, NUP>();
+    double e_l = 0.0;
+    if (w < W)
+        e_l = kw_eval_walker<NE, NUP, NNUC>(S, scr, gpos, gdinv, glog, gsign, gel, w, Wcap, write_state, out_grad, out_lap,
+                                            flags);
+    if (partial) warp_block_partial<WPB>(e_l, partial, blockIdx.x);
+}
+template <int NE, int NUP, int NNUC, int WPB>
+__global__ void __launch_bounds__(32 * WPB) kwb_eval(const BatchTile* __restrict__ tiles, int ntiles,
+                                                     const BatchRec* __restrict__ recs, double* tile_partial) {
+    using TAB = EvalTab<NNUC, NUP>;
     extern __shared__ __align__(16) unsigned char wsm[];
     if ((int)blockIdx.x >= ntiles) return;
-    const int wib = threadIdx.x >> 5;
-    TC* Mrow = reinterpret_cast<TC*>(wsm) + (size_t)wib * NM * MRS;
     const BatchTile tl = tiles[blockIdx.x];
     const BatchRec& R = recs[tl.rec];
-    load_sysw(&S, static_cast<const SysW<TC>*>(R.tab_d));
-    const int w = tl.w0 + wib;
-    double e_l = kw_measure_walker<NE, NUP, NNUC, TC, TS>(S, Mrow, (const TS*)R.pos, (TS*)R.dinv, R.logabs, R.sign,
-                                                          R.el, w, w < R.W, R.Wcap, 1, nullptr, nullptr, R.flags);
+    TAB& S = *reinterpret_cast<TAB*>(wsm);
+    load_tab(&S, static_cast<const TAB*>(R.tab_d));
+    const int wib = threadIdx.x >> 5, w = tl.w0 + wib;
+    double* scr = reinterpret_cast<double*>(wsm + TAB::bytes(S.n_ao)) + (size_t)wib * eval_scratch<NE, NUP>();
+    double e_l = 0.0;
+    if (w < R.W)
+        e_l = kw_eval_walker<NE, NUP, NNUC>(S, scr, (const double*)R.pos, (double*)R.dinv, R.logabs, R.sign, R.el, w, R.Wcap,
+                                            1, nullptr, nullptr, R.flags);
     warp_block_partial<WPB>(e_l, tile_partial, blockIdx.x);
 }
 
@@ -2271,47 +2640,58 @@ struct WarpShapeOps {
         return launch_sum_partials(partial, nb, 1, dw.partial + dw.partial_cap - 1, st);
     }
 
-    // Refresh of FP32 walkers: its table (device copy cached like the others) and
-    // shared memory.  12 warps per SM at up to 168 registers.
+    // The kernels' own tables, filled from a SysW of their precision: device copies
+    // cached like the others.
     using PT = PairTab<NNUC, NUP>;
-    static int pair_table(const HostSys& hs, const PT** out) {
-        constexpr int slot = 2;
-        if (!hs.dev_table[slot] || hs.dev_table_version[slot] != hs.version) {
-            SysW<ff>* w = new SysW<ff>;
-            PT* h = new PT;
-            const bool good = fill_sysw<ff>(hs, NE, NUP, NNUC, *w);
-            if (good) fill_pairtab<NNUC, NUP>(*w, *h);
-            int rc = good ? 0 : 7;
-            if (!rc && !hs.dev_table[slot] && cudaMalloc(&hs.dev_table[slot], sizeof(PT)) != cudaSuccess) rc = 8;
-            if (!rc && cudaMemcpy(hs.dev_table[slot], h, sizeof(PT), cudaMemcpyHostToDevice) != cudaSuccess) rc = 2;
-            delete w;
-            delete h;
-            if (rc) return rc;
-            hs.dev_table_version[slot] = hs.version;
-        }
-        *out = static_cast<const PT*>(hs.dev_table[slot]);
-        return 0;
-    }
-    // FP32 Gaussian sweeps: their table and launches.
     using GT = GaussTab<NNUC, NM>;
-    static int gauss_table(const HostSys& hs, const GT** out) {
-        constexpr int slot = 4;
+    using ET = EvalTab<NNUC, NUP>;
+    template <class T, class TAB>
+    static int own_table(const HostSys& hs, int slot, void (*fill)(const SysW<T>&, TAB&), const TAB** out) {
         if (!hs.dev_table[slot] || hs.dev_table_version[slot] != hs.version) {
-            SysW<float>* w = new SysW<float>;
-            GT* h = new GT;
-            const bool good = fill_sysw<float>(hs, NE, NUP, NNUC, *w);
-            if (good) fill_gausstab<NNUC, NM>(*w, *h);
+            SysW<T>* w = new SysW<T>;
+            TAB* h = new TAB;
+            const bool good = fill_sysw<T>(hs, NE, NUP, NNUC, *w);
+            if (good) fill(*w, *h);
             int rc = good ? 0 : 7;
-            if (!rc && !hs.dev_table[slot] && cudaMalloc(&hs.dev_table[slot], sizeof(GT)) != cudaSuccess) rc = 8;
-            if (!rc && cudaMemcpy(hs.dev_table[slot], h, sizeof(GT), cudaMemcpyHostToDevice) != cudaSuccess) rc = 2;
+            if (!rc && !hs.dev_table[slot] && cudaMalloc(&hs.dev_table[slot], sizeof(TAB)) != cudaSuccess) rc = 8;
+            if (!rc && cudaMemcpy(hs.dev_table[slot], h, sizeof(TAB), cudaMemcpyHostToDevice) != cudaSuccess) rc = 2;
             delete w;
             delete h;
             if (rc) return rc;
             hs.dev_table_version[slot] = hs.version;
         }
-        *out = static_cast<const GT*>(hs.dev_table[slot]);
+        *out = static_cast<const TAB*>(hs.dev_table[slot]);
         return 0;
     }
+    static int pair_table(const HostSys& hs, const PT** out) { return own_table<ff, PT>(hs, 2, fill_pairtab<NNUC, NUP>, out); }
+    static int gauss_table(const HostSys& hs, const GT** out) { return own_table<float, GT>(hs, 4, fill_gausstab<NNUC, NM>, out); }
+    static int eval_table(const HostSys& hs, const ET** out) { return own_table<double, ET>(hs, 5, fill_evaltab<NNUC, NUP>, out); }
+
+    // FP64 evaluation.
+    static int eval(const HostSys& hs, DevWalkers& dw, bool ws, const MeasureOut& out, cudaStream_t st) {
+        const ET* S;
+        const int rc = eval_table(hs, &S);
+        if (rc) return rc;
+        const int nb = (dw.W + WPB - 1) / WPB;
+        auto kern = kw_eval<NE, NUP, NNUC, WPB>;
+        static bool attr = false;
+        if (!attr) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)eval_smem<NE, NUP, NNUC, WPB>(WMAX_AO)) != cudaSuccess)
+                return 2;
+            attr = true;
+        }
+        double* partial = (ws && dw.partial && dw.partial_cap >= 2 * nb + 1) ? dw.partial : nullptr;
+        kern<<<nb, 32 * WPB, eval_smem<NE, NUP, NNUC, WPB>(hs.n_ao), st>>>(
+            S, (const double*)dw.pos, (double*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W, dw.Wcap, ws ? 1 : 0, out.grad, out.lap,
+            partial, dw.flags);
+        ++g_launch_count;
+        if (cudaGetLastError() != cudaSuccess) return 2;
+        if (!partial) return 0;
+        return launch_sum_partials(partial, nb, 1, dw.partial + dw.partial_cap - 1, st);
+    }
+
+    // FP32 Gaussian sweeps.
     static int gauss(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, uint64_t seed, cudaStream_t st) {
         const GT* S;
         const int rc = gauss_table(hs, &S);
@@ -2373,7 +2753,7 @@ struct WarpShapeOps {
     static int measure(const HostSys& hs, DevWalkers& dw, int cp, bool ws, const MeasureOut& out, cudaStream_t st) {
         if (out.O || out.fhf || out.omega) return 7;
         // FP32 walkers refresh in float-float arithmetic on the FP32 pipe
-        if (cp == 0 && dw.prec == 0) return measure_w<double, double, WPB>(hs, dw, ws, out, st);
+        if (cp == 0 && dw.prec == 0) return eval(hs, dw, ws, out, st);
         if (cp == 0) return out.grad || out.lap ? 7 : refresh(hs, dw, ws, st);
         if (dw.prec == 1) return measure_w<float, float, WPB>(hs, dw, ws, out, st);
         return 7;
@@ -2407,9 +2787,12 @@ struct WarpShapeOps {
         r.ktab = nullptr;
         if (prec == 0) {
             const SysW<double>* d;
+            const ET* e;
             int rc = table<double>(hs, &d);
+            if (!rc) rc = eval_table(hs, &e);
             if (rc) return rc;
-            r.tab_d = r.tab_s = d;
+            r.tab_d = e;
+            r.tab_s = d;
             return 0;
         }
         const PT* m;
@@ -2452,13 +2835,13 @@ struct WarpShapeOps {
         return 7;
     }
 
-    template <class TC, class TS>
-    static int batch_measure_t(const BatchClass& bc, cudaStream_t st, int* occ) {
-        const size_t smem = sizeof(TC) * BTW * NM * MRS;
-        auto kern = kwb_measure<NE, NUP, NNUC, TC, TS, BTW>;
+    static int batch_eval(const BatchClass& bc, cudaStream_t st, int* occ) {
+        auto kern = kwb_eval<NE, NUP, NNUC, BTW>;
+        const size_t smem = eval_smem<NE, NUP, NNUC, BTW>(bc.n_ao);
         static bool attr = false;
         if (!attr) {
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)eval_smem<NE, NUP, NNUC, BTW>(WMAX_AO)) != cudaSuccess)
                 return 2;
             attr = true;
         }
@@ -2470,7 +2853,7 @@ struct WarpShapeOps {
     }
 
     static int batch_measure(const BatchClass& bc, cudaStream_t st, int* occ = nullptr) {
-        if (bc.prec == 0) return batch_measure_t<double, double>(bc, st, occ);
+        if (bc.prec == 0) return batch_eval(bc, st, occ);
         auto kern = kwb_refresh<NE, NUP, NNUC, RWPB>;
         const size_t smem = refresh_smem(WMAX_AO);
         static bool attr = false;
