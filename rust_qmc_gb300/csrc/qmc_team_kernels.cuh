@@ -508,7 +508,8 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
         for (int k = 0; k < NM; ++k) v[k] += S.C[T.sig][a][k] * chi;
         if (NR > 0) {
 #pragma unroll
-            for (int q = 0; q < NR; ++q) dv[q] += S.dC[q][a] * chi;
+            for (int q = 0; q < NR; ++q)
+                if (q < S.n_rot) dv[q] += S.dC[q][a] * chi;
         }
     }
 #pragma unroll
@@ -564,8 +565,9 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
         // rotation rows: d ln|D| / d theta = sum_q psi(r_q) D^-1[c][q]
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
+            if (q >= S.n_rot) break;
             dv[q] = T.part_sum(dv[q]);
-            if (q < S.n_rot && T.on && T.part == 0) {
+            if (T.on && T.part == 0) {
                 const int c = S.rot_col[q][T.sig];
                 double b = 0;
 #pragma unroll
@@ -628,14 +630,13 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
                 const int c = (m < TM::NUP) == (T.e < TM::NUP) ? 1 : 0;
                 const double b = el ? S.b_ee[c] : S.enB[I], a = el ? S.a_ee[c] : -S.enA[I];
                 const double i1 = recip_full(1.0 + b * d), i2 = i1 * i1, i3 = i2 * i1;
-                const double s = el ? 1.0 : -S.Z[I];
-                const double fa = s * i2 * ri, la = 2.0 * fa - 2.0 * s * b * i3;
-                const double fb = -2.0 * a * i3, lb = 3.0 * fb * i1;
-                const double gd = 2.0 * (Gx * dx + Gy * dy + Gz * dz);
+                // f = -2 a i3, l = 3 f i1 for b; f = s i2 / r, l = 2 f - 2 s b i3 for a
+                const double ms = el ? -1.0 : S.Z[I];
+                const double h = Gx * dx + Gy * dy + Gz * dz;
                 const int k = el ? c : 4 + S.species[I];
                 if (use && !d_below(d, 1e-10)) {
-                    mine[k] -= 0.5 * (lb + fb * gd);
-                    mine[k + 2] -= 0.5 * (la + fa * gd);
+                    mine[k] += a * i3 * fma(3.0, i1, 2.0 * h);
+                    mine[k + 2] += ms * fma(i2 * ri, 1.0 + h, -b * i3);
                 }
             }
             // rotation columns: with beta = D^-1 psi (over the sector's rows) and
@@ -1278,7 +1279,8 @@ struct TeamOps {
         if (rc) return rc;
         if (dw.W == 0) return 0;
         const int nb = (dw.W + NT - 1) / NT;
-        double* partial = ws && dw.partial && dw.partial_cap >= 2 * nb + 1 ? dw.partial : nullptr;
+        // the sums of the sampled rows include E_L's: no partials beside them
+        double* partial = ws && NR == 0 && !FORCE && dw.partial && dw.partial_cap >= 2 * nb + 1 ? dw.partial : nullptr;
         k_team_measure<SH, G, NR, DEL, FORCE, TPB><<<nb, TPB, 0, st>>>(
             tab, (const double*)dw.pos, (double*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W, dw.Wcap, ws ? 1 : 0, out,
             hs.n_params(), partial, dw.flags);

@@ -3,12 +3,17 @@
 //
 // One warp owns one walker.  Lane j holds column j of each inverse Slater
 // matrix in registers (Dinv[k][j], k = 0..n-1) and the positions of
-// electrons j and j+32.  AOs are evaluated lane-parallel from tables in
-// shared memory; the AO->MO contraction, the determinant ratio and the
-// Sherman-Morrison update broadcast one lane's values with shuffles, so every
-// register index stays static.  The FP64 refresh is a warp-cooperative
-// Gauss-Jordan elimination in which lane j carries column j of [D | I] and
-// ends holding column j of D^-1 -- exactly the sweep kernel's layout.
+// electrons j and j+32.  The kernels:
+//   kw_gauss    FP32 Gaussian sweeps (packed FP32 instructions)
+//   kw_sweep    drift-diffusion sweeps, and FP64 Gaussian sweeps
+//   kw_refresh  float-float refresh of FP32 walkers (packed, both sectors)
+//   kw_eval     FP64 evaluation and refresh
+//   kw_measure  FP32 refresh of FP32 walkers
+// and kwb_* their batched forms.  Tables lie in shared memory; what all lanes need of
+// one lane or of one proposal (inverse column, orbital values) is broadcast from
+// there or by shuffles, so every register index stays static.  Inverses come from a
+// warp-cooperative Gauss-Jordan elimination in which lane j ends holding column j of
+// D^-1 -- exactly the sweep kernels' layout.
 #pragma once
 #include <algorithm>
 #include <cstddef>
@@ -981,7 +986,10 @@ __device__ __forceinline__ float wsum_order(const float* v) {
     return s[0];
 }
 
-// FP32 Gaussian sweeps.  kw_sweep_walker's operations in its order on every value;
+// FP32 Gaussian sweeps.  Issue slots and the latency of the proposal chain bound them:
+// at 16 warps per SM (128 registers) 272 warp instructions a proposal, issue 62 % busy,
+// shared-memory pipe 68 %, where the shuffle form had 315; 8 sweeps of 16 384 benzene
+// walkers take 1.93 ms after 2.39 ms.  kw_sweep_walker's operations in its order on every value;
 // here a lane's inverse columns lie in row pairs, so that ratio, update, orbital
 // contraction and the two rounds of Jastrow partners take packed FP32 instructions,
 // and a proposal's position and draw and the moving electron's column are read from
@@ -1328,7 +1336,7 @@ __global__ void __launch_bounds__(32 * WPB, sizeof(T) == 4 ? 16 / WPB : 1) kwb_s
     kw_sweep_walker<NE, NUP, NNUC, T, MOVE>(S, a, w, ph);
 }
 
-// Full evaluation from positions (refresh + E_L), one warp per walker.
+// Full evaluation from positions (refresh + E_L) in FP32, one warp per walker.
 // Per-warp shared scratch holds the sector's D rows, then the rows of its
 // inverse; orbital derivatives are evaluated in a second pass.
 // Row stride of the refresh's per-warp matrix scratch: lane q writes row q
@@ -1433,8 +1441,6 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
             P.z[r] = ok ? (TC)gpos[(3 * j + 2) * (size_t)Wcap + w] : TC(0);
         }
         double logdet = 0.0;
-        ff pmag = ff(1.0f);                       // float-float form: |det| = pmag 2^pexp
-        int pexp = 0;
         int sg = 1;
         bool ok = true;
         // per-lane electron results: lane owns electron (sig*NUP + lane) of each sector
@@ -1492,12 +1498,7 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
                 TC piv = wshfl(A[0], k);
                 if (!(piv != TC(0))) { ok = false; piv = TC(1); }
                 if (piv < 0) sg = -sg;
-                if constexpr (std::is_same<TC, ff>::value) {
-                    pmag = pmag * fabs(piv);           // |det| as a rescaled product
-                    ff_rescale(pmag, pexp);
-                } else {
-                    logdet += log(fabs((double)piv));
-                }
+                logdet += log(fabs((double)piv));
                 const TC ip = TC(1) / piv;
                 const TC t = (lane == k) ? TC(1) + ip : A[0] * ip;
                 A[0] = (lane == k) ? ip : t;
@@ -1597,8 +1598,6 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
         u = wsum(u);
         V = wsum(V);
         kin = wsum(kin);
-        if constexpr (std::is_same<TC, ff>::value)
-            logdet = log((double)pmag) + (double)pexp * 0.6931471805599453;
         e_l = (double)(TC(-0.5) * kin + V + S.v_nn);
         if (lane == 0) {
             int fl = 0;
@@ -1619,7 +1618,8 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
 // where one lane per electron of a sector took two rounds of 21 lanes over all
 // shells; pairs and nucleus terms are evaluated once each and added to per-electron
 // sums; pivots are compared, and |det| is kept, on exponent and high-word bits, with
-// one logarithm a walker.
+// one logarithm a walker.  500 configurations: 641 us before, about 330 us now (the
+// host call 797 us and 484 us).
 // ---------------------------------------------------------------------------
 template <int NNUC, int NM>
 struct EvalTab {
@@ -1960,7 +1960,11 @@ __device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, cons
 // pairs are evaluated once, two per lane and instruction.  The kernel is an
 // instruction stream of several loops, each longer than the instruction cache likes
 // to hold beside the others: the block's warps (one block per SM) walk the phases
-// together, so that one loop is in use at a time.
+// together, so that one loop is in use at a time (16 384 walkers: 2.16 ms, 2.69 ms in
+// four-warp blocks that do not wait for each other, 3.15 ms for one sector at a time).
+// The FP32 pipe bounds it, 74 % busy; of the cycles 30 % are orbital values, 25 % the
+// inversion, 29 % derivatives, 16 % pairs and nuclei.  1.94 ms with the derivatives as
+// (electron pair, third) tasks.
 // ---------------------------------------------------------------------------
 struct PairTabHead {                // sizes and scalars; the arrays follow in the block's shared memory
     int n_ao, n_sh, n_third, quirk_lap;
@@ -2590,7 +2594,7 @@ struct WarpShapeOps {
     static int table(const HostSys& hs, const SysW<T>** out) {
         // device copies of the table, cached per system and rebuilt when the
         // parameters or nuclei change (HostSys::version)
-        const int slot = std::is_same<T, double>::value ? 0 : (std::is_same<T, float>::value ? 1 : 2);
+        const int slot = std::is_same<T, double>::value ? 0 : 1;
         if (!hs.dev_table[slot] || hs.dev_table_version[slot] != hs.version) {
             SysW<T>* h = new SysW<T>;
             if (!fill_sysw<T>(hs, NE, NUP, NNUC, *h)) { delete h; return 7; }
@@ -2617,14 +2621,14 @@ struct WarpShapeOps {
         return cudaGetLastError() == cudaSuccess ? 0 : 2;
     }
 
-    template <class TC, class TS, int WB>
+    template <class TC, class TS>
     static int measure_w(const HostSys& hs, DevWalkers& dw, bool ws, const MeasureOut& out, cudaStream_t st) {
         const SysW<TC>* S;
         int rc = table<TC>(hs, &S);
         if (rc) return rc;
-        int nb = (dw.W + WB - 1) / WB;
-        size_t smem = sizeof(TC) * WB * NM * MRS;
-        auto kern = kw_measure<NE, NUP, NNUC, TC, TS, WB>;
+        int nb = (dw.W + WPB - 1) / WPB;
+        size_t smem = sizeof(TC) * WPB * NM * MRS;
+        auto kern = kw_measure<NE, NUP, NNUC, TC, TS, WPB>;
         static bool attr = false;
         if (!attr) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -2632,7 +2636,7 @@ struct WarpShapeOps {
             attr = true;
         }
         double* partial = (ws && dw.partial && dw.partial_cap >= 2 * nb + 1) ? dw.partial : nullptr;
-        kern<<<nb, 32 * WB, smem, st>>>(S, (const TS*)dw.pos, (TS*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W, dw.Wcap,
+        kern<<<nb, 32 * WPB, smem, st>>>(S, (const TS*)dw.pos, (TS*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W, dw.Wcap,
                                         ws ? 1 : 0, out.grad, out.lap, partial, dw.flags);
         ++g_launch_count;
         if (cudaGetLastError() != cudaSuccess) return 2;
@@ -2755,7 +2759,7 @@ struct WarpShapeOps {
         // FP32 walkers refresh in float-float arithmetic on the FP32 pipe
         if (cp == 0 && dw.prec == 0) return eval(hs, dw, ws, out, st);
         if (cp == 0) return out.grad || out.lap ? 7 : refresh(hs, dw, ws, st);
-        if (dw.prec == 1) return measure_w<float, float, WPB>(hs, dw, ws, out, st);
+        if (dw.prec == 1) return measure_w<float, float>(hs, dw, ws, out, st);
         return 7;
     }
 
