@@ -193,6 +193,24 @@ __device__ __forceinline__ void team_ao(const TeamTab<SH>& S, int a, bool ok, do
     }
 }
 
+// |psi| = pm 2^pe exp(u): a step compares these without a logarithm.
+struct PsiAbs {
+    double pm, u;
+    int pe;
+    __device__ __forceinline__ double log_abs() const { return d_log(pm) + (double)pe * 0.6931471805599453 + u; }
+    // From log|psi| (pm = 1).
+    static __device__ __forceinline__ PsiAbs of_log(double l) {
+        const int pe = __float2int_rn(fminf(fmaxf((float)l * 1.44269504f, -1e6f), 1e6f));
+        return {1.0, fma(-(double)pe, 0.6931471805599453, l), pe};
+    }
+};
+// Whether uniform ua is below |a|^2 / |b|^2 (bm2 = b.pm^2).
+__device__ __forceinline__ bool below_ratio2(double ua, const PsiAbs& a, const PsiAbs& b, double bm2) {
+    const double e = d_exp(2.0 * (a.u - b.u));
+    const int k = max(-900, min(900, 2 * (a.pe - b.pe)));     // 2^-900 is below every uniform
+    return ua * bm2 < a.pm * a.pm * __hiloint2double((1023 + k) << 20, 0) * e;
+}
+
 // Lanes of a walker (team) and the pieces of an evaluation.
 template <class SH, int G>
 struct Team {
@@ -326,10 +344,6 @@ struct Team {
         ok = shfl(g, base) && (NDN == 0 || shfl(g, base + NUP));
         sg = s ? -1 : 1;
     }
-    static __device__ __forceinline__ double log_det(double pm, int pe) {
-        return d_log(pm) + (double)pe * 0.6931471805599453;
-    }
-
     // Jastrow u alone: the pairs and electron-nucleus terms spread over the lanes.
     __device__ __forceinline__ double jastrow_value(const Tab& S, double x, double y, double z) const {
         double u = 0;
@@ -390,6 +404,8 @@ struct Team {
             double d, ri;
             dist(r2, d, ri);
             V += ok ? (el ? 0.5 : -S.Z[I]) * ri : 0.0;
+            // nuclei alone in a round, and no electron-nucleus Jastrow terms
+            if (SH::JAS == JAS_PADE_F && PARTS * r >= NE) continue;
             double inv = 0, f = 0, l = 0, uu = 0, up = 0;
             const int c = (m < NUP) == (e < NUP) ? 1 : 0;
             if (SH::JAS == JAS_PADE_EEN) {
@@ -433,10 +449,10 @@ __device__ __forceinline__ void stage_team(TAB* dst, const TAB* __restrict__ src
     __syncthreads();
 }
 
-// log|psi| and sign at the team's positions; ok false for a singular matrix.
+// |psi| and sign at the team's positions; ok false for a singular matrix.
 template <class SH, int G>
-__device__ __forceinline__ double team_logpsi(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double x, double y,
-                                              double z, int& sg, bool& ok) {
+__device__ __forceinline__ PsiAbs team_psi(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double x, double y,
+                                           double z, int& sg, bool& ok) {
     using TM = Team<SH, G>;
     double v[TM::NM], w[TM::NM], u0, u1, u2, u3;
 #pragma unroll
@@ -451,10 +467,10 @@ __device__ __forceinline__ double team_logpsi(const Team<SH, G>& T, const TeamTa
     }
 #pragma unroll
     for (int k = 0; k < TM::NM; ++k) v[k] = T.part_sum(v[k]);
-    double pm;
-    int pe;
-    T.template det<false>(v, sh, w, pm, pe, sg, ok);
-    return TM::log_det(pm, pe) + T.jastrow_value(S, x, y, z);
+    PsiAbs a;
+    T.template det<false>(v, sh, w, a.pm, a.pe, sg, ok);
+    a.u = T.jastrow_value(S, x, y, z);
+    return a;
 }
 
 // a[q] of a register array.
@@ -479,7 +495,7 @@ struct TeamOut {
 
 template <class SH, int G, int NR, bool DEL, bool FORCE, class Store>
 __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double* red,
-                                                double x, double y, double z, double& logabs, int& sg, bool& ok,
+                                                double x, double y, double z, PsiAbs& psi, int& sg, bool& ok,
                                                 const TeamOut& out, bool act, Store store) {
     using TM = Team<SH, G>;
     constexpr int NM = TM::NM, NNUC = TM::NNUC, SLOTS = TM::SLOTS;
@@ -514,9 +530,7 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
     }
 #pragma unroll
     for (int k = 0; k < NM; ++k) v[k] = T.part_sum(v[k]);
-    double pm;
-    int pe;
-    T.template det<true>(v, sh, w, pm, pe, sg, ok);
+    T.template det<true>(v, sh, w, psi.pm, psi.pe, sg, ok);
     store(w);
     // grad ln D and lap D / D of the electron from c'_a
     double gx = 0, gy = 0, gz = 0, ld = 0;
@@ -587,7 +601,7 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
         if (out.lap) out.lap[T.e] = lp;
     }
     const double e_l = TM::sum(V - (first ? 0.5 * lp : 0.0)) + S.v_nn;
-    logabs = TM::log_det(pm, pe) + TM::sum(u);
+    psi.u = TM::sum(u);
     // sums over the lanes' rows of red, column by column (a whole warp: half of
     // the rows by lane p and half by lane p + 16)
     auto reduce = [&](int n, double* to, auto map) {
@@ -745,7 +759,8 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
         y = act ? gpos[i + Wcap] : (T.e + 1) * 1.37;
         z = act ? gpos[i + 2 * (size_t)Wcap] : (T.e + 1) * 2.37;
     }
-    double lp = act ? glog[w] : 0.0;
+    PsiAbs cur = PsiAbs::of_log(act ? glog[w] : 0.0);
+    double pm2 = 1.0;                          // cur.pm^2
     int sg = act ? gsign[w] : 1;
     double el = act ? gel[w] : 0.0;
     unsigned acc = 0;
@@ -775,19 +790,20 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
             ny = y + step * (d_u32(r.y) - 0.5);
             nz = z + step * (d_u32(r.z) - 0.5);
         }
-        double ln, en = 0;
+        PsiAbs next;
+        double en = 0;
         int sn;
         bool ok;
         if constexpr (REC)
-            en = team_evaluate<SH, G, 0, false, false>(T, S, sh, nullptr, nx, ny, nz, ln, sn, ok, none, false, nostore);
+            en = team_evaluate<SH, G, 0, false, false>(T, S, sh, nullptr, nx, ny, nz, next, sn, ok, none, false, nostore);
         else
-            ln = team_logpsi(T, S, sh, nx, ny, nz, sn, ok);
+            next = team_psi(T, S, sh, nx, ny, nz, sn, ok);
         const U4 a = rng_draw(seed, (uint32_t)w, st, 0, TAG_ACCEPT);
-        const double prob = d_exp(2.0 * (ln - lp));
-        const int take = act && ok && d_u32(a.x) < prob;
+        const int take = act && ok && below_ratio2(d_u32(a.x), next, cur, pm2);
         if (TM::shfl(take, T.base)) {
             x = nx; y = ny; z = nz;
-            lp = ln;
+            cur = next;
+            pm2 = next.pm * next.pm;
             sg = sn;
             ++acc;
             if (REC) {
@@ -812,10 +828,10 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
         }
     }
     if (!REC && __any_sync(0xffffffffu, acc > 0)) {
-        double ln;
+        PsiAbs again;
         int sn;
         bool ok;
-        const double en = team_evaluate<SH, G, 0, false, false>(T, S, sh, nullptr, x, y, z, ln, sn, ok, none, false, nostore);
+        const double en = team_evaluate<SH, G, 0, false, false>(T, S, sh, nullptr, x, y, z, again, sn, ok, none, false, nostore);
         if (acc) {
             el = en;
             if (!isfinite(el)) flg |= FLAG_NONFINITE;
@@ -829,7 +845,7 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
             gpos[i + 2 * (size_t)Wcap] = z;
         }
         if (T.t == 0) {
-            glog[w] = lp;
+            if (acc) glog[w] = cur.log_abs();
             gsign[w] = sg;
             gel[w] = el;
             if (acc) atomicAdd(acc_out, (unsigned long long)acc);
@@ -868,16 +884,16 @@ __device__ __forceinline__ double team_measure(const Team<SH, G>& T, const TeamT
         for (int k = 0; k < TM::NM; ++k)
             if (k < NS) dinv[((size_t)(T.sig * TM::NM * TM::NM + k * TM::NM + T.q)) * Wcap + w] = d[k];
     };
-    double ln;
+    PsiAbs psi;
     int sg;
     bool ok;
-    const double e = team_evaluate<SH, G, NR, DEL, FORCE>(T, S, sh, red, x, y, z, ln, sg, ok, out, act, store);
+    const double e = team_evaluate<SH, G, NR, DEL, FORCE>(T, S, sh, red, x, y, z, psi, sg, ok, out, act, store);
     if (act && T.t == 0) {
         int fl = 0;
         if (!ok) fl |= FLAG_SINGULAR;
         if (!isfinite(e)) fl |= FLAG_NONFINITE;
         if (fl) atomicOr(flags, fl);
-        if (write_state) { logabs[w] = ln; sign[w] = sg; el[w] = e; }
+        if (write_state) { logabs[w] = psi.log_abs(); sign[w] = sg; el[w] = e; }
     }
     return act ? e : 0.0;
 }
