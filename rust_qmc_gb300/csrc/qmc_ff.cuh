@@ -48,6 +48,15 @@ struct F2 {
     __device__ __forceinline__ explicit F2(float a) : F2(a, a) {}
     __device__ __forceinline__ void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 };
+// Two pairs in a 16-byte word of shared memory.
+__device__ __forceinline__ void load2x2(const void* p, F2& a, F2& b) {
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
+    a.v = t.x;
+    b.v = t.y;
+}
+__device__ __forceinline__ void store2x2(void* p, F2 a, F2 b) {
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a.v, b.v);
+}
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     F2 r;
     asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));

@@ -710,6 +710,12 @@ __device__ __forceinline__ void khw_gauss_walker(const SysH<float>& S, A& a, flo
             };
             propose(0);
             __syncwarp();
+            // the lane's column for the sector's turn: rows 2r, 2r + 1 (re, re') and (im, im')
+            F2 dre[NR], dim[NR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                load2x2(D + r * NC + col, dre[r], dim[r]);
+            }
             for (int q = 0; q < NS; ++q) {
                 const int e = sig * NUP + q;
                 const float4* ph = D + NM + 2 * (q & 1);
@@ -719,12 +725,12 @@ __device__ __forceinline__ void khw_gauss_walker(const SysH<float>& S, A& a, flo
                 float tr = 0, ti = 0;
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
-                    const float4 p = ph[r * NC], d = D[r * NC + col];
-                    const float2 n = *reinterpret_cast<const float2*>(ph + r * NC + 1);
-                    const F2 pr(p.x, p.y), pi(p.z, p.w), np(n.x, n.y), dx(d.x, d.y), dy(d.z, d.w);
+                    F2 pr, pi, np;
+                    load2x2(ph + r * NC, pr, pi);
+                    np.v = *reinterpret_cast<const unsigned long long*>(ph + r * NC + 1);
                     float a0, a1, b0, b1;
-                    fma2(pr, dx, mul2(np, dy)).get(a0, a1);
-                    fma2(pr, dy, mul2(pi, dx)).get(b0, b1);
+                    fma2(pr, dre[r], mul2(np, dim[r])).get(a0, a1);
+                    fma2(pr, dim[r], mul2(pi, dre[r])).get(b0, b1);
                     tr += a0; ti += b0;
                     if (2 * r + 1 < NM) { tr += a1; ti += b1; }
                 }
@@ -751,28 +757,31 @@ __device__ __forceinline__ void khw_gauss_walker(const SysH<float>& S, A& a, flo
                     const float iRr = Rr * iR2, iRi = -Ri * iR2;              // 1/R
                     const float fr = tr * iRr - ti * iRi, fi = tr * iRi + ti * iRr;   // t_l / R
                     if (lane == q) { csr = iRr; csi = iRi; }
-                    const bool store = lane < NM && lane != q;
-                    const F2 f(fi), nfr(-fr), nfi(-fi);
+                    if (lane != q) {
+                        const F2 f(fi), nfr(-fr), nfi(-fi);
 #pragma unroll
-                    for (int r = 0; r < NR; ++r) {
-                        const float4 c = D[r * NC + q];
-                        float4 d = D[r * NC + col];
-                        const F2 qr(c.x, c.y), qi(c.z, c.w);
-                        // d - (qr fr - qi fi) and d - (qr fi + qi fr)
-                        const F2 x = add2(F2(d.x, d.y), fma2(qr, nfr, mul2(qi, f)));
-                        const F2 y = add2(F2(d.z, d.w), fma2(qr, nfi, mul2(qi, nfr)));
-                        x.get(d.x, d.y);
-                        y.get(d.z, d.w);
-                        if (store) D[r * NC + lane] = d;
+                        for (int r = 0; r < NR; ++r) {
+                            F2 qr, qi;
+                            load2x2(D + r * NC + q, qr, qi);
+                            // d - (qr fr - qi fi) and d - (qr fi + qi fr)
+                            dre[r] = add2(dre[r], fma2(qr, nfr, mul2(qi, f)));
+                            dim[r] = add2(dim[r], fma2(qr, nfi, mul2(qi, nfr)));
+                        }
                     }
                     ++acc;
+                }
+                // the next moving electron's column, for the others to read
+                if (lane == q + 1 && lane < NS) {
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) store2x2(D + r * NC + lane, dre[r], dim[r]);
                 }
                 __syncwarp();                          // this proposal's reads before the next one's writes
             }
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                const float4 d = D[r * NC + col];
-                float4 n;
+                float4 d, n;
+                dre[r].get(d.x, d.y);
+                dim[r].get(d.z, d.w);
                 n.x = d.x * csr - d.z * csi; n.z = d.x * csi + d.z * csr;
                 n.y = d.y * csr - d.w * csi; n.w = d.y * csi + d.w * csr;
                 if (lane < NM) D[r * NC + lane] = n;
