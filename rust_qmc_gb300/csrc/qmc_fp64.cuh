@@ -8,11 +8,11 @@
 // by powers of two run on the bits of the value, arguments are reduced with
 // tables, and reciprocals and square roots start from FP32 seeds.
 // Measured cycles per call, one warp (these functions / CUDA's, the latter
-// compiled with the library's flags): exp 503 / 1062, log 731 / 2035,
-// sqrt 446 / 623, sincos of 2 pi u 810 / 1884, 1/x 190 / 383 and 1/sqrt 265 / 511
-// (both sides one Newton step).  Errors against 64 bits: exp, log and sqrt
-// below 1 ulp, sine and cosine below 3e-16 absolute
-// (tests/test_fp64_functions.py).
+// compiled with the library's flags): exp 687 / 1062, log 790 / 2035,
+// sqrt 475 / 623, 1/x 188 / 383 and 1/sqrt 250 / 511 (both sides one Newton
+// step), 1/x to the last bits 288 / 378; a Box-Muller pair 2340.  Errors against
+// 64 bits: exp 0.55 ulp, log 1.54 ulp, sqrt and the full reciprocal 0.5 ulp, sine
+// and cosine 1.7e-16 absolute (tests/test_fp64_functions.py has the bounds).
 // Argument reduction of exp after Tang, ACM TOMS 15 (1989), of log after Tang,
 // ACM TOMS 16 (1990).
 #pragma once
