@@ -329,7 +329,7 @@ def other_configs(ctx, args, fp32_peak, fp64_peak, cpu=True, cpu_seconds=2.0):
                        "value": moves / ((statistics.mean(sw) + statistics.mean(rf)) / 1e3), "unit": UNIT,
                        "sweep_moves_per_s": moves / (statistics.mean(sw) / 1e3), "sweep_ms": statistics.mean(sw),
                        "refresh_ms": statistics.mean(rf), "acceptance": acc,
-                       "roofline": {"bound": "fp32_simt", "kernel": "kw_sweep", "achieved": tf, "peak": fp32_peak,
+                       "roofline": {"bound": "fp32_simt", "kernel": "kw_gauss", "achieved": tf, "peak": fp32_peak,
                                     "unit": "TFLOP/s", "frac": tf / fp32_peak if fp32_peak else None,
                                     "flops_per_move": c["sweep_flops_per_move"]}}
     e_ref = wk.refresh() / W

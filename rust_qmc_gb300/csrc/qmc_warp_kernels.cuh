@@ -1618,8 +1618,8 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
 // where one lane per electron of a sector took two rounds of 21 lanes over all
 // shells; pairs and nucleus terms are evaluated once each and added to per-electron
 // sums; pivots are compared, and |det| is kept, on exponent and high-word bits, with
-// one logarithm a walker.  500 configurations: 641 us before, about 330 us now (the
-// host call 797 us and 484 us).
+// one logarithm a walker.  500 configurations: 641 us before, 321 us now (the host
+// call 797 us and 484 us).
 // ---------------------------------------------------------------------------
 template <int NNUC, int NM>
 struct EvalTab {
@@ -1963,7 +1963,7 @@ __device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, cons
 // together, so that one loop is in use at a time (16 384 walkers: 2.16 ms, 2.69 ms in
 // four-warp blocks that do not wait for each other, 3.15 ms for one sector at a time).
 // The FP32 pipe bounds it, 74 % busy; of the cycles 30 % are orbital values, 25 % the
-// inversion, 29 % derivatives, 16 % pairs and nuclei.  1.94 ms with the derivatives as
+// inversion, 29 % derivatives, 16 % pairs and nuclei.  1.98 ms with the derivatives as
 // (electron pair, third) tasks.
 // ---------------------------------------------------------------------------
 struct PairTabHead {                // sizes and scalars; the arrays follow in the block's shared memory

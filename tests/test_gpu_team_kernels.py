@@ -131,3 +131,21 @@ def test_refresh_and_recorded_steps_across_the_size_rule(ctx, oracle, name, W):
     np.testing.assert_allclose(r["energies"], means, rtol=1e-9, atol=0)
     wk.close()
     sysh.close()
+
+
+@pytest.mark.parametrize("name", ["ch4_gto", "ch4_min"])
+def test_sr_rows_do_not_depend_on_the_batch(ctx, name):
+    """Rows of a batch above the team kernels' size (24 576) against the same
+    configurations in a small batch: two FP64 routes, 1e-9 of the norm each as above."""
+    spec = SPECS[name]()
+    sysh = Q.System(ctx, spec)
+    pos = random_configs(spec, 24577, seed=3)
+    big = sysh.logderiv_batch(pos, el_derivs=True)
+    rows = np.r_[0:40, 24537:24577]
+    small = sysh.logderiv_batch(pos[rows], el_derivs=True)
+    for a, b in zip(big, small):
+        a = np.asarray(a)[rows]
+        for x, y in zip(a, b):
+            _close(x, y, 1e-7)
+        _close(a, b)
+    sysh.close()
