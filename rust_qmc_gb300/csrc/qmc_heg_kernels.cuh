@@ -40,6 +40,10 @@ struct SysH {
     T k2sum;                       // (1/2) sum over occupied |k|^2 of both sectors
     T kvec[2][32][3];              // [sector][column][xyz]
     T k2[2][32];                   // |k|^2 of each
+    // columns by opposite wave vectors: column rep[sig][i] and, unless 255, column
+    // mate[sig][i] with the negated vector
+    int n_rep[2];
+    unsigned char rep[2][32], mate[2][32];
     int nt;                        // octant vectors of the reciprocal sum
     int kmax;                      // their largest component
     float aL, rc2u;                // alpha L and the squared real-space cutoff, in box units
@@ -152,18 +156,31 @@ static bool fill_sysh(const HostSys& hs, int NE, int NUP, SysH<T>& S, KTable& KT
     }
     double k2s = 0.0;
     for (int sig = 0; sig < 2; ++sig) {
-        int col = 0;
+        int col = 0, of[32];                       // orbital of each column
         for (int ei = 0; ei < hs.N; ++ei) {
             int e = hs.perm[ei];
             if ((hs.spins[e] > 0) != (sig == 0)) continue;
             int k = hs.occ[e];
             if (col >= 32) return false;
+            of[col] = k;
             for (int c = 0; c < 3; ++c) S.kvec[sig][col][c] = (T)hs.kvec[3 * k + c];
             const double k2 = hs.kvec[3 * k] * hs.kvec[3 * k] + hs.kvec[3 * k + 1] * hs.kvec[3 * k + 1] +
                               hs.kvec[3 * k + 2] * hs.kvec[3 * k + 2];
             S.k2[sig][col] = (T)k2;
             k2s += k2;
             ++col;
+        }
+        bool taken[32] = {};
+        for (int j = 0; j < col; ++j) {
+            if (taken[j]) continue;
+            const double* k = &hs.kvec[3 * of[j]];
+            int m = j + 1;
+            while (m < col && (taken[m] || hs.kvec[3 * of[m]] != -k[0] || hs.kvec[3 * of[m] + 1] != -k[1] ||
+                               hs.kvec[3 * of[m] + 2] != -k[2]))
+                ++m;
+            S.rep[sig][S.n_rep[sig]] = (unsigned char)j;
+            S.mate[sig][S.n_rep[sig]++] = (unsigned char)(m < col ? m : 255);
+            if (m < col) taken[m] = true;
         }
     }
     S.k2sum = (T)(0.5 * k2s);
@@ -1311,14 +1328,43 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
 #pragma unroll 1
         for (int sig = 0; sig < 2; ++sig) {
             const int NS = NUP == NDN || sig == 0 ? NUP : NDN;
-            const TC kx = S.kvec[sig][lane][0], ky = S.kvec[sig][lane][1], kz = S.kvec[sig][lane][2];
-            for (int q = 0; q < NS; ++q) {
-                TC rx, ry, rz;
-                P.get(sig * NUP + q, rx, ry, rz);
-                TC s, c;
-                fsincos(kx * rx + ky * ry + kz * rz, &s, &c);
-                Mr[q * HRS + lane] = c;
-                Mi[q * HRS + lane] = s;
+            if constexpr (std::is_same<TC, ff>::value) {
+                // opposite wave vectors share a sine and cosine (every step of fsincos
+                // is odd or even in its argument, to the bit): (pair of columns,
+                // electron) tasks over the lanes, 378 of them for an untwisted cell's 27
+                // columns where a lane per column took 27 rounds
+                float* pos = reinterpret_cast<float*>(bc);
+                if (lane < NS) {
+                    const int e = sig * NUP + lane;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) pos[3 * lane + c] = a.pos[(3 * e + c) * (size_t)a.Wcap + w];
+                }
+                __syncwarp();
+                const int nr = S.n_rep[sig];
+#pragma unroll 1
+                for (int t = lane; t < nr * NS; t += 32) {
+                    const int q = t / nr, i = t - q * nr, col = S.rep[sig][i], mate = S.mate[sig][i];
+                    const TC kx = S.kvec[sig][col][0], ky = S.kvec[sig][col][1], kz = S.kvec[sig][col][2];
+                    const TC rx = TC(pos[3 * q]), ry = TC(pos[3 * q + 1]), rz = TC(pos[3 * q + 2]);
+                    TC s, c;
+                    fsincos(kx * rx + ky * ry + kz * rz, &s, &c);
+                    Mr[q * HRS + col] = c;
+                    Mi[q * HRS + col] = s;
+                    if (mate != 255) {
+                        Mr[q * HRS + mate] = c;
+                        Mi[q * HRS + mate] = -s;
+                    }
+                }
+            } else {
+                const TC kx = S.kvec[sig][lane][0], ky = S.kvec[sig][lane][1], kz = S.kvec[sig][lane][2];
+                for (int q = 0; q < NS; ++q) {
+                    TC rx, ry, rz;
+                    P.get(sig * NUP + q, rx, ry, rz);
+                    TC s, c;
+                    fsincos(kx * rx + ky * ry + kz * rz, &s, &c);
+                    Mr[q * HRS + lane] = c;
+                    Mi[q * HRS + lane] = s;
+                }
             }
             __syncwarp();
             // complex Gauss-Jordan in place: lane j carries column j of D and
