@@ -714,11 +714,11 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     // the warp kernels give E_L, a per-walker kernel the Jastrow derivatives;
     // MO-rotation angles would need the determinant and are not compiled.
     // Large batches of the molecules without rotations go the same way, E_L from a
-    // thread per walker.  MethaneGTO, host call: 20 000 configurations 1.73 ms this
-    // way and 1.62 ms by teams, 65 536 4.01 and 5.09 ms.
+    // thread per walker.  MethaneGTO, host call: 9300 configurations 0.79 ms this way
+    // and 0.88 ms by teams, 20 000 1.26 and 1.62 ms, 65 536 3.30 and 5.09 ms.
     const bool benzene = hs.shape == SHAPE_C6H6;
     if (benzene && P != 8) return QMC_ERR_UNSUPPORTED;
-    const bool split = benzene || (P == 8 && W > 24576);
+    const bool split = benzene || (P == 8 && !team_measures(W));
     // device scratch: O [W][P], the SR sums and their block partials, the
     // Jastrow table (jas[8], nuclei [n_nuc][5]), then with dEL: dEL [W][P] and
     // (split form) grad ln|psi| [W][N][3]

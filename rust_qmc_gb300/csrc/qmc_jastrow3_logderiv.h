@@ -1,6 +1,7 @@
 // qmc_jastrow3_logderiv.h -- parameter log-derivatives of the Jastrow3 factor
-// for one configuration, compiled for the device (k_jastrow3_logderiv) and,
-// unchanged, for the host checks of this header.
+// for one configuration, term by term: the sums that the device kernel
+// k_jastrow3_logderiv takes with a warp, in the plain form that the host checks
+// compile.
 //
 // u = sum_{i<j} a_s r_ij / (1 + b_s r_ij) - sum_{i,I} A_t Z_I r_iI / (1 + B_t r_iI)
 // (src/correlation/jastrow.rs:138-449) with a and b per spin class s

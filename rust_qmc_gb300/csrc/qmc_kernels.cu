@@ -6,7 +6,6 @@
 #include <algorithm>
 #include "qmc_internal.h"
 #include "qmc_device.cuh"
-#include "qmc_jastrow3_logderiv.h"
 
 namespace qmc {
 
@@ -308,33 +307,75 @@ int launch_hf_force_walkers(const DevWalkers& dw, int N, int n_nuc, const double
     return cuda_status(cudaGetLastError());
 }
 
-// Jastrow3 parameter log-derivatives, one thread per walker, for the shapes
-// whose evaluation kernels carry no O_p outputs (qmc_jastrow3_logderiv.h):
-// O[w][0..7] with row stride P (skipped when O is null); par = p[8],
-// nuc = [n_nuc][5] (x, y, z, Z, species 0 or 1: the host rejects other
-// species when it builds a system).  With grad ([W][N][3], grad_i ln|psi| in
-// the internal electron order) the Jastrow-parameter derivatives of the
-// local energy go to dEL[w][0..7], same stride.
-template <class TS>
-__global__ void k_jastrow3_logderiv(const TS* __restrict__ pos, int W, int Wcap, int N, int n_up, int n_nuc,
-                                    const double* __restrict__ nuc, const double* __restrict__ par, int P,
-                                    double* __restrict__ O, const double* __restrict__ grad,
-                                    double* __restrict__ dEL) {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= W) return;
-    auto at = [&](int i, int c) { return (double)pos[(size_t)(3 * i + c) * Wcap + w]; };
-    double o[8];
-    if (O) {
-        jastrow3_log_derivatives(N, n_up, n_nuc, nuc, par, at, o);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) O[(size_t)w * P + k] = o[k];
+// Jastrow3 parameter log-derivatives, a warp per walker, for the shapes whose
+// evaluation kernels carry no O_p outputs: O[w][0..7] with row stride P (skipped when
+// O is null); par = p[8], nuc = [n_nuc][5] (x, y, z, Z, species 0 or 1: the host
+// rejects other species when it builds a system).  With grad ([W][N][3],
+// grad_i ln|psi| in the internal electron order) the Jastrow-parameter derivatives of
+// the local energy go to dEL[w][0..7], same stride.  The sums of
+// qmc_jastrow3_logderiv.h, with the common factors of a pair's two parameters taken
+// out.  An FP64 instruction costs the same for 1 and 32 lanes: a thread per walker
+// spent a serial chain of 1365 benzene terms on 19 warps, the lanes of a warp take
+// them 32 at a time: 94 us for 600 walkers (their SR call 0.54 ms after 5.66 ms).
+constexpr int J3_MAX_N = 64;
+template <class TS, int TPB>
+__global__ void __launch_bounds__(TPB) k_jastrow3_logderiv(const TS* __restrict__ pos, int W, int Wcap, int N, int n_up,
+                                                           int n_nuc, const double* __restrict__ nuc,
+                                                           const double* __restrict__ par, int P, double* __restrict__ O,
+                                                           const double* __restrict__ grad, double* __restrict__ dEL) {
+    __shared__ double rs[TPB / 32][3 * J3_MAX_N], gs[TPB / 32][3 * J3_MAX_N], sums[TPB / 32][16][32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, w = blockIdx.x * (TPB / 32) + wib;
+    if (w >= W) return;                               // whole warps only
+    double *r = rs[wib], *g = gs[wib];
+    double(*acc)[32] = sums[wib];                     // O, then dE_L/dp, a column per lane
+    const bool del = grad && dEL;
+    for (int i = lane; i < 3 * N; i += 32) {
+        r[i] = (double)pos[(size_t)i * Wcap + w];
+        g[i] = del ? grad[(size_t)w * N * 3 + i] : 0.0;
     }
-    if (grad && dEL) {
-        const double* g = grad + (size_t)w * N * 3;
-        auto gr = [&](int i, int c) { return g[3 * i + c]; };
-        jastrow3_el_derivatives(N, n_up, n_nuc, nuc, par, at, gr, o);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) dEL[(size_t)w * P + k] = o[k];
+    for (int k = 0; k < 16; ++k) acc[k][lane] = 0.0;
+    __syncwarp();
+    // terms: pairs (p mod N with p mod N + p / N + 1, the last N / 2 pairs of an even N
+    // opposite electrons), then electrons by nuclei
+    const int n_pair = N * (N - 1) / 2, full = N * ((N - 1) / 2), n_term = n_pair + N * n_nuc;
+#pragma unroll 1
+    for (int t = lane; t < n_term; t += 32) {
+        const bool ee = t < n_pair;
+        const int q = ee ? t : t - n_pair;
+        const int i = ee && q >= full ? q - full : q % N;
+        int j = ee ? (q < full ? i + q / N + 1 : i + N / 2) : 0;
+        j = j >= N ? j - N : j;
+        const double* n = nuc + 5 * (ee ? 0 : q / N);
+        const double dx = r[3 * i] - (ee ? r[3 * j] : n[0]), dy = r[3 * i + 1] - (ee ? r[3 * j + 1] : n[1]),
+                     dz = r[3 * i + 2] - (ee ? r[3 * j + 2] : n[2]);
+        // class: spin pair or species; parameters b, a at p[k], p[k + 2]
+        const int k = ee ? ((i < n_up) == (j < n_up) ? 1 : 0) : 4 + (n[4] == 0.0 ? 0 : 1);
+        const double z = ee ? 1.0 : -n[3], b = par[k], a = z * par[k + 2];     // u = a r / (1 + b r)
+        const double d = d_sqrt(dx * dx + dy * dy + dz * dz);
+        const double i1 = d_rcp_full(1.0 + b * d), s = d * i1;
+        acc[k][lane] -= a * s * s;
+        acc[k + 2][lane] += z * s;
+        if (del && !d_below(d, 1e-10)) {
+            // -1/2 sum over the ends of l + 2 f G.dr: two ends with G_i - G_j, or one
+            const double h = (g[3 * i] - (ee ? g[3 * j] : 0.0)) * dx + (g[3 * i + 1] - (ee ? g[3 * j + 1] : 0.0)) * dy +
+                             (g[3 * i + 2] - (ee ? g[3 * j + 2] : 0.0)) * dz;
+            const double i2 = i1 * i1, i3 = i2 * i1, e = ee ? 2.0 : 1.0;
+            acc[8 + k][lane] += a * i3 * (3.0 * e * i1 + 2.0 * h);
+            acc[8 + k + 2][lane] -= z * (i2 * d_rcp_full(d) * (e + h) - e * b * i3);
+        }
+    }
+    __syncwarp();
+    // column sums: half of the lanes' terms by lane k and half by lane k + 16
+    const int k = lane & 15, from = lane & 16;
+    double v = 0.0;
+#pragma unroll
+    for (int l = 0; l < 16; ++l) v += acc[k][from + ((l + k) & 15)];
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    if (lane < 8) {
+        if (O) O[(size_t)w * P + k] = v;
+    } else if (lane < 16 && del) {
+        dEL[(size_t)w * P + k - 8] = v;
     }
 }
 
@@ -342,15 +383,15 @@ int launch_jastrow3_logderiv(const DevWalkers& dw, int N, int n_up, int n_nuc, c
                              const double* d_par, int P, double* d_O, cudaStream_t st, const double* d_grad,
                              double* d_dEL) {
     if (dw.W <= 0) return 0;
-    if (P < 8) return 1;
-    const int tpb = 128;
-    const int nb = (dw.W + tpb - 1) / tpb;
+    if (P < 8 || N > J3_MAX_N) return 1;
+    constexpr int TPB = 128;
+    const int nb = (dw.W + TPB / 32 - 1) / (TPB / 32);
     if (dw.prec == 0)
-        k_jastrow3_logderiv<double><<<nb, tpb, 0, st>>>((const double*)dw.pos, dw.W, dw.Wcap, N, n_up, n_nuc, d_nuc,
-                                                        d_par, P, d_O, d_grad, d_dEL);
+        k_jastrow3_logderiv<double, TPB><<<nb, TPB, 0, st>>>((const double*)dw.pos, dw.W, dw.Wcap, N, n_up, n_nuc, d_nuc,
+                                                             d_par, P, d_O, d_grad, d_dEL);
     else
-        k_jastrow3_logderiv<float><<<nb, tpb, 0, st>>>((const float*)dw.pos, dw.W, dw.Wcap, N, n_up, n_nuc, d_nuc,
-                                                       d_par, P, d_O, d_grad, d_dEL);
+        k_jastrow3_logderiv<float, TPB><<<nb, TPB, 0, st>>>((const float*)dw.pos, dw.W, dw.Wcap, N, n_up, n_nuc, d_nuc,
+                                                            d_par, P, d_O, d_grad, d_dEL);
     ++g_launch_count;
     return cuda_status(cudaGetLastError());
 }

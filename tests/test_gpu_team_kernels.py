@@ -135,13 +135,13 @@ def test_refresh_and_recorded_steps_across_the_size_rule(ctx, oracle, name, W):
 
 @pytest.mark.parametrize("name", ["ch4_gto", "ch4_min"])
 def test_sr_rows_do_not_depend_on_the_batch(ctx, name):
-    """Rows of a batch above the team kernels' size (24 576) against the same
+    """Rows of a batch above the team kernels' size (9216) against the same
     configurations in a small batch: two FP64 routes, 1e-9 of the norm each as above."""
     spec = SPECS[name]()
     sysh = Q.System(ctx, spec)
-    pos = random_configs(spec, 24577, seed=3)
+    pos = random_configs(spec, 9217, seed=3)
     big = sysh.logderiv_batch(pos, el_derivs=True)
-    rows = np.r_[0:40, 24537:24577]
+    rows = np.r_[0:40, 9177:9217]
     small = sysh.logderiv_batch(pos[rows], el_derivs=True)
     for a, b in zip(big, small):
         a = np.asarray(a)[rows]

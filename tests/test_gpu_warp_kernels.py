@@ -202,3 +202,25 @@ def test_sr_sums(ctx, W):
     np.testing.assert_allclose(f, f2 - E.mean() * Om, rtol=0, atol=1e-12 * np.abs(E).max() * np.abs(O).max())
     assert abs(em - E.mean()) <= 1e-12 * np.abs(E).max()
     sysh.close()
+
+
+@pytest.mark.parametrize("W", [1, 3, 5])
+def test_benzene_sr_rows(ctx, oracle, W):
+    """A warp per configuration, partial blocks of four: O_p against the oracle, dE_L/dp
+    against differences of E_L (step 1e-4 of a parameter: 1e-5 of the largest)."""
+    spec = Q.benzene_gto(2.0, 3.0)
+    sysh = Q.System(ctx, spec)
+    pos = random_configs(spec, W, seed=40 + W)
+    O, E, dE = sysh.logderiv_batch(pos, el_derivs=True)
+    _close(O, oracle.log_derivatives(spec, pos))
+    p, h = sysh.get_params(), 1e-4
+    for k in range(len(p)):
+        e = []
+        for s in (h, -h):
+            q = p.copy()
+            q[k] += s
+            sysh.set_params(q)
+            e.append(sysh.eval_batch(pos)["e_local"])
+        want = (e[0] - e[1]) / (2 * h)
+        assert np.max(np.abs(dE[:, k] - want)) <= 1e-5 * max(1.0, np.max(np.abs(dE)))
+    sysh.close()
