@@ -18,7 +18,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--use_fast_math", "-Xcompiler", "-fPIC",
               "-I" + os.path.join(ROOT, "include")]
 CU_SOURCES = ["qmc_kernels.cu", "qmc_shape_h2.cu", "qmc_shape_li.cu", "qmc_shape_ch4_measure.cu",
-              "qmc_shape_ch4_sweep.cu", "qmc_shape_ch4_allstep.cu", "qmc_shape_ch4min_measure.cu",
+              "qmc_shape_ch4_sweep.cu", "qmc_shape_ch4_split.cu", "qmc_shape_ch4_allstep.cu", "qmc_shape_ch4min_measure.cu",
               "qmc_shape_ch4min_sweep.cu", "qmc_shape_c6h6.cu", "qmc_shape_heg.cu",
               "qmc_shape_ch4_batch.cu", "qmc_shape_ch4min_batch.cu", "qmc_shape_c6h6_batch.cu",
               "qmc_shape_heg_batch.cu", "qmc_noalloc.cu"]

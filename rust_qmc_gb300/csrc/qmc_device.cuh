@@ -33,6 +33,17 @@ struct LayoutCH4Min {
     __host__ __device__ static constexpr int ao0(int s) { return s < 2 ? s : s + 3; }
 };
 
+// The layout of a 6-31G CH4 (MethaneGTO): carbon 6 (s), 3 and 1 (sp), each hydrogen 3
+// and 1 (s).
+struct LayoutCH4Split {
+    static constexpr int NSHELL = 11;
+    __host__ __device__ static constexpr int nuc(int s) { return s < 3 ? 0 : (s - 1) / 2; }
+    __host__ __device__ static constexpr int np(int s) { return s == 0 ? 6 : (s == 1 || (s > 2 && s % 2 == 1) ? 3 : 1); }
+    __host__ __device__ static constexpr int kind(int s) { return s == 1 || s == 2 ? 2 : 1; }
+    __host__ __device__ static constexpr int p0(int s) { return s == 0 ? 0 : p0(s - 1) + np(s - 1); }
+    __host__ __device__ static constexpr int ao0(int s) { return s == 0 ? 0 : ao0(s - 1) + (kind(s - 1) == 2 ? 4 : 1); }
+};
+
 template <int NE_, int NUP_, int NNUC_, int NSH_, int NAO_, int NPRIM_, int BASIS_, int JAS_, int NROT_,
           class LAYOUT_ = void>
 struct ShapeT {
@@ -49,6 +60,8 @@ using ShapeH2 = ShapeT<2, 1, 2, 2, 2, 2, BASIS_STO, JAS_PADE_F, 1>;
 using ShapeLi = ShapeT<3, 2, 1, 1, 2, 8, BASIS_STO, JAS_PADE_F, 1>;
 // CH4 (src/systems/methane.rs:600-776): up to 17 Gaussian AOs, 5 up + 5 down.
 using ShapeCH4 = ShapeT<10, 5, 5, 12, 17, 28, BASIS_GTO, JAS_PADE_EEN, 4>;
+// The same with the 6-31G layout fixed at compile time, for the FP32 Gaussian sweeps.
+using ShapeCH4Split = ShapeT<10, 5, 5, 12, 17, 28, BASIS_GTO, JAS_PADE_EEN, 4, LayoutCH4Split>;
 // The 9-function CH4 workload with its basis layout fixed at compile time.
 using ShapeCH4Min = ShapeT<10, 5, 5, 6, 9, 18, BASIS_GTO, JAS_PADE_EEN, 4, LayoutCH4Min>;
 
