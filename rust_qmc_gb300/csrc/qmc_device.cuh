@@ -44,6 +44,13 @@ struct LayoutCH4Split {
     __host__ __device__ static constexpr int ao0(int s) { return s == 0 ? 0 : ao0(s - 1) + (kind(s - 1) == 2 ? 4 : 1); }
 };
 
+// One nucleus with one Slater-type shell of seven primitives for two s AOs (the Li
+// atom), r^pow e^{-zeta r}.
+struct LayoutSto7 {
+    static constexpr int NSHELL = 1, NPRIM = 7;
+    __host__ __device__ static constexpr int pow(int p) { return p < 2 ? 1 : (p < 6 ? 2 : 3); }
+};
+
 template <int NE_, int NUP_, int NNUC_, int NSH_, int NAO_, int NPRIM_, int BASIS_, int JAS_, int NROT_,
           class LAYOUT_ = void>
 struct ShapeT {
@@ -58,6 +65,8 @@ struct ShapeT {
 using ShapeH2 = ShapeT<2, 1, 2, 2, 2, 2, BASIS_STO, JAS_PADE_F, 1>;
 // Li atom (src/systems/lithium.rs, src/main.rs:37-48): STO-7G 1s/2s, 2 up + 1 down.
 using ShapeLi = ShapeT<3, 2, 1, 1, 2, 8, BASIS_STO, JAS_PADE_F, 1>;
+// The same with its shell fixed at compile time, for the FP32 Gaussian sweeps.
+using ShapeLiSto7 = ShapeT<3, 2, 1, 1, 2, 8, BASIS_STO, JAS_PADE_F, 1, LayoutSto7>;
 // CH4 (src/systems/methane.rs:600-776): up to 17 Gaussian AOs, 5 up + 5 down.
 using ShapeCH4 = ShapeT<10, 5, 5, 12, 17, 28, BASIS_GTO, JAS_PADE_EEN, 4>;
 // The same with the 6-31G layout fixed at compile time, for the FP32 Gaussian sweeps.
@@ -253,7 +262,25 @@ struct MOEval {
     __device__ __forceinline__ void run(const SysT<SH, T>& S, T x, T y, T z) {
 #pragma unroll
         for (int k = 0; k < SH::NMAX; ++k) { v[k] = 0; gx[k] = 0; gy[k] = 0; gz[k] = 0; l[k] = 0; }
-        if constexpr (!std::is_void<typename SH::Layout>::value) {
+        constexpr bool sto7 = std::is_same<typename SH::Layout, LayoutSto7>::value;
+        if constexpr (sto7 && MODE == 0) {
+            // run_tables' operations, the primitives and their powers unrolled
+            using LY = LayoutSto7;
+            const T dx = x - S.nuc[0][0], dy = y - S.nuc[0][1], dz = z - S.nuc[0][2];
+            const T d = fsqrt(dx * dx + dy * dy + dz * dz);
+            T v0 = 0, v1 = 0;
+#pragma unroll
+            for (int p = 0; p < LY::NPRIM; ++p) {
+                T dn = 1;
+#pragma unroll
+                for (int t = 0; t < LY::pow(p); ++t) dn *= d;
+                const T val = dn * fexp(-S.pexp[p] * d);
+                v0 += S.cs0[p] * val;
+                v1 += S.cs1[p] * val;
+            }
+            add(S, 0, v0, T(0), T(0), T(0), T(0));
+            add(S, 1, v1, T(0), T(0), T(0), T(0));
+        } else if constexpr (!sto7 && !std::is_void<typename SH::Layout>::value) {
             using LY = typename SH::Layout;
 #pragma unroll
             for (int sh = 0; sh < LY::NSHELL; ++sh) {

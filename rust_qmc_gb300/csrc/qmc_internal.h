@@ -117,6 +117,8 @@ size_t refresh_rows_bytes(int shape);
 int dinv_elems_of_shape(int shape);
 // True when the system's shells match the compile-time 9-function CH4 layout.
 bool layout_matches_ch4min(const HostSys& hs);
+int shape_sweep_gauss_li_sto7(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, uint64_t seed,
+                              cudaStream_t st);
 int shape_sweep_gauss_ch4_split(const HostSys& hs, DevWalkers& dw, int n, uint64_t s0, double step, uint64_t seed,
                                 cudaStream_t st);
 

@@ -77,6 +77,15 @@ static bool layout_matches(const HostSys& hs, int n_ao) {
     return true;
 }
 bool layout_matches_ch4min(const HostSys& hs) { return layout_matches<LayoutCH4Min>(hs, 9); }
+static bool layout_matches_sto7(const HostSys& hs) {
+    using LY = LayoutSto7;
+    if (hs.shells.size() != 1 || hs.n_ao != 2 || hs.shells[0].exps.size() != LY::NPRIM) return false;
+    const HostShell& h = hs.shells[0];
+    if (h.s_ao[0] < 0 || h.s_ao[1] < 0 || h.p_ao[0] >= 0 || hs.ao_int[h.s_ao[0]] != 0 || hs.ao_int[h.s_ao[1]] != 1) return false;
+    for (int p = 0; p < LY::NPRIM; ++p)
+        if (h.pows.empty() || h.pows[p] != LY::pow(p)) return false;
+    return true;
+}
 
 #define QMC_SHAPE_SWITCH(shape, CALL)                  \
     switch (shape) {                                   \
@@ -130,6 +139,8 @@ int launch_sweep(const HostSys& hs, DevWalkers& dw, int move_kind, int n_sweeps,
     // 1024 walkers 0.42 ms against 1.19, 65 536 walkers 1.51 against 2.71).
     if (hs.shape == SHAPE_CH4 && dw.prec == 1 && move_kind == MOVE_ONE_GAUSS && layout_matches<LayoutCH4Split>(hs, 17))
         return shape_sweep_gauss_ch4_split(hs, dw, n_sweeps, step0, step, seed, st);
+    if (hs.shape == SHAPE_LI && dw.prec == 1 && move_kind == MOVE_ONE_GAUSS && layout_matches_sto7(hs))
+        return shape_sweep_gauss_li_sto7(hs, dw, n_sweeps, step0, step, seed, st);
 #define C_(n) shape_sweep_one_##n(hs, dw, move_kind, n_sweeps, step0, step, tau, max_drift, seed, st)
     QMC_SHAPE_SWITCH(hs.shape, C_)
 #undef C_
