@@ -1613,20 +1613,23 @@ __device__ __forceinline__ double kw_measure_walker(const SysW<TC>& S, TC* Mrow,
 // ---------------------------------------------------------------------------
 // FP64 evaluation and refresh, one warp per walker.  An FP64 instruction holds its
 // sub-partition for 64 cycles however many of its lanes are active, so the work is
-// laid out to fill lanes: the orbital values and the derivative sums are (electron,
-// third of the shells) tasks in rounds of 32, 126 tasks for benzene's 42 electrons,
-// where one lane per electron of a sector took two rounds of 21 lanes over all
-// shells; pairs and nucleus terms are evaluated once each and added to per-electron
-// sums; pivots are compared, and |det| is kept, on exponent and high-word bits, with
-// one logarithm a walker.  500 configurations: 641 us before, 321 us now (the host
-// call 797 us and 484 us).
+// laid out to fill lanes, where one lane per electron of a sector left 11 of 32 idle:
+// radial parts are (electron, shell) tasks, orbital values (electron, third of the
+// columns), derivative sums (electron, third of the shells); pairs and nucleus terms
+// are evaluated once each and added to per-electron sums; pivots are compared, and
+// |det| is kept, on the bits, with one logarithm a walker.  Orbital matrices and
+// inverses keep the rounding of a lane per electron with the CUDA library's
+// exponential, so that configurations next to a node, which amplify it, keep their
+// values (largest change over 30 000 configurations 4e-13).  500 configurations
+// through the host call: 797 us before, 521 us now (484 us with d_exp and the values
+// summed in thirds, which moved such configurations by up to 1e-8).
 // ---------------------------------------------------------------------------
 template <int NNUC, int NM>
 struct EvalTab {
-    int n_ao, n_third, quirk_lap, pad;
+    int n_ao, n_sh, n_third, quirk_lap;
     double qa, v_nn, a_ee[2], b_ee[2];
     double nuc[NNUC][6];                      // x, y, z, Z, enA, enB
-    int third[WMAX_THIRD];
+    int sh[WMAX_AO], third[WMAX_THIRD];       // shells in AO order; the same in thirds
     // exponent; c, c a, c a^2 of the s or lone p part; the same of an sp shell's p part
     alignas(16) double prim[WMAX_PRIM][8];
     double C[WMAX_AO][2][NM + 1];             // [AO][sector][column], rows of whole 16-byte words
@@ -1642,6 +1645,8 @@ static void fill_evaltab(const SysW<double>& w, EvalTab<NNUC, NM>& S) {
     std::memset(static_cast<void*>(&S), 0, sizeof(S));
     const ShellList<double> L(w);
     S.n_ao = w.n_ao;
+    S.n_sh = (int)L.desc.size();
+    for (int g = 0; g < S.n_sh; ++g) S.sh[g] = L.desc[g];
     S.n_third = deal_thirds(L.desc, S.third);
     S.quirk_lap = w.quirk_lap;
     S.qa = w.qa;
@@ -1662,11 +1667,13 @@ static void fill_evaltab(const SysW<double>& w, EvalTab<NNUC, NM>& S) {
 
 // Shared doubles of a warp: row e of the electron's orbital values, then of its column
 // of the inverse, later positions [3][NE] and sums [5][NE] over the same storage; then
-// the derivative sums [4][NE].
+// the derivative sums [4][NE]; then radial parts [EVAL_SH][2][NM] of a sector's
+// electrons (six shells: 126 tasks, four rounds of lanes).
+constexpr int EVAL_SH = 6;
 template <int NE, int NM>
 __host__ __device__ constexpr int eval_rows() { return (NE * NM > 8 * NE ? NE * NM : 8 * NE) + (NE * NM) % 2; }
 template <int NE, int NM>
-__host__ __device__ constexpr int eval_scratch() { return eval_rows<NE, NM>() + 4 * NE; }
+__host__ __device__ constexpr int eval_scratch() { return eval_rows<NE, NM>() + 4 * NE + 2 * NM * EVAL_SH; }
 
 template <int NE, int NUP, int NNUC, class TAB>
 __device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, const double* __restrict__ gpos,
@@ -1686,46 +1693,79 @@ __device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, cons
         return 32 * round + lane < 3 * NE;
     };
     auto coord = [&](int e, int c) { return gpos[(size_t)(3 * e + c) * Wcap + w]; };
-    // orbital values, row e of the electron's matrix
+    // Orbital values, row e of the electron's matrix, in the plain order of operations
+    // (the sum over a shell's primitives, then the sum over the AOs as they come):
+    // next to a node their rounding is what the inverse amplifies, so another order
+    // would be another, equally good, value there.  The radial parts are (electron,
+    // shell) tasks, the contraction (electron, third of the columns) tasks.
+    static_assert(NM % 3 == 0 && 3 * NM <= 64, "columns in thirds, two tasks a lane");
+    constexpr int NC = NM / 3;
+    double* rad = der + 4 * NE;
 #pragma unroll 1
-    for (int round = 0; round < ROUNDS; ++round) {
-        int e, t3;
-        const bool on = task_of(round, e, t3);
-        const int sig = e >= NUP;
-        const double x = coord(e, 0), y = coord(e, 1), z = coord(e, 2);
-        double v[NM];
+    for (int sig = 0; sig < 2; ++sig) {
+        double v[2][NC];                       // the lane's tasks `lane` and `lane + 32`
 #pragma unroll
-        for (int k = 0; k < NM; ++k) v[k] = 0;
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < NC; ++k) v[h][k] = 0;
 #pragma unroll 1
-        for (int g = 0; g < S.n_third; ++g) {
-            const int d = S.third[3 * g + t3];
-            const int I = shell_nuc(d), np = shell_np(d), p0 = shell_p0(d), a0 = shell_a0(d);
-            const int ns = (d & SHELL_S) ? 1 : 0, na = ns + ((d & SHELL_P) ? 3 : 0);
-            const bool sp = na == 4;
-            const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            double s0 = 0, s1 = 0;
-            for (int p = p0; p < p0 + np; ++p) {
-                const double ex = d_exp(-S.prim[p][0] * r2);
-                s0 += S.prim[p][1] * ex;
-                if (sp) s1 += S.prim[p][4] * ex;
+        for (int g0 = 0; g0 < S.n_sh; g0 += EVAL_SH) {
+            const int ng = min(EVAL_SH, S.n_sh - g0);
+#pragma unroll 1
+            for (int t = lane; t < NM * ng; t += 32) {
+                const int g = t / NM, q = t - g * NM, e = sig * NUP + q, d = S.sh[g0 + g];
+                const int I = shell_nuc(d), np = shell_np(d), p0 = shell_p0(d);
+                const bool sp = (d & SHELL_S) && (d & SHELL_P);
+                const double dx = coord(e, 0) - S.nuc[I][0], dy = coord(e, 1) - S.nuc[I][1], dz = coord(e, 2) - S.nuc[I][2];
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                double s0 = 0, s1 = 0;
+                for (int p = p0; p < p0 + np; ++p) {
+                    const double ex = exp(-S.prim[p][0] * r2);
+                    s0 += S.prim[p][1] * ex;
+                    if (sp) s1 += S.prim[p][4] * ex;
+                }
+                rad[2 * g * NM + q] = s0;
+                rad[(2 * g + 1) * NM + q] = sp ? s1 : s0;
             }
-            if (!sp) s1 = s0;
-#pragma unroll 1
-            for (int m = 0; m < na; ++m) {
-                const int c3 = m - ns;
-                const double chi = c3 < 0 ? s0 : (c3 == 0 ? dx : (c3 == 1 ? dy : dz)) * s1;
-                const double* c = S.C[a0 + m][sig];
+            __syncwarp();
 #pragma unroll
-                for (int k = 0; k < NM; ++k) v[k] += c[k] * chi;
+            for (int h = 0; h < 2; ++h) {
+                const int t = min(lane + 32 * h, 3 * NM - 1), third = t / NM, q = t - third * NM, e = sig * NUP + q;
+                const double x = coord(e, 0), y = coord(e, 1), z = coord(e, 2);
+#pragma unroll 1
+                for (int g = 0; g < ng; ++g) {
+                    const int d = S.sh[g0 + g], I = shell_nuc(d);
+                    const double s0 = rad[2 * g * NM + q], s1 = rad[(2 * g + 1) * NM + q];
+                    const double* c = &S.C[shell_a0(d)][sig][third * NC];
+                    constexpr int row = 2 * (NM + 1);
+                    if (d & SHELL_S) {
+#pragma unroll
+                        for (int k = 0; k < NC; ++k) v[h][k] += c[k] * s0;
+                        c += row;
+                    }
+                    if (d & SHELL_P) {
+                        const double cx = (x - S.nuc[I][0]) * s1, cy = (y - S.nuc[I][1]) * s1, cz = (z - S.nuc[I][2]) * s1;
+#pragma unroll
+                        for (int k = 0; k < NC; ++k) v[h][k] += c[k] * cx;
+#pragma unroll
+                        for (int k = 0; k < NC; ++k) v[h][k] += c[row + k] * cy;
+#pragma unroll
+                        for (int k = 0; k < NC; ++k) v[h][k] += c[2 * row + k] * cz;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int t = lane + 32 * h, third = t / NM, q = t - third * NM;
+            if (t < 3 * NM) {
+#pragma unroll
+                for (int k = 0; k < NC; ++k) scr[(sig * NUP + q) * NM + third * NC + k] = v[h][k];
             }
         }
-        if (on) {
-#pragma unroll
-            for (int k = 0; k < NM; ++k) scr[e * NM + k] = t3 == 0 ? v[k] : scr[e * NM + k] + v[k];
-        }
-        __syncwarp();
     }
+    __syncwarp();
     // Gauss-Jordan of each sector (kw_measure_walker's steps), lane j with column j
     double det = 1.0, logdet = 0.0;            // |det| = det 2^ex exp(logdet)
     int ex = 0, sg = 1;
@@ -1740,10 +1780,15 @@ __device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, cons
         int src = lane;
 #pragma unroll 1
         for (int k = 0; k < NM; ++k) {
-            int p = 0, best = d_hi(A[0]) & 0x7fffffff;
+            // magnitudes to 24 bits, on the bits (a conversion is an FP64 instruction)
+            auto mag = [](double a) {
+                return (((unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull) + 0x10000000ull) >> 29;
+            };
+            int p = 0;
+            unsigned long long best = mag(A[0]);
 #pragma unroll
             for (int r = 1; r < NM; ++r) {
-                const int m = d_hi(A[r]) & 0x7fffffff;
+                const unsigned long long m = mag(A[r]);
                 if (r < NM - k && m > best) { best = m; p = r; }
             }
             p = wshfl(p, k);
@@ -1767,7 +1812,7 @@ __device__ __forceinline__ double kw_eval_walker(const TAB& S, double* scr, cons
                 det *= __hiloint2double((h & 0x000fffff) | 0x3ff00000, d_lo(piv));
                 ex += f - 1023;
             }
-            const double ip = d_rcp_full(piv);
+            const double ip = 1.0 / piv;
             const double t = lane == k ? 1.0 + ip : A[0] * ip, first = lane == k ? ip : t;
 #pragma unroll
             for (int i = 1; i < NM; ++i) A[i - 1] = A[i] - wshfl(A[i], k) * t;
