@@ -36,6 +36,7 @@ struct TeamTab {
     double pown[NPT];                      // Slater-type powers
     int powi[NPT];
     int ao[SH::NAO];                       // nucleus | type << 4 | primitives << 8 | first primitive << 16
+    int ord[SH::NAO];                      // position here of the AOs in shell order
     int term[NTERM > 0 ? NTERM : 1];       // Jastrow value terms: i | partner << 8 | class << 16 | nucleus flag << 24
     int species[SH::NNUC];
     int rot_col[SH::NROT][2];
@@ -105,6 +106,7 @@ static bool fill_team(const HostSys& hs, TeamTab<SH>& S) {
     const std::vector<double> Ce = hs.effective_mo(), dC = hs.rotation_derivative_rows();
     for (int a = 0; a < hs.n_ao; ++a) {
         S.ao[a] = aos[a].packed;
+        S.ord[hs.ao_int[aos[a].caller]] = a;
         int col[2] = {0, 0};
         for (int ei = 0; ei < hs.N; ++ei) {
             const int e = hs.perm[ei], sig = hs.spins[e] > 0 ? 0 : 1;
@@ -132,8 +134,8 @@ static bool fill_team(const HostSys& hs, TeamTab<SH>& S) {
 }
 
 // AO a at (x, y, z): value and, with MODE >= 1 / 2, gradient / Laplacian; zero
-// unless ok.
-template <class SH, int MODE>
+// unless ok.  LIB: the CUDA library's exponential (see team_evaluate).
+template <class SH, int MODE, bool LIB = false>
 __device__ __forceinline__ void team_ao(const TeamTab<SH>& S, int a, bool ok, double x, double y, double z, double& v,
                                         double& gx, double& gy, double& gz, double& l) {
     const int d = S.ao[ok ? a : 0];
@@ -144,7 +146,7 @@ __device__ __forceinline__ void team_ao(const TeamTab<SH>& S, int a, bool ok, do
     if constexpr (SH::BASIS == BASIS_GTO) {
         for (int p = p0; p < p0 + np; ++p) {
             const double2 pr = S.prim[p];
-            const double f = pr.y * d_exp(-pr.x * r2);
+            const double f = pr.y * (LIB ? exp(-pr.x * r2) : d_exp(-pr.x * r2));
             s0 += f;
             if (MODE >= 1) {
                 const double fa = pr.x * f;
@@ -255,20 +257,21 @@ struct Team {
     }
 
     // AO of this lane's slot at (x, y, z) (zero past the basis).
-    template <bool DER>
+    template <bool DER, bool LIB = false>
     __device__ __forceinline__ void ao(const Tab& S, int slot, double x, double y, double z, double& v, double& gx,
                                        double& gy, double& gz, double& l) const {
         const int a = slot * PARTS + part;
-        team_ao<SH, DER ? 2 : 0>(S, a, on && a < S.n_ao, x, y, z, v, gx, gy, gz, l);
+        team_ao<SH, DER ? 2 : 0, LIB>(S, a, on && a < S.n_ao, x, y, z, v, gx, gy, gz, l);
     }
 
     // Determinants of both sectors from the electrons' orbital rows v (part 0's),
     // by elimination with partial pivoting on lane-columns; with INV in place, so
-    // that w[k] = D^-1[k][q] of the lane's electron.  |det| = pm 2^pe.
-    template <bool INV>
+    // that w[k] = D^-1[k][q] of the lane's electron.  |det| = pm 2^pe.  READY: the rows
+    // are in sh already (and pivots are inverted by a division).
+    template <bool INV, bool READY = false>
     __device__ __forceinline__ void det(const double (&v)[NM], double* sh, double (&w)[NM], double& pm, int& pe,
                                         int& sg, bool& ok) const {
-        if (on && part == 0) {
+        if (!READY && on && part == 0) {
 #pragma unroll
             for (int k = 0; k < NM; ++k) sh[e * NM + k] = v[k];
         }
@@ -312,7 +315,7 @@ struct Team {
                 m = d_scale(m, 1023 - be);
             }
             if (INV || k + 1 < NM) {
-                const double ip = d_rcp_full(piv);
+                const double ip = READY ? 1.0 / piv : d_rcp_full(piv);
                 if (INV) {
                     const bool own = q == k;
                     const double x = own ? ip : w[k] * ip;
@@ -483,7 +486,12 @@ __device__ __forceinline__ double pick(const double (&a)[N], int q) {
 }
 
 // Full evaluation.  NR: MO-rotation rows, DEL: with dE_L/dp, FORCE: with forces;
-// `red` is the team's [32][RED] reduction scratch of those.
+// `red` is the team's [32][RED] reduction scratch of those.  LIB (Gaussian bases; `chi`
+// is the team's [NE][NAO] scratch): the orbital matrix with the CUDA library's
+// exponential and every element's sum in AO order by one lane, and pivots inverted by
+// a division -- the rounding of a thread per walker.  Configurations next to a node
+// amplify the matrix's rounding: over 60 sets of 5000 CH4 configurations another order
+// moved SR rows by 7e-12 of their norm in the median and 6.5e-9 at worst.
 struct TeamOut {
     double* grad;                          // [N][3] of this walker, or null
     double* lap;
@@ -493,8 +501,8 @@ struct TeamOut {
     double* omega;
 };
 
-template <class SH, int G, int NR, bool DEL, bool FORCE, class Store>
-__device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double* red,
+template <class SH, int G, int NR, bool DEL, bool FORCE, bool LIB, class Store>
+__device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double* red, double* chis,
                                                 double x, double y, double z, PsiAbs& psi, int& sg, bool& ok,
                                                 const TeamOut& out, bool act, Store store) {
     using TM = Team<SH, G>;
@@ -518,19 +526,41 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) {
         double chi;
-        T.template ao<true>(S, s, x, y, z, chi, ax[s], ay[s], az[s], al[s]);
+        T.template ao<true, LIB>(S, s, x, y, z, chi, ax[s], ay[s], az[s], al[s]);
         const int a = min(s * TM::PARTS + T.part, SH::NAO - 1);
+        if constexpr (LIB) {
+            if (T.on && s * TM::PARTS + T.part < S.n_ao) chis[T.e * SH::NAO + a] = chi;
+        } else {
 #pragma unroll
-        for (int k = 0; k < NM; ++k) v[k] += S.C[T.sig][a][k] * chi;
+            for (int k = 0; k < NM; ++k) v[k] += S.C[T.sig][a][k] * chi;
+        }
         if (NR > 0) {
 #pragma unroll
             for (int q = 0; q < NR; ++q)
                 if (q < S.n_rot) dv[q] += S.dC[q][a] * chi;
         }
     }
+    if constexpr (LIB) {
+        __syncwarp();
+        constexpr int KP = (NM + TM::PARTS - 1) / TM::PARTS;        // columns part, part + PARTS, ... of the row
+        double vk[KP];
 #pragma unroll
-    for (int k = 0; k < NM; ++k) v[k] = T.part_sum(v[k]);
-    T.template det<true>(v, sh, w, psi.pm, psi.pe, sg, ok);
+        for (int i = 0; i < KP; ++i) vk[i] = 0;
+#pragma unroll 1
+        for (int i = 0; i < S.n_ao; ++i) {
+            const int a = S.ord[i];
+            const double chi = chis[T.e * SH::NAO + a];
+#pragma unroll
+            for (int c = 0; c < KP; ++c) vk[c] += S.C[T.sig][a][min(T.part + TM::PARTS * c, NM - 1)] * chi;
+        }
+#pragma unroll
+        for (int c = 0; c < KP; ++c)
+            if (T.on && T.part + TM::PARTS * c < NM) sh[T.e * NM + T.part + TM::PARTS * c] = vk[c];
+    } else {
+#pragma unroll
+        for (int k = 0; k < NM; ++k) v[k] = T.part_sum(v[k]);
+    }
+    T.template det<true, LIB>(v, sh, w, psi.pm, psi.pe, sg, ok);
     store(w);
     // grad ln D and lap D / D of the electron from c'_a
     double gx = 0, gy = 0, gz = 0, ld = 0;
@@ -795,7 +825,7 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
         int sn;
         bool ok;
         if constexpr (REC)
-            en = team_evaluate<SH, G, 0, false, false>(T, S, sh, nullptr, nx, ny, nz, next, sn, ok, none, false, nostore);
+            en = team_evaluate<SH, G, 0, false, false, false>(T, S, sh, nullptr, nullptr, nx, ny, nz, next, sn, ok, none, false, nostore);
         else
             next = team_psi(T, S, sh, nx, ny, nz, sn, ok);
         const U4 a = rng_draw(seed, (uint32_t)w, st, 0, TAG_ACCEPT);
@@ -831,7 +861,7 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
         PsiAbs again;
         int sn;
         bool ok;
-        const double en = team_evaluate<SH, G, 0, false, false>(T, S, sh, nullptr, x, y, z, again, sn, ok, none, false, nostore);
+        const double en = team_evaluate<SH, G, 0, false, false, false>(T, S, sh, nullptr, nullptr, x, y, z, again, sn, ok, none, false, nostore);
         if (acc) {
             el = en;
             if (!isfinite(el)) flg |= FLAG_NONFINITE;
@@ -858,9 +888,18 @@ __global__ void __launch_bounds__(TPB) k_team_steps(const TeamTab<SH>* __restric
 template <class SH, int G, int NR, bool FORCE>
 __host__ __device__ constexpr int team_red() { return NR > 0 ? G * (8 + NR) : (FORCE ? G * 3 * SH::NNUC : 1); }
 
+// Whether an evaluation keeps a thread per walker's rounding (team_evaluate): SR rows,
+// whose derivatives amplify it most (5000 configurations 461 us through the host call,
+// 440 us without).  Forces would pay more (531 and 434 us) for less: 60 sets moved by
+// 3e-12 in the median and 4e-10 at worst.
+template <class SH, int NR>
+__host__ __device__ constexpr bool team_lib() { return SH::BASIS == BASIS_GTO && NR > 0; }
+template <class SH, int NR>
+__host__ __device__ constexpr int team_chi() { return team_lib<SH, NR>() ? SH::NE * SH::NAO : 1; }
+
 // Refresh or evaluation of walker w by its team; E_L (0 for an idle team).
 template <class SH, int G, int NR, bool DEL, bool FORCE>
-__device__ __forceinline__ double team_measure(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double* red,
+__device__ __forceinline__ double team_measure(const Team<SH, G>& T, const TeamTab<SH>& S, double* sh, double* red, double* chis,
                                                const double* __restrict__ pos, double* __restrict__ dinv,
                                                double* __restrict__ logabs, int* __restrict__ sign,
                                                double* __restrict__ el, int w, bool act, int Wcap, int write_state,
@@ -887,7 +926,7 @@ __device__ __forceinline__ double team_measure(const Team<SH, G>& T, const TeamT
     PsiAbs psi;
     int sg;
     bool ok;
-    const double e = team_evaluate<SH, G, NR, DEL, FORCE>(T, S, sh, red, x, y, z, psi, sg, ok, out, act, store);
+    const double e = team_evaluate<SH, G, NR, DEL, FORCE, team_lib<SH, NR>()>(T, S, sh, red, chis, x, y, z, psi, sg, ok, out, act, store);
     if (act && T.t == 0) {
         int fl = 0;
         if (!ok) fl |= FLAG_SINGULAR;
@@ -909,10 +948,11 @@ __global__ void __launch_bounds__(TPB) k_team_measure(const TeamTab<SH>* __restr
     __shared__ TeamTab<SH> S;
     __shared__ double rows[NT][TM::ROWS];
     __shared__ double red[NT][team_red<SH, G, NR, FORCE>()];
+    __shared__ double chis[NT][team_chi<SH, NR>()];
     stage_team(&S, tab);
     const TM T;
     const int tm = threadIdx.x / G, w = blockIdx.x * NT + tm;
-    const double e = team_measure<SH, G, NR, DEL, FORCE>(T, S, rows[tm], red[tm], pos, dinv, logabs, sign, el, w, w < W,
+    const double e = team_measure<SH, G, NR, DEL, FORCE>(T, S, rows[tm], red[tm], chis[tm], pos, dinv, logabs, sign, el, w, w < W,
                                                          Wcap, write_state, out, P, flags);
     if (partial) team_block_partial<G, TPB>(e, partial, blockIdx.x);
 }
@@ -937,7 +977,7 @@ __global__ void __launch_bounds__(TPB) kb_team_measure(const BatchTile* __restri
     const MeasureOut none{};
     for (int i = tm; i < TW; i += NT) {
         const int w = tl.w0 + i;
-        const double e = team_measure<SH, G, 0, false, false>(T, S, rows[tm], nullptr, (const double*)R.pos,
+        const double e = team_measure<SH, G, 0, false, false>(T, S, rows[tm], nullptr, nullptr, (const double*)R.pos,
                                                               (double*)R.dinv, R.logabs, R.sign, R.el, w, w < R.W,
                                                               R.Wcap, 1, none, 0, R.flags);
         if (T.t == 0) es[i] = e;
