@@ -116,9 +116,8 @@ __device__ __forceinline__ double flog(double x) { return d_log(x); }
 __device__ __forceinline__ float flog(float x) { return __logf(x); }
 __device__ __forceinline__ double fsqrt(double x) { return d_sqrt(x); }
 __device__ __forceinline__ float fsqrt(float x) { return sqrtf(x); }
-// Reciprocal (and frsqrt below) of a positive double within single-precision
-// range: FP32 seed and one Newton-Raphson step, which squares the seed's
-// ~2^-22 relative error to ~1e-14.
+// Reciprocal (and frsqrt below) of a double: FP32 seed and one Newton-Raphson
+// step, which squares the seed's ~2^-22 relative error to ~1e-14.
 __device__ __forceinline__ double frcp(double x) { return d_rcp(x); }
 __device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
 // 2^x by the PTX approximate base-2 exponential (flush-to-zero).

@@ -44,18 +44,26 @@ __device__ __forceinline__ double d_scale(double x, int k) { return __hiloint2do
 __device__ __forceinline__ bool d_below(double x, double c) { return d_hi(x) < d_hi(c); }
 __device__ __forceinline__ bool d_positive(double x) { return d_hi(x) > 0; }
 
-// 1/x for positive x in FP32's normal range: FP32 seed and one Newton step,
-// relative error ~1e-14.
+// 1/x for normal x of either sign below 2^1022 (zero, subnormal and larger x, inf and
+// NaN give NaN): FP32 seed on the mantissa and one Newton step, relative error ~1e-14.
+// Sign and exponent are put back on the bits, which costs no FP64 instruction.
 __device__ __forceinline__ double d_rcp(double x) {
-    const double y = d_of_float(__fdividef(1.0f, float_of_pos(x)));
-    const double e = fma(-x, y, 1.0);
-    return fma(e, y, y);
+    const int hi = d_hi(x), ex = (hi >> 20) & 0x7ff;
+    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, d_lo(x));
+    const double y = d_of_float(__fdividef(1.0f, float_of_pos(m)));
+    const double e = fma(-m, y, 1.0);
+    const double r = fma(e, y, y);
+    const int rh = (d_hi(r) - ((ex - 1023) << 20)) ^ (hi & 0x80000000);
+    return __hiloint2double((unsigned)(ex - 1) < 2044u ? rh : 0x7ff80000, d_lo(r));
 }
-// 1/sqrt(x), the same way: y + (y/2)(1 - x y^2).
+// 1/sqrt(x) for positive normal x, the same way on x 4^-k in [1/2, 2): y + (y/2)(1 - x y^2).
 __device__ __forceinline__ double d_rsqrt(double x) {
-    const double y = d_of_float(rsqrtf(float_of_pos(x)));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(d_scale(y, -1), e, y);
+    const int hi = d_hi(x), k = (hi >> 21) - 511;
+    const double m = __hiloint2double(hi - (k << 21), d_lo(x));
+    const double y = d_of_float(rsqrtf(float_of_pos(m)));
+    const double e = fma(-m * y, y, 1.0);
+    const double r = fma(d_scale(y, -1), e, y);
+    return __hiloint2double((unsigned)(hi - 0x00100000) < 0x7fe00000u ? d_hi(r) - (k << 20) : 0x7ff80000, d_lo(r));
 }
 
 // 1/x to the last bit or two, any normal x: seed on the mantissa, two Newton

@@ -1,0 +1,58 @@
+"""The FP64 elementary functions of csrc/qmc_fp64.cuh outside the arguments of
+test_fp64_functions.py: negative numbers, the whole exponent range, zero,
+infinities and NaN.  The header is compiled for the host with that test's
+device intrinsics.  Bounds as there: one Newton step on a seed of relative error
+2^-22 leaves less than 2e-13."""
+import subprocess
+
+import pytest
+
+from tests.test_fp64_functions import CSRC, SHIM
+
+MAIN = r"""
+static bool isn(double x) { return x != x; }
+int main() {
+    std::mt19937_64 g(11);
+    auto U = [&](double a, double b) { return a + (b - a) * ((g() >> 11) * 0x1p-53); };
+    auto mx = [](double& m, double v) { if (!(v <= m)) m = v; };
+    const double inf = INFINITY, nan = NAN;
+    double e_rcp = 0, e_rsq = 0;
+    for (int i = 0; i < 400000; ++i) {
+        seed_err = U(-1, 1) * 0x1p-22;
+        const double x = (i & 1 ? -1 : 1) * std::ldexp(U(1, 2), (int)U(i % 3 ? -8 : -1021, i % 3 ? 8 : 1022));
+        mx(e_rcp, std::fabs((double)((ld)d_rcp(x) * (ld)x - 1)));
+        const double y = std::ldexp(U(1, 2), (int)U(-1021, 1023));
+        mx(e_rsq, std::fabs((double)((ld)d_rsqrt(y) * sqrtl((ld)y) - 1)));
+    }
+    seed_err = 0;
+    const bool special = isn(d_rcp(0.0)) && isn(d_rcp(-0.0)) && isn(d_rcp(inf)) && isn(d_rcp(-inf)) && isn(d_rcp(nan)) &&
+                         isn(d_rcp(1e-310)) && isn(d_rsqrt(0.0)) && isn(d_rsqrt(-2.0)) && isn(d_rsqrt(inf)) &&
+                         isn(d_rsqrt(nan)) && isn(d_rsqrt(1e-310)) && d_rcp(-2.0) == -0.5 && d_rsqrt(0x1p-400) == 0x1p200;
+    std::printf("%g %g %d\n", e_rcp, e_rsq, (int)special);
+    return 0;
+}
+"""
+
+
+def run_host(tmp, main):
+    """Output of `main` compiled with the functions under test."""
+    (tmp / "cuda_runtime.h").write_text("")
+    (tmp / "t.cpp").write_text(SHIM.split("int main")[0] + main)
+    exe = str(tmp / "t")
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-std=c++17", "-I", str(tmp), "-I", CSRC, str(tmp / "t.cpp"), "-o", exe],
+                   check=True)
+    return [float(v) for v in subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()]
+
+
+@pytest.fixture(scope="module")
+def one_step(tmp_path_factory):
+    return run_host(tmp_path_factory.mktemp("domains"), MAIN)
+
+
+@pytest.mark.parametrize("k, name", [(0, "reciprocal"), (1, "reciprocal square root")])
+def test_one_newton_step_over_all_exponents(one_step, k, name):
+    assert one_step[k] <= 2e-13, (name, one_step[k])
+
+
+def test_one_newton_step_special_values(one_step):
+    assert one_step[2] == 1
