@@ -66,10 +66,12 @@ __device__ __forceinline__ double d_rsqrt(double x) {
     return __hiloint2double((unsigned)(hi - 0x00100000) < 0x7fe00000u ? d_hi(r) - (k << 20) : 0x7ff80000, d_lo(r));
 }
 
-// 1/x to the last bit or two, any normal x: seed on the mantissa, two Newton
-// steps in one (y (1 + e + e^2)).
+// 1/x to the last bit or two: seed on the mantissa, two Newton steps in one
+// (y (1 + e + e^2)); arguments whose reciprocal is not a normal number, or that are
+// none themselves, are divided.
 __device__ __forceinline__ double d_rcp_full(double x) {
     const int hi = d_hi(x), ex = ((hi >> 20) & 0x7ff) - 1023;
+    if ((unsigned)(ex + 1022) >= 2044u) return 1.0 / x;               // zero, subnormal, from 2^1022 on, inf, NaN
     const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, d_lo(x));
     double y = d_of_float(__fdividef(1.0f, float_of_pos(m)));
     const double e = fma(-m, y, 1.0);

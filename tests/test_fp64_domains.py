@@ -56,3 +56,38 @@ def test_one_newton_step_over_all_exponents(one_step, k, name):
 
 def test_one_newton_step_special_values(one_step):
     assert one_step[2] == 1
+
+
+FULL = r"""
+int main() {
+    std::mt19937_64 g(13);
+    auto U = [&](double a, double b) { return a + (b - a) * ((g() >> 11) * 0x1p-53); };
+    double worst = 0;
+    const double inf = INFINITY, nan = NAN;
+    const double xs[] = {0.0, -0.0, inf, -inf, 5e-324, -1e-310, 0x1.8p1022, -0x1p1023, 0x1.fffffffffffffp1023, 0x1p-1022, 0x1p1021};
+    bool special = d_rcp_full(nan) != d_rcp_full(nan);
+    for (double x : xs) special = special && (std::isinf(1 / x) ? d_rcp_full(x) == 1 / x : std::fabs(d_rcp_full(x) - 1 / x) <= 2 * ulp(1 / x) || d_rcp_full(x) == 1 / x);
+    for (int i = 0; i < 200000; ++i) {
+        seed_err = U(-1, 1) * 0x1p-22;
+        const double x = (i & 1 ? -1 : 1) * std::ldexp(U(1, 2), (int)U(-1022, 1022));
+        const double e = std::fabs((double)((ld)d_rcp_full(x) - 1 / (ld)x)) / ulp(1 / x);
+        if (!(e <= worst)) worst = e;
+    }
+    std::printf("%g %d\n", worst, (int)special);
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def full(tmp_path_factory):
+    return run_host(tmp_path_factory.mktemp("full"), FULL)
+
+
+def test_full_reciprocal_over_all_exponents(full):
+    assert full[0] <= 2.0
+
+
+def test_full_reciprocal_special_values(full):
+    """Zero, subnormal numbers, the largest exponents, infinities and NaN as a division gives them."""
+    assert full[1] == 1
