@@ -97,7 +97,8 @@ __device__ __forceinline__ double d_sqrt(double x) {
 
 // e^x: x = (256 k + j) ln2/256 + r, |r| < 1.4e-3; e^x = 2^k 2^(j/256) e^r with
 // e^r through r^4 and the r^3 coefficient raised by 0.87 max|r|^2 / 120, which
-// leaves an eighth of the r^5 term (5e-18).  Results below 2^-1021 are returned as 0, above 2^1023 as inf.
+// leaves an eighth of the r^5 term (5e-18).  From |x| = 708 on the result is scaled in
+// two steps, so that it may be subnormal, 0 or inf.
 __device__ __forceinline__ double d_exp(double x) {
     const int hi = d_hi(x), mag = hi & 0x7fffffff;
     const bool out = mag >= 0x40862000;                               // |x| >= 708, inf, NaN
@@ -113,8 +114,10 @@ __device__ __forceinline__ double d_exp(double x) {
     double p = fma(r, 1.0 / 24.0, 1.0 / 6.0 + 1.3288e-8);
     p = fma(r, p, 0.5);
     const double s = fma(r * r, p, r);
-    const double v = d_scale(t.x + fma(t.x, s, t.y), n >> 8);
-    if (!out) return v;
+    const double v = t.x + fma(t.x, s, t.y);
+    if (!out) return d_scale(v, n >> 8);
+    if (mag < 0x40880000)                                             // |x| < 768
+        return d_scale(v, (n >> 8) + (hi < 0 ? 128 : -128)) * __hiloint2double(hi < 0 ? (1023 - 128) << 20 : (1023 + 128) << 20, 0);
     return mag > 0x7ff00000 ? x : (hi < 0 ? 0.0 : __hiloint2double(0x7ff00000, 0));
 }
 

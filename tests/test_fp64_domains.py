@@ -91,3 +91,35 @@ def test_full_reciprocal_over_all_exponents(full):
 def test_full_reciprocal_special_values(full):
     """Zero, subnormal numbers, the largest exponents, infinities and NaN as a division gives them."""
     assert full[1] == 1
+
+
+EXP = r"""
+int main() {
+    std::mt19937_64 g(17);
+    auto U = [&](double a, double b) { return a + (b - a) * ((g() >> 11) * 0x1p-53); };
+    double hi = 0, lo = 0;
+    auto mx = [](double& m, double v) { if (!(v <= m)) m = v; };
+    for (int i = 0; i < 100000; ++i) {
+        const double x = U(700.0, 709.78), y = U(-745.13, -700.0);
+        mx(hi, std::fabs((double)((ld)d_exp(x) - expl((ld)x))) / ulp(std::exp(x)));
+        const double want = std::exp(y);
+        mx(lo, std::fabs((double)((ld)d_exp(y) - expl((ld)y))) / std::fmax(want >= 0x1p-1022 ? ulp(want) : 0, 0x1p-1074));
+    }
+    const bool ends = std::isinf(d_exp(709.79)) && std::isinf(d_exp(767.9)) && std::isinf(d_exp(768.0)) && std::isinf(d_exp(1e300)) &&
+                      d_exp(-745.2) == 0 && d_exp(-767.9) == 0 && d_exp(-768.0) == 0 && d_exp(-1e300) == 0;
+    std::printf("%g %g %d\n", hi, lo, (int)ends);
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def ends_of_exp(tmp_path_factory):
+    return run_host(tmp_path_factory.mktemp("exp"), EXP)
+
+
+def test_exp_at_the_ends_of_its_range(ends_of_exp):
+    """Up to the largest double and down to the smallest subnormal one (2 ulp; a
+    subnormal result is rounded once more, in units of 2^-1074)."""
+    assert ends_of_exp[0] <= 2.0 and ends_of_exp[1] <= 2.0
+    assert ends_of_exp[2] == 1
