@@ -6,7 +6,10 @@ mpmath at 40 digits and rounded to doubles (printed as hexadecimal literals):
               that the leading bits of z select; 1/c_i is the rounded
               reciprocal of the interval's midpoint and log c_i is
               -log of that rounded value, so z (1/c_i) - 1 and log c_i belong
-              together; the two intervals that meet at 1 have c_i = 1
+              together; the two intervals that meet at 1 have c_i = 1; log c_i
+              is rounded to a multiple of 2^-42, as is kLn2Hi, so that
+              k kLn2Hi + log c_i is exact
+  kLogLo[i]   what that rounding of log c_i leaves; kLn2Lo the same of ln 2
   kSinCosT[j] (cos, sin) of 2 pi j / 256, j = 0..63
 
 Run: python gen_fp64_tables.py > qmc_fp64_tables.cuh"""
@@ -17,6 +20,11 @@ mp.mp.dps = 40
 
 def hexd(v):
     return float(v).hex()
+
+
+def grid(v):
+    """v to a multiple of 2^-42."""
+    return mp.nint(v * 2 ** 42) / 2 ** 42
 
 
 def log_rows():
@@ -51,7 +59,9 @@ if __name__ == "__main__":
     print("namespace qmc {")
     powers = [mp.mpf(2) ** (mp.mpf(j) / 256) for j in range(256)]
     table("double2", "kExp2T", ["{%s, %s}" % (hexd(v), hexd(v - mp.mpf(float(v)))) for v in powers], 2)
-    table("double2", "kLogT", ["{%s, %s}" % (hexd(a), hexd(b)) for a, b in log_rows()], 2)
+    table("double2", "kLogT", ["{%s, %s}" % (hexd(a), hexd(grid(b))) for a, b in log_rows()], 2)
+    table("double", "kLogLo", [hexd(b - grid(b)) for _, b in log_rows()], 4)
+    print("constexpr double kLn2Hi = %s, kLn2Lo = %s;" % (hexd(grid(mp.log(2))), hexd(mp.log(2) - grid(mp.log(2)))))
     table("double2", "kSinCosT", ["{%s, %s}" % (hexd(mp.cos(2 * mp.pi * j / 256)), hexd(mp.sin(2 * mp.pi * j / 256)))
                                   for j in range(64)], 2)
     print("}  // namespace qmc")

@@ -8,11 +8,12 @@
 // by powers of two run on the bits of the value, arguments are reduced with
 // tables, and reciprocals and square roots start from FP32 seeds.
 // Measured cycles per call, one warp (these functions / CUDA's, the latter
-// compiled with the library's flags): exp 687 / 1062, log 790 / 2035,
-// sqrt 475 / 623, 1/x 188 / 383 and 1/sqrt 250 / 511 (both sides one Newton
-// step), 1/x to the last bits 288 / 378; a Box-Muller pair 2340.  Errors against
-// 64 bits: exp 0.55 ulp, log 1.54 ulp, sqrt and the full reciprocal 0.5 ulp, sine
-// and cosine 1.7e-16 absolute (tests/test_fp64_functions.py has the bounds).
+// compiled with the library's flags): exp 709 / 1062, log 907 / 2035,
+// sqrt 476 / 623, 1/x 225 / 383 and 1/sqrt 291 / 511 (both sides one Newton
+// step), 1/x to the last bits 289 / 378; a Box-Muller pair 2466.  Errors against
+// 64 bits: exp 0.55 ulp, log 0.9 ulp, sqrt and the full reciprocal 0.5 ulp, sine
+// and cosine 1.7e-16 absolute (tests/test_fp64_functions.py and
+// tests/test_fp64_domains.py have the bounds).
 // Argument reduction of exp after Tang, ACM TOMS 15 (1989), of log after Tang,
 // ACM TOMS 16 (1990).
 #pragma once
@@ -123,13 +124,17 @@ __device__ __forceinline__ double d_exp(double x) {
 
 // log x: x = 2^k z with z in [0.6875, 1.375), log x = k ln2 + log c + log(1 + r)
 // with r = z (1/c) - 1, |r| <= 2^-7 next to 1 (where c = 1 keeps the result
-// relatively exact) and below 4e-3 elsewhere.
+// relatively exact) and below 4e-3 elsewhere.  k ln2 + log c is exact in its leading
+// parts (multiples of 2^-42); what these leave goes with the polynomial.  The interval
+// bounds (z from 0x3fe60000 of the high word, seven more bits) are those of the
+// logarithm in ARM's optimized-routines.
 __device__ __forceinline__ double d_log(double x) {
     const int hi = d_hi(x);
     if ((unsigned)(hi - 0x00100000) >= 0x7fe00000u) return log(x);    // zero, subnormal, negative, inf, NaN
     const int tmp = hi - 0x3fe60000, k = tmp >> 20;
     const double z = __hiloint2double(hi - (tmp & 0xfff00000), d_lo(x));
-    const double2 c = kLogT[(tmp >> 13) & 127];
+    const int i = (tmp >> 13) & 127;
+    const double2 c = kLogT[i];
     const double r = fma(z, c.x, -1.0);
     double p = fma(r, -1.0 / 8.0, 1.0 / 7.0);
     p = fma(r, p, -1.0 / 6.0);
@@ -137,7 +142,8 @@ __device__ __forceinline__ double d_log(double x) {
     p = fma(r, p, -1.0 / 4.0);
     p = fma(r, p, 1.0 / 3.0);
     p = fma(r, p, -0.5);
-    return fma(d_of_float((float)k), 0.6931471805599453, c.y) + fma(r * r, p, r);
+    const double kd = d_of_float((float)k);
+    return fma(kd, kLn2Hi, c.y) + (r + fma(r * r, p, fma(kd, kLn2Lo, kLogLo[i])));
 }
 
 // (sin, cos) of 2 pi (j + rem scale) with integer j / 256 of a turn and the odd

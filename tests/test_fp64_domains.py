@@ -123,3 +123,26 @@ def test_exp_at_the_ends_of_its_range(ends_of_exp):
     subnormal result is rounded once more, in units of 2^-1074)."""
     assert ends_of_exp[0] <= 2.0 and ends_of_exp[1] <= 2.0
     assert ends_of_exp[2] == 1
+
+
+LOG = r"""
+int main() {
+    std::mt19937_64 g(19);
+    auto U = [&](double a, double b) { return a + (b - a) * ((g() >> 11) * 0x1p-53); };
+    double worst = 0;
+    for (int i = 0; i < 1000000; ++i) {
+        const double y = i % 4 == 0 ? U(0.6, 1.5) : (i % 4 == 1 ? std::ldexp(U(1, 2), (int)U(-1000, 1000)) : (i % 4 == 2 ? U(0.0, 1.0) : 1.0 + U(-1, 1) * 0x1p-6));
+        const ld l = logl((ld)y);
+        const double e = std::fabs((double)((ld)d_log(y) - l)) / ulp((double)l);
+        if (!(e <= worst)) worst = e;
+    }
+    std::printf("%g\n", worst);
+    return 0;
+}
+"""
+
+
+def test_logarithm_is_as_exact_as_the_librarys(tmp_path):
+    """1 ulp, the documented bound of CUDA's log."""
+    err, = run_host(tmp_path, LOG)
+    assert err <= 1.0, err
