@@ -412,13 +412,15 @@ __device__ __forceinline__ void heg_u(const SysH<T>& S, T r, T a, T& u, T& du, T
 }
 
 // Refresh pair geometry: minimum image of xi - xj.  FP32 walkers' positions are
-// floats (the low parts are zero), so the difference is one exact TwoSum.
+// floats (the low parts are zero), so the difference is one exact TwoSum.  Positions
+// need not lie in the box: n L is a two-product for any n.
 template <class T>
 __device__ __forceinline__ T pair_image(T a, T b, const SysH<T>& S) { return min_img(a - b, S); }
 __device__ __forceinline__ ff pair_image(ff a, ff b, const SysH<ff>& S) {
     const ff d = ff_two_sum(a.hi, -b.hi);
     const float n = rintf(__fmul_rn(d.hi, S.invL.hi));
-    return d + ff(__fmul_rn(-n, S.L.hi), __fmul_rn(-n, S.L.lo));
+    const float p = __fmul_rn(-n, S.L.hi);
+    return d + ff_fast_two_sum(p, __fmaf_rn(-n, S.L.lo, __fmaf_rn(-n, S.L.hi, -p)));
 }
 
 // Squared length; the float-float form sums the exact squares lazily.
