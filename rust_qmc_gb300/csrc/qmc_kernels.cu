@@ -217,10 +217,12 @@ __global__ void k_flush(uint4* buf, size_t n, unsigned v) {
 int launch_sr_sums(const double* E, const double* O, int W, int P, double* d_out, double* d_scratch,
                    int scratch_cap, cudaStream_t st) {
     int M = 2 + 2 * P + P * (P + 1) / 2;
-    int nblk = sr_blocks(W);
+    // a smaller scratch takes longer chunks, up to 256 walkers
+    const int room = scratch_cap / (2 * M);
+    if (room < std::min(1024, (W + 255) / 256)) return 8;
+    int nblk = std::min(sr_blocks(W), room);
     int chunk = (W + nblk - 1) / nblk;
     nblk = (W + chunk - 1) / chunk;
-    if ((size_t)2 * M * nblk > (size_t)scratch_cap) return 8;
     int tpb = ((M + 31) / 32) * 32;
     if (tpb > 1024) return 1;
     k_sr_partials<<<nblk, tpb, 0, st>>>(E, O, W, P, M, chunk, d_scratch, nblk);

@@ -53,7 +53,8 @@ extern "C" int qmc_sr_sums_noalloc(const double* d_E, const double* d_O, int W, 
                      QMC_NOALLOC_MAX_PARAMS);
         return QMC_ERR_ARG;
     }
-    // Same blocking as launch_sr_sums: ceil(W/256) chunks, at most 1024.
+    // launch_sr_sums needs a chunk per 256 walkers, at most 1024 (it takes shorter
+    // chunks where the scratch has room for them).
     long long M = 2 + 2LL * P + (long long)P * (P + 1) / 2;
     long long nblk = (W + 255) / 256;
     if (nblk > 1024) nblk = 1024;
