@@ -206,11 +206,16 @@ struct PsiAbs {
         return {1.0, fma(-(double)pe, 0.6931471805599453, l), pe};
     }
 };
-// Whether uniform ua is below |a|^2 / |b|^2 (bm2 = b.pm^2).
+// Whether uniform ua is below |a|^2 / |b|^2 (bm2 = b.pm^2).  A power of two or an
+// exponential out of range by itself (a kept |psi| has its Jastrow exponent in pe, a new
+// one in u) is joined with the other factor first.
 __device__ __forceinline__ bool below_ratio2(double ua, const PsiAbs& a, const PsiAbs& b, double bm2) {
-    const double e = d_exp(2.0 * (a.u - b.u));
-    const int k = max(-900, min(900, 2 * (a.pe - b.pe)));     // 2^-900 is below every uniform
-    return ua * bm2 < a.pm * a.pm * __hiloint2double((1023 + k) << 20, 0) * e;
+    const double t = 2.0 * (a.u - b.u);
+    const int k = 2 * (a.pe - b.pe);
+    // (two calls: one with joined arguments took 6.48 ms for 20-walker CH4 sampling, 6.34 so)
+    if ((unsigned)(k + 900) <= 1800u && (d_hi(t) & 0x7fffffff) < 0x40860000)         // |t| < 704
+        return ua * bm2 < a.pm * a.pm * __hiloint2double((1023 + k) << 20, 0) * d_exp(t);
+    return ua * bm2 < a.pm * a.pm * d_exp(fma((double)k, 0.6931471805599453, t));
 }
 
 // Lanes of a walker (team) and the pieces of an evaluation.
