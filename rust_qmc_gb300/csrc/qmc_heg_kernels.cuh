@@ -434,6 +434,12 @@ __device__ __forceinline__ ff length2(ff x, ff y, ff z) {
     return ff_norm(r);
 }
 
+// Reciprocal of a pair term: to the last bits in FP64 (one Newton step is 1e-14 off, the
+// same way in each of the 1431 pairs: log|psi| was 1.3e-12 off in the median, 5e-14 now).
+__device__ __forceinline__ float pair_rcp(float a) { return frcp(a); }
+__device__ __forceinline__ ff pair_rcp(ff a) { return frcp(a); }
+__device__ __forceinline__ double pair_rcp(double a) { return d_rcp_full(a); }
+
 // Pair function of the refresh: u, u'(r)/r and u'' + 2u'/r of heg_u inside its
 // cutoff, from r, r^2 and 1/r, with one reciprocal for the RPA form.
 template <class T>
@@ -445,7 +451,7 @@ __device__ __forceinline__ void heg_pair(const SysH<T>& S, T r, T r2, T ri, T a,
         return;
     }
     const T cr = S.pc * r, cr2 = S.pc * r2, q = T(1) - cr2;
-    const T inv = frcp(T(1) + S.pb * r + cr2);
+    const T inv = pair_rcp(T(1) + S.pb * r + cr2);
     const T ai = a * inv, ai2 = ai * inv;
     u = ai * r;
     f = ai2 * q * ri;
@@ -1508,7 +1514,7 @@ __device__ __forceinline__ double khw_measure_walker(const SysH<TC>& S, A& a, TC
                 const TC r2 = length2(dx, dy, dz);
                 const TC r = fsqrt(r2);
                 const bool apart = on && r > TC(1e-10);
-                const TC ri = apart ? frcp(r) : TC(0);
+                const TC ri = apart ? pair_rcp(r) : TC(0);
                 TC uu, f, l;
                 heg_pair(S, r, r2, ri, S.a_ee[((j < NUP) == (i < NUP)) ? 1 : 0], uu, f, l);
                 if (on) u += uu;
