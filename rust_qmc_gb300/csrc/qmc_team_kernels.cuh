@@ -605,7 +605,9 @@ __device__ __forceinline__ double team_evaluate(const Team<SH, G>& T, const Team
         if (FORCE) {
             // Jastrow part of d ln|psi| / dR_I
             if (use && !near && !el && SH::JAS == JAS_PADE_EEN) {
-                const double f = S.enA[I] * ri * inv * inv;
+                // (full precision: ri and inv are one Newton step, 1e-14 each)
+                const double r = d_sqrt(dx * dx + dy * dy + dz * dz), den = 1.0 + S.enB[I] * r;
+                const double f = S.enA[I] * d_rcp_full(r * den * den);
                 mine[3 * I] += f * dx; mine[3 * I + 1] += f * dy; mine[3 * I + 2] += f * dz;
             }
         }
