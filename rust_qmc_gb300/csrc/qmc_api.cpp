@@ -714,8 +714,8 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     // the warp kernels give E_L, a per-walker kernel the Jastrow derivatives;
     // MO-rotation angles would need the determinant and are not compiled.
     // Large batches of the molecules without rotations go the same way, E_L from a
-    // thread per walker.  MethaneGTO, host call: 9300 configurations 0.79 ms this way
-    // and 0.88 ms by teams, 20 000 1.26 and 1.62 ms, 65 536 3.30 and 5.09 ms.
+    // thread per walker.  MethaneGTO, host call: 9300 configurations 0.85 ms this way
+    // and 1.02 ms by teams, 20 000 1.37 and 1.62 ms, 65 536 3.60 and 5.09 ms.
     const bool benzene = hs.shape == SHAPE_C6H6;
     if (benzene && P != 8) return QMC_ERR_UNSUPPORTED;
     const bool split = benzene || (P == 8 && !team_measures(W));
@@ -739,6 +739,7 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     if (split) CU(cudaMemcpyAsync(d_tab, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice, st));
     MeasureOut mo;
     mo.grad = d_grad;
+    mo.lib = split;
     if (split) {
         CK(launch_measure(hs, wk->dw, 0, true, mo, st));          // FP64 refresh: E_L (and grad) on the device
         if (launch_jastrow3_logderiv(wk->dw, hs.N, hs.n_up, hs.n_nuc, d_tab + 8, d_tab, P, wk->d_out, st, d_grad,

@@ -223,15 +223,18 @@ __device__ __forceinline__ MoveDraw<T> draw_of(const MoveDraw<T>& d, int q) {
 // 91-145 for Slater-type radial functions).
 // ---------------------------------------------------------------------------
 // Gaussian primitive p at squared distance r2: exp(-alpha r^2); FP32 uses
-// the pre-scaled exponent and one base-2 exponential.
-template <class SH, class T>
-__device__ __forceinline__ T gauss_prim(const SysT<SH, T>& S, int p, T r2) { return fexp(-S.pexp[p] * r2); }
-template <class SH>
+// the pre-scaled exponent and one base-2 exponential, LIB the CUDA library's.
+template <bool LIB = false, class SH, class T>
+__device__ __forceinline__ T gauss_prim(const SysT<SH, T>& S, int p, T r2) {
+    if constexpr (LIB) return exp(-S.pexp[p] * r2);
+    else return fexp(-S.pexp[p] * r2);
+}
+template <bool LIB = false, class SH>
 __device__ __forceinline__ float gauss_prim(const SysT<SH, float>& S, int p, float r2) {
     return ex2_approx(S.pexp2[p] * r2);
 }
 
-template <class SH, class T, int SIG, int MODE>
+template <class SH, class T, int SIG, int MODE, bool LIB = false>
 struct MOEval {
     static constexpr int NS = SIG == 0 ? SH::NUP : SH::NDN;
     T v[SH::NMAX], gx[SH::NMAX], gy[SH::NMAX], gz[SH::NMAX], l[SH::NMAX];
@@ -291,7 +294,7 @@ struct MOEval {
 #pragma unroll
                 for (int p = p0; p < p0 + LY::np(sh); ++p) {
                     T al = S.pexp[p];
-                    T e = gauss_prim(S, p, r2);
+                    T e = gauss_prim<LIB>(S, p, r2);
                     T e0 = S.cs0[p] * e;
                     a0 += e0;
                     if (MODE >= 1) b0 += al * e0;
@@ -322,7 +325,7 @@ struct MOEval {
                     T a0 = 0, a1 = 0, ap = 0, b0 = 0, b1 = 0, bp = 0, c0 = 0, c1 = 0, cpp = 0;
                     for (int p = p0; p < p1; ++p) {
                         T al = S.pexp[p];
-                        T e = gauss_prim(S, p, r2);
+                        T e = gauss_prim<LIB>(S, p, r2);
                         T e0 = S.cs0[p] * e, e1 = S.cs1[p] * e, ep = S.cp[p] * e;
                         a0 += e0; a1 += e1; ap += ep;
                         if (MODE >= 1) { b0 += al * e0; b1 += al * e1; bp += al * ep; }
@@ -428,8 +431,9 @@ __device__ __forceinline__ int pivot_mag(double a) { return d_hi(a) & 0x7fffffff
 template <class T>
 __device__ __forceinline__ T recip_full(T a) { return T(1) / a; }
 __device__ __forceinline__ double recip_full(double a) { return d_rcp_full(a); }
-// on_pivot(|pivot|) receives each pivot magnitude for the determinant.
-template <int N, class T, class OnPivot>
+// on_pivot(|pivot|) receives each pivot magnitude for the determinant.  LIB: whole
+// magnitudes are compared and pivots inverted by a division.
+template <int N, class T, class OnPivot, bool LIB = false>
 __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], int& sign, OnPivot on_pivot) {
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -437,13 +441,17 @@ __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], i
         for (int j = 0; j < N; ++j) Ainv[i][j] = (i == j) ? T(1) : T(0);
     sign = 1;
     bool ok = true;
+    auto mag = [](T a) {
+        if constexpr (LIB) return fabs(a);
+        else return pivot_mag(a);
+    };
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         int p = k;
-        auto best = pivot_mag(A[k][k]);
+        auto best = mag(A[k][k]);
 #pragma unroll
         for (int i = k + 1; i < N; ++i) {
-            const auto a = pivot_mag(A[i][k]);
+            const auto a = mag(A[i][k]);
             if (a > best) { best = a; p = i; }
         }
 #pragma unroll
@@ -462,7 +470,7 @@ __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], i
         if (!(piv != T(0))) { ok = false; piv = T(1); }
         if (piv < 0) sign = -sign;
         on_pivot(fabs(piv));
-        T ip = recip_full(piv);
+        T ip = LIB ? T(1) / piv : recip_full(piv);
 #pragma unroll
         for (int j = 0; j < N; ++j) { A[k][j] *= ip; Ainv[k][j] *= ip; }
 #pragma unroll
@@ -476,10 +484,11 @@ __device__ __forceinline__ bool gj_inverse_core(T (&A)[N][N], T (&Ainv)[N][N], i
     return ok;
 }
 
-template <int N, class T>
+template <int N, class T, bool LIB = false>
 __device__ __forceinline__ bool gj_inverse(T (&A)[N][N], T (&Ainv)[N][N], double& logdet, int& sign) {
     logdet = 0.0;
-    return gj_inverse_core<N, T>(A, Ainv, sign, [&](T p) { logdet += d_log((double)p); });
+    auto on_pivot = [&](T p) { logdet += d_log((double)p); };
+    return gj_inverse_core<N, T, decltype(on_pivot), LIB>(A, Ainv, sign, on_pivot);
 }
 
 // Float-float form: |det| accumulated as a rescaled product (one logarithm

@@ -100,6 +100,9 @@ struct MeasureOut {
     double* fhf = nullptr;               // [W][n_nuc][3]
     double* omega = nullptr;             // [W][n_nuc][3]
     double* dEL = nullptr;               // [W][P] d E_L / dp: rotation columns 8.. (with O)
+    // rows that belong to an SR batch: a thread per walker keeps the rounding of the
+    // orbital matrix that the team kernels give O_p and dE_L/dp
+    bool lib = false;
     // only the inverse, sign and log|psi| are wanted (E_L may be skipped)
     bool inverse_only = false;
 };

@@ -361,7 +361,7 @@ struct FullEval {
 };
 
 // One spin sector.
-template <class SH, class TC, int SIG, class DinvStore>
+template <class SH, class TC, int SIG, bool LIB, class DinvStore>
 __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], double& logdet,
                                             int& sg, bool& ok, TC (&gdx)[SH::NE], TC (&gdy)[SH::NE],
                                             TC (&gdz)[SH::NE], TC (&ld)[SH::NE], DinvStore store) {
@@ -372,7 +372,7 @@ __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)
 #pragma unroll 1
     for (int q = 0; q < NS; ++q) {
         const int e = SIG * SH::NUP + q;
-        MOEval<SH, TC, SIG, 2> m;
+        MOEval<SH, TC, SIG, 2, LIB> m;
         m.run(S, r[e][0], r[e][1], r[e][2]);
 #pragma unroll
         for (int k = 0; k < NS; ++k) { D[q][k] = m.v[k]; Gx[q][k] = m.gx[k]; Gy[q][k] = m.gy[k]; Gz[q][k] = m.gz[k]; L[q][k] = m.l[k]; }
@@ -380,7 +380,7 @@ __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)
     TC Di[NSa][NSa];
     double lg;
     int s;
-    ok = gj_inverse<NSa, TC>(D, Di, lg, s) && ok;
+    ok = gj_inverse<NSa, TC, LIB>(D, Di, lg, s) && ok;
     logdet += lg;
     sg *= s;
 #pragma unroll
@@ -455,7 +455,9 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
     return u;
 }
 
-template <class SH, class TC, class DinvStore>
+// LIB (Gaussian bases in FP64): the orbital matrix with the CUDA library's exponential
+// and pivots inverted by a division (see team_evaluate).
+template <class SH, class TC, bool LIB = false, class DinvStore>
 __device__ __forceinline__ void evaluate_config(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], FullEval<SH, TC>& out,
                                                 DinvStore store) {
     TC gjx[SH::NE], gjy[SH::NE], gjz[SH::NE], lu[SH::NE], gsq[SH::NE];
@@ -465,8 +467,8 @@ __device__ __forceinline__ void evaluate_config(const SysT<SH, TC>& S, const TC 
     double logdet = 0.0;
     int sg = 1;
     bool ok = true;
-    eval_sector<SH, TC, 0>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
-    eval_sector<SH, TC, 1>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
+    eval_sector<SH, TC, 0, LIB>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
+    eval_sector<SH, TC, 1, LIB>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
     TC kin = 0;
 #pragma unroll
     for (int e = 0; e < SH::NE; ++e) {
@@ -509,7 +511,7 @@ __global__ void k_init(const __grid_constant__ SysT<SH, double> S, TS* __restric
 // asked for, gradients and Laplacians); returns E_L (0 for an inactive lane, which
 // still runs the arithmetic on a dummy configuration so that the block stays
 // converged).
-template <class SH, class TC, class TS>
+template <class SH, class TC, class TS, bool LIB = false>
 __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS* __restrict__ pos,
                                                  TS* __restrict__ dinv, double* __restrict__ logabs,
                                                  int* __restrict__ sign, double* __restrict__ el, int w, bool act,
@@ -524,7 +526,7 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
         if (act && write_state) dinv[((size_t)(sig * NM * NM + k * NM + j)) * Wcap + w] = (TS)v;
     };
     FullEval<SH, TC> ev;
-    evaluate_config<SH, TC>(S, r, ev, store);
+    evaluate_config<SH, TC, LIB>(S, r, ev, store);
     double e_l = (double)ev.el;
     if (act) {
         int fl = 0;
@@ -548,14 +550,14 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
     return act ? e_l : 0.0;
 }
 
-template <class SH, class T, int TPB>
+template <class SH, class T, int TPB, bool LIB>
 __global__ void __launch_bounds__(TPB) k_measure(const __grid_constant__ SysT<SH, T> S,
                                                  const T* __restrict__ pos, T* __restrict__ dinv,
                                                  double* __restrict__ logabs, int* __restrict__ sign,
                                                  double* __restrict__ el, int W, int Wcap, int write_state,
                                                  MeasureOut out, double* partial, int* flags) {
     const int w = blockIdx.x * TPB + threadIdx.x;
-    double e_l = measure_walker<SH, T, T>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out, flags);
+    double e_l = measure_walker<SH, T, T, LIB>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out, flags);
     if (partial) block_partial<TPB>(e_l, partial, blockIdx.x);
 }
 
@@ -1433,7 +1435,7 @@ struct ShapeOps {
     }
 
     // Evaluation in the walkers' precision, a thread per walker.
-    template <class T>
+    template <class T, bool LIB = false>
     static int measure1(const HostSys& hs, DevWalkers& dw, bool write_state, const MeasureOut& out, cudaStream_t st) {
         SysT<SH, T> S;
         if (!fill_sys(hs, S)) return 7;
@@ -1441,7 +1443,7 @@ struct ShapeOps {
         int nb = (dw.W + TPB - 1) / TPB;
         double* partial = nullptr;
         if (write_state && dw.partial && dw.partial_cap >= 2 * nb + 1) partial = dw.partial;
-        k_measure<SH, T, TPB><<<nb, TPB, 0, st>>>(S, (const T*)dw.pos, (T*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W,
+        k_measure<SH, T, TPB, LIB><<<nb, TPB, 0, st>>>(S, (const T*)dw.pos, (T*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W,
                                                   dw.Wcap, write_state ? 1 : 0, out, partial, dw.flags);
         ++g_launch_count;
         int rc = cuda_status(cudaGetLastError());
@@ -1478,6 +1480,8 @@ struct ShapeOps {
     static int measure(const HostSys& hs, DevWalkers& dw, int cp, bool ws, const MeasureOut& out, cudaStream_t st) {
         if (cp == 0 && dw.prec == 0) {
             const bool plain = !out.O && !out.fhf && !out.omega;
+            if constexpr (team_lib<SH, 1>())
+                if (out.lib && !team_measures(dw.W)) return measure1<double, true>(hs, dw, ws, out, st);
             return plain && !team_measures(dw.W) ? measure1<double>(hs, dw, ws, out, st)
                                                  : Teams::measure(hs, dw, ws, out, st);
         }
