@@ -713,12 +713,11 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     // benzene (OptimizableWfn of BenzeneGTO, src/systems/benzene.rs:726-756):
     // the warp kernels give E_L, a per-walker kernel the Jastrow derivatives;
     // MO-rotation angles would need the determinant and are not compiled.
-    // Large batches of the molecules without rotations go the same way, E_L from a
-    // thread per walker.  MethaneGTO, host call: 9300 configurations 0.85 ms this way
-    // and 1.02 ms by teams, 20 000 1.37 and 1.62 ms, 65 536 3.60 and 5.09 ms.
+    // Large batches of CH4 go the same way, E_L and the rotation columns from a thread
+    // per walker.
     const bool benzene = hs.shape == SHAPE_C6H6;
     if (benzene && P != 8) return QMC_ERR_UNSUPPORTED;
-    const bool split = benzene || (P == 8 && !team_measures(W));
+    const bool split = benzene || !team_sr(W, P > 8);
     // device scratch: O [W][P], the SR sums and their block partials, the
     // Jastrow table (jas[8], nuclei [n_nuc][5]), then with dEL: dEL [W][P] and
     // (split form) grad ln|psi| [W][N][3]
@@ -739,8 +738,12 @@ int qmc_logderiv_batch(qmc_sys_t s, int W, const double* pos, double* O, double*
     if (split) CU(cudaMemcpyAsync(d_tab, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice, st));
     MeasureOut mo;
     mo.grad = d_grad;
-    mo.lib = split;
     if (split) {
+        mo.lib = !benzene;
+        if (P > 8) {
+            mo.O = wk->d_out;
+            mo.dEL = d_dEL;
+        }
         CK(launch_measure(hs, wk->dw, 0, true, mo, st));          // FP64 refresh: E_L (and grad) on the device
         if (launch_jastrow3_logderiv(wk->dw, hs.N, hs.n_up, hs.n_nuc, d_tab + 8, d_tab, P, wk->d_out, st, d_grad,
                                      d_dEL))

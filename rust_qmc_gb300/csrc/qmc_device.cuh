@@ -234,10 +234,23 @@ __device__ __forceinline__ float gauss_prim(const SysT<SH, float>& S, int p, flo
     return ex2_approx(S.pexp2[p] * r2);
 }
 
-template <class SH, class T, int SIG, int MODE, bool LIB = false>
+// MO-rotation rows: d phi / d theta of each angle, and the column of the rotated MO in
+// each sector (-1 none).
+template <class SH>
+struct RotTab {
+    double dC[SH::NROT][SH::NAO];
+    int col[SH::NROT][2];
+    int n;
+};
+
+// With NR, the values, gradients and Laplacians of the rotation rows as well.
+template <class SH, class T, int SIG, int MODE, bool LIB = false, int NR = 0>
 struct MOEval {
     static constexpr int NS = SIG == 0 ? SH::NUP : SH::NDN;
+    static constexpr int NRa = NR > 0 ? NR : 1;
     T v[SH::NMAX], gx[SH::NMAX], gy[SH::NMAX], gz[SH::NMAX], l[SH::NMAX];
+    T dv[NRa], dgx[NRa], dgy[NRa], dgz[NRa], dl[NRa];
+    const RotTab<SH>* rot = nullptr;
 
     __device__ __forceinline__ void add(const SysT<SH, T>& S, int a, T chi, T ax, T ay, T az, T la) {
 #pragma unroll
@@ -246,6 +259,11 @@ struct MOEval {
             v[k] += c * chi;
             if (MODE >= 1) { gx[k] += c * ax; gy[k] += c * ay; gz[k] += c * az; }
             if (MODE >= 2) l[k] += c * la;
+        }
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            const T c = rot->dC[q][a];
+            dv[q] += c * chi; dgx[q] += c * ax; dgy[q] += c * ay; dgz[q] += c * az; dl[q] += c * la;
         }
     }
 
@@ -264,6 +282,8 @@ struct MOEval {
     __device__ __forceinline__ void run(const SysT<SH, T>& S, T x, T y, T z) {
 #pragma unroll
         for (int k = 0; k < SH::NMAX; ++k) { v[k] = 0; gx[k] = 0; gy[k] = 0; gz[k] = 0; l[k] = 0; }
+#pragma unroll
+        for (int q = 0; q < NR; ++q) { dv[q] = 0; dgx[q] = 0; dgy[q] = 0; dgz[q] = 0; dl[q] = 0; }
         constexpr bool sto7 = std::is_same<typename SH::Layout, LayoutSto7>::value;
         if constexpr (sto7 && MODE == 0) {
             // run_tables' operations, the primitives and their powers unrolled

@@ -99,9 +99,9 @@ struct MeasureOut {
     double* O = nullptr;                 // [W][P]
     double* fhf = nullptr;               // [W][n_nuc][3]
     double* omega = nullptr;             // [W][n_nuc][3]
-    double* dEL = nullptr;               // [W][P] d E_L / dp: rotation columns 8.. (with O)
-    // rows that belong to an SR batch: a thread per walker keeps the rounding of the
-    // orbital matrix that the team kernels give O_p and dE_L/dp
+    double* dEL = nullptr;               // [W][P] d E_L / dp (with O)
+    // SR rows by a thread per walker (FP64 CH4), with the rounding of the orbital matrix
+    // that the team kernels give them; O and dEL then take the rotation columns only
     bool lib = false;
     // only the inverse, sign and log|psi| are wanted (E_L may be skipped)
     bool inverse_only = false;
@@ -260,6 +260,11 @@ inline bool team_sweeps(int W, bool drift) { return W <= (drift ? 10240 : 6144);
 // CH4 6-31G at 1000 walkers 0.08 ms by teams and 0.64 ms by threads, at 20 000
 // 1.15 and 0.9 ms.
 inline bool team_measures(int W) { return W <= 9216; }
+// SR rows of CH4, the same choice.  Host calls in ms, threads / teams, without rotations
+// (MethaneGTO): 9300 configurations 0.85 / 1.02, 20 000 1.37 / 1.62, 65 536 3.60 / 5.09;
+// with four (9 functions): 9300 0.77 / 0.73, 12 000 0.87 / 0.89, 20 000 1.24 / 1.40,
+// 65 536 3.25 / 4.38.
+inline bool team_sr(int W, bool rotations) { return W <= (rotations ? 10240 : 9216); }
 inline bool has_team_kernels(int shape) { return shape != SHAPE_C6H6 && shape != SHAPE_HEG54; }
 // Walkers per tile for a shape: threads per block for the thread-per-walker
 // shapes, a multiple of the warps per sweep block for the warp-per-walker ones.

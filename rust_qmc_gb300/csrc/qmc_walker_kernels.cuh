@@ -360,22 +360,41 @@ struct FullEval {
     TC gx[SH::NE], gy[SH::NE], gz[SH::NE], lap[SH::NE];   // grad psi/psi, lap psi/psi
 };
 
-// One spin sector.
-template <class SH, class TC, int SIG, bool LIB, class DinvStore>
+// Derivatives by the rotation angles: of ln|psi| and of E_L.
+template <class SH, class TC>
+struct RotEval {
+    const RotTab<SH>* tab;
+    TC O[SH::NROT], dE[SH::NROT];
+};
+
+// One spin sector.  With NR also the rotation columns: for column c of the sector rotated
+// by theta_q, with B = D^-1 and beta = B (d phi_c / d theta)(r_.), d ln|D| = beta_c and
+//   d (X B)_ii = X_psi(r_i) B_ci - B_ci sum_k X_k(r_i) beta_k   (X = grad, lap),
+//   d E_L / d theta_q += -1/2 sum_i [ d (lap B)_ii + 2 d (grad B)_ii . j_i ],
+// j_i the Jastrow gradient of electron i (gjx, gjy, gjz).
+template <class SH, class TC, int SIG, bool LIB, int NR, class DinvStore>
 __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], double& logdet,
                                             int& sg, bool& ok, TC (&gdx)[SH::NE], TC (&gdy)[SH::NE],
-                                            TC (&gdz)[SH::NE], TC (&ld)[SH::NE], DinvStore store) {
+                                            TC (&gdz)[SH::NE], TC (&ld)[SH::NE], DinvStore store,
+                                            const TC (&gjx)[SH::NE], const TC (&gjy)[SH::NE], const TC (&gjz)[SH::NE],
+                                            RotEval<SH, TC>* rot) {
     constexpr int NS = SIG == 0 ? SH::NUP : SH::NDN;
     if (NS == 0) return;
     constexpr int NSa = NS > 0 ? NS : 1;
     TC D[NSa][NSa], Gx[NSa][NSa], Gy[NSa][NSa], Gz[NSa][NSa], L[NSa][NSa];
+    TC X[NSa][NR > 0 ? NR : 1][5];             // rotation rows: value, gradient, Laplacian
 #pragma unroll 1
     for (int q = 0; q < NS; ++q) {
         const int e = SIG * SH::NUP + q;
-        MOEval<SH, TC, SIG, 2, LIB> m;
+        MOEval<SH, TC, SIG, 2, LIB, NR> m;
+        if constexpr (NR > 0) m.rot = rot->tab;
         m.run(S, r[e][0], r[e][1], r[e][2]);
 #pragma unroll
         for (int k = 0; k < NS; ++k) { D[q][k] = m.v[k]; Gx[q][k] = m.gx[k]; Gy[q][k] = m.gy[k]; Gz[q][k] = m.gz[k]; L[q][k] = m.l[k]; }
+#pragma unroll
+        for (int a = 0; a < NR; ++a) {
+            X[q][a][0] = m.dv[a]; X[q][a][1] = m.dgx[a]; X[q][a][2] = m.dgy[a]; X[q][a][3] = m.dgz[a]; X[q][a][4] = m.dl[a];
+        }
     }
     TC Di[NSa][NSa];
     double lg;
@@ -397,6 +416,40 @@ __device__ __forceinline__ void eval_sector(const SysT<SH, TC>& S, const TC (&r)
             ax += Gx[q][k] * w; ay += Gy[q][k] * w; az += Gz[q][k] * w; al += L[q][k] * w;
         }
         gdx[e] = ax; gdy[e] = ay; gdz[e] = az; ld[e] = al;
+    }
+    if constexpr (NR > 0) {
+#pragma unroll 1
+        for (int a = 0; a < rot->tab->n; ++a) {
+            const int c = rot->tab->col[a][SIG];
+            if (c < 0) continue;
+            TC beta[NSa], Bc[NSa], dlog = 0, acc = 0;
+#pragma unroll
+            for (int k = 0; k < NS; ++k) {
+                beta[k] = 0;
+#pragma unroll
+                for (int row = 0; row < NS; ++row) beta[k] += Di[k][row] * X[row][a][0];
+                dlog = k == c ? beta[k] : dlog;
+            }
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                Bc[q] = 0;
+#pragma unroll
+                for (int k = 0; k < NS; ++k) Bc[q] = k == c ? Di[k][q] : Bc[q];
+            }
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                const int e = SIG * SH::NUP + q;
+                TC tx = 0, ty = 0, tz = 0, tl = 0;
+#pragma unroll
+                for (int k = 0; k < NS; ++k) {
+                    tx += Gx[q][k] * beta[k]; ty += Gy[q][k] * beta[k]; tz += Gz[q][k] * beta[k]; tl += L[q][k] * beta[k];
+                }
+                acc += Bc[q] * ((X[q][a][4] - tl) + 2 * ((X[q][a][1] - tx) * gjx[e] + (X[q][a][2] - ty) * gjy[e] +
+                                                         (X[q][a][3] - tz) * gjz[e]));
+            }
+            rot->O[a] += dlog;
+            rot->dE[a] -= TC(0.5) * acc;
+        }
     }
 }
 
@@ -457,9 +510,9 @@ __device__ __forceinline__ TC jastrow_coulomb(const SysT<SH, TC>& S, const TC (&
 
 // LIB (Gaussian bases in FP64): the orbital matrix with the CUDA library's exponential
 // and pivots inverted by a division (see team_evaluate).
-template <class SH, class TC, bool LIB = false, class DinvStore>
+template <class SH, class TC, bool LIB = false, int NR = 0, class DinvStore>
 __device__ __forceinline__ void evaluate_config(const SysT<SH, TC>& S, const TC (&r)[SH::NE][3], FullEval<SH, TC>& out,
-                                                DinvStore store) {
+                                                DinvStore store, RotEval<SH, TC>* rot = nullptr) {
     TC gjx[SH::NE], gjy[SH::NE], gjz[SH::NE], lu[SH::NE], gsq[SH::NE];
     TC V;
     const TC u = jastrow_coulomb<SH, TC>(S, r, gjx, gjy, gjz, lu, gsq, V);
@@ -467,8 +520,8 @@ __device__ __forceinline__ void evaluate_config(const SysT<SH, TC>& S, const TC 
     double logdet = 0.0;
     int sg = 1;
     bool ok = true;
-    eval_sector<SH, TC, 0, LIB>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
-    eval_sector<SH, TC, 1, LIB>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store);
+    eval_sector<SH, TC, 0, LIB, NR>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store, gjx, gjy, gjz, rot);
+    eval_sector<SH, TC, 1, LIB, NR>(S, r, logdet, sg, ok, gdx, gdy, gdz, ld, store, gjx, gjy, gjz, rot);
     TC kin = 0;
 #pragma unroll
     for (int e = 0; e < SH::NE; ++e) {
@@ -511,11 +564,12 @@ __global__ void k_init(const __grid_constant__ SysT<SH, double> S, TS* __restric
 // asked for, gradients and Laplacians); returns E_L (0 for an inactive lane, which
 // still runs the arithmetic on a dummy configuration so that the block stays
 // converged).
-template <class SH, class TC, class TS, bool LIB = false>
+template <class SH, class TC, class TS, bool LIB = false, int NR = 0>
 __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS* __restrict__ pos,
                                                  TS* __restrict__ dinv, double* __restrict__ logabs,
                                                  int* __restrict__ sign, double* __restrict__ el, int w, bool act,
-                                                 int Wcap, int write_state, const MeasureOut& out, int* flags) {
+                                                 int Wcap, int write_state, const MeasureOut& out, int* flags,
+                                                 const RotTab<SH>* tab = nullptr) {
     TC r[SH::NE][3];
 #pragma unroll
     for (int e = 0; e < SH::NE; ++e)
@@ -526,7 +580,8 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
         if (act && write_state) dinv[((size_t)(sig * NM * NM + k * NM + j)) * Wcap + w] = (TS)v;
     };
     FullEval<SH, TC> ev;
-    evaluate_config<SH, TC, LIB>(S, r, ev, store);
+    RotEval<SH, TC> rot{tab, {}, {}};
+    evaluate_config<SH, TC, LIB, NR>(S, r, ev, store, &rot);
     double e_l = (double)ev.el;
     if (act) {
         int fl = 0;
@@ -546,6 +601,13 @@ __device__ __forceinline__ double measure_walker(const SysT<SH, TC>& S, const TS
 #pragma unroll
             for (int e = 0; e < SH::NE; ++e) out.lap[(size_t)w * SH::NE + e] = (double)ev.lap[e];
         }
+        if constexpr (NR > 0) {
+            const size_t row = (size_t)w * (8 + tab->n) + 8;
+            for (int a = 0; a < tab->n; ++a) {
+                out.O[row + a] = (double)rot.O[a];
+                if (out.dEL) out.dEL[row + a] = (double)rot.dE[a];
+            }
+        }
     }
     return act ? e_l : 0.0;
 }
@@ -559,6 +621,19 @@ __global__ void __launch_bounds__(TPB) k_measure(const __grid_constant__ SysT<SH
     const int w = blockIdx.x * TPB + threadIdx.x;
     double e_l = measure_walker<SH, T, T, LIB>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out, flags);
     if (partial) block_partial<TPB>(e_l, partial, blockIdx.x);
+}
+
+// The same with the rotation columns (from 8 on) of O_p and dE_L/dp, for large SR batches.
+template <class SH, int TPB>
+__global__ void __launch_bounds__(TPB) k_measure_rot(const __grid_constant__ SysT<SH, double> S,
+                                                     const __grid_constant__ RotTab<SH> R,
+                                                     const double* __restrict__ pos, double* __restrict__ dinv,
+                                                     double* __restrict__ logabs, int* __restrict__ sign,
+                                                     double* __restrict__ el, int W, int Wcap, int write_state,
+                                                     MeasureOut out, int* flags) {
+    const int w = blockIdx.x * TPB + threadIdx.x;
+    measure_walker<SH, double, double, true, SH::NROT>(S, pos, dinv, logabs, sign, el, w, w < W, Wcap, write_state, out,
+                                                       flags, &R);
 }
 
 // Bytes of a system table staged in shared memory (16-byte multiple).
@@ -1451,6 +1526,31 @@ struct ShapeOps {
         return launch_sum_partials(partial, nb, 1, dw.partial + dw.partial_cap - 1, st);
     }
 
+    // SR rows of a large batch with rotations: E_L, grad ln|psi| and the rotation columns.
+    static int measure_rot(const HostSys& hs, DevWalkers& dw, bool write_state, const MeasureOut& out, cudaStream_t st) {
+        SysT<SH, double> S;
+        RotTab<SH> R{};
+        if (!fill_sys(hs, S) || (int)hs.rot_occ.size() > SH::NROT) return 7;
+        R.n = (int)hs.rot_occ.size();
+        const std::vector<double> dC = hs.rotation_derivative_rows();
+        for (int q = 0; q < R.n; ++q) {
+            for (int a = 0; a < hs.n_ao; ++a) R.dC[q][hs.ao_int[a]] = dC[(size_t)q * hs.n_ao + a];
+            int col[2] = {0, 0};
+            R.col[q][0] = R.col[q][1] = -1;
+            for (int ei = 0; ei < hs.N; ++ei) {
+                const int e = hs.perm[ei], sig = hs.spins[e] > 0 ? 0 : 1;
+                if (hs.occ[e] == hs.rot_occ[q]) R.col[q][sig] = col[sig];
+                ++col[sig];
+            }
+        }
+        constexpr int TPB = 64;
+        k_measure_rot<SH, TPB><<<(dw.W + TPB - 1) / TPB, TPB, 0, st>>>(S, R, (const double*)dw.pos, (double*)dw.dinv,
+                                                                       dw.logabs, dw.sign, dw.el, dw.W, dw.Wcap,
+                                                                       write_state ? 1 : 0, out, dw.flags);
+        ++g_launch_count;
+        return cuda_status(cudaGetLastError());
+    }
+
     template <bool VALUES>
     static int measure_split(const HostSys& hs, DevWalkers& dw, bool write_state, cudaStream_t st) {
         SysT<SH, ff> S;
@@ -1481,7 +1581,7 @@ struct ShapeOps {
         if (cp == 0 && dw.prec == 0) {
             const bool plain = !out.O && !out.fhf && !out.omega;
             if constexpr (team_lib<SH, 1>())
-                if (out.lib && !team_measures(dw.W)) return measure1<double, true>(hs, dw, ws, out, st);
+                if (out.lib) return out.O ? measure_rot(hs, dw, ws, out, st) : measure1<double, true>(hs, dw, ws, out, st);
             return plain && !team_measures(dw.W) ? measure1<double>(hs, dw, ws, out, st)
                                                  : Teams::measure(hs, dw, ws, out, st);
         }
