@@ -1010,6 +1010,9 @@ struct Adapt {
     }
 };
 
+// Memory of the recorded all-electron steps' block partials in a vmc_run.
+constexpr size_t kStepPartialBytes = (size_t)256 << 20;
+
 int read_acc(qmc_walkers_s* wk, unsigned long long* acc) {
     cudaStream_t st = wk->sys->ctx->stream;
     CU(cudaMemcpyAsync(acc, wk->dw.acc, 8, cudaMemcpyDeviceToHost, st));
@@ -1047,26 +1050,37 @@ int qmc_vmc_run(qmc_sys_t s, const qmc_run_params* p, uint64_t seed, qmc_run_res
         const int total = p->n_burnin + p->n_steps;
         const int nblk = step_all_blocks(hs, wk->dw);
         if (nblk <= 0) return QMC_ERR_UNSUPPORTED;
+        // block partials of at most `rows` steps, summed into d_mean when they are full
+        // (a long run's partials of every step would take as much memory as it has)
+        const int rows = (int)std::min<size_t>(p->n_steps, std::max<size_t>(1, kStepPartialBytes / (16 * (size_t)nblk)));
         double* d_part = nullptr;
         double* d_mean = nullptr;
-        CU(cudaMalloc((void**)&d_part, 16 * (size_t)nblk * p->n_steps));
+        CU(cudaMalloc((void**)&d_part, 16 * (size_t)nblk * rows));
         cudaError_t e = cudaMalloc((void**)&d_mean, 8 * (size_t)p->n_steps);
         if (e != cudaSuccess) { cudaFree(d_part); return cuda_rc(e); }
         struct Bufs { double* a; double* b; ~Bufs() { cudaFree(a); cudaFree(b); } } bufs{d_part, d_mean};
-        // steps t = 0 .. total-1 in launches that end at adaptation points and
-        // at the end of the burn-in; production steps record their mean E_L
-        int t = 0;
+        // steps t = 0 .. total-1 in launches that end at adaptation points, at
+        // the end of the burn-in and when the partials are full; production steps
+        // record their mean E_L
+        int t = 0, kept = 0;
         while (t < total) {
             int end = total;
             if (t < p->n_burnin) end = std::min(end, p->n_burnin);
             if (ad.on) end = std::min(end, (t / ad.interval + 1) * ad.interval);
+            const bool record = t >= p->n_burnin;
+            if (record) end = std::min(end, t + rows - kept);
             const int n = end - t;
-            if (t >= p->n_burnin)
+            if (record)
                 CK(launch_step_all(hs, wk->dw, p->move_kind, n, (uint64_t)t, ad.value, seed,
-                                   d_part + 2 * (size_t)nblk * (t - p->n_burnin), st));
+                                   d_part + 2 * (size_t)nblk * kept, st));
             else
                 CK(launch_sweep(hs, wk->dw, p->move_kind, n, (uint64_t)t, ad.value, 0, 0, seed, st));
             t = end;
+            if (record) kept += n;
+            if (kept == rows || (t == total && kept)) {
+                CK(launch_sum_partials(d_part, nblk, kept, d_mean + (t - p->n_burnin - kept), st));
+                kept = 0;
+            }
             if (t == p->n_burnin) CK(read_acc(wk, &acc_prod0));
             if (ad.on && t % ad.interval == 0) {
                 unsigned long long acc;
@@ -1074,7 +1088,6 @@ int qmc_vmc_run(qmc_sys_t s, const qmc_run_params* p, uint64_t seed, qmc_run_res
                 ad.update(acc, (double)ad.interval * W);
             }
         }
-        CK(launch_sum_partials(d_part, nblk, p->n_steps, d_mean, st));
         series.resize(p->n_steps);
         CU(cudaMemcpyAsync(series.data(), d_mean, 8 * (size_t)p->n_steps, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
