@@ -1499,13 +1499,11 @@ int batch_sync_tables(qmc_batch_s* b) {
         }
         if (dirty) CU(cudaMemcpy(c.d_recs, c.recs.data(), sizeof(BatchRec) * c.recs.size(), cudaMemcpyHostToDevice));
         // the electron-gas refresh sizes its shared memory by the largest
-        // reciprocal component: a larger one needs new attributes and graphs
+        // reciprocal component: a larger one needs new graphs
         int kmax = c.bc.kmax;
         for (int i : c.members) kmax = std::max(kmax, reciprocal_kmax(b->wk[i]->sys->hs));
         if (kmax > c.bc.kmax) {
             c.bc.kmax = kmax;
-            const int occ = batch_occupancy(c.bc.shape, c.bc.prec, 0, true, kmax);
-            if (occ < 0) return -occ;
             for (auto& g : b->graph)
                 if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         }

@@ -25,6 +25,7 @@ template <> struct HComplex<float> { using type = float2; };
 template <> struct HComplex<double> { using type = double2; };
 
 constexpr int HMAX_K = 1800;      // reciprocal half-space vectors (|n_i| <= 7 cube: 1687)
+constexpr int HMAX_KMAX = 9;      // largest component they leave room for (|n| <= 10: 2084)
 
 template <class T>
 struct SysH {
@@ -81,6 +82,7 @@ static bool fill_sysh(const HostSys& hs, int NE, int NUP, SysH<T>& S, KTable& KT
     const bool qe = (hs.quirks & 4) != 0;
     const double alpha = qe ? 5.0 / L : hs.jas[4] / L;
     const int K = reciprocal_kmax(hs);
+    if (K > HMAX_KMAX) return false;
     S.alpha = (T)alpha;
     S.real_images = qe ? 0 : 1;
     S.rcut = (T)(5.6 / alpha);
@@ -1804,8 +1806,14 @@ struct HegShapeOps {
     static int batch_measure_t(const BatchClass& bc, cudaStream_t st, int* occ) {
         const size_t smem = measure_smem<TC, TS, PART>(bc.kmax);
         auto kern = khwb_measure<NE, NUP, TC, TS, WPB, PART>;
-        static size_t attr = 0;
-        if (attr < smem) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = smem; }
+        // the largest cutoff's, whatever this one: a limit that depends on the call could be
+        // lowered again by another thread's
+        static bool attr = false;
+        if (!attr) {
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)measure_smem<TC, TS, PART>(HMAX_KMAX));
+            attr = true;
+        }
         if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, 32 * WPB, smem) == cudaSuccess ? 0 : 2;
         if (bc.ntiles == 0) return 0;
         kern<<<bc.ntiles, 32 * WPB, smem, st>>>(bc.tiles, bc.ntiles, bc.recs, bc.tile_partial);
@@ -1845,8 +1853,14 @@ struct HegShapeOps {
                                    const MeasureOut& out, double* partial, int nb, cudaStream_t st) {
         const size_t smem = measure_smem<TC, TS, PART>(kmax);
         auto kern = khw_measure<NE, NUP, TC, TS, WPB, PART>;
-        static size_t attr = 0;
-        if (attr < smem) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = smem; }
+        // the largest cutoff's, whatever this one: a limit that depends on the call could be
+        // lowered again by another thread's
+        static bool attr = false;
+        if (!attr) {
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)measure_smem<TC, TS, PART>(HMAX_KMAX));
+            attr = true;
+        }
         kern<<<nb, 32 * WPB, smem, st>>>(S, KT, (const TS*)dw.pos, (TS*)dw.dinv, dw.logabs, dw.sign, dw.el, dw.W,
                                          dw.Wcap, ws ? 1 : 0, out.grad, out.lap, partial, dw.flags, dw.rows);
         ++g_launch_count;
