@@ -13,6 +13,7 @@
 // G: 4 for H2, 8 for Li, 32 for CH4 (30 lanes busy).
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <vector>
 #include "qmc_internal.h"
@@ -1286,6 +1287,18 @@ __global__ void __launch_bounds__(32) kb_team_sweep(const BatchTile* __restrict_
                                 batch_system_seed(ctl->seed, R.index), R.fixed_node, R.acc, R.flags);
 }
 
+// SMs of the current device, asked for once per device.
+inline int device_sms() {
+    constexpr int N = 64;
+    static std::atomic<int> known[N];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= N) dev = 0;
+    n = known[dev].load(std::memory_order_relaxed);
+    if (!n && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+        known[dev].store(n, std::memory_order_relaxed);
+    return n > 0 ? n : 1;
+}
+
 // Launchers of a shape with teams of G lanes.
 template <class SH, int G>
 struct TeamOps {
@@ -1303,9 +1316,9 @@ struct TeamOps {
     }
 
     // One warp per block while every warp can have a sub-partition of its own
-    // (152 SMs x 4), so that the block scheduler spreads them over the SMs;
+    // (four an SM), so that the block scheduler spreads them over the SMs;
     // four beyond that, which share one copy of the table.
-    static bool spread(int W) { return (long long)W * G <= 32LL * 152 * 4; }
+    static bool spread(int W) { return (long long)W * G <= 32LL * 4 * device_sms(); }
 
     static int step_blocks(int W) {
         const int nt = (spread(W) ? 32 : 128) / G;
