@@ -1,7 +1,7 @@
 // qmc_jastrow3_logderiv.h -- parameter log-derivatives of the Jastrow3 factor
-// for one configuration, term by term: the sums that the device kernel
-// k_jastrow3_logderiv takes with a warp, in the plain form that the host checks
-// compile.
+// for one configuration: the terms that the device kernel k_jastrow3_logderiv deals
+// to the lanes of a warp (jastrow3_term), and the plain sums over all of them that the
+// host checks compare with.  Compiled for the device and, unchanged, for the host.
 //
 // u = sum_{i<j} a_s r_ij / (1 + b_s r_ij) - sum_{i,I} A_t Z_I r_iI / (1 + B_t r_iI)
 // (src/correlation/jastrow.rs:138-449) with a and b per spin class s
@@ -119,6 +119,49 @@ QMC_JHD inline void jastrow3_el_derivatives(int N, int n_up, int n_nuc, const do
         }
     }
     for (int k = 0; k < 8; ++k) dE[k] = -0.5 * acc[k];
+}
+
+// Terms of a configuration: the electron pairs, then electrons by nuclei.  Pair t joins
+// electron t mod N with the one t / N + 1 after it (mod N); the last N / 2 pairs of an
+// even N join opposite electrons.
+QMC_JHD inline int jastrow3_terms(int N, int n_nuc) { return N * (N - 1) / 2 + N * n_nuc; }
+QMC_JHD inline void jastrow3_pair(int t, int N, int& i, int& j) {
+    const int full = N * ((N - 1) / 2);
+    i = t < full ? t % N : t - full;
+    j = t < full ? i + t / N + 1 : i + N / 2;
+    j = j >= N ? j - N : j;
+}
+
+// Term t of the sums of jastrow3_log_derivatives and, with DEL, of
+// jastrow3_el_derivatives, the common factors of the term's two parameters taken out:
+// add(k, v) adds v to sum k (O 0..7, dE 8..15).  sqrt_ and rcp are the square root and
+// the reciprocal.
+template <class Pos, class Grad, class Sqrt, class Rcp, class Add>
+QMC_JHD inline void jastrow3_term(int t, int N, int n_up, const double* nuc, const double* p, const Pos& pos,
+                                  const Grad& grad, bool del, const Sqrt& sqrt_, const Rcp& rcp, const Add& add) {
+    const int n_pair = N * (N - 1) / 2;
+    const bool ee = t < n_pair;
+    const int q = ee ? t : t - n_pair;
+    int i = q % N, j = 0;
+    if (ee) jastrow3_pair(q, N, i, j);
+    const double* n = nuc + 5 * (ee ? 0 : q / N);
+    const double dx = pos(i, 0) - (ee ? pos(j, 0) : n[0]), dy = pos(i, 1) - (ee ? pos(j, 1) : n[1]),
+                 dz = pos(i, 2) - (ee ? pos(j, 2) : n[2]);
+    // class: spin pair or species; parameters b, a at p[k], p[k + 2]
+    const int k = ee ? ((i < n_up) == (j < n_up) ? 1 : 0) : 4 + (n[4] == 0.0 ? 0 : 1);
+    const double z = ee ? 1.0 : -n[3], b = p[k], a = z * p[k + 2];        // u = a r / (1 + b r)
+    const double d = sqrt_(dx * dx + dy * dy + dz * dz);
+    const double i1 = rcp(1.0 + b * d), s = d * i1;
+    add(k, -(a * s * s));
+    add(k + 2, z * s);
+    if (del && !(d < 1e-10)) {
+        // -1/2 sum over the ends of l + 2 f G.dr: two ends with G_i - G_j, or one
+        const double h = (grad(i, 0) - (ee ? grad(j, 0) : 0.0)) * dx + (grad(i, 1) - (ee ? grad(j, 1) : 0.0)) * dy +
+                         (grad(i, 2) - (ee ? grad(j, 2) : 0.0)) * dz;
+        const double i2 = i1 * i1, i3 = i2 * i1, e = ee ? 2.0 : 1.0;
+        add(8 + k, a * i3 * (3.0 * e * i1 + 2.0 * h));
+        add(8 + k + 2, -(z * (i2 * rcp(d) * (e + h) - e * b * i3)));
+    }
 }
 
 }  // namespace qmc

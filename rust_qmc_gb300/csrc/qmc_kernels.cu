@@ -6,6 +6,7 @@
 #include <algorithm>
 #include "qmc_internal.h"
 #include "qmc_device.cuh"
+#include "qmc_jastrow3_logderiv.h"
 
 namespace qmc {
 
@@ -331,11 +332,11 @@ int launch_hf_force_walkers(const DevWalkers& dw, int N, int n_nuc, const double
 // O is null); par = p[8], nuc = [n_nuc][5] (x, y, z, Z, species 0 or 1: the host
 // rejects other species when it builds a system).  With grad ([W][N][3],
 // grad_i ln|psi| in the internal electron order) the Jastrow-parameter derivatives of
-// the local energy go to dEL[w][0..7], same stride.  The sums of
-// qmc_jastrow3_logderiv.h, with the common factors of a pair's two parameters taken
-// out.  An FP64 instruction costs the same for 1 and 32 lanes: a thread per walker
-// spent a serial chain of 1365 benzene terms on 19 warps, the lanes of a warp take
-// them 32 at a time: 94 us for 600 walkers (their SR call 0.54 ms after 5.66 ms).
+// the local energy go to dEL[w][0..7], same stride.  The terms are jastrow3_term's
+// (qmc_jastrow3_logderiv.h).  An FP64 instruction costs the same for 1 and 32 lanes: a
+// thread per walker spent a serial chain of 1365 benzene terms on 19 warps, the lanes of
+// a warp take them 32 at a time: 94 us for 600 walkers (their SR call 0.54 ms after
+// 5.66 ms).
 constexpr int J3_MAX_N = 64;
 template <class TS, int TPB>
 __global__ void __launch_bounds__(TPB) k_jastrow3_logderiv(const TS* __restrict__ pos, int W, int Wcap, int N, int n_up,
@@ -355,35 +356,14 @@ __global__ void __launch_bounds__(TPB) k_jastrow3_logderiv(const TS* __restrict_
 #pragma unroll
     for (int k = 0; k < 16; ++k) acc[k][lane] = 0.0;
     __syncwarp();
-    // terms: pairs (p mod N with p mod N + p / N + 1, the last N / 2 pairs of an even N
-    // opposite electrons), then electrons by nuclei
-    const int n_pair = N * (N - 1) / 2, full = N * ((N - 1) / 2), n_term = n_pair + N * n_nuc;
+    const int n_term = jastrow3_terms(N, n_nuc);
+    auto at = [&](int i, int c) { return r[3 * i + c]; };
+    auto gr = [&](int i, int c) { return g[3 * i + c]; };
+    auto root = [](double x) { return d_sqrt(x); };
+    auto rcp = [](double x) { return d_rcp_full(x); };
+    auto add = [&](int k, double v) { acc[k][lane] += v; };
 #pragma unroll 1
-    for (int t = lane; t < n_term; t += 32) {
-        const bool ee = t < n_pair;
-        const int q = ee ? t : t - n_pair;
-        const int i = ee && q >= full ? q - full : q % N;
-        int j = ee ? (q < full ? i + q / N + 1 : i + N / 2) : 0;
-        j = j >= N ? j - N : j;
-        const double* n = nuc + 5 * (ee ? 0 : q / N);
-        const double dx = r[3 * i] - (ee ? r[3 * j] : n[0]), dy = r[3 * i + 1] - (ee ? r[3 * j + 1] : n[1]),
-                     dz = r[3 * i + 2] - (ee ? r[3 * j + 2] : n[2]);
-        // class: spin pair or species; parameters b, a at p[k], p[k + 2]
-        const int k = ee ? ((i < n_up) == (j < n_up) ? 1 : 0) : 4 + (n[4] == 0.0 ? 0 : 1);
-        const double z = ee ? 1.0 : -n[3], b = par[k], a = z * par[k + 2];     // u = a r / (1 + b r)
-        const double d = d_sqrt(dx * dx + dy * dy + dz * dz);
-        const double i1 = d_rcp_full(1.0 + b * d), s = d * i1;
-        acc[k][lane] -= a * s * s;
-        acc[k + 2][lane] += z * s;
-        if (del && !d_below(d, 1e-10)) {
-            // -1/2 sum over the ends of l + 2 f G.dr: two ends with G_i - G_j, or one
-            const double h = (g[3 * i] - (ee ? g[3 * j] : 0.0)) * dx + (g[3 * i + 1] - (ee ? g[3 * j + 1] : 0.0)) * dy +
-                             (g[3 * i + 2] - (ee ? g[3 * j + 2] : 0.0)) * dz;
-            const double i2 = i1 * i1, i3 = i2 * i1, e = ee ? 2.0 : 1.0;
-            acc[8 + k][lane] += a * i3 * (3.0 * e * i1 + 2.0 * h);
-            acc[8 + k + 2][lane] -= z * (i2 * d_rcp_full(d) * (e + h) - e * b * i3);
-        }
-    }
+    for (int t = lane; t < n_term; t += 32) jastrow3_term(t, N, n_up, nuc, par, at, gr, del, root, rcp, add);
     __syncwarp();
     // column sums: half of the lanes' terms by lane k and half by lane k + 16
     const int k = lane & 15, from = lane & 16;
