@@ -1,9 +1,10 @@
-"""Coefficients of the float-float erfc of the electron-gas Ewald sum
-(qmc_heg_kernels.cuh, erfc_ff): Chebyshev interpolation of erfc on [0, 6]
-at 64 first-kind nodes, computed with mpmath at 40 digits.  erfc(x) =
-c_0 / 2 + sum_{k=1..42} c_k T_k(t), t = x / 3 - 1; |c_k| < 2e-18 for k > 42.
-Prints the table as C++ initialisers (float-float pairs for k < 24, FP32
-beyond).  Run: python gen_erfc_table.py"""
+"""Coefficients of a Chebyshev interpolant of erfc on [0, 6] at 64 first-kind
+nodes, computed with mpmath at 40 digits: erfc(x) = c_0 / 2 + sum_{k=1..42}
+c_k T_k(t), t = x / 3 - 1; |c_k| < 2e-18 for k > 42.  tests/test_ff_algorithms.py
+sums it by Clenshaw's recurrence in float-float arithmetic; the library's own erfc
+is the Taylor table of qmc_ewald.cuh.  Prints the coefficients as C++
+initialisers (float-float pairs for k < 24, FP32 beyond).
+Run: python gen_erfc_table.py"""
 import mpmath as mp
 
 N_NODES, DEG, FF_TERMS = 64, 42, 24

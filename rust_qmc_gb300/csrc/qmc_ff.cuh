@@ -37,6 +37,7 @@ struct ff {
     __host__ __device__ explicit constexpr operator float() const { return hi + lo; }
 };
 
+#if defined(__CUDACC__)
 // ---- packed FP32 -------------------------------------------------------------
 // Two FP32 values in a 64-bit register, for the packed instructions (one issue
 // for two IEEE operations; subnormals are flushed, as the library's FP32 code is
@@ -72,6 +73,8 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b) {
     asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
+
+#endif
 
 // ---- error-free transformations ---------------------------------------------
 __device__ __forceinline__ ff ff_two_sum(float a, float b) {
@@ -245,6 +248,7 @@ __device__ __forceinline__ ff ff_load(const float2* p) {
     return ff(t.x, t.y);
 }
 
+#if defined(__CUDACC__)
 // Warp shuffle of a float-float value (two FP32 shuffles).
 __device__ __forceinline__ ff wshfl(ff v, int src) {
     return ff(__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src));
@@ -354,5 +358,6 @@ __device__ __forceinline__ ff2 ff2_fexp(ff2 a) {
                 a1 < -87.0f ? 0.0f : __int_as_float(((n1 >> 5) + 127) << 23));
     return ff2(mul2(m.hi, sc), mul2(m.lo, sc));
 }
+#endif
 
 }  // namespace qmc
