@@ -349,8 +349,10 @@ struct Team {
         pm = shfl(m, base) * (NDN > 0 ? shfl(m, base + NUP) : 1.0);
         pe = shfl(ex, base) + (NDN > 0 ? shfl(ex, base + NUP) : 0);
         s = shfl(s, base) ^ (NDN > 0 ? shfl(s, base + NUP) : 0);
-        const int g = good;
-        ok = shfl(g, base) && (NDN == 0 || shfl(g, base + NUP));
+        // every lane takes both shuffles: a team with a singular matrix that skipped the second
+        // would leave the warp's other teams waiting in it
+        const int g = good, g0 = shfl(g, base), g1 = NDN > 0 ? shfl(g, base + NUP) : 1;
+        ok = g0 != 0 && g1 != 0;
         sg = s ? -1 : 1;
     }
     // Jastrow u alone: the pairs and electron-nucleus terms spread over the lanes.
