@@ -46,7 +46,7 @@ inline void fill_erfc_table(float4 (*tab)[3]) {
 // against 75 and three 16-byte loads).
 __device__ __forceinline__ ff erfc_ff(const float4 (*__restrict__ tab)[3], ff x) {
     if (!(x.hi < 6.0f)) return ff(0.0f);
-    const int j = min((int)(x.hi * 32.0f), HERFC_N - 1);
+    const int j = max(0, min((int)(x.hi * 32.0f), HERFC_N - 1));   // set_params takes any splitting: x may be negative
     const ff d = x + ff(-((float)j + 0.5f) * 0.03125f);
     const float4 a = tab[j][0], b = tab[j][1], c = tab[j][2];
     const float t = __fmaf_rn(d.hi, __fmaf_rn(d.hi, __fmaf_rn(d.hi, c.w, c.z), c.y), c.x);

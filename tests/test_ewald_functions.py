@@ -39,12 +39,16 @@ static float __fdividef(float a, float b) { return (float)(a / (double)b * (1.0 
 static float rsqrtf(float a) { return (float)(1.0 / std::sqrt((double)a)); }
 static int __float_as_int(float f) { int i; memcpy(&i, &f, 4); return i; }
 static float __int_as_float(int i) { float f; memcpy(&f, &i, 4); return f; }
+using std::max;
 using std::min;
 #include "qmc_ewald.cuh"
 using namespace qmc;
 typedef long double ld;
-static float4 tab[HERFC_N][3];
+static float4 room[3 * HERFC_N][3];                  // the table between rows of NaN
+static float4 (*tab)[3] = room + HERFC_N;
 int main() {
+    for (auto& row : room)
+        for (auto& v : row) v = {NAN, NAN, NAN, NAN};
     std::mt19937_64 g(5);
     auto U = [&](double a, double b) { return a + (b - a) * ((g() >> 11) * 0x1p-53); };
     auto mx = [](double& m, double v) { if (!(v <= m)) m = v; };
@@ -90,7 +94,9 @@ int main() {
         mx(e_img, std::fmax(0.0, (double)(fabsl(got - want) - 1e-13L)) / (double)want);
         if (exact) { bias += e * (want > 1e-6L); n += want > 1e-6L; }
     }
-    std::printf("%g %g %g %g\n", e_erfc, e_exp, e_img, std::fabs(bias / n));
+    bool inside = true;                              // every argument reads the table's own rows
+    for (double v : {-1e-6, -0.02, -3.0, -5.99, -6.0, -11.0, 6.0, 1e30}) inside = inside && std::isfinite(erfc_ff(tab, ff(v)).hi);
+    std::printf("%g %g %g %g %d\n", e_erfc, e_exp, e_img, std::fabs(bias / n), (int)inside);
 }
 """
 
@@ -110,3 +116,7 @@ def errors(tmp_path_factory):
                                             (2, "image sum (relative)", 1.1e-6), (3, "image sum, mean", 2e-7)])
 def test_error_bound(errors, k, name, bound):
     assert errors[k] <= bound, (name, errors[k])
+
+
+def test_no_argument_reads_past_the_table(errors):
+    assert errors[4] == 1
