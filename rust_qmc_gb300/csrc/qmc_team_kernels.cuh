@@ -49,6 +49,10 @@ static bool fill_team(const HostSys& hs, TeamTab<SH>& S) {
     std::memset(&S, 0, sizeof(S));
     if (hs.N != SH::NE || hs.n_up != SH::NUP || hs.n_nuc != SH::NNUC) return false;
     if (hs.n_ao > SH::NAO || (int)hs.rot_occ.size() > SH::NROT) return false;
+    // the limits of the other kernels' table (this one has room for more primitives)
+    size_t prims = 0;
+    for (const HostShell& sh : hs.shells) prims += sh.exps.size();
+    if (hs.shells.size() > SH::NSH || prims > SH::NPRIM) return false;
     for (int I = 0; I < SH::NNUC; ++I) {
         const int sp = hs.species[I];
         for (int c = 0; c < 3; ++c) S.nuc[I][c] = hs.R[3 * I + c];
